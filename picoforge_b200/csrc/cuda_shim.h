@@ -19,11 +19,14 @@ typedef struct {
     uint32_t k_storage, k_logical, n_out, n_experts;
     uint32_t row_bytes;
     uint64_t expert_bytes;
-    /* tile kernels, gate / up tensors: tensor maps (CUtensorMap, 128 bytes each) of the sections of the resident image
-     * (Q4_K and IQ2_XXS: the packed rows; Q2_K: codes, scale bytes, super-scales), made by qw4sh_tile_prepare; with them
-     * the eight row pieces of a section come as one request.  0 sections: the kernel copies row by row. */
-    unsigned char tile_maps[3][128];
-    int tile_sections;
+    /* tensor-core expert products (experts_tc.cu), made by qw4sh_tile_prepare: tensor maps (CUtensorMap, 128 bytes each) of the
+     * resident image, and the format the kernel reads it in (a GGUF type id, or the wide form; 0: the kernel cannot take it) */
+    unsigned char tc_maps[2][128];
+    uint32_t tc_format;
+    /* wide form of a shared-expert tensor in any other format: fp16 hi / lo rows and a power of two per row, owned by the layer */
+    void *wide;
+    float *wide_scale;
+    size_t wide_bytes;
 } QW4ShTensor;
 
 typedef struct {
@@ -38,6 +41,10 @@ typedef struct {
     void *fused_alt[8];
     size_t fused_alt_bytes;
 } QW4ShLayer;
+
+/* Activation rows as the tensor-core products read them: fp16 hi / lo after a power-of-two scale, column sums (hi / lo) for
+ * the minima, and what undoes the scale (one float per row, or per 128 columns of an activation). */
+typedef struct { void *hi, *lo, *sum_hi, *sum_lo; float *scale; } QW4ShSplit;
 
 /* Device scratch of one workspace, sized for `cap` tokens. */
 typedef struct {
@@ -63,8 +70,7 @@ typedef struct {
     void *groups, *shared_groups; /* [cap * k], [cap / 4 + 1] groups of <= 4 rows (16 bytes each) */
     uint32_t *n_groups;           /* [2]: routed, shared */
     uint32_t *status;             /* [4]: error bits, first bad row, spare */
-    /* tensor-core prefill: fp16 hi / lo images and 32-column sums (hi, lo) of x [0-3], act [4-7], shared act [8-11] */
-    void *half[12];
+    QW4ShSplit split_x, split_act, split_shared;   /* [cap, hidden], [cap * k, inter], [cap, shared_inter] */
     void *groups32, *shared_groups32;  /* groups of <= 32 rows (16 bytes each): routed, shared */
     uint32_t *n_groups32;         /* [2]: routed, shared */
     uint32_t *dispatch_scratch;   /* [2 * experts * ceil(cap / 32) + experts]: token bitmaps, word prefixes, counts */
@@ -174,8 +180,6 @@ int qw4sh_fused_repairs(const QW4ShWork *work, uint32_t *count);
 void qw4sh_set_wrong_speculation(int on);
 void qw4sh_fused_scratch_sizes(const QW4ShLayer *layer, size_t *aq_bytes, size_t *asc_bytes, size_t *fast_bytes);
 
-/* Tensor-core prefill path (prefill_tc.cu): Q4_K experts, groups of <= 32 token rows, tcgen05
- * MMAs with TMEM accumulators.  supported: 1 when a tensor fits it. */
 /* Stable per-expert lists of plain rows (one id per row; 0xffffffff: none), one CTA. */
 int qw4sh_group_rows(uint32_t experts, size_t rows, const uint32_t *ids, uint32_t *offsets, uint32_t *pair_to_row,
                      uint32_t *row_to_pair, uint32_t *active, uint32_t *status, void *stream);
@@ -210,26 +214,20 @@ int qw4sh_quantize_rows_pitched(const float *x, uint32_t pitch, uint32_t rows, u
                                 float *xscale, void *stream);
 void qw4sh_launch_log_begin(void);
 size_t qw4sh_launch_log(char *out, size_t cap);
-/* Tile kernels (experts_tile.cu): int8 tensor-core products for groups of <= 16 rows. */
-int qw4sh_tile_supported(const QW4ShTensor *w, int mode);
+/* Tensor-core expert products (experts_tc.cu): groups of <= 32 rows of one expert. */
+int qw4sh_tile_supported(const QW4ShTensor *w);
+void qw4sh_tile_release(QW4ShLayer *layer);
 void qw4sh_set_tile_path(int path);         /* -1 automatic (default), 0 never, 1 every batch of > 4 rows */
+void qw4sh_set_prefill_path(int path);      /* -1 automatic (default), 0 never */
+/* Profiling aid: device array of 64 x 8 bytes (or NULL); CTA 0 of later launches stores the cycles its five roles spent in
+ * their waits: [32 * mode + 4 * role + kind], kind 3 = the role's total. */
+void qw4sh_prefill_debug(void *device_words);
+int qw4sh_split_rows(const float *x, uint32_t pitch, uint32_t rows, uint32_t k, const QW4ShSplit *to, void *stream);
 int qw4sh_build_tile_groups(const uint32_t *offsets, const uint32_t *active, void *groups, uint32_t *n_groups, void *stream);
 int qw4sh_build_dense_tile_groups(uint32_t tokens, void *groups, uint32_t *n_groups, void *stream);
-int qw4sh_expert_tiles(int mode, const QW4ShTensor *w0, const QW4ShTensor *w1, const void *groups, const uint32_t *n_groups,
-                       const uint32_t *row_to_pair, uint32_t k_div, const int8_t *digits, const int *sums, const float *scale,
-                       float *out, uint32_t *status, int ctas, void *stream);
-int qw4sh_prefill_supported(const QW4ShTensor *w, int mode);
-void qw4sh_set_prefill_path(int path);      /* -1 automatic (default), 0 never */
-/* Profiling aid: device array of 64 x 8 bytes (or NULL); CTA 0 of later prefill launches stores the cycles its
- * five roles spent in their waits: [32 * mode + 4 * role + kind], kind 3 = the role's total. */
-void qw4sh_prefill_debug(void *device_words);
-int qw4sh_split_rows(const float *x, uint32_t rows, uint32_t k, void *hi, void *lo, void *sum_hi, void *sum_lo, void *stream);
-int qw4sh_build_groups32(const uint32_t *offsets, const uint32_t *active, void *groups, uint32_t *n_groups, void *stream);
-int qw4sh_build_dense_groups32(uint32_t tokens, void *groups, uint32_t *n_groups, void *stream);
-int qw4sh_prefill_tc(int mode, const QW4ShTensor *w0, const QW4ShTensor *w1, const void *groups, const uint32_t *n_groups,
-                     const uint32_t *row_to_pair, uint32_t k_div, const void *in_hi, const void *in_lo, const void *sum_hi,
-                     const void *sum_lo, void *out_hi, void *out_lo, void *osum_hi, void *osum_lo, float *out, uint32_t *status,
-                     int ctas, void *stream);
+int qw4sh_expert_tc(int mode, int prefill, const QW4ShTensor *w0, const QW4ShTensor *w1, const void *groups, const uint32_t *n_groups,
+                    const uint32_t *row_to_pair, uint32_t k_div, const QW4ShSplit *in, const QW4ShSplit *act, float *out, uint32_t *status,
+                    int ctas, void *stream);
 
 /* The layer stage by stage in the reference's order, every stage copied back and shown to `observer`
  * (observed_forward.cu).  The observer has the signature of QW4MoeObserver. */

@@ -1513,30 +1513,33 @@ static bool mma_path(const QW4ShLayer *layer, size_t tokens) {
            qw4sh_mma_supported(&layer->w[4], 0) && qw4sh_mma_supported(&layer->w[5], 0) && qw4sh_mma_supported(&layer->w[6], 1);
 }
 
-// Batches of more than MMA_MAX_TOKENS rows take the tcgen05 prefill kernels when every expert tensor is Q4_K.
+// Every layer whose six expert tensors fit the tensor-core products (experts_tc.cu) runs on them, whatever the batch: large
+// all-Q4_K batches under one name (prefill), everything else under the other (tile).  The four-row grouped kernels stay for
+// callers that ask for them (qw4cu_set_tile_path(0), qw4cu_set_expert_path(1)); the CUDA-core kernels for the rest.
 static int g_prefill_path = -1;                    // -1 automatic, 0 never
 extern "C" void qw4sh_set_prefill_path(int path) { g_prefill_path = path; }
-static bool prefill_path(const QW4ShLayer *layer, size_t tokens) {
-    if (g_prefill_path == 0 || g_expert_path == 0 || tokens <= MMA_MAX_TOKENS) return false;
-    for (int i = 1; i <= 6; i++) if (!qw4sh_prefill_supported(&layer->w[i], i == 3 || i == 6)) return false;
-    return layer->inter % 32 == 0 && layer->shared_inter % 32 == 0;
-}
-
-// Batches of more than four rows (and any batch the one-kernel decode or the tcgen05 prefill cannot take) run the
-// expert products on the tile kernels: weight fragments built once per 32-row group instead of once per 4 rows.
 static int g_tile_path = -1;                       // -1 automatic, 0 never, 1 whenever the types allow
 extern "C" void qw4sh_set_tile_path(int path) { g_tile_path = path; }
-static bool tile_types(const QW4ShLayer *layer) {
-    return layer->w[1].type == layer->w[2].type && qw4sh_tile_supported(&layer->w[1], 0) && qw4sh_tile_supported(&layer->w[2], 0) &&
-           qw4sh_tile_supported(&layer->w[3], 1);
+static bool tc_routed(const QW4ShLayer *l) {
+    return l->w[1].tc_format == l->w[2].tc_format && qw4sh_tile_supported(&l->w[1]) && qw4sh_tile_supported(&l->w[3]);
+}
+static bool tc_shared(const QW4ShLayer *l) {
+    return l->w[4].tc_format == l->w[5].tc_format && qw4sh_tile_supported(&l->w[4]) && qw4sh_tile_supported(&l->w[6]);
+}
+static bool prefill_path(const QW4ShLayer *layer, size_t tokens) {
+    if (g_prefill_path == 0 || g_expert_path == 0 || tokens <= MMA_MAX_TOKENS) return false;
+    for (int i = 1; i <= 6; i++) if (layer->w[i].tc_format != T_Q4_K) return false;
+    return true;
 }
 static bool tile_path(const QW4ShLayer *layer, size_t tokens) {
     if (g_tile_path == 0 || g_expert_path == 0 || (g_tile_path > 0 && tokens <= 4)) return false;
-    // automatic: batches that neither the four-row kernels (<= 64 rows, Q4_K / IQ2_XXS) nor the tcgen05 prefill
-    // (Q4_K) can take: IQ2_XXS beyond 64 rows, Q2_K at any size; 1: every batch of more than four rows
-    if (g_tile_path < 0 && (tokens <= MMA_MAX_TOKENS ? mma_path(layer, tokens) : prefill_path(layer, tokens))) return false;
-    return tile_types(layer) && layer->w[4].type == layer->w[5].type && qw4sh_tile_supported(&layer->w[4], 0) &&
-           qw4sh_tile_supported(&layer->w[5], 0) && qw4sh_tile_supported(&layer->w[6], 1);
+    if (g_tile_path < 0) {
+        if (prefill_path(layer, tokens)) return false;
+        // IQ2_XXS at up to 64 rows: two table reads for eight weights bound its dequantiser (2000 cycles for 128 columns of 256
+        // rows), and with a row or two per expert the four-row kernel's int8 table form is faster (23 tokens: 158 against 176 us)
+        if (mma_path(layer, tokens) && (g_expert_path == 1 || layer->w[1].type == T_IQ2_XXS)) return false;
+    }
+    return tc_routed(layer) && tc_shared(layer);
 }
 
 static cudaStream_t g_side_stream[64] = {nullptr};
@@ -1604,55 +1607,59 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
         if (fused_rc != (int)cudaErrorCooperativeLaunchTooLarge) return fused_rc;
         (void)cudaGetLastError();
     }
-    const bool tile = tile_path(layer, tokens);
-    const bool mma = tile || mma_path(layer, tokens);
-    const bool fused_route = mma && T <= 64 && E <= 512 && k <= E && T * k < 4096;
+    const bool prefill = prefill_path(layer, tokens), tc = prefill || tile_path(layer, tokens), mma = !tc && mma_path(layer, tokens);
+    const bool fused_route = (tc || mma) && T <= 64 && E <= 512 && k <= E && T * k < 4096;
     int rc, stage = 0;
 #define STAGE_MARK() do { if (timed) CU(cudaEventRecord(g_stage_event[stage++], stream)); } while (0)
     STAGE_MARK();
-    // The shared expert and the quantisation of x need only x: they run on a second stream
+    // The shared expert and the conversion of x need only x: they run on a second stream
     // beside router and route, and join before the routed experts / the combine.  (Serial when
     // timing stages.)
     cudaStream_t side = stream;
-    cudaEvent_t *ev = nullptr;                          // [0] fork, [1] x digits ready, [2] routes ready, [3] shared expert done
-    const bool overlap = mma && !timed;
+    cudaEvent_t *ev = nullptr;                          // [0] fork, [1] converted x ready, [2] routes ready, [3] shared expert done
+    const bool overlap = (tc || mma) && !timed;
     uint8_t *shared_groups = (uint8_t *)work->groups + (size_t)T * k * 16;      // behind the routed groups
     if (overlap) {
         if ((rc = side_stream(&side, &ev))) return rc;
         CU(cudaEventRecord(ev[0], stream));
         CU(cudaStreamWaitEvent(side, ev[0], 0));
     }
-    if (mma) {
-        if (STEP(1) && (rc = qw4sh_quantize_rows(x, T, H, work->xq, work->xneg, work->xsum, work->xscale, side))) return rc;
-        if (overlap) CU(cudaEventRecord(ev[1], side));
-    }
+    if (tc && (rc = qw4sh_split_rows(x, H, T, H, &work->split_x, side))) return rc;
+    if (mma && STEP(1) && (rc = qw4sh_quantize_rows(x, T, H, work->xq, work->xneg, work->xsum, work->xscale, side))) return rc;
+    if (overlap) CU(cudaEventRecord(ev[1], side));
     const int ctas = sm_count();
-    // expert products of one stage: tile kernels over groups of <= 32 rows, or the 4-row grouped kernel
-    auto products = [&](int mode, const QW4ShTensor *w0, const QW4ShTensor *w1, bool shared, const uint32_t *r2p, uint32_t k_div, const int8_t *q,
-                        const int8_t *neg, const int *sums, const float *scale, float *out, cudaStream_t strm) -> int {
-        if (tile)
-            return qw4sh_expert_tiles(mode, w0, w1, shared ? (void *)shared_groups : work->groups, work->n_groups + (shared ? 1 : 0), r2p, k_div,
-                                      q, sums, scale, out, work->status, ctas, strm);
+    // expert products of one stage: mode 0 gate/up, 1 down
+    auto products = [&](int mode, bool shared, cudaStream_t strm) -> int {
+        const QW4ShTensor *w0 = &layer->w[(shared ? 4 : 1) + (mode ? 2 : 0)], *w1 = mode ? nullptr : w0 + 1;
+        const uint32_t *r2p = shared ? nullptr : work->row_to_pair;
+        const uint32_t k_div = shared || mode ? 1 : k;
+        float *out = shared ? work->shared_out : work->out;
+        if (tc) {
+            const QW4ShSplit *act = shared ? &work->split_shared : &work->split_act;
+            return qw4sh_expert_tc(mode, prefill, w0, w1, shared ? work->shared_groups32 : work->groups32, work->n_groups32 + (shared ? 1 : 0), r2p, k_div,
+                                   mode ? act : &work->split_x, mode ? nullptr : act, mode ? out : nullptr, work->status, ctas, strm);
+        }
+        const int8_t *q = mode == 0 ? work->xq : shared ? work->sq : work->aq, *neg = mode == 0 ? work->xneg : shared ? work->sneg : work->aneg;
+        const int *sums = mode == 0 ? work->xsum : shared ? work->ssum : work->asum;
+        const float *scale = mode == 0 ? work->xscale : shared ? work->sscale : work->ascale;
         return qw4sh_grouped_mma(mode, w0, w1, shared ? (void *)shared_groups : work->groups, work->n_groups + (shared ? 1 : 0), r2p, k_div, q, neg,
-                                 sums, scale, out, work->status, ctas, strm);
+                                 sums, scale, mode ? out : shared ? work->shared_act : work->act, work->status, ctas, strm);
     };
     auto shared_branch = [&](int which) -> int {
         if (which == 0) {
-            if (tile) { if ((rc = qw4sh_build_dense_tile_groups(T, shared_groups, work->n_groups + 1, side))) return rc; }
+            if (tc) { if ((rc = qw4sh_build_dense_tile_groups(T, work->shared_groups32, work->n_groups32 + 1, side))) return rc; }
             else if (!fused_route && (rc = qw4sh_build_dense_groups(T, shared_groups, work->n_groups + 1, side))) return rc;
-            if (!STEP(4)) return 0;
-            return products(0, &layer->w[4], &layer->w[5], true, nullptr, 1, work->xq, work->xneg, work->xsum, work->xscale, work->shared_act, side);
+            return STEP(4) ? products(0, true, side) : 0;
         }
-        if (STEP(7) && (rc = qw4sh_quantize_rows(work->shared_act, T, layer->shared_inter, work->sq, work->sneg, work->ssum, work->sscale, side))) return rc;
-        if (!STEP(8)) return 0;
-        return products(1, &layer->w[6], nullptr, true, nullptr, 1, work->sq, work->sneg, work->ssum, work->sscale, work->shared_out, side);
+        if (mma && STEP(7) && (rc = qw4sh_quantize_rows(work->shared_act, T, layer->shared_inter, work->sq, work->sneg, work->ssum, work->sscale, side))) return rc;
+        return STEP(8) ? products(1, true, side) : 0;
     };
     if (STEP(0) && (rc = launch_router(layer, x, tokens, work->logits, work->shared_logit, work->status, router_mode, stream))) return rc;
     STAGE_MARK();
     if (fused_route) {
         if (STEP(2) && (rc = launch_route_group_small(layer, work, T, stream))) return rc;
         STAGE_MARK(); STAGE_MARK();
-        if (overlap) {                                // shared groups are written by the fused kernel
+        if (overlap && mma) {                         // shared groups are written by the fused kernel
             CU(cudaEventRecord(ev[2], stream));
             CU(cudaStreamWaitEvent(side, ev[2], 0));
         }
@@ -1663,51 +1670,27 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
             if ((rc = qw4sh_group_large(E, k, tokens, work->ids, work->offsets, work->pair_to_row, work->row_to_pair, work->active,
                                         work->dispatch_scratch, work->status, stream))) return rc;
         } else if ((rc = qw4sh_group(E, k, tokens, work->ids, work->offsets, work->pair_to_row, work->row_to_pair, work->active, work->status, stream))) return rc;
-        if (mma && !tile && (rc = qw4sh_build_groups(work->offsets, work->active, work->groups, work->n_groups, stream))) return rc;
+        if (mma && (rc = qw4sh_build_groups(work->offsets, work->active, work->groups, work->n_groups, stream))) return rc;
         STAGE_MARK();
     }
-    if (tile && (rc = qw4sh_build_tile_groups(work->offsets, work->active, work->groups, work->n_groups, stream))) return rc;
-    if (mma) {
+    if (tc && (rc = qw4sh_build_tile_groups(work->offsets, work->active, work->groups32, work->n_groups32, stream))) return rc;
+    if (tc || mma) {
         if (overlap) {
             if ((rc = shared_branch(0)) || (rc = shared_branch(1))) return rc;
             CU(cudaEventRecord(ev[3], side));
             CU(cudaStreamWaitEvent(stream, ev[1], 0));
         }
-        if (STEP(3) && (rc = products(0, &layer->w[1], &layer->w[2], false, work->row_to_pair, k, work->xq, work->xneg, work->xsum, work->xscale,
-                                      work->act, stream))) return rc;
+        if (STEP(3) && (rc = products(0, false, stream))) return rc;
         STAGE_MARK();
         if (!overlap && (rc = shared_branch(0))) return rc;
         STAGE_MARK();
-        if (STEP(5) && (rc = qw4sh_quantize_rows(work->act, T * k, layer->inter, work->aq, work->aneg, work->asum, work->ascale, stream))) return rc;
-        if (STEP(6) && (rc = products(1, &layer->w[3], nullptr, false, work->row_to_pair, 1, work->aq, work->aneg, work->asum, work->ascale,
-                                      work->out, stream))) return rc;
+        if (mma && STEP(5) && (rc = qw4sh_quantize_rows(work->act, T * k, layer->inter, work->aq, work->aneg, work->asum, work->ascale, stream))) return rc;
+        if (STEP(6) && (rc = products(1, false, stream))) return rc;
         STAGE_MARK();
         if (!overlap && (rc = shared_branch(1))) return rc;
         STAGE_MARK();
         if (overlap) CU(cudaStreamWaitEvent(stream, ev[3], 0));
         if (STEP(9) && (rc = qw4sh_combine(work->out, work->shared_out, work->weights, work->shared_logit, k, H, T, y, work->routed, work->status, work->hc_residual, work->hc_inject,
-                                             work->hc_streams, stream))) return rc;
-        STAGE_MARK();
-    } else if (prefill_path(layer, tokens)) {
-        // tensor-core prefill: groups of <= 32 rows, tcgen05 MMAs on exact integer codes.  (The shared expert on a second
-        // stream beside router and dispatch was measured and made the step slower: its persistent CTAs hold every SM.)
-        void *const *hf = work->half;
-        if ((rc = qw4sh_build_groups32(work->offsets, work->active, work->groups32, work->n_groups32, stream))) return rc;
-        if ((rc = qw4sh_build_dense_groups32(T, work->shared_groups32, work->n_groups32 + 1, stream))) return rc;
-        if ((rc = qw4sh_split_rows(x, T, H, hf[0], hf[1], hf[2], hf[3], stream))) return rc;
-        if ((rc = qw4sh_prefill_tc(0, &layer->w[1], &layer->w[2], work->groups32, work->n_groups32, work->row_to_pair, k, hf[0], hf[1], hf[2],
-                                   hf[3], hf[4], hf[5], hf[6], hf[7], nullptr, work->status, ctas, stream))) return rc;
-        STAGE_MARK();
-        if ((rc = qw4sh_prefill_tc(0, &layer->w[4], &layer->w[5], work->shared_groups32, work->n_groups32 + 1, nullptr, 1, hf[0], hf[1], hf[2],
-                                   hf[3], hf[8], hf[9], hf[10], hf[11], nullptr, work->status, ctas, stream))) return rc;
-        STAGE_MARK();
-        if ((rc = qw4sh_prefill_tc(1, &layer->w[3], nullptr, work->groups32, work->n_groups32, work->row_to_pair, 1, hf[4], hf[5], hf[6], hf[7],
-                                   nullptr, nullptr, nullptr, nullptr, work->out, work->status, ctas, stream))) return rc;
-        STAGE_MARK();
-        if ((rc = qw4sh_prefill_tc(1, &layer->w[6], nullptr, work->shared_groups32, work->n_groups32 + 1, nullptr, 1, hf[8], hf[9], hf[10],
-                                   hf[11], nullptr, nullptr, nullptr, nullptr, work->shared_out, work->status, ctas, stream))) return rc;
-        STAGE_MARK();
-        if ((rc = qw4sh_combine(work->out, work->shared_out, work->weights, work->shared_logit, k, H, T, y, work->routed, work->status, work->hc_residual, work->hc_inject,
                                              work->hc_streams, stream))) return rc;
         STAGE_MARK();
     } else {
@@ -1809,39 +1792,36 @@ static bool shared_on_mma(const QW4ShLayer *layer) {
     return layer->w[4].type == layer->w[5].type && qw4sh_mma_supported(&layer->w[4], 0) && qw4sh_mma_supported(&layer->w[5], 0) &&
            qw4sh_mma_supported(&layer->w[6], 1);
 }
-static bool shared_on_tiles(const QW4ShLayer *layer) {
-    return layer->w[4].type == layer->w[5].type && qw4sh_tile_supported(&layer->w[4], 0) && qw4sh_tile_supported(&layer->w[5], 0) &&
-           qw4sh_tile_supported(&layer->w[6], 1);
-}
 
 // The shared expert of `tokens` own tokens, on the side stream: it needs only x, so it runs under the exchange.
-// Its x digits live in the LAST rows of the quantisation buffers (rows 0 .. total-1 belong to the gathered rows).
+// Its converted x lives in the LAST rows of the buffers (rows 0 .. total-1 belong to the gathered rows).
 static int ep_shared_begin(const QW4ShLayer *layer, const QW4ShWork *work, const float *x, size_t tokens) {
     if (!tokens) return 0;
-    const bool tiles = tokens > MMA_MAX_TOKENS || !shared_on_mma(layer);
-    if (tiles ? !shared_on_tiles(layer) : !shared_on_mma(layer))
-        return fail(cudaErrorNotSupported, "expert-parallel step needs a Q4_K, IQ2_XXS or Q2_K shared expert");
+    const bool tiles = g_tile_path != 0 && tc_shared(layer);
+    if (!tiles && !shared_on_mma(layer)) return fail(cudaErrorNotSupported, "expert-parallel step: no tensor-core kernel takes the shared expert");
     cudaStream_t stream = (cudaStream_t)work->stream, side;
     cudaEvent_t *ev;
     int rc;
     if ((rc = side_stream(&side, &ev))) return rc;
     const uint32_t T = (uint32_t)tokens, H = layer->hidden;
     const size_t off = work->cap - tokens;
-    int8_t *xq = work->xq + off * 2 * H, *xneg = work->xneg + off * 2 * H;
-    int *xsum = work->xsum + off * (H / 32) * 2;
-    float *xscale = work->xscale + off;
     const int ctas = sm_count();
     CU(cudaEventRecord(ev[0], stream));
     CU(cudaStreamWaitEvent(side, ev[0], 0));
-    if ((rc = qw4sh_quantize_rows(x, T, H, xq, xneg, xsum, xscale, side))) return rc;
     if (tiles) {
-        if ((rc = qw4sh_build_dense_tile_groups(T, work->shared_groups, work->n_groups + 3, side))) return rc;
-        if ((rc = qw4sh_expert_tiles(0, &layer->w[4], &layer->w[5], work->shared_groups, work->n_groups + 3, nullptr, 1, xq, xsum, xscale,
-                                     work->shared_act, work->status, ctas, side))) return rc;
-        if ((rc = qw4sh_quantize_rows(work->shared_act, T, layer->shared_inter, work->sq, work->sneg, work->ssum, work->sscale, side))) return rc;
-        if ((rc = qw4sh_expert_tiles(1, &layer->w[6], nullptr, work->shared_groups, work->n_groups + 3, nullptr, 1, work->sq, work->ssum,
-                                     work->sscale, work->shared_out, work->status, ctas, side))) return rc;
+        const QW4ShSplit own = {(uint16_t *)work->split_x.hi + off * H, (uint16_t *)work->split_x.lo + off * H, (uint16_t *)work->split_x.sum_hi + off * (H / 16),
+                                (uint16_t *)work->split_x.sum_lo + off * (H / 16), work->split_x.scale + off};
+        if ((rc = qw4sh_split_rows(x, H, T, H, &own, side))) return rc;
+        if ((rc = qw4sh_build_dense_tile_groups(T, work->shared_groups32, work->n_groups32 + 1, side))) return rc;
+        if ((rc = qw4sh_expert_tc(0, 0, &layer->w[4], &layer->w[5], work->shared_groups32, work->n_groups32 + 1, nullptr, 1, &own, &work->split_shared, nullptr,
+                                  work->status, ctas, side))) return rc;
+        if ((rc = qw4sh_expert_tc(1, 0, &layer->w[6], nullptr, work->shared_groups32, work->n_groups32 + 1, nullptr, 1, &work->split_shared, nullptr,
+                                  work->shared_out, work->status, ctas, side))) return rc;
     } else {
+        int8_t *xq = work->xq + off * 2 * H, *xneg = work->xneg + off * 2 * H;
+        int *xsum = work->xsum + off * (H / 32) * 2;
+        float *xscale = work->xscale + off;
+        if ((rc = qw4sh_quantize_rows(x, T, H, xq, xneg, xsum, xscale, side))) return rc;
         if ((rc = qw4sh_build_dense_groups(T, work->shared_groups, work->n_groups + 3, side))) return rc;
         if ((rc = qw4sh_grouped_mma(0, &layer->w[4], &layer->w[5], work->shared_groups, work->n_groups + 3, nullptr, 1, xq, xneg, xsum, xscale,
                                     work->shared_act, work->status, ctas, side))) return rc;
@@ -1880,16 +1860,24 @@ extern "C" int qw4sh_ep_experts(const QW4ShLayer *layer, const QW4ShWork *work, 
     uint32_t *local = work->ids + own * k;                                  // behind this rank's own routes
     int rc;
     if ((rc = qw4sh_ep_trace_mark(3, stream))) return rc;                   // stage 2 was the all-gather
-    // the digits of the gathered rows depend on the rows alone: they are made on a stream of their own beside the lists
-    // (in one stream, as before, while stages are being timed)
+    const bool mma_types = layer->w[1].type == layer->w[2].type && qw4sh_mma_supported(&layer->w[1], 0) && qw4sh_mma_supported(&layer->w[2], 0) &&
+                           qw4sh_mma_supported(&layer->w[3], 1);
+    const bool tiles = g_tile_path != 0 && tc_routed(layer);
+    if (!tiles && !mma_types) return fail(cudaErrorNotSupported, "expert-parallel step: no tensor-core kernel takes the expert tensors");
+    // the gathered rows are converted on a stream of their own beside the lists: that needs the rows alone
+    // (in one stream while stages are being timed)
     cudaStream_t aux = stream;
     cudaEvent_t *aux_ev = nullptr;
     const bool beside = !qw4sh_ep_trace_on();
+    auto convert = [&](cudaStream_t strm) -> int {
+        return tiles ? qw4sh_split_rows(msg_all, pitch, T, H, &work->split_x, strm)
+                     : qw4sh_quantize_rows_pitched(msg_all, pitch, T, H, work->xq, work->xneg, work->xsum, work->xscale, strm);
+    };
     if (beside) {
         if ((rc = aux_stream(&aux, &aux_ev))) return rc;
         CU(cudaEventRecord(aux_ev[0], stream));
         CU(cudaStreamWaitEvent(aux, aux_ev[0], 0));
-        if ((rc = qw4sh_quantize_rows_pitched(msg_all, pitch, T, H, work->xq, work->xneg, work->xsum, work->xscale, aux))) return rc;
+        if ((rc = convert(aux))) return rc;
         CU(cudaEventRecord(aux_ev[1], aux));
     }
     // Lists.  Small batches: the foreign ids are masked out and one CTA sorts the rest.  Large batches: the bitmap
@@ -1910,26 +1898,19 @@ extern "C" int qw4sh_ep_experts(const QW4ShLayer *layer, const QW4ShWork *work, 
         if ((rc = qw4sh_group_rows(local_experts, (size_t)T * k, local, work->offsets, work->pair_to_row, work->row_to_pair, work->active,
                                    work->status, stream))) return rc;
     }
-    const bool mma_types = layer->w[1].type == layer->w[2].type && qw4sh_mma_supported(&layer->w[1], 0) && qw4sh_mma_supported(&layer->w[2], 0) &&
-                           qw4sh_mma_supported(&layer->w[3], 1);
-    const bool tiles = g_tile_path != 0 && tile_types(layer) && (g_tile_path > 0 || !mma_types || total > MMA_MAX_TOKENS);
-    if (!tiles && !mma_types) return fail(cudaErrorNotSupported, "expert-parallel step needs Q4_K, IQ2_XXS or Q2_K expert tensors");
     const int ctas = sm_count();
     const uint32_t *row_end = offsets + local_experts;                      // rows of this rank's experts: [*row_begin (or 0), *row_end)
     if ((rc = qw4sh_ep_trace_mark(4, stream))) return rc;
     if (beside) CU(cudaStreamWaitEvent(stream, aux_ev[1], 0));
-    else if ((rc = qw4sh_quantize_rows_pitched(msg_all, pitch, T, H, work->xq, work->xneg, work->xsum, work->xscale, stream))) return rc;
+    else if ((rc = convert(stream))) return rc;
     if ((rc = qw4sh_ep_trace_mark(5, stream))) return rc;
     if (tiles) {
-        if ((rc = qw4sh_build_tile_groups(offsets, active, work->groups, work->n_groups, stream))) return rc;
-        if ((rc = qw4sh_expert_tiles(0, &layer->w[1], &layer->w[2], work->groups, work->n_groups, work->row_to_pair, k, work->xq, work->xsum,
-                                     work->xscale, work->act, work->status, ctas, stream))) return rc;
-        if ((rc = qw4sh_ep_trace_mark(6, stream))) return rc;
-        if ((rc = qw4sh_quantize_rows_listed(work->act, layer->inter, T * k, layer->inter, work->row_to_pair, row_begin, row_end, work->aq, work->aneg,
-                                             work->asum, work->ascale, stream))) return rc;
-        if ((rc = qw4sh_ep_trace_mark(7, stream))) return rc;
-        if ((rc = qw4sh_expert_tiles(1, &layer->w[3], nullptr, work->groups, work->n_groups, work->row_to_pair, 1, work->aq, work->asum,
-                                     work->ascale, work->out, work->status, ctas, stream))) return rc;
+        if ((rc = qw4sh_build_tile_groups(offsets, active, work->groups32, work->n_groups32, stream))) return rc;
+        if ((rc = qw4sh_expert_tc(0, 0, &layer->w[1], &layer->w[2], work->groups32, work->n_groups32, work->row_to_pair, k, &work->split_x, &work->split_act,
+                                  nullptr, work->status, ctas, stream))) return rc;
+        if ((rc = qw4sh_ep_trace_mark(6, stream)) || (rc = qw4sh_ep_trace_mark(7, stream))) return rc;        // no separate digits of the activation
+        if ((rc = qw4sh_expert_tc(1, 0, &layer->w[3], nullptr, work->groups32, work->n_groups32, work->row_to_pair, 1, &work->split_act, nullptr, work->out,
+                                  work->status, ctas, stream))) return rc;
     } else {
         if ((rc = qw4sh_build_groups(offsets, active, work->groups, work->n_groups, stream))) return rc;
         if ((rc = qw4sh_grouped_mma(0, &layer->w[1], &layer->w[2], work->groups, work->n_groups, work->row_to_pair, k, work->xq, work->xneg,

@@ -175,6 +175,7 @@ static void release(Qwen4Moe *m) {
     if (m && --m->refs == 0) {
         for (int a = 0; a < 8; a++) qw4sh_free(m->image[a]);
         qw4sh_fused_release(&m->layer);
+        qw4sh_tile_release(&m->layer);
         free(m);
     }
 }
@@ -219,6 +220,7 @@ static Qwen4Status create_shard(const Qwen4MoeConfig *c, const Qwen4MoeWeights *
             .row_bytes = (uint32_t)l->row_bytes, .expert_bytes = l->expert_bytes};
     }
     (void)qw4sh_tile_prepare(&m->layer);
+    for (size_t a = 4; a <= 6; a++) m->device_bytes += m->layer.w[a].wide_bytes;
     if (qw4sh_fused_prepare(&m->layer)) { release(m); return cuda_failure(err, "decode path images"); }
     m->device_bytes += m->layer.fused_alt_bytes;
     *out = m;
@@ -269,22 +271,23 @@ static Qwen4Status plan_work(const Qwen4Moe *m, size_t cap, size_t *chunk, Plan 
     const size_t g32 = pairs / 32 + e + 2;                   /* groups of <= 32 rows: at most pairs/32 + experts */
     size_t fused_aq = 0, fused_asc = 0, fused_fast = 0;
     qw4sh_fused_scratch_sizes(&m->layer, &fused_aq, &fused_asc, &fused_fast);
-    const size_t count[52] = {t * h, t * h, t * e, t * e, t, pairs, pairs, e + 1, pairs, pairs, e + 1,
+    const size_t count[55] = {t * h, t * h, t * e, t * e, t, pairs, pairs, e + 1, pairs, pairs, e + 1,
         pairs * i, t * si, t * h, 4,
         pairs * h, t * h,                                   /* 15 out, 16 shared_out */
         t * h / 2 + 8, t * h / 2 + 8, t * (h / 32 + 1) * 2, t,                 /* 17 xq, 18 xneg, 19 xsum, 20 xscale */
         pairs * i / 2 + 8, pairs * i / 2 + 8, pairs * (i / 32 + 1) * 2, pairs,  /* 21 aq, 22 aneg, 23 asum, 24 ascale */
         t * si / 2 + 8, t * si / 2 + 8, t * (si / 32 + 1) * 2, t,              /* 25 sq, 26 sneg, 27 ssum, 28 sscale */
         pairs * 4 + t + 16, t + 8, 4, 1024, 0,
-        /* 34.. tensor-core prefill: fp16 hi/lo images (2 bytes per value) and 32-column sums of x, act, shared act; groups */
-        t * h / 2 + 8, t * h / 2 + 8, t * (h / 32) / 2 + 8, t * (h / 32) / 2 + 8,               /* 34 xh_hi, 35 xh_lo, 36 xs_hi, 37 xs_lo */
-        pairs * i / 2 + 8, pairs * i / 2 + 8, pairs * (i / 32 + 1) / 2 + 8, pairs * (i / 32 + 1) / 2 + 8,   /* 38-41 act */
-        t * si / 2 + 8, t * si / 2 + 8, t * (si / 32 + 1) / 2 + 8, t * (si / 32 + 1) / 2 + 8,           /* 42-45 shared act */
-        g32 * 4 + (t / 32 + 2) * 4, 8,
-        2 * e * (t / 32 + 1) + e + 8,
-        fused_aq / 4, fused_asc / 4, fused_fast / 4};                                    /* 49-51 one-kernel decode path */                                                      /* 48 dispatch scratch */                                                      /* 46 groups32 (routed, then shared), 47 counts */                                  /* 29 groups, 30 spare, 31 n_groups, 32 sync */
+        /* 34.. tensor-core products: fp16 hi / lo (2 bytes per value) and column sums of x (16 columns), act and shared act (8) */
+        t * h / 2 + 8, t * h / 2 + 8, t * (h / 16 + 1) / 2 + 8, t * (h / 16 + 1) / 2 + 8,                   /* 34-37 x */
+        pairs * i / 2 + 8, pairs * i / 2 + 8, pairs * (i / 8 + 1) / 2 + 8, pairs * (i / 8 + 1) / 2 + 8,     /* 38-41 act */
+        t * si / 2 + 8, t * si / 2 + 8, t * (si / 8 + 1) / 2 + 8, t * (si / 8 + 1) / 2 + 8,                 /* 42-45 shared act */
+        g32 * 4 + (t / 32 + 2) * 4, 8,                      /* 46 groups of <= 32 rows (routed, then shared), 47 their counts */
+        2 * e * (t / 32 + 1) + e + 8,                       /* 48 dispatch scratch */
+        fused_aq / 4, fused_asc / 4, fused_fast / 4,        /* 49-51 one-kernel decode path */
+        t, pairs * (i / 128 + 1), t * (si / 128 + 1)};      /* 52-54 what undoes the scales of x, act, shared act */
     size_t at = 0;
-    for (int j = 0; j < 52; j++) {
+    for (int j = 0; j < 55; j++) {
         if (count[j] > (SIZE_MAX >> 4)) return report(err, QW4_OVERFLOW, "scratch size overflow");
         plan->offset[j] = at;
         at += align256(count[j] * 4 + 4);
@@ -358,7 +361,10 @@ Qwen4Status qwen4_moe_work_create(const Qwen4Moe *m, size_t cap, size_t budget, 
     w->d.groups = base + plan.offset[29]; w->d.shared_groups = base + plan.offset[30];
     w->d.n_groups = (uint32_t *)(base + plan.offset[31]);
     w->d.sync = (uint32_t *)(base + plan.offset[32]);
-    for (int j = 0; j < 12; j++) w->d.half[j] = base + plan.offset[34 + j];
+    QW4ShSplit *const split[3] = {&w->d.split_x, &w->d.split_act, &w->d.split_shared};
+    for (int j = 0; j < 3; j++)
+        *split[j] = (QW4ShSplit){base + plan.offset[34 + 4 * j], base + plan.offset[35 + 4 * j], base + plan.offset[36 + 4 * j],
+                                 base + plan.offset[37 + 4 * j], (float *)(base + plan.offset[52 + j])};
     w->d.groups32 = base + plan.offset[46];
     w->d.shared_groups32 = (char *)w->d.groups32 + (pairs_of(m, chunk) / 32 + m->c.experts + 2) * 16;
     w->d.n_groups32 = (uint32_t *)(base + plan.offset[47]);
