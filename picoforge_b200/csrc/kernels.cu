@@ -269,138 +269,70 @@ __global__ void __launch_bounds__(32 * TT) router_exact_kernel(DevTensor router,
     }
 }
 
-// Exact, mid-sized batches: 16 router rows x 16 tokens per CTA of four warps (one per scheduler), every thread two
-// serial chains (one row x two tokens), so that three 128-bit shared-memory reads feed eight chain steps.  Measured
-// here: with one chain per thread (256 threads) the kernel is bound by shared-memory bandwidth, with four chains in
-// a lone warp per SM by that warp's issue rate (a warp issues at most every other cycle); this is the middle.
-// Both tiles go through a four-stage cp.async ring in chunks of 128 columns (three chunks are in flight ahead of
-// the adds: more than a DRAM round trip); row pitch 132 floats keeps the reads free of bank conflicts.
-constexpr int RC_ROWS = 16, RC_TOK = 16, RC_K = 128, RC_PITCH = 132, RC_STAGES = 4, RC_THREADS = 128;
-constexpr size_t RC_SMEM = (size_t)RC_STAGES * (RC_ROWS + RC_TOK) * RC_PITCH * sizeof(float);
-__device__ __forceinline__ void rc_copy16(void *dst_smem, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src) : "memory");
-}
-__global__ void __launch_bounds__(RC_THREADS) router_chain_kernel(DevTensor router, DevTensor srouter, const float *__restrict__ x, uint32_t tokens,
+// Exact, up to 128 tokens: ROWS router rows x TOK tokens per CTA, one thread and one serial chain per pair.  A chain is K
+// dependent additions of four cycles each (4.3 us at K = 2048) whatever else happens, so the tile is sized to keep everything
+// else under it: a warp issues eight instructions per four columns (two 128-bit shared-memory reads, two packed multiplies, each
+// half rounded like a scalar one, four adds) against sixteen cycles of additions, and the grid covers the SMs once.  Both
+// operands come by bulk copies in chunks of 512 columns through a ring that holds all of K = 2048 where the tile is small: the copies
+// of the whole chain are then in flight at once, and nothing waits but the first chunk.  (Before: 16 x 16 tiles through
+// a four-stage cp.async ring with two CTA barriers per 128 columns, 33 CTAs for up to 16 tokens: 22 us at 7 tokens.)
+constexpr uint32_t RC_K = 512, RC_PITCH = RC_K * 4 + 16;                      // bytes per row and chunk; the pad keeps 128-bit reads of eight rows apart
+__host__ __device__ constexpr uint32_t rc_stage_bytes(uint32_t rows) { return rows * RC_PITCH; }
+template <int ROWS, int TOK, int STAGES>
+__global__ void __launch_bounds__(ROWS * TOK) router_chain_kernel(DevTensor router, DevTensor srouter, const float *__restrict__ x, uint32_t tokens,
                                                                   float *__restrict__ logits, float *__restrict__ shared_logit, uint32_t *status) {
-    extern __shared__ __align__(16) uint8_t rc_smem[];
-    float (*tile)[RC_ROWS + RC_TOK][RC_PITCH] = reinterpret_cast<float (*)[RC_ROWS + RC_TOK][RC_PITCH]>(rc_smem);   // rows 0-15 router rows, 16-31 tokens
+    extern __shared__ __align__(128) uint8_t rc_smem[];                       // [STAGES][ROWS + TOK][RC_PITCH]
+    __shared__ uint64_t bars[STAGES];
     const uint32_t experts = router.n_out, K = router.k_logical, tid = threadIdx.x;
-    const uint32_t e0 = blockIdx.x * RC_ROWS, t0 = blockIdx.y * RC_TOK;
-    const uint32_t chunks = K / RC_K;
-    // loader role: thread t copies the 16-byte piece t % 32 of rows t / 32, t / 32 + 4, ... (32 pieces = 128 columns)
-    const uint32_t piece = (tid & 31u) * 4, lrow = tid >> 5;
-    const float *srcs[(RC_ROWS + RC_TOK) / 4];
-#pragma unroll
-    for (int j = 0; j < (RC_ROWS + RC_TOK) / 4; j++) {
-        const uint32_t r = lrow + 4 * j;
-        if (r < RC_ROWS) {
-            const uint32_t e = e0 + r;
-            srcs[j] = (e < experts ? (const float *)(router.data + (uint64_t)e * router.row_bytes) : (const float *)srouter.data) + piece;
-        } else srcs[j] = x + (uint64_t)min(t0 + r - RC_ROWS, tokens - 1) * K + piece;
-    }
-    auto load = [&](uint32_t c) {
-        if (c < chunks) {
-#pragma unroll
-            for (int j = 0; j < (RC_ROWS + RC_TOK) / 4; j++) rc_copy16(&tile[c % RC_STAGES][lrow + 4 * j][piece], srcs[j] + c * RC_K);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    for (uint32_t c = 0; c + 1 < RC_STAGES; c++) load(c);
-    const uint32_t er = tid >> 3, tc = tid & 7u;                                 // worker role: row er x tokens tc, tc + 8
-    float s0 = 0.0f, s1 = 0.0f;
-    for (uint32_t c = 0; c < chunks; c++) {
-        load(c + RC_STAGES - 1);
-        asm volatile("cp.async.wait_group %0;" ::"n"(RC_STAGES - 1) : "memory");
-        __syncthreads();
-        const float4 *w4 = reinterpret_cast<const float4 *>(tile[c % RC_STAGES][er]);
-        const float4 *x0 = reinterpret_cast<const float4 *>(tile[c % RC_STAGES][RC_ROWS + tc]), *x1 = reinterpret_cast<const float4 *>(tile[c % RC_STAGES][RC_ROWS + tc + 8]);
-#pragma unroll 8
-        for (int i = 0; i < RC_K / 4; i++) {
-            const float4 a = w4[i], u = x0[i], v = x1[i];
-            const float p0 = __fmul_rn(a.x, u.x), p1 = __fmul_rn(a.x, v.x), p2 = __fmul_rn(a.y, u.y), p3 = __fmul_rn(a.y, v.y);
-            const float p4 = __fmul_rn(a.z, u.z), p5 = __fmul_rn(a.z, v.z), p6 = __fmul_rn(a.w, u.w), p7 = __fmul_rn(a.w, v.w);
-            s0 = __fadd_rn(s0, p0); s1 = __fadd_rn(s1, p1); s0 = __fadd_rn(s0, p2); s1 = __fadd_rn(s1, p3);
-            s0 = __fadd_rn(s0, p4); s1 = __fadd_rn(s1, p5); s0 = __fadd_rn(s0, p6); s1 = __fadd_rn(s1, p7);
-        }
-        __syncthreads();
-    }
-    const uint32_t e = e0 + er;
-    bool bad = false;
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-        const uint32_t t = t0 + tc + 8 * j;
-        const float sum = j ? s1 : s0;
-        if (t < tokens && e <= experts) {
-            bad |= !finite_f32(sum);
-            if (e < experts) logits[(uint64_t)t * experts + e] = sum;
-            else shared_logit[t] = sum;
-        }
-    }
-    if (bad) atomicOr(status, QW4SH_ERR_NONFINITE);
-}
-
-// Exact, few tokens: one warp per (32 router rows, token).  The serial chain of separately
-// rounded multiply-adds (the reference's order) is the critical path: K dependent additions.
-// To keep operands ahead of the chain, the 32 rows are staged through shared memory by bulk
-// copies (one per lane and chunk of 512 columns, three chunks in flight); rows are padded by
-// 16 bytes so that the lanes' 128-bit reads fall in different banks.
-__device__ __forceinline__ uint32_t rsm_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-constexpr uint32_t RS_CHUNK = 512, RS_PITCH = RS_CHUNK * 4 + 16, RS_STAGES = 3;
-__global__ void __launch_bounds__(32) router_exact_small_kernel(DevTensor router, DevTensor srouter, const float *__restrict__ x,
-                                                                float *__restrict__ logits, float *__restrict__ shared_logit,
-                                                                uint32_t *status) {
-    extern __shared__ __align__(128) uint8_t rs_smem[];       // [STAGES][32][PITCH] | x [K] floats | barriers
-    const uint32_t experts = router.n_out, K = router.k_logical, lane = threadIdx.x;
-    const uint32_t e = blockIdx.x * 32 + lane, t = blockIdx.y;
-    const uint8_t *row = e < experts ? router.data + (uint64_t)e * router.row_bytes : (e == experts ? srouter.data : router.data);
-    float *xs = reinterpret_cast<float *>(rs_smem + RS_STAGES * 32 * RS_PITCH);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(rs_smem + RS_STAGES * 32 * RS_PITCH + ((K * 4 + 15) & ~15u));
-    const uint32_t chunks = (K + RS_CHUNK - 1) / RS_CHUNK;
-    if (lane == 0) {
-        for (uint32_t s = 0; s < RS_STAGES; s++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(rsm_u32(&bar[s])), "r"(1u) : "memory");
+    const uint32_t e0 = blockIdx.x * ROWS, t0 = blockIdx.y * TOK, chunks = (K + RC_K - 1) / RC_K;
+    auto saddr = [](const void *p) { return (uint32_t)__cvta_generic_to_shared(p); };
+    if (tid < STAGES) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(&bars[tid])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncwarp();
-    auto issue = [&](uint32_t c) {
-        const uint32_t s = c % RS_STAGES, bytes = min(RS_CHUNK, K - c * RS_CHUNK) * 4;
-        if (lane == 0)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(rsm_u32(&bar[s])), "r"(bytes * 32) : "memory");
+    __syncthreads();
+    auto issue = [&](uint32_t c) {                                            // by the first warp
+        const uint32_t bytes = min(RC_K, K - c * RC_K) * 4u, bar = saddr(&bars[c % STAGES]);
+        if (tid == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes * (ROWS + TOK)) : "memory");
         __syncwarp();
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(rsm_u32(rs_smem + (s * 32 + lane) * RS_PITCH)), "l"(row + (uint64_t)c * RS_CHUNK * 4), "r"(bytes), "r"(rsm_u32(&bar[s])) : "memory");
+        for (uint32_t r = tid; r < ROWS + TOK; r += 32) {
+            const uint32_t e = min(e0 + r, experts);
+            const uint8_t *src = r >= ROWS ? reinterpret_cast<const uint8_t *>(x + (uint64_t)min(t0 + r - ROWS, tokens - 1) * K)
+                                           : e < experts ? router.data + (uint64_t)e * router.row_bytes : srouter.data;
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(saddr(rc_smem + ((c % STAGES) * (ROWS + TOK) + r) * RC_PITCH)), "l"(src + (uint64_t)c * RC_K * 4), "r"(bytes), "r"(bar) : "memory");
+        }
     };
-    for (uint32_t c = 0; c < RS_STAGES && c < chunks; c++) issue(c);
-    for (uint32_t k = lane * 4; k < K; k += 128) *reinterpret_cast<float4 *>(xs + k) = *reinterpret_cast<const float4 *>(x + (uint64_t)t * K + k);
-    __syncwarp();
+    if (tid < 32) for (uint32_t c = 0; c < STAGES && c < chunks; c++) issue(c);
+    const uint32_t er = tid / TOK, tc = tid % TOK;
     float sum = 0.0f;
     bool alive = true;
     for (uint32_t c = 0; c < chunks; c++) {
-        const uint32_t s = c % RS_STAGES, parity = (c / RS_STAGES) & 1u, cols = min(RS_CHUNK, K - c * RS_CHUNK);
-        if (alive) {                                           // bounded wait (~1 s), then give up with an error bit
-            const long long start = clock64();
-            uint32_t ok = 0;
-            while (!ok) {
-                asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                             : "=r"(ok) : "r"(rsm_u32(&bar[s])), "r"(parity) : "memory");
-                if (!ok && clock64() - start > (1ll << 31)) { atomicOr(status, QW4SH_ERR_STATE); alive = false; break; }
-            }
+        const uint32_t bar = saddr(&bars[c % STAGES]), parity = (c / STAGES) & 1u;
+        const long long start = clock64();
+        for (uint32_t ok = 0; alive && !ok;) {                                // bounded (about a second), then the error bit
+            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+            if (!ok && clock64() - start > (1ll << 31)) { atomicOr(status, QW4SH_ERR_STATE); alive = false; }
         }
-        alive = __all_sync(0xffffffffu, alive);
-        if (alive) {
-            const float4 *w = reinterpret_cast<const float4 *>(rs_smem + (s * 32 + lane) * RS_PITCH);
-            const float4 *xv = reinterpret_cast<const float4 *>(xs + c * RS_CHUNK);
+        const uint8_t *stage = rc_smem + (c % STAGES) * rc_stage_bytes(ROWS + TOK);
+        const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(stage + er * RC_PITCH), *v = reinterpret_cast<const ulonglong2 *>(stage + (ROWS + tc) * RC_PITCH);
+        const uint32_t quads = min(RC_K, K - c * RC_K) / 4;
 #pragma unroll 8
-            for (uint32_t i = 0; i < cols / 4; i++) {
-                const float4 a = w[i], b = xv[i];
-                sum = __fadd_rn(sum, __fmul_rn(a.x, b.x)); sum = __fadd_rn(sum, __fmul_rn(a.y, b.y));
-                sum = __fadd_rn(sum, __fmul_rn(a.z, b.z)); sum = __fadd_rn(sum, __fmul_rn(a.w, b.w));
-            }
+        for (uint32_t i = 0; i < quads; i++) {
+            const ulonglong2 a = w[i], b = v[i];
+            unsigned long long p, q;
+            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(a.x), "l"(b.x));
+            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(a.y), "l"(b.y));
+            sum = __fadd_rn(sum, __uint_as_float((uint32_t)p)); sum = __fadd_rn(sum, __uint_as_float((uint32_t)(p >> 32)));
+            sum = __fadd_rn(sum, __uint_as_float((uint32_t)q)); sum = __fadd_rn(sum, __uint_as_float((uint32_t)(q >> 32)));
         }
-        __syncwarp();
-        if (alive && c + RS_STAGES < chunks) issue(c + RS_STAGES);
+        if (chunks > STAGES) {                                                // the ring turns only for longer rows or larger tiles
+            __syncthreads();
+            if (tid < 32 && c + STAGES < chunks) { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); issue(c + STAGES); }
+        }
     }
-    if (e <= experts && alive) {
+    const uint32_t e = e0 + er, t = t0 + tc;
+    if (e <= experts && t < tokens && alive) {
         if (!finite_f32(sum)) atomicOr(status, QW4SH_ERR_NONFINITE);
         if (e < experts) logits[(uint64_t)t * experts + e] = sum;
         else shared_logit[t] = sum;
@@ -1291,17 +1223,26 @@ static int launch_router(const QW4ShLayer *layer, const float *x, size_t tokens,
                          uint32_t *status, int mode, cudaStream_t stream) {
     const DevTensor router = as_dev(layer->w[0]), srouter = as_dev(layer->w[7]);
     const uint32_t rows = layer->experts + 1;
-    if (mode == 0 && tokens > 4 && tokens <= 128 && router.k_logical % RC_K == 0 && ((uintptr_t)x & 15u) == 0 && router.row_bytes % 16 == 0 &&
-               ((uintptr_t)router.data & 15u) == 0 && ((uintptr_t)srouter.data & 15u) == 0) {
-        if (allow_smem(router_chain_kernel, RC_SMEM)) return -1;
-        router_chain_kernel<<<dim3((rows + RC_ROWS - 1) / RC_ROWS, (unsigned)((tokens + RC_TOK - 1) / RC_TOK)), RC_THREADS, RC_SMEM, stream>>>(
-            router, srouter, x, (uint32_t)tokens, logits, shared_logit, status);
+    const bool aligned = ((uintptr_t)x & 15u) == 0 && router.k_logical % 4 == 0 && router.row_bytes % 16 == 0 && ((uintptr_t)router.data & 15u) == 0 &&
+                         ((uintptr_t)srouter.data & 15u) == 0;
+    if (mode == 0 && tokens <= 128 && aligned) {
+        // the tile: as many chains per CTA as leave one CTA per SM (513 rows)
+#define ROUTER_CHAIN(ROWS, TOK, STAGES) do { \
+        static bool configured[64] = {false}; \
+        const size_t smem = (size_t)STAGES * rc_stage_bytes(ROWS + TOK); \
+        int device = 0; \
+        CU(cudaGetDevice(&device)); \
+        if (device < 0 || device >= 64) return fail(cudaErrorInvalidDevice, "device index"); \
+        if (!configured[device]) { if (allow_smem(router_chain_kernel<ROWS, TOK, STAGES>, smem)) return -1; configured[device] = true; } \
+        router_chain_kernel<ROWS, TOK, STAGES><<<dim3((rows + ROWS - 1) / ROWS, (unsigned)((tokens + TOK - 1) / TOK)), ROWS * TOK, smem, stream>>>( \
+            router, srouter, x, (uint32_t)tokens, logits, shared_logit, status); } while (0)
+        if (tokens <= 8) ROUTER_CHAIN(4, 8, 4);
+        else if (tokens <= 16) ROUTER_CHAIN(4, 16, 4);
+        else if (tokens <= 32) ROUTER_CHAIN(8, 16, 4);
+        else if (tokens <= 64) ROUTER_CHAIN(16, 16, 3);
+        else ROUTER_CHAIN(32, 16, 2);
+#undef ROUTER_CHAIN
         LAUNCHED("router_chain_kernel");
-    } else if (mode == 0 && tokens <= 16 && router.k_logical % 4 == 0 && router.k_logical <= 4096) {
-        const size_t smem = RS_STAGES * 32 * RS_PITCH + (((size_t)router.k_logical * 4 + 15) & ~(size_t)15) + 64;
-        if (allow_smem(router_exact_small_kernel, smem)) return -1;
-        router_exact_small_kernel<<<dim3((rows + 31) / 32, (unsigned)tokens), 32, smem, stream>>>(router, srouter, x, logits, shared_logit, status);
-        LAUNCHED("router_exact_small_kernel");
     } else if (tokens > 16 && router.k_logical % 64 == 0 && ((uintptr_t)x & 15u) == 0 && router.row_bytes % 16 == 0) {
 #define ROUTER_GEMM(TI, TJ) do { \
         const dim3 grid((unsigned)((tokens + 16 * TI - 1) / (16 * TI)), (rows + 16 * TJ - 1) / (16 * TJ)); \
