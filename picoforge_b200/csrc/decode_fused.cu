@@ -66,8 +66,9 @@ constexpr uint32_t FZP = FMAXE + 4;             // pitch of a logit row in share
 constexpr int CROWS = 32;                       // router rows per chain CTA (lane = row).  64 rows (two chain warps per token, nine
                                                 // chain CTAs) evened out the streaming CTAs' shares but ran the chains at 42 k cycles
                                                 // instead of 25 k, and the step at 44.4 us instead of 42.0
-constexpr int CSTG = 16;                        // chunks in flight in a chain CTA
-constexpr int CCH = 64;                         // columns per chunk: 256 bytes per row
+constexpr int CCH = 512;                        // columns per chunk: a bulk copy of 2 KB per row
+constexpr int CSTG = 2;                         // chunks in flight in a chain CTA: 128 KB, half of K = 2048, before the first addition
+constexpr uint32_t CPITCH = CCH * 4 + 16;       // bytes per row of a chunk: the pad keeps the lanes' 128-bit reads apart
 // words of the sync array
 enum : uint32_t { S_FAST = 0, S_CHAIN = 1, S_ROUTED = 2, S_ACT0 = 3, S_ACT1 = 4, S_EXITS = 5, S_ROUTE_FAIL = 6, S_CLOCKS = 8, S_REPAIRS = 48, S_MARKS = 256 };
 
@@ -157,19 +158,18 @@ __host__ __device__ inline FPlan make_fplan(uint32_t hidden, uint32_t inter_max,
     return p;
 }
 // Shared-memory plan of a chain CTA.
-struct CPlan { uint32_t bars, misc, ids, wts, xf, xf_pitch, ring, zs, total; };
+struct CPlan { uint32_t bars, misc, xf, xf_pitch, ring, route, total; };
 __host__ __device__ inline CPlan make_cplan(uint32_t hidden) {
     CPlan p;
     uint32_t at = 0;
     p.bars = at; at += 512;
-    p.misc = at; at += 1024;
-    p.ids = at; at += FMAXK * 4 * FTOK;
-    p.wts = at; at += FMAXK * 4 * FTOK;
+    p.misc = at; at += 512;
     p.xf_pitch = hidden * 4 + 16;
     p.xf = at; at += FTOK * p.xf_pitch;
     at = (at + 127) & ~127u;
-    p.ring = at; at += CSTG * CROWS * CCH * 4;
-    p.zs = at; at += FTOK * FZP * 4;
+    p.ring = at; p.route = at;                  // the routing starts when the chains are done
+    const uint32_t ring = CSTG * CROWS * CPITCH, route = (uint32_t)sizeof(RouteShared) + RT_PITCH * 4;
+    at += ring > route ? ring : route;
     p.total = at;
     return p;
 }
@@ -627,179 +627,6 @@ __device__ __forceinline__ float fast_sigmoid(float v) {
     return v >= 0.0f ? __fdividef(1.0f, 1.0f + e) : __fdividef(e, 1.0f + e);
 }
 
-// Top-k of up to 32 * PL ordered keys held in registers, one warp: lane L holds the keys of elements
-// L, L + 32, ... (0: absent).  Sequential selection (k dependent warp reductions) costs a lone warp
-// several hundred cycles per round, so the work is arranged in parallel steps instead:
-//   1. every lane's maximum, and the k-th largest of those 32 maxima: at least k elements reach it;
-//   2. the elements that reach it (typically a dozen or two) are compacted into `cand` (shared memory);
-//   3. every candidate counts the candidates that beat it (larger key, or equal key and lower element):
-//      that count is its place, and places below k are written out.
-// Returns false when more than 64 elements qualify (heavy ties): the caller then selects sequentially.
-// cand: 128 words.  ids_out[place] = element, keys_out[place] = key (either may alias nothing else).
-template <int PL>
-__device__ __forceinline__ bool warp_topk(const uint32_t (&key)[PL], uint32_t lane, uint32_t k, uint32_t *cand, uint32_t *ids_out,
-                                          uint32_t *keys_out) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int i = 0; i < PL; i++) m = max(m, key[i]);
-    uint32_t ahead = 0;                                                     // lanes whose maximum beats this lane's
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-        const uint32_t v = __shfl_sync(0xffffffffu, m, j);
-        ahead += (v > m || (v == m && (uint32_t)j < lane)) ? 1u : 0u;
-    }
-    const uint32_t holder = __ballot_sync(0xffffffffu, ahead == min(k, 32u) - 1u);
-    const uint32_t bound = max(__shfl_sync(0xffffffffu, m, __ffs(holder) - 1), 1u);
-    uint32_t count = 0;
-    const uint32_t below = (1u << lane) - 1u;
-#pragma unroll
-    for (int i = 0; i < PL; i++) {
-        const bool in = key[i] >= bound;
-        const uint32_t votes = __ballot_sync(0xffffffffu, in);
-        const uint32_t at = count + __popc(votes & below);
-        if (in && at < 64) { cand[at] = key[i]; cand[64 + at] = lane + 32u * i; }
-        count += __popc(votes);
-    }
-    if (count > 64) return false;
-    __syncwarp();
-    const uint32_t k0 = lane < count ? cand[lane] : 0u, e0 = cand[64 + lane];
-    const uint32_t k1 = lane + 32 < count ? cand[lane + 32] : 0u, e1 = cand[96 + lane];
-    uint32_t place0 = 0, place1 = 0;
-#pragma unroll 4
-    for (uint32_t j = 0; j < count; j++) {
-        const uint32_t kj = cand[j], ej = cand[64 + j];
-        place0 += (kj > k0 || (kj == k0 && ej < e0)) ? 1u : 0u;
-        place1 += (kj > k1 || (kj == k1 && ej < e1)) ? 1u : 0u;
-    }
-    if (lane < count && place0 < k) { ids_out[place0] = e0; if (keys_out) keys_out[place0] = k0; }
-    if (lane + 32 < count && place1 < k) { ids_out[place1] = e1; if (keys_out) keys_out[place1] = k1; }
-    __syncwarp();
-    return true;
-}
-// The sequential form: every lane keeps its best three (key, element) pairs, so a selection step is one
-// warp maximum and a ballot, and a lane rescans its registers only when it has won three times.
-template <int PL>
-__device__ __forceinline__ void topk_scan(const uint32_t (&key)[PL], uint32_t lane, uint32_t &b1, uint32_t &e1, uint32_t &b2, uint32_t &e2,
-                                          uint32_t &b3, uint32_t &e3) {
-    b1 = 0; e1 = 0xffffffffu; b2 = 0; e2 = 0xffffffffu; b3 = 0; e3 = 0xffffffffu;
-#pragma unroll
-    for (int i = 0; i < PL; i++) {                                         // ascending element: the lowest wins among equals
-        const uint32_t k = key[i], e = lane + 32u * i;
-        if (k > b1) { b3 = b2; e3 = e2; b2 = b1; e2 = e1; b1 = k; e1 = e; }
-        else if (k > b2) { b3 = b2; e3 = e2; b2 = k; e2 = e; }
-        else if (k > b3) { b3 = k; e3 = e; }
-    }
-}
-template <int PL>
-__device__ __forceinline__ void topk_clear(uint32_t (&key)[PL], uint32_t index) {
-#pragma unroll
-    for (int i = 0; i < PL; i++) if ((uint32_t)i == index) key[i] = 0;
-}
-template <int PL>
-__device__ __noinline__ void warp_topk_sequential(uint32_t (&key)[PL], uint32_t lane, uint32_t k, uint32_t *ids_out, uint32_t *keys_out) {
-    uint32_t b1, e1, b2, e2, b3, e3, spare = 2;
-    topk_scan<PL>(key, lane, b1, e1, b2, e2, b3, e3);
-#pragma unroll 1
-    for (uint32_t slot = 0; slot < k; slot++) {
-        const uint32_t top = __reduce_max_sync(0xffffffffu, b1);
-        const uint32_t e_win = __reduce_min_sync(0xffffffffu, b1 == top ? e1 : 0xffffffffu);
-        if (lane == 0) { ids_out[slot] = e_win; if (keys_out) keys_out[slot] = top; }
-        if ((e_win & 31u) == lane) {
-            topk_clear<PL>(key, e_win >> 5);
-            if (spare) { b1 = b2; e1 = e2; b2 = b3; e2 = e3; spare--; }
-            else { topk_scan<PL>(key, lane, b1, e1, b2, e2, b3, e3); spare = 2; }
-        }
-    }
-    __syncwarp();
-}
-
-// Softmax, top-k and renormalisation of ONE row of logits in shared memory (zs), CTA-wide;
-// src/qwen4_moe.c:209-247 with its order of operations: ties go to the lower id, and with `exact`
-// the exp-sum runs serially over e = 0..E-1 (the reference's bits); otherwise it is a warp tree
-// sum.  Returns false (CTA-uniform) when a logit is not finite; the row is recorded.
-__device__ __forceinline__ bool route_row(float *zs, uint32_t E, uint32_t k, int norm, uint32_t row, bool exact, uint32_t *ids_s, float *wts_s,
-                                       float *scratch, const unsigned long long *exp_table, uint32_t *flag, uint32_t *status) {
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    if (tid == 0) *flag = 1;
-    __syncthreads();
-    if (warp == 0) {                                                      // row maximum and finiteness
-        float m = -CUDART_INF_F;
-        bool bad = false;
-#pragma unroll 4
-        for (uint32_t e = lane; e < E; e += 32) { const float v = zs[e]; bad |= !finite_f32(v); m = fmaxf(m, v); }
-        for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        bad = __any_sync(0xffffffffu, bad);
-        if (lane == 0) {
-            scratch[0] = m;
-            if (bad) { atomicOr(status, QW4SH_ERR_NONFINITE); atomicMin(status + 1, row); *flag = 0; }
-        }
-    }
-    __syncthreads();
-    if (!*flag) return false;
-    {
-        const float m = scratch[0];
-#pragma unroll 1
-        for (uint32_t e = tid; e < E; e += FT) zs[e] = expf_libm_table(__fsub_rn(zs[e], m), exp_table);   // p = expf(z - max)
-    }
-    __syncthreads();
-    if (warp == 0) {
-        float sum = 0.0f;
-        if (exact) {
-            if (lane == 0) {                                               // the reference's serial sum
-                // 32 values per pass: the loads of the next pass are issued before the 32 dependent adds of this
-                // one, and the loop overhead hides under the add chain
-                uint32_t e = 0;
-                float4 v[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = E >= 32 ? *reinterpret_cast<const float4 *>(zs + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-                for (; e + 32 <= E; e += 32) {
-                    float4 w[8];
-#pragma unroll
-                    for (int j = 0; j < 8; j++) w[j] = e + 64 <= E ? *reinterpret_cast<const float4 *>(zs + e + 32 + 4 * j) : v[j];
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        sum = __fadd_rn(sum, v[j].x); sum = __fadd_rn(sum, v[j].y); sum = __fadd_rn(sum, v[j].z); sum = __fadd_rn(sum, v[j].w);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] = w[j];
-                }
-                for (; e < E; e++) sum = __fadd_rn(sum, zs[e]);
-            }
-            sum = __shfl_sync(0xffffffffu, sum, 0);
-        } else {
-#pragma unroll 4
-            for (uint32_t e = lane; e < E; e += 32) sum += zs[e];
-            for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        }
-        if (lane == 0) scratch[1] = sum;
-    }
-    __syncthreads();
-    {
-        const float sum = scratch[1];
-#pragma unroll 1
-        for (uint32_t e = tid; e < E; e += FT) zs[e] = __fdiv_rn(zs[e], sum);
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // keys: bits of p / sum (>= 0, so ordered as integers) + 1
-        constexpr int PL = FMAXE / 32;
-        uint32_t key[PL];
-#pragma unroll
-        for (int i = 0; i < PL; i++) { const uint32_t e = lane + 32u * i; key[i] = e < E ? __float_as_uint(zs[e]) + 1u : 0u; }
-        __syncwarp();
-        uint32_t *cand = reinterpret_cast<uint32_t *>(zs), *keys_out = cand + 128;     // the probabilities are in registers now
-        if (!warp_topk<PL>(key, lane, k, cand, ids_s, keys_out)) warp_topk_sequential<PL>(key, lane, k, ids_s, keys_out);
-        const float mine = lane < k ? __uint_as_float(keys_out[lane] - 1u) : 0.0f;
-        float selected = 0.0f;
-#pragma unroll 1
-        for (uint32_t slot = 0; slot < k; slot++) selected = __fadd_rn(selected, __shfl_sync(0xffffffffu, mine, slot));   // slot order
-        if (lane < k) wts_s[lane] = norm ? __fdiv_rn(mine, selected) : mine;
-    }
-    __syncthreads();
-    return true;
-}
-
 // The k largest of one row of logits by VALUE (ties to the lower id), one warp; the row is turned
 // read into ordered integer keys (its memory then serves as scratch).  `extra`: choose k + 1 and put the last one in slot k - 1 (a
 // deliberately wrong set, for the test of the repair path).  Returns false on a nonfinite logit.
@@ -840,6 +667,12 @@ __device__ __forceinline__ bool speculate_row(float *zs, uint32_t E, uint32_t k,
 // ---- chain CTA -----------------------------------------------------------------------------------
 // Exact logits of router rows [32 c, 32 c + 32) (row E is the shared expert's router) for every
 // token, then, in CTA t < T, the routing of token t.
+//
+// A chain is H dependent additions of four cycles (8.2 k cycles at H = 2048), and everything else of it is kept under them: the
+// rows come by bulk copies of 512 columns, two chunks at once, and a lane reads the operands of
+// the next sixteen columns while the products of the current ones are added.  (Before: 64-column chunks through a
+// 16-stage cp.async ring, with a barrier wait and exposed read latency per chunk: 20 k cycles with resident
+// rows, 35 k when the rows came from HBM.)
 __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
     const uint32_t T = a.tokens, H = a.hidden, E = a.experts, k = a.top_k;
     const CPlan p = make_cplan(H);
@@ -847,53 +680,45 @@ __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + p.bars);              // [CSTG]
     uint64_t *empty = full + CSTG;                                             // [CSTG]
     uint64_t *xbar = empty + CSTG;
-    float *misc_f = reinterpret_cast<float *>(smem + p.misc);
-    uint32_t *misc_u = reinterpret_cast<uint32_t *>(smem + p.misc) + 16;
-    unsigned long long *exp_table = reinterpret_cast<unsigned long long *>(smem + p.misc + 256);
+    uint32_t *misc_u = reinterpret_cast<uint32_t *>(smem + p.misc);
     const bool exact = a.router_mode != 1;
-    const uint32_t loaders = 64;                                               // two loader warps: the rest sleep at the CTA barrier
-    if (tid < CSTG) { fbar_init(&full[tid], loaders); fbar_init(&empty[tid], T); }
+    if (tid < CSTG) { fbar_init(&full[tid], 1); fbar_init(&empty[tid], T); }
     if (tid == CSTG) fbar_init(xbar, 1);
     if (tid <= CSTG) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (tid < 32) exp_table[tid] = c_exp2_table[tid];
     __syncthreads();
     const uint32_t r0 = cta * CROWS;
     const uint32_t nr = exact && r0 <= E ? min((uint32_t)CROWS, E + 1 - r0) : 0;
+    const uint32_t chunks = (H + CCH - 1) / CCH;
+    uint8_t *ring = smem + p.ring;
     bool alive = true;
-    if (nr && warp >= T && warp < T + 2) {
-        // loader warps (weights only: they start before the previous launch has drained): 16-byte pieces of the
-        // chunk, piece q of row r stored at position q ^ (r & 7)
-        uint8_t *ring = smem + p.ring;
-        const uint32_t lt = tid - 32 * T, pieces = nr * (CCH / 4), chunks = H / CCH;
-#pragma unroll 1
-        for (uint32_t i = 0; i < chunks && alive; i++) {
-            const uint32_t st = i % CSTG;
-            if (i >= CSTG) {
-                const uint32_t parity = ((i / CSTG) - 1u) & 1u;
-                const long long start = clock64();
-                while (!fbar_try(&empty[st], parity)) {                         // the chain warps share the schedulers: poll gently
-                    __nanosleep(200);
-                    if (clock64() - start > (1ll << 31)) { atomicOr(a.status, QW4SH_ERR_STATE); alive = false; break; }
-                }
-            }
-            if (!alive) break;
-#pragma unroll 1
-            for (uint32_t pc = lt; pc < pieces; pc += loaders) {
-                const uint32_t r = pc / (CCH / 4), q = pc % (CCH / 4), gr = r0 + r;
-                const uint8_t *src = (gr < E ? a.w[0].data + (uint64_t)gr * a.w[0].row_bytes : a.w[7].data) + (uint64_t)i * (CCH * 4) + q * 16u;
-                const uint32_t dst = fs_u32(ring + (st * CROWS + r) * (CCH * 4) + ((q ^ (r & 7u)) << 4));
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(fs_u32(&full[st])) : "memory");
-        }
-    }
+    auto issue = [&](uint32_t c) {                                             // by warp T: lane = row
+        const uint32_t st = c % CSTG, bytes = min((uint32_t)CCH, H - c * CCH) * 4u, gr = r0 + lane;
+        if (lane == 0) fbar_expect(&full[st], bytes * nr);
+        __syncwarp();
+        if (lane < nr)
+            fbulk(ring + (st * CROWS + lane) * CPITCH, (gr < E ? a.w[0].data + (uint64_t)gr * a.w[0].row_bytes : a.w[7].data) + (uint64_t)c * CCH * 4, bytes, &full[st]);
+    };
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tid == 0) a.t0 = clock64();                                            // read back by thread 0 only
+    if (nr && warp == T) {
+        // not before the previous launch has drained: its last phase is bound by memory, and the chains have slack (ahead of the
+        // wait, four tokens took 40.9 us a layer instead of 40.0)
+        for (uint32_t c = 0; c < CSTG && c < chunks; c++) issue(c);
+        for (uint32_t c = CSTG; c < chunks && alive; c++) {
+            const long long start = clock64();
+            while (alive && !fbar_try(&empty[c % CSTG], (c / CSTG - 1u) & 1u)) {
+                __nanosleep(100);                                              // the chain warps share the schedulers: poll gently
+                if (clock64() - start > (1ll << 31)) { atomicOr(a.status, QW4SH_ERR_STATE); alive = false; }
+            }
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            fproxy_fence();
+            issue(c);
+        }
+    }
     if (nr && warp < T) {
         // chain warp: token = warp, lane = row.  Multiplies and adds are separately rounded.
         uint8_t *xf = smem + p.xf;
-        const uint8_t *ring = smem + p.ring;
-        const uint32_t chunks = H / CCH;
         if (tid == 0) {
             fbar_expect(xbar, T * H * 4u);
             for (uint32_t q = 0; q < T; q++) fbulk(xf + q * p.xf_pitch, a.x + (uint64_t)q * H, H * 4u, xbar);
@@ -901,29 +726,40 @@ __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
         alive = fbar_wait(xbar, 0, a.status);
         MARK(2);
         long long waited = 0;
-        const float4 *xv = reinterpret_cast<const float4 *>(xf + warp * p.xf_pitch);
         float sum = 0.0f;
 #pragma unroll 1
-        for (uint32_t i = 0; i < chunks; i++) {
-            const uint32_t st = i % CSTG;
+        for (uint32_t c = 0; c < chunks; c++) {
+            const uint32_t st = c % CSTG;
             const long long w0 = clock64();
-            if (alive) alive = fbar_wait(&full[st], (i / CSTG) & 1u, a.status);
+            if (alive) alive = fbar_wait(&full[st], (c / CSTG) & 1u, a.status);
             alive = __all_sync(0xffffffffu, alive);
             waited += clock64() - w0;
             if (!alive) break;
-            const uint8_t *row = ring + (st * CROWS + lane) * (CCH * 4);
-            // a lone warp issues every other cycle: the products go two at a time (mul.rn.f32x2 rounds each half
-            // like a scalar multiply), which leaves load + 2 packed multiplies + 4 adds per four columns, just
-            // under the adds' own latency
+            const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(ring + (st * CROWS + lane) * CPITCH);
+            const ulonglong2 *v = reinterpret_cast<const ulonglong2 *>(xf + warp * p.xf_pitch) + c * (CCH / 4);
+            const uint32_t quads = min((uint32_t)CCH, H - c * CCH) / 4;       // a multiple of four
+            ulonglong2 wa[4], va[4];
 #pragma unroll
-            for (uint32_t q = 0; q < CCH / 4; q++) {
-                const ulonglong2 w4 = *reinterpret_cast<const ulonglong2 *>(row + ((q ^ (lane & 7u)) << 4));
-                const ulonglong2 x4 = *reinterpret_cast<const ulonglong2 *>(&xv[i * (CCH / 4) + q]);
-                unsigned long long p01, p23;
-                asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p01) : "l"(w4.x), "l"(x4.x));
-                asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p23) : "l"(w4.y), "l"(x4.y));
-                sum = __fadd_rn(sum, __uint_as_float((uint32_t)p01)); sum = __fadd_rn(sum, __uint_as_float((uint32_t)(p01 >> 32)));
-                sum = __fadd_rn(sum, __uint_as_float((uint32_t)p23)); sum = __fadd_rn(sum, __uint_as_float((uint32_t)(p23 >> 32)));
+            for (int j = 0; j < 4; j++) { wa[j] = w[j]; va[j] = v[j]; }
+            // a lone warp issues every other cycle: the products go two at a time (mul.rn.f32x2 rounds each half
+            // like a scalar multiply), which leaves two loads + 2 packed multiplies + 4 adds per four columns, just
+            // under the adds' own latency
+#pragma unroll 2
+            for (uint32_t q = 0; q < quads; q += 4) {
+                ulonglong2 wb[4], vb[4];
+                const uint32_t next = q + 4 < quads ? q + 4 : q;
+#pragma unroll
+                for (int j = 0; j < 4; j++) { wb[j] = w[next + j]; vb[j] = v[next + j]; }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    unsigned long long p01, p23;
+                    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p01) : "l"(wa[j].x), "l"(va[j].x));
+                    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p23) : "l"(wa[j].y), "l"(va[j].y));
+                    sum = __fadd_rn(sum, __uint_as_float((uint32_t)p01)); sum = __fadd_rn(sum, __uint_as_float((uint32_t)(p01 >> 32)));
+                    sum = __fadd_rn(sum, __uint_as_float((uint32_t)p23)); sum = __fadd_rn(sum, __uint_as_float((uint32_t)(p23 >> 32)));
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) { wa[j] = wb[j]; va[j] = vb[j]; }
             }
             __syncwarp();
             if (lane == 0) fbar_arrive(&empty[st]);
@@ -942,27 +778,20 @@ __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
     const uint32_t waited = exact ? S_CHAIN : S_FAST;
     const uint32_t expected = exact ? a.chain_ctas : gridDim.x - a.chain_ctas;
     bool ok = wait_counter(a.sync + waited, expected, a.status, misc_u);
-    float *zs = reinterpret_cast<float *>(smem + p.zs);
-    uint32_t *ids_s = reinterpret_cast<uint32_t *>(smem + p.ids);
-    float *wts_s = reinterpret_cast<float *>(smem + p.wts);
     if (ok) {
         const float *from = exact ? a.logits + (uint64_t)cta * E : a.logits_fast + (uint64_t)cta * a.fast_pitch;
-#pragma unroll 1
-        for (uint32_t e = tid; e < E; e += FT) {
-            const float v = __ldcg(from + e);
-            zs[e] = v;
-            if (!exact) a.logits[(uint64_t)cta * E + e] = v;
+        if (!exact) {
+            for (uint32_t e = tid; e < E; e += FT) a.logits[(uint64_t)cta * E + e] = __ldcg(from + e);
+            if (tid == 0) a.shared_logit[cta] = __ldcg(from + E);
         }
-        if (!exact && tid == 0) a.shared_logit[cta] = __ldcg(a.logits_fast + (uint64_t)cta * a.fast_pitch + E);
-        __syncthreads();
-        ok = route_row(zs, E, k, a.norm, cta, exact, ids_s, wts_s, misc_f + 8, exp_table, misc_u + 1, a.status);
-    }
-    if (ok && tid < k) {
-        const uint32_t e = ids_s[tid];
-        const float w = wts_s[tid];
-        a.ids[cta * k + tid] = e; a.weights[cta * k + tid] = w;
-        if (a.ids_out) a.ids_out[cta * k + tid] = e;
-        if (a.weights_out) a.weights_out[cta * k + tid] = w;
+        RouteShared &rs = *reinterpret_cast<RouteShared *>(smem + p.route);
+        ok = route_rows<FW>(cta, 1, E, k, a.norm, exact, reinterpret_cast<float *>(smem + p.route + sizeof(RouteShared)), rs, a.status, nullptr,
+                            [&](uint32_t, uint32_t e) { return __ldcg(from + e); },
+                            [&](uint32_t t, uint32_t slot, uint32_t id, float w) {
+                                a.ids[t * k + slot] = id; a.weights[t * k + slot] = w;
+                                if (a.ids_out) a.ids_out[t * k + slot] = id;
+                                if (a.weights_out) a.weights_out[t * k + slot] = w;
+                            }) == 0;
     }
     if (!ok && tid == 0) atomicOr(a.sync + S_ROUTE_FAIL, 1u);
     __threadfence();

@@ -304,7 +304,9 @@ __global__ void __launch_bounds__(ROWS * TOK) router_chain_kernel(DevTensor rout
         }
     };
     if (tid < 32) for (uint32_t c = 0; c < STAGES && c < chunks; c++) issue(c);
-    const uint32_t er = tid / TOK, tc = tid % TOK;
+    // a warp is 8 rows x 4 tokens (4 x 8 in the narrowest tile): its 128-bit reads of either operand then take one pass over the banks
+    constexpr uint32_t WR = ROWS < 8 ? ROWS : 8, WT = 32 / WR;
+    const uint32_t wi = tid >> 5, li = tid & 31u, er = wi % (ROWS / WR) * WR + li / WT, tc = wi / (ROWS / WR) * WT + li % WT;
     float sum = 0.0f;
     bool alive = true;
     for (uint32_t c = 0; c < chunks; c++) {
@@ -502,7 +504,7 @@ __device__ __forceinline__ void route_token(uint32_t experts, uint32_t k, int no
     for (uint32_t e = lane; e < experts; e += 32) {
         const float v = __fdiv_rn(p[e], sum);
         p[e] = v;
-        probs[(uint64_t)t * experts + e] = v;
+        if (probs) probs[(uint64_t)t * experts + e] = v;
     }
     __syncwarp();
     float selected = 0.0f;
@@ -529,6 +531,7 @@ __device__ __forceinline__ void route_token(uint32_t experts, uint32_t k, int no
             weights[(uint64_t)t * k + slot] = __fdiv_rn(weights[(uint64_t)t * k + slot], selected);
 }
 
+// Shapes beyond route_batch_kernel's (more than 512 experts or k > 32): one warp per token.
 __global__ void __launch_bounds__(128) route_kernel(uint32_t experts, uint32_t k, int norm, const float *__restrict__ logits,
                                                     uint64_t pitch, uint32_t tokens, float *__restrict__ probs,
                                                     uint32_t *__restrict__ ids, float *__restrict__ weights, uint32_t *status) {
@@ -536,164 +539,106 @@ __global__ void __launch_bounds__(128) route_kernel(uint32_t experts, uint32_t k
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, warps = blockDim.x >> 5;
     const uint32_t t = blockIdx.x * warps + warp;
     if (t >= tokens) return;
-    if (experts <= 512 && k <= 32) route_token_regs<16>(experts, k, norm, logits + (uint64_t)t * pitch, t, probs, ids, weights, status, lane);
-    else route_token(experts, k, norm, logits + (uint64_t)t * pitch, t, route_smem + (uint64_t)warp * experts, probs, ids, weights, status, lane);
+    route_token(experts, k, norm, logits + (uint64_t)t * pitch, t, route_smem + (uint64_t)warp * experts, probs, ids, weights, status, lane);
 }
 
-// Few tokens: one CTA of 512 threads per token routes it (thread e owns expert e, experts <=
-// 512), and the CTA that finishes last builds the stable per-expert lists and the groups of
-// <= 4 rows for all tokens (no CTA waits for another: the last one to arrive is found with an
-// atomic counter).  One lone warp per token would be bound by its own instruction latency;
-// spreading exp, division and the k arg-max rounds over 16 warps leaves only the exp-sum serial
-// (512 dependent additions in expert order, the reference's order).
+// Routes of a batch (experts <= 512, k <= 32), each CTA `per` tokens (route_rows above), and, where `offsets` is given, the
+// dispatch of all of them: the stable per-expert lists (src/qwen4_moe.c:285-301; order inside an expert by ascending pair) and
+// the groups of up to 2^group_log rows that the expert products walk.  The CTA that arrives last at an atomic counter builds them; no CTA
+// waits for another.  An expert takes a token at most once, so its list is a set of tokens: one bit per (expert, token)
+// in shared memory, a prefix count per word, and a pair's row is its expert's first row plus the bits below its token.
+// All of it is latency, not work (2048 tokens: 20480 pairs, 40 per thread), which is why it is one launch: 1024 tokens took 17 us to route
+// with a warp per token, 22 us in a clear and four launches for the lists and 4 us for the groups.
 struct Group4 { uint32_t expert, first, count, pad; };
-__global__ void __launch_bounds__(512) route_group_small_kernel(uint32_t experts, uint32_t k, int norm, const float *__restrict__ logits,
-                                                                uint32_t tokens, float *__restrict__ probs, uint32_t *__restrict__ ids,
-                                                                float *__restrict__ weights, uint32_t *__restrict__ offsets,
-                                                                uint32_t *__restrict__ pair_to_row, uint32_t *__restrict__ row_to_pair,
-                                                                uint32_t *__restrict__ active, Group4 *__restrict__ groups,
-                                                                uint32_t *__restrict__ n_groups, uint32_t *status) {
-    __shared__ __align__(16) float p[512];
-    __shared__ float wred[16];
-    __shared__ float s_sum;
-    __shared__ uint32_t s_bad, s_last, wsum[16];
-    extern __shared__ uint32_t sids[];                         // [tokens * k] for the dispatch step
-    const uint32_t t = blockIdx.x, e = threadIdx.x, lane = e & 31u, warp = e >> 5;
-    if (e == 0) s_bad = 0;
-    __syncthreads();
-    float z = e < experts ? logits[(uint64_t)t * experts + e] : -CUDART_INF_F;
-    if (e < experts && !finite_f32(z)) s_bad = 1;
-    float m = z;
-    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) wred[warp] = m;
-    __syncthreads();
-    const bool bad = s_bad != 0;
-    if (bad && e == 0) { atomicOr(status, QW4SH_ERR_NONFINITE); atomicMin(status + 1, t); }
-    float value = -1.0f;
-    if (!bad) {
-        float maximum = wred[0];
-        for (int w = 1; w < 16; w++) maximum = fmaxf(maximum, wred[w]);
-        p[e] = e < experts ? expf_libm(__fsub_rn(z, maximum)) : 0.0f;
-        __syncthreads();
-        if (e == 0) {                                          // the reference's serial sum, e = 0, 1, 2, ...
-            float sum = 0.0f;
-            uint32_t i = 0;
-            for (; i + 16 <= experts; i += 16) {
-                const float4 a = *reinterpret_cast<const float4 *>(p + i), b = *reinterpret_cast<const float4 *>(p + i + 4);
-                const float4 c = *reinterpret_cast<const float4 *>(p + i + 8), d = *reinterpret_cast<const float4 *>(p + i + 12);
-                sum = __fadd_rn(sum, a.x); sum = __fadd_rn(sum, a.y); sum = __fadd_rn(sum, a.z); sum = __fadd_rn(sum, a.w);
-                sum = __fadd_rn(sum, b.x); sum = __fadd_rn(sum, b.y); sum = __fadd_rn(sum, b.z); sum = __fadd_rn(sum, b.w);
-                sum = __fadd_rn(sum, c.x); sum = __fadd_rn(sum, c.y); sum = __fadd_rn(sum, c.z); sum = __fadd_rn(sum, c.w);
-                sum = __fadd_rn(sum, d.x); sum = __fadd_rn(sum, d.y); sum = __fadd_rn(sum, d.z); sum = __fadd_rn(sum, d.w);
-            }
-            for (; i < experts; i++) sum = __fadd_rn(sum, p[i]);
-            s_sum = sum;
-        }
-        __syncthreads();
-        if (e < experts) { value = __fdiv_rn(p[e], s_sum); probs[(uint64_t)t * experts + e] = value; }
-        // Selection by one warp over the row in shared memory: lane L owns experts L, L + 32, ... and keeps the best
-        // three of them in registers (keys: float bits + 1, a chosen entry becomes -1 = key 0), so a slot costs two
-        // warp reductions; a lane rescans its experts only when it wins a third time after its last scan.  Ties go
-        // to the lower id, the sum of the chosen probabilities runs in slot order (the reference's order).
-        __syncthreads();                                       // every thread has read its exp value out of p
-        p[e] = e < experts ? value : -1.0f;
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t b1, e1, b2, e2, b3, e3;
-            auto scan3 = [&]() {
-                b1 = 0; e1 = 0xffffffffu; b2 = 0; e2 = 0xffffffffu; b3 = 0; e3 = 0xffffffffu;
-#pragma unroll 4
-                for (uint32_t i = lane; i < experts; i += 32) {            // ascending ids: the lowest wins among equals
-                    const float v = p[i];
-                    const uint32_t key = v < 0.0f ? 0u : __float_as_uint(v) + 1u;
-                    if (key > b1) { b3 = b2; e3 = e2; b2 = b1; e2 = e1; b1 = key; e1 = i; }
-                    else if (key > b2) { b3 = b2; e3 = e2; b2 = key; e2 = i; }
-                    else if (key > b3) { b3 = key; e3 = i; }
-                }
-            };
-            scan3();
-            uint32_t spare = 2;
-            float selected = 0.0f;
-            for (uint32_t slot = 0; slot < k; slot++) {
-                const uint32_t top = __reduce_max_sync(0xffffffffu, b1);
-                const uint32_t e_win = __reduce_min_sync(0xffffffffu, b1 == top ? e1 : 0xffffffffu);
-                const float best = __uint_as_float(top - 1u);
-                if (lane == 0) { ids[(uint64_t)t * k + slot] = e_win; sids[slot] = top - 1u; }    // sids: free until the dispatch step
-                if ((e_win & 31u) == lane) {
-                    p[e_win] = -1.0f;
-                    if (spare) { b1 = b2; e1 = e2; b2 = b3; e2 = e3; spare--; }
-                    else { scan3(); spare = 2; }
-                }
-                selected = __fadd_rn(selected, best);
-            }
-            __syncwarp();
-            for (uint32_t slot = lane; slot < k; slot += 32) {
-                const float raw = __uint_as_float(sids[slot]);
-                weights[(uint64_t)t * k + slot] = norm ? __fdiv_rn(raw, selected) : raw;
-            }
-        }
-    }
+struct RouteArgs {
+    const float *logits;
+    uint64_t pitch;
+    uint32_t experts, k, tokens, per;
+    int norm;
+    float *probs;                                               // nullptr: not wanted
+    uint32_t *ids; float *weights;
+    uint32_t *ids_out; float *weights_out;                      // a caller's copies, or nullptr
+    uint32_t *status;
+    uint32_t *offsets, *pair_to_row, *row_to_pair, *active;     // offsets nullptr: routes only
+    Group4 *groups; uint32_t *n_groups, group_log;
+    Group4 *dense; uint32_t *n_dense;                           // the shared expert's groups: all rows in turn (or nullptr)
+    uint32_t *ticket;                                           // zero between launches
+};
+static size_t route_smem_bytes(size_t tokens, uint32_t per, bool dispatch) {
+    const size_t route = sizeof(RouteShared) + (size_t)per * RT_PITCH * 4, words = ((tokens + 31) / 32) | 1;
+    const size_t lists = dispatch ? 512 * words * 6 : 0;
+    return route > lists ? route : lists;
+}
+__global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant__ RouteArgs a) {
+    extern __shared__ __align__(16) uint8_t rb_smem[];
+    __shared__ uint32_t s_last, wrows[16], wgroups[16], s_first[512];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, E = a.experts, k = a.k;
+    const uint32_t row0 = blockIdx.x * a.per;
+    route_rows<16>(row0, min(a.per, a.tokens - row0), E, k, a.norm, true, reinterpret_cast<float *>(rb_smem + sizeof(RouteShared)),
+                   *reinterpret_cast<RouteShared *>(rb_smem), a.status, a.probs,
+                   [&](uint32_t t, uint32_t e) { return __ldg(a.logits + (uint64_t)t * a.pitch + e); },
+                   [&](uint32_t t, uint32_t slot, uint32_t id, float w) {
+                       const uint64_t at = (uint64_t)t * k + slot;
+                       a.ids[at] = id; a.weights[at] = w;
+                       if (a.ids_out) a.ids_out[at] = id;
+                       if (a.weights_out) a.weights_out[at] = w;
+                   });
+    if (!a.offsets) return;
     // ---- the CTA that arrives last does the dispatch for all tokens ----
     __threadfence();
     __syncthreads();
-    if (e == 0) s_last = atomicAdd(n_groups + 2, 1u) == tokens - 1 ? 1u : 0u;
+    if (tid == 0) s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
     __syncthreads();
     if (!s_last) return;
-    if (e == 0) n_groups[2] = 0;                                // ready for the next call
+    if (tid == 0) *a.ticket = 0;                                // ready for the next call
     __threadfence();
-    // An expert takes a token at most once, so its list is a 64-bit set of tokens (tokens <= 64): thread q marks
-    // pair q, thread e counts its set, and every pair finds its own row with one popcount.
-    const uint32_t pairs = tokens * k;
-    __shared__ unsigned long long s_tokens[512];
-    __shared__ uint32_t s_first[512];
-    s_tokens[e] = 0ull;
+    const uint32_t words = (a.tokens + 31) / 32, pitch = words | 1u, pairs = a.tokens * k;      // odd pitch: thread e reads words of expert e
+    uint32_t *bits = reinterpret_cast<uint32_t *>(rb_smem);
+    uint16_t *before = reinterpret_cast<uint16_t *>(bits + 512 * pitch);
+    for (uint32_t i = tid; i < 512 * pitch; i += 512) bits[i] = 0;
     __syncthreads();
-    for (uint32_t q = e; q < pairs; q += blockDim.x) {
-        const uint32_t id = __ldcg(ids + q);
-        sids[q] = id;
-        if (id < experts) atomicOr(&s_tokens[id], 1ull << (q / k));
+#pragma unroll 4
+    for (uint32_t q = tid; q < pairs; q += 512) {
+        const uint32_t id = __ldcg(a.ids + q), t = q / k;
+        if (id < E) atomicOr(&bits[id * pitch + (t >> 5)], 1u << (t & 31u));
     }
     __syncthreads();
-    const unsigned long long my_tokens = e < experts ? s_tokens[e] : 0ull;
-    const uint32_t count = __popcll(my_tokens);
-    // packed: bits 0-11 rows, 12-21 groups of four, 22-31 non-empty flag
-    const uint32_t packed = count | (((count + 3) >> 2) << 12) | ((count ? 1u : 0u) << 22);
-    uint32_t scan = packed;
-    for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(0xffffffffu, scan, o); if (lane >= (uint32_t)o) scan += v; }
-    if (lane == 31) wsum[warp] = scan;
+    uint32_t count = 0;
+#pragma unroll 4
+    for (uint32_t w = 0; w < words; w++) { before[tid * pitch + w] = (uint16_t)count; count += __popc(bits[tid * pitch + w]); }
+    const uint32_t per_group = 1u << a.group_log, n_groups = (count + per_group - 1) >> a.group_log;
+    const uint32_t listed = n_groups | (count ? 1u << 20 : 0u);                                // groups, then experts with rows from bit 20
+    uint32_t rows = count, groups = listed;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, rows, o), u = __shfl_up_sync(0xffffffffu, groups, o);
+        if (lane >= (uint32_t)o) { rows += v; groups += u; }
+    }
+    if (lane == 31) { wrows[warp] = rows; wgroups[warp] = groups; }
     __syncthreads();
-    if (warp == 0) {
-        uint32_t v = lane < 16 ? wsum[lane] : 0, sc = v;
-        for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(0xffffffffu, sc, o); if (lane >= (uint32_t)o) sc += u; }
-        if (lane < 16) wsum[lane] = sc - v;
+    for (uint32_t w = 0; w < warp; w++) { rows += wrows[w]; groups += wgroups[w]; }
+    const uint32_t first = rows - count, at = groups - listed;
+    s_first[tid] = first;
+    if (tid < E) {
+        a.offsets[tid] = first;
+        if (count) a.active[1 + (at >> 20)] = tid;
+        for (uint32_t j = 0; j < n_groups; j++)
+            a.groups[(at & 0xfffffu) + j] = Group4{tid, first + (j << a.group_log), min(per_group, count - (j << a.group_log)), 0};
+    }
+    if (tid == 511) { a.offsets[E] = rows; *a.n_groups = groups & 0xfffffu; a.active[0] = groups >> 20; }
+    if (a.dense) {
+        const uint32_t n = (a.tokens + per_group - 1) >> a.group_log;
+        for (uint32_t j = tid; j < n; j += 512) a.dense[j] = Group4{0, j << a.group_log, min(per_group, a.tokens - (j << a.group_log)), 0};
+        if (tid == 0) *a.n_dense = n;
     }
     __syncthreads();
-    const uint32_t exclusive = scan - packed + wsum[warp];
-    const uint32_t first = exclusive & 0xfffu, gfirst = (exclusive >> 12) & 0x3ffu, arank = exclusive >> 22;
-    if (e < experts) {
-        offsets[e] = first;
-        if (count) {
-            active[1 + arank] = e;
-            for (uint32_t j = 0; j < (count + 3) >> 2; j++) groups[gfirst + j] = Group4{e, first + 4 * j, min(4u, count - 4 * j), 0};
+#pragma unroll 4
+    for (uint32_t q = tid; q < pairs; q += 512) {
+        const uint32_t id = __ldcg(a.ids + q), t = q / k;
+        if (id < E) {
+            const uint32_t w = id * pitch + (t >> 5), row = s_first[id] + before[w] + __popc(bits[w] & ((1u << (t & 31u)) - 1u));
+            a.pair_to_row[q] = row; a.row_to_pair[row] = q;
         }
     }
-    // placement by pair: a pair's row is its expert's first row plus the number of lower tokens in the expert's set
-    s_first[e] = first;
-    __syncthreads();
-    for (uint32_t q = e; q < pairs; q += blockDim.x) {
-        const uint32_t id = sids[q];
-        if (id < experts) {
-            const uint32_t row = s_first[id] + __popcll(s_tokens[id] & ((1ull << (q / k)) - 1ull));
-            pair_to_row[q] = row; row_to_pair[row] = q;
-        }
-    }
-    if (e == blockDim.x - 1) {                                   // inclusive total sits in the last thread
-        const uint32_t total = exclusive + packed;
-        offsets[experts] = total & 0xfffu; n_groups[0] = (total >> 12) & 0x3ffu; active[0] = total >> 22;
-    }
-    for (uint32_t j = e; j < (tokens + 3) / 4; j += blockDim.x)   // the shared expert's groups: rows four at a time
-        groups[pairs + j] = Group4{0, 4 * j, min(4u, tokens - 4 * j), 0};
-    if (e == 0) n_groups[1] = (tokens + 3) / 4;
 }
 
 // ------------------------------------------------------------------------------------
@@ -1195,10 +1140,39 @@ static int allow_smem(Kernel kernel, size_t smem) {
     return 0;
 }
 
+static int g_sm_count[64] = {0};
+static int sm_count() {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 148;
+    if (!g_sm_count[device] && cudaDeviceGetAttribute(&g_sm_count[device], cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        g_sm_count[device] = 148;
+    return g_sm_count[device];
+}
+// Tokens per CTA: as few as cover the SMs once, sixteen at most (one lane of a warp sums one row, and one warp ranks one).
+static int launch_route_batch(RouteArgs &a, cudaStream_t stream) {
+    static bool configured[64] = {false};
+    const uint32_t sms = (uint32_t)sm_count();
+    a.per = (a.tokens + sms - 1) / sms;
+    if (a.per > 16) a.per = 16;
+    int device = 0;
+    CU(cudaGetDevice(&device));
+    if (device < 0 || device >= 64) return fail(cudaErrorInvalidDevice, "device index");
+    if (!configured[device]) { if (allow_smem(route_batch_kernel, 220u * 1024u)) return -1; configured[device] = true; }
+    route_batch_kernel<<<(a.tokens + a.per - 1) / a.per, 512, route_smem_bytes(a.tokens, a.per, a.offsets != nullptr), stream>>>(a);
+    LAUNCHED("route_batch_kernel");
+    return 0;
+}
+
 extern "C" int qw4sh_route(uint32_t experts, uint32_t k, int norm, const float *logits, size_t pitch, size_t tokens,
                            float *probs, uint32_t *ids, float *weights, uint32_t *status, void *stream) {
     if (!tokens) return 0;
     if (ensure_constants()) return -1;
+    if (experts <= 512 && k <= 32) {
+        RouteArgs a = {};
+        a.logits = logits; a.pitch = pitch; a.experts = experts; a.k = k; a.tokens = (uint32_t)tokens; a.norm = norm;
+        a.probs = probs; a.ids = ids; a.weights = weights; a.status = status;
+        return launch_route_batch(a, (cudaStream_t)stream);
+    }
     const size_t per_warp = (size_t)experts * sizeof(float);
     int warps = 4;
     while (warps > 1 && per_warp * warps > 96u * 1024u) warps >>= 1;
@@ -1429,14 +1403,6 @@ extern "C" int qw4sh_combine(const float *out, const float *shared_out, const fl
 extern "C" int qw4sh_build_groups(const uint32_t *offsets, const uint32_t *active, void *groups, uint32_t *n_groups, void *stream);
 extern "C" int qw4sh_build_dense_groups(uint32_t tokens, void *groups, uint32_t *n_groups, void *stream);
 
-static int g_sm_count[64] = {0};
-static int sm_count() {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 148;
-    if (!g_sm_count[device] && cudaDeviceGetAttribute(&g_sm_count[device], cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-        g_sm_count[device] = 148;
-    return g_sm_count[device];
-}
 static int g_only_step = -1;                       // profiling: launch just one step of the layer (-1: all)
 extern "C" void qw4sh_set_only_step(int step) { g_only_step = step; }
 #define STEP(id) (g_only_step < 0 || g_only_step == (id))
@@ -1513,15 +1479,6 @@ static int aux_stream(cudaStream_t *stream, cudaEvent_t **events) {
     return 0;
 }
 
-static int launch_route_group_small(const QW4ShLayer *layer, const QW4ShWork *work, uint32_t T, cudaStream_t stream) {
-    const uint32_t E = layer->experts, k = layer->top_k;
-    route_group_small_kernel<<<T, 512, (size_t)T * k * 4, stream>>>(E, k, layer->norm, work->logits, T, work->probs, work->ids,
-                                                                    work->weights, work->offsets, work->pair_to_row, work->row_to_pair,
-                                                                    work->active, (Group4 *)work->groups, work->n_groups, work->status);
-    LAUNCHED("route_group_small_kernel");
-    return 0;
-}
-
 static bool takes_fused(const QW4ShLayer *layer, const QW4ShWork *work, const float *x, const float *y, size_t tokens) {
     return g_only_step < 0 && g_expert_path != 0 && !work->routed && qw4sh_fused_supported(layer, tokens, x, y, sm_count());
 }
@@ -1549,7 +1506,7 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
         (void)cudaGetLastError();
     }
     const bool prefill = prefill_path(layer, tokens), tc = prefill || tile_path(layer, tokens), mma = !tc && mma_path(layer, tokens);
-    const bool fused_route = (tc || mma) && T <= 64 && E <= 512 && k <= E && T * k < 4096;
+    const bool listed = (tc || mma) && E <= 512 && k <= 32 && T <= 2048;      // routes and lists in one launch
     int rc, stage = 0;
 #define STAGE_MARK() do { if (timed) CU(cudaEventRecord(g_stage_event[stage++], stream)); } while (0)
     STAGE_MARK();
@@ -1589,7 +1546,7 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
     auto shared_branch = [&](int which) -> int {
         if (which == 0) {
             if (tc) { if ((rc = qw4sh_build_dense_tile_groups(T, work->shared_groups32, work->n_groups32 + 1, side))) return rc; }
-            else if (!fused_route && (rc = qw4sh_build_dense_groups(T, shared_groups, work->n_groups + 1, side))) return rc;
+            else if (!listed && (rc = qw4sh_build_dense_groups(T, shared_groups, work->n_groups + 1, side))) return rc;
             return STEP(4) ? products(0, true, side) : 0;
         }
         if (mma && STEP(7) && (rc = qw4sh_quantize_rows(work->shared_act, T, layer->shared_inter, work->sq, work->sneg, work->ssum, work->sscale, side))) return rc;
@@ -1597,24 +1554,31 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
     };
     if (STEP(0) && (rc = launch_router(layer, x, tokens, work->logits, work->shared_logit, work->status, router_mode, stream))) return rc;
     STAGE_MARK();
-    if (fused_route) {
-        if (STEP(2) && (rc = launch_route_group_small(layer, work, T, stream))) return rc;
+    if (listed) {
+        RouteArgs a = {};
+        a.logits = work->logits; a.pitch = E; a.experts = E; a.k = k; a.tokens = T; a.norm = layer->norm;
+        a.ids = work->ids; a.weights = work->weights; a.ids_out = ids_out; a.weights_out = weights_out; a.status = work->status;
+        a.offsets = work->offsets; a.pair_to_row = work->pair_to_row; a.row_to_pair = work->row_to_pair; a.active = work->active;
+        a.groups = (Group4 *)(tc ? work->groups32 : work->groups); a.n_groups = tc ? work->n_groups32 : work->n_groups; a.group_log = tc ? 5 : 2;
+        if (mma) { a.dense = (Group4 *)shared_groups; a.n_dense = work->n_groups + 1; }
+        a.ticket = work->n_groups + 2;
+        if (STEP(2) && (rc = launch_route_batch(a, stream))) return rc;
         STAGE_MARK(); STAGE_MARK();
-        if (overlap && mma) {                         // shared groups are written by the fused kernel
+        if (overlap && mma) {                         // shared groups are written by the same kernel
             CU(cudaEventRecord(ev[2], stream));
             CU(cudaStreamWaitEvent(side, ev[2], 0));
         }
     } else {
-        if ((rc = qw4sh_route(E, k, layer->norm, work->logits, E, tokens, work->probs, work->ids, work->weights, work->status, stream))) return rc;
+        if ((rc = qw4sh_route(E, k, layer->norm, work->logits, E, tokens, nullptr, work->ids, work->weights, work->status, stream))) return rc;
         STAGE_MARK();
         if (tokens > 64 && work->dispatch_scratch) {
             if ((rc = qw4sh_group_large(E, k, tokens, work->ids, work->offsets, work->pair_to_row, work->row_to_pair, work->active,
                                         work->dispatch_scratch, work->status, stream))) return rc;
         } else if ((rc = qw4sh_group(E, k, tokens, work->ids, work->offsets, work->pair_to_row, work->row_to_pair, work->active, work->status, stream))) return rc;
         if (mma && (rc = qw4sh_build_groups(work->offsets, work->active, work->groups, work->n_groups, stream))) return rc;
+        if (tc && (rc = qw4sh_build_tile_groups(work->offsets, work->active, work->groups32, work->n_groups32, stream))) return rc;
         STAGE_MARK();
     }
-    if (tc && (rc = qw4sh_build_tile_groups(work->offsets, work->active, work->groups32, work->n_groups32, stream))) return rc;
     if (tc || mma) {
         if (overlap) {
             if ((rc = shared_branch(0)) || (rc = shared_branch(1))) return rc;
@@ -1651,7 +1615,7 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
         STAGE_MARK(); STAGE_MARK(); STAGE_MARK();
     }
 #undef STAGE_MARK
-    if (ids_out || weights_out) {
+    if (!listed && (ids_out || weights_out)) {
         copy_routes_kernel<<<(T * k + 255) / 256, 256, 0, stream>>>(work->ids, work->weights, T * k, ids_out, weights_out);
         LAUNCHED("copy_routes_kernel");
     }
