@@ -37,7 +37,7 @@ typedef struct {
      * qw4sh_fused_prepare once the images are resident; ready = 0 when the layer does not fit that path */
     unsigned char fused_maps[4][128];
     int fused_maps_ready;
-    /* the same path: expanded images (4-bit codes) of the IQ2_XXS expert tensors, owned by the layer */
+    /* the same path: expanded images (3-bit codes) of the IQ2_XXS expert tensors, owned by the layer */
     void *fused_alt[8];
     size_t fused_alt_bytes;
 } QW4ShLayer;

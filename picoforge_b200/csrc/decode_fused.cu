@@ -24,7 +24,7 @@
 //   B  work unit = 8 gate rows + the same 8 up rows of one expert (gate in MMA rows 0-7, up in
 //      8-15); a unit is cut into slices of 512 columns dealt to the CTA's warps, each warp fetching
 //      slices into its own ring (Q4_K: one 3-D tensor-map request per matrix; IQ2_XXS: one bulk copy
-//      of a contiguous span of its expanded image) and feeding int8 tensor-core MMAs with the codes.
+//      of a block of its expanded image) and feeding int8 tensor-core MMAs with the codes.
 //      Units come in granules of four (32 activation columns): the warp that sums a granule's
 //      slices applies SwiGLU and writes the activation as int8 digit pairs with ONE SCALE PER
 //      32-COLUMN CHUNK, so that no row maximum has to cross the grid and phase C starts with a
@@ -61,7 +61,7 @@ constexpr int FMAXSRC = FTOK * FMAXK + 1;       // shared expert + distinct rout
 constexpr int FRMAX = 4;                        // router rows per streaming CTA
 constexpr int FNS = 2;                          // ring stages per warp, gate/up phase (three stages fit and were measured: no faster)
 constexpr int FNC = 2;                          // ring stages per warp, down phase
-constexpr uint32_t FSTAGE = 4608;               // bytes per ring stage: 16 rows x 288 bytes (512 columns of either format)
+constexpr uint32_t FSTAGE = 4608;               // bytes per ring stage: sixteen rows x 512 columns (4608 of Q4_K, 3392 of the expanded IQ2_XXS image)
 constexpr uint32_t FZP = FMAXE + 4;             // pitch of a logit row in shared memory (floats)
 constexpr int CROWS = 32;                       // router rows per chain CTA (lane = row).  64 rows (two chain warps per token, nine
                                                 // chain CTAs) evened out the streaming CTAs' shares but ran the chains at 42 k cycles
@@ -281,8 +281,7 @@ __device__ __forceinline__ void q4k_scales(const uint4 h0, uint32_t hb, uint32_t
 
 // Q4_K: r0 / r1 point at the first 144-byte block of the two rows; `halves` half blocks follow.
 template <> struct Halves<T_Q4_K> {
-    static __device__ __forceinline__ void run(const uint8_t *r0, const uint8_t *r1, uint32_t halves, uint32_t, const uint16_t *,
-                                            const uint16_t *, const uint8_t *, uint32_t t, const uint8_t *xq, const int2 *xsum,
+    static __device__ __forceinline__ void run(const uint8_t *r0, const uint8_t *r1, uint32_t halves, uint32_t t, const uint8_t *xq, const int2 *xsum,
                                             float &f0, float &f1) {
 #pragma unroll 1
         for (uint32_t h = 0; h < halves; h++, xq += 128, xsum += 4) {
@@ -320,8 +319,7 @@ template <> struct Halves<T_Q4_K> {
     }
 };
 template <> struct HalvesS<T_Q4_K> {
-    static __device__ __forceinline__ void run(const uint8_t *r0, const uint8_t *r1, uint32_t halves, uint32_t, const uint16_t *,
-                                            const uint16_t *, const uint8_t *, uint32_t t, const uint8_t *aq, const float2 *asc,
+    static __device__ __forceinline__ void run(const uint8_t *r0, const uint8_t *r1, uint32_t halves, uint32_t t, const uint8_t *aq, const float2 *asc,
                                             float &f0, float &f1) {
 #pragma unroll 1
         for (uint32_t h = 0; h < halves; h++, aq += 128, asc += 4) {
@@ -360,28 +358,32 @@ template <> struct HalvesS<T_Q4_K> {
     }
 };
 
-// IQ2_XXS on this path is read from a second resident image, made at create (iq2_expand_kernel below): every
-// weight as a 4-bit code (level | sign << 2), laid out for this kernel.  2.06 bits per weight become 4.5, and in
-// exchange a lane turns eight weights into MMA operands with one shift and two byte permutes against an 8-byte
-// table held in two registers (the codebook and sign look-ups of the packed form cost four shared-memory reads per
-// eight weights and bound the whole kernel).  Decoded values are the same bits.
+// IQ2_XXS on this path is read from a second resident image, made at create (iq2_expand_kernel below): every weight as
+// a 2-bit level and a sign bit, laid out for this kernel.  2.06 bits per weight become 3.31, and in exchange a lane turns eight
+// weights into MMA operands with shifts, masks and two byte permutes against an 8-byte table held in two registers (the codebook and
+// sign look-ups of the packed form cost four shared-memory reads per eight weights and bound the whole kernel).  Decoded values
+// are the same bits.  The kernel's weight phases are bound by the bytes they stream: with whole 4-bit codes (4.5 bits per
+// weight, one shift and two permutes) four tokens read 65 MB and took 39.3 us a layer.
 //
-// Block of 512 columns, 288 bytes (the geometry of two Q4_K blocks, so slices, stages and tensor-map boxes are
-// shared with that format):
-//   [0, 256)    codes: the 32-bit word of lane t for 32-column chunk j of half h (columns 128 h + 32 j + 8 t .. + 7,
-//               nibble i = column + i) sits at 64 h + 16 t + 4 j, so a lane reads its four chunks of a half with
-//               one 128-bit load;
-//   [256, 272)  2 * scale + 1 of the sixteen 32-column chunks, one byte each;
-//   [272, 276)  the fp16 super-scales of the two 256-column source blocks;  [276, 288) zero.
+// Block of sixteen rows x 512 columns, 3392 bytes: a slice of a gate/up unit (8 gate rows, 8 up rows) or a down tile.  With row r, half h
+// (128 columns) and lane t of the consumer (columns 128 h + 32 j + 8 t .. + 7 of chunk j):
+//   [0, 2048)     levels: words at 512 h + 32 r + 8 t; nibble n of word w: column n of chunk 2 w in its low, of chunk 2 w + 1 in its high two bits;
+//   [2048, 3072)  signs: word at 256 h + 16 r + 4 t; nibble n, bit j: column n of chunk j;
+//   [3072, 3328)  2 * scale + 1 of the chunks: byte at 16 r + 4 h + j;
+//   [3328, 3392)  the fp16 super-scales of the two 256-column source blocks: 4 r + 2 (h >> 1).
+// The lanes of a warp read consecutive words of each part.
 constexpr uint32_t T_IQ2N = 116;                        // not a GGUF type: the expanded image of an IQ2_XXS tensor
 constexpr uint32_t IQ2N_LO = 8u | 25u << 8 | 43u << 16 | 60u << 24;                                  // iq2_magnitude(0..3)
 constexpr uint32_t IQ2N_HI = (256u - 8u) | (256u - 25u) << 8 | (256u - 43u) << 16 | (256u - 60u) << 24;   // the same, negated
-
-__device__ __forceinline__ uint4 lds_ring4(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
+constexpr uint32_t IQ2N_SIGNS = 2048, IQ2N_SCALES = 3072, IQ2N_D = 3328, IQ2N_BLOCK = 3392;
+// Permute selectors (level | sign << 2 per nibble) of chunk j.
+template <int J>
+__device__ __forceinline__ uint32_t iq2n_select(uint2 levels, uint32_t signs) {
+    const uint32_t l = J < 2 ? levels.x : levels.y;
+    const uint32_t s = J < 2 ? signs << (2 - J) : signs >> (J - 2);
+    return ((J & 1 ? l >> 2 : l) & 0x33333333u) | (s & 0x44444444u);
 }
+
 __device__ __forceinline__ uint32_t lds_ring1(uint32_t a) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
@@ -389,18 +391,18 @@ __device__ __forceinline__ uint32_t lds_ring1(uint32_t a) {
 }
 
 template <> struct Halves<T_IQ2N> {
-    static __device__ __forceinline__ void run(const uint8_t *r0, const uint8_t *r1, uint32_t halves, uint32_t, const uint16_t *,
-                                            const uint16_t *, const uint8_t *, uint32_t t, const uint8_t *xq, const int2 *,
-                                            float &f0, float &f1) {
-        const uint32_t a0s = fs_u32(r0) + 16u * t, a1s = fs_u32(r1) + 16u * t;
+    static __device__ __forceinline__ void run(const uint8_t *block, uint32_t g, uint32_t t, const uint8_t *xq, float &f0, float &f1) {
+        const uint32_t base = fs_u32(block), lv = base + 32u * g + 8u * t, sg = base + IQ2N_SIGNS + 16u * g + 4u * t, sc = base + IQ2N_SCALES + 16u * g,
+                       dd = base + IQ2N_D + 4u * g;
         uint32_t xs = fs_u32(xq);
 #pragma unroll 1
-        for (uint32_t h = 0; h < halves; h++, xs += 128) {
-            const uint32_t at = (h >> 2) * 288u, hh = h & 3u;
-            const uint4 w0 = lds_ring4(a0s + at + 64u * hh), w1 = lds_ring4(a1s + at + 64u * hh);
-            const uint32_t s0 = lds_ring1(a0s - 16u * t + at + 256u + 4u * hh), s1 = lds_ring1(a1s - 16u * t + at + 256u + 4u * hh);
-            const uint32_t dh0 = lds_ring_u16(a0s - 16u * t + at + 272u + (hh >> 1) * 2u), dh1 = lds_ring_u16(a1s - 16u * t + at + 272u + (hh >> 1) * 2u);
-            const uint32_t c0[4] = {w0.x, w0.y, w0.z, w0.w}, c1[4] = {w1.x, w1.y, w1.z, w1.w};
+        for (uint32_t h = 0; h < 4; h++, xs += 128) {
+            const uint2 l0 = lds_ring2(lv + 512u * h), l1 = lds_ring2(lv + 512u * h + 256u);
+            const uint32_t g0 = lds_ring1(sg + 256u * h), g1 = lds_ring1(sg + 256u * h + 128u);
+            const uint32_t s0 = lds_ring1(sc + 4u * h), s1 = lds_ring1(sc + 4u * h + 128u);
+            const uint32_t dh0 = lds_ring_u16(dd + (h >> 1) * 2u), dh1 = lds_ring_u16(dd + (h >> 1) * 2u + 32u);
+            const uint32_t c0[4] = {iq2n_select<0>(l0, g0), iq2n_select<1>(l0, g0), iq2n_select<2>(l0, g0), iq2n_select<3>(l0, g0)};
+            const uint32_t c1[4] = {iq2n_select<0>(l1, g1), iq2n_select<1>(l1, g1), iq2n_select<2>(l1, g1), iq2n_select<3>(l1, g1)};
             int iacc[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -419,28 +421,28 @@ template <> struct Halves<T_IQ2N> {
     }
 };
 template <> struct HalvesS<T_IQ2N> {
-    static __device__ __forceinline__ void run(const uint8_t *r0, const uint8_t *r1, uint32_t halves, uint32_t, const uint16_t *,
-                                            const uint16_t *, const uint8_t *, uint32_t t, const uint8_t *aq, const float2 *asc,
-                                            float &f0, float &f1) {
-        const uint32_t a0s = fs_u32(r0) + 16u * t, a1s = fs_u32(r1) + 16u * t;
+    static __device__ __forceinline__ void run(const uint8_t *block, uint32_t g, uint32_t t, const uint8_t *aq, const float2 *asc, float &f0, float &f1) {
+        const uint32_t base = fs_u32(block), lv = base + 32u * g + 8u * t, sg = base + IQ2N_SIGNS + 16u * g + 4u * t, sc = base + IQ2N_SCALES + 16u * g,
+                       dd = base + IQ2N_D + 4u * g;
         uint32_t xs = fs_u32(aq), ss = fs_u32(asc);
 #pragma unroll 1
-        for (uint32_t h = 0; h < halves; h++, xs += 128, ss += 32) {
-            const uint32_t at = (h >> 2) * 288u, hh = h & 3u;
-            const uint4 w0 = lds_ring4(a0s + at + 64u * hh), w1 = lds_ring4(a1s + at + 64u * hh);
-            const uint32_t s0 = lds_ring1(a0s - 16u * t + at + 256u + 4u * hh), s1 = lds_ring1(a1s - 16u * t + at + 256u + 4u * hh);
-            const uint32_t dh0 = lds_ring_u16(a0s - 16u * t + at + 272u + (hh >> 1) * 2u), dh1 = lds_ring_u16(a1s - 16u * t + at + 272u + (hh >> 1) * 2u);
-            const uint32_t c0[4] = {w0.x, w0.y, w0.z, w0.w}, c1[4] = {w1.x, w1.y, w1.z, w1.w};
+        for (uint32_t h = 0; h < 4; h++, xs += 128, ss += 32) {
+            const uint2 l0 = lds_ring2(lv + 512u * h), l1 = lds_ring2(lv + 512u * h + 256u);
+            const uint32_t g0 = lds_ring1(sg + 256u * h), g1 = lds_ring1(sg + 256u * h + 128u);
+            const uint32_t s0 = lds_ring1(sc + 4u * h), s1 = lds_ring1(sc + 4u * h + 128u);
+            const uint32_t dh0 = lds_ring_u16(dd + (h >> 1) * 2u), dh1 = lds_ring_u16(dd + (h >> 1) * 2u + 32u);
+            const uint32_t c0[4] = {iq2n_select<0>(l0, g0), iq2n_select<1>(l0, g0), iq2n_select<2>(l0, g0), iq2n_select<3>(l0, g0)};
+            const uint32_t c1[4] = {iq2n_select<0>(l1, g1), iq2n_select<1>(l1, g1), iq2n_select<2>(l1, g1), iq2n_select<3>(l1, g1)};
             float fa0 = 0.0f, fa1 = 0.0f;
             const float lo = 1.0f / 254.0f;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const uint2 bq = lds_ring2(xs + j * 32), sc = lds_ring2(ss + j * 8);
+                const uint2 bq = lds_ring2(xs + j * 32), as = lds_ring2(ss + j * 8);
                 int c[4];
                 fmma_zero(c, __byte_perm(IQ2N_LO, IQ2N_HI, c0[j]), __byte_perm(IQ2N_LO, IQ2N_HI, c1[j]),
                           __byte_perm(IQ2N_LO, IQ2N_HI, c0[j] >> 16), __byte_perm(IQ2N_LO, IQ2N_HI, c1[j] >> 16), bq.x, bq.y);
                 const float k0 = (float)((s0 >> (8 * j)) & 0xffu), k1 = (float)((s1 >> (8 * j)) & 0xffu);       // 2 * scale + 1
-                const float a = __uint_as_float(sc.x);
+                const float a = __uint_as_float(as.x);
                 fa0 = fmaf(k0 * a, fmaf((float)c[1], lo, (float)c[0]), fa0);
                 fa1 = fmaf(k1 * a, fmaf((float)c[3], lo, (float)c[2]), fa1);
             }
@@ -451,36 +453,50 @@ template <> struct HalvesS<T_IQ2N> {
     }
 };
 
-// One thread per 32-column chunk of a row: the chunk's 32 codes, its scale byte, and (first chunk of a 256-column
-// source block) the block's super-scale, from the resident IQ2_XXS image into the expanded one.
-// which < 0: rows in order, [expert][row][blocks] (down tiles: sixteen rows are one contiguous span).  which = 0 / 1
-// (gate / up): unit slices, [expert][unit of 8 rows][block][gate rows | up rows][288 bytes], so that the sixteen row
-// pieces of one ring stage are ONE contiguous span of 4608 bytes.
+// One thread per 128-column half of a row, from the resident IQ2_XXS image into the expanded one.
+// which < 0: [expert][tile of 16 rows][block] (down; one block where a tile is 512 columns deep).  which = 0 / 1 (gate / up):
+// unit slices, [expert][unit of 8 rows][block], the gate's rows in block rows 0-7, the up's in 8-15.
+__device__ __forceinline__ uint8_t *iq2n_block(uint8_t *image, uint32_t n_out, uint32_t nb5, uint32_t expert, uint32_t row, uint32_t block, int which, uint32_t &r) {
+    const uint32_t rows_log = which < 0 ? 4 : 3;
+    r = which < 0 ? row & 15u : (row & 7u) + 8u * (uint32_t)which;
+    return image + (((uint64_t)expert * (n_out >> rows_log) + (row >> rows_log)) * nb5 + block) * IQ2N_BLOCK;
+}
 __global__ void __launch_bounds__(256) iq2_expand_kernel(DevTensor t, uint8_t *__restrict__ out, int which) {
-    const uint32_t nb = t.k_storage >> 8, chunks = t.k_storage >> 5;
-    const uint64_t rows = (uint64_t)t.n_out * t.n_experts, total = rows * chunks;
+    const uint32_t nb = t.k_storage >> 8, halves = t.k_storage >> 7;
+    const uint64_t rows = (uint64_t)t.n_out * t.n_experts, total = rows * halves;
     const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= total) return;
-    const uint64_t grow = i / chunks;                                          // expert * n_out + row
-    const uint32_t q = (uint32_t)(i % chunks), expert = (uint32_t)(grow / t.n_out), row = (uint32_t)(grow % t.n_out);
+    const uint64_t grow = i / halves;                                          // expert * n_out + row
+    const uint32_t q = (uint32_t)(i % halves), expert = (uint32_t)(grow / t.n_out), row = (uint32_t)(grow % t.n_out);
     const uint8_t *mat = t.data + (uint64_t)expert * t.expert_bytes;
-    const uint32_t blk = q >> 3, ch = q & 7u;
-    const uint8_t *group = mat + ((uint64_t)row * nb * 8u + ((blk * 8u + ch) ^ iq2_swizzle(row, nb))) * 8u;
-    const uint32_t bits = load_u32(group + 4);
-    const uint32_t nb5 = t.k_storage >> 9;                                      // 512-column blocks per row
-    uint8_t *block = which < 0 ? out + (grow * nb5 + (q >> 4)) * 288u           // the 512-column block of this chunk
-                               : out + ((((uint64_t)expert * (t.n_out >> 3) + (row >> 3)) * nb5 + (q >> 4)) * 2u + (uint32_t)which) * 2304u + (row & 7u) * 288u;
-    const uint32_t h = (q >> 2) & 3u, j = q & 3u;
-    for (uint32_t slot = 0; slot < 4; slot++) {                                 // slot = lane t of the consumer: columns 8 t .. 8 t + 7
-        const uint32_t levels = c_iq2_levels[group[slot]], signs = iq2_signs8((bits >> (7 * slot)) & 127u);
-        uint32_t word = 0;
-        for (uint32_t c = 0; c < 8; c++) word |= (((levels >> (2 * c)) & 3u) | (((signs >> c) & 1u) << 2)) << (4 * c);
-        *reinterpret_cast<uint32_t *>(block + 64u * h + 16u * slot + 4u * j) = word;
+    uint32_t r;
+    uint8_t *block = iq2n_block(out, t.n_out, t.k_storage >> 9, expert, row, q >> 2, which, r);
+    const uint32_t h = q & 3u, blk = q >> 1;                                    // half of the 512-column block; 256-column source block
+    uint32_t levels[4][2] = {}, signs[4] = {}, scales = 0;                      // by slot = lane t of the consumer: columns 8 t .. 8 t + 7
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+        const uint8_t *group = mat + ((uint64_t)row * nb * 8u + ((blk * 8u + (q & 1u) * 4u + j) ^ iq2_swizzle(row, nb))) * 8u;
+        const uint32_t bits = load_u32(group + 4), codes = load_u32(group);
+#pragma unroll
+        for (uint32_t slot = 0; slot < 4; slot++) {
+            const uint32_t lv = c_iq2_levels[(codes >> (8 * slot)) & 0xffu], sg = iq2_signs8((bits >> (7 * slot)) & 127u);
+#pragma unroll
+            for (uint32_t c = 0; c < 8; c++) {
+                levels[slot][j >> 1] |= ((lv >> (2 * c)) & 3u) << (4 * c + 2 * (j & 1u));
+                signs[slot] |= ((sg >> c) & 1u) << (4 * c + j);
+            }
+        }
+        scales |= (2u * (bits >> 28) + 1u) << (8 * j);
     }
-    block[256u + 4u * h + j] = (uint8_t)(2u * (bits >> 28) + 1u);
-    if (ch == 0) {
+#pragma unroll
+    for (uint32_t slot = 0; slot < 4; slot++) {
+        *reinterpret_cast<uint2 *>(block + 512u * h + 32u * r + 8u * slot) = make_uint2(levels[slot][0], levels[slot][1]);
+        *reinterpret_cast<uint32_t *>(block + IQ2N_SIGNS + 256u * h + 16u * r + 4u * slot) = signs[slot];
+    }
+    *reinterpret_cast<uint32_t *>(block + IQ2N_SCALES + 16u * r + 4u * h) = scales;
+    if (!(q & 1u)) {
         const uint64_t blocks = (uint64_t)t.n_out * nb;
-        *reinterpret_cast<uint16_t *>(block + 272u + (blk & 1u) * 2u) = (uint16_t)load_u16(mat + blocks * 64u + ((uint64_t)row * nb + blk) * 2u);
+        *reinterpret_cast<uint16_t *>(block + IQ2N_D + 4u * r + h) = (uint16_t)load_u16(mat + blocks * 64u + ((uint64_t)row * nb + blk) * 2u);      // h is 0 or 2
     }
 }
 
@@ -491,13 +507,15 @@ __global__ void __launch_bounds__(256) iq2n_decode_rows_kernel(const uint8_t *__
                                                                uint32_t row0, uint32_t rows, int which, float *__restrict__ out) {
     const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= (uint64_t)rows * k) return;
-    const uint32_t row = row0 + (uint32_t)(i / k), col = (uint32_t)(i % k), nb5 = k >> 9;
-    const uint8_t *block = which < 0 ? image + (((uint64_t)expert * n_out + row) * nb5 + (col >> 9)) * 288u
-                                     : image + ((((uint64_t)expert * (n_out >> 3) + (row >> 3)) * nb5 + (col >> 9)) * 2u + (uint32_t)which) * 2304u + (row & 7u) * 288u;
+    const uint32_t row = row0 + (uint32_t)(i / k), col = (uint32_t)(i % k);
+    uint32_t r;
+    const uint8_t *block = iq2n_block(const_cast<uint8_t *>(image), n_out, k >> 9, expert, row, col >> 9, which, r);
     const uint32_t c = col & 511u, h = c >> 7, j = (c >> 5) & 3u, t = (c >> 3) & 3u, n = c & 7u;
-    const uint32_t word = *reinterpret_cast<const uint32_t *>(block + 64u * h + 16u * t + 4u * j), code = (word >> (4 * n)) & 15u;
-    const uint32_t twice_plus_one = block[256u + 4u * h + j];
-    const float d = half_bits_to_float(*reinterpret_cast<const uint16_t *>(block + 272u + (h >> 1) * 2u));
+    const uint32_t word = *reinterpret_cast<const uint32_t *>(block + 512u * h + 32u * r + 8u * t + 4u * (j >> 1));
+    const uint32_t sign = (*reinterpret_cast<const uint32_t *>(block + IQ2N_SIGNS + 256u * h + 16u * r + 4u * t) >> (4 * n + j)) & 1u;
+    const uint32_t code = ((word >> (4 * n + 2 * (j & 1u))) & 3u) | sign << 2;
+    const uint32_t twice_plus_one = block[IQ2N_SCALES + 16u * r + 4u * h + j];
+    const float d = half_bits_to_float(*reinterpret_cast<const uint16_t *>(block + IQ2N_D + 4u * r + (h >> 1) * 2u));
     const float scale = __fmul_rn(__fmul_rn(d, (float)twice_plus_one), 0.125f);
     const float value = __fmul_rn(scale, (float)iq2_magnitude(code & 3u));
     out[i] = (code & 4u) ? -value : value;
@@ -505,8 +523,8 @@ __global__ void __launch_bounds__(256) iq2n_decode_rows_kernel(const uint8_t *__
 
 // Geometry of one format inside the rings.
 template <uint32_t TYPE> struct FGeo;
-template <> struct FGeo<T_Q4_K> { static constexpr uint32_t SLICE_BLOCKS = 2, BLOCK_BYTES = 144; };      // 512 columns, 288 B per row
-template <> struct FGeo<T_IQ2N> { static constexpr uint32_t SLICE_BLOCKS = 2, BLOCK_BYTES = 144; };      // the same: one 288-byte block of 512 columns
+template <> struct FGeo<T_Q4_K> { static constexpr uint32_t SLICE_BLOCKS = 2, SLICE_BYTES = 16 * 288; };      // sixteen rows x 512 columns
+template <> struct FGeo<T_IQ2N> { static constexpr uint32_t SLICE_BLOCKS = 2, SLICE_BYTES = IQ2N_BLOCK; };
 
 // Copies of slice `s` of a gate/up unit (8 gate rows + 8 up rows from row `row0` of expert `expert`) into `stage`:
 // row r at r * slice bytes.  The eight row pieces of a
@@ -515,45 +533,48 @@ template <uint32_t TYPE>
 __device__ __forceinline__ void issue_unit_slice(const CUtensorMap *gate_map, const CUtensorMap *up_map, const uint8_t *gate_mat,
                                               const uint8_t *up_mat, uint32_t expert, uint32_t n_out, uint32_t nb, uint32_t row0, uint32_t s,
                                               uint8_t *stage, uint64_t *bar, uint32_t lane) {
-    constexpr uint32_t slice_bytes = FGeo<TYPE>::SLICE_BLOCKS * FGeo<TYPE>::BLOCK_BYTES;
+    constexpr uint32_t bytes = FGeo<TYPE>::SLICE_BYTES;
     if (TYPE == T_IQ2N) {
         // the expanded image keeps a unit slice (gate rows, then up rows) as one span: gate_mat is the image's base
         if (lane == 0) {
-            fbar_expect(bar, 16 * slice_bytes);
-            fbulk(stage, gate_mat + ((((uint64_t)expert * (n_out >> 3) + (row0 >> 3)) * (nb >> 1) + s) * 16u) * slice_bytes, 16 * slice_bytes, bar);
+            fbar_expect(bar, bytes);
+            fbulk(stage, gate_mat + (((uint64_t)expert * (n_out >> 3) + (row0 >> 3)) * (nb >> 1) + s) * bytes, bytes, bar);
         }
         return;
     }
-    if (lane == 0) fbar_expect(bar, 16 * slice_bytes);
+    if (lane == 0) fbar_expect(bar, bytes);
     __syncwarp();
-    if (lane < 2) ftma_rows(stage + lane * 8 * slice_bytes, lane ? up_map : gate_map, s * (slice_bytes / 4), row0, expert, bar);
+    if (lane < 2) ftma_rows(stage + lane * (bytes / 2), lane ? up_map : gate_map, s * (bytes / 64), row0, expert, bar);
 }
 template <uint32_t TYPE>
 __device__ __forceinline__ void consume_unit_slice(const uint8_t *stage, uint32_t nb, uint32_t s, const uint8_t *xq_lane,
                                                    const int2 *xsum_tok, uint32_t g, uint32_t t, float &f0, float &f1) {
-    constexpr uint32_t SB = FGeo<TYPE>::SLICE_BLOCKS, slice_bytes = SB * FGeo<TYPE>::BLOCK_BYTES;
-    const uint16_t *d = reinterpret_cast<const uint16_t *>(stage + 16 * slice_bytes);
-    Halves<TYPE>::run(stage + g * slice_bytes, stage + (8 + g) * slice_bytes, SB * 2, iq2_swizzle(g, nb), d + g * nb + s * SB,
-                      d + (8 + g) * nb + s * SB, nullptr, t, xq_lane + s * SB * 256u, xsum_tok + s * SB * 8u, f0, f1);
+    constexpr uint32_t SB = FGeo<TYPE>::SLICE_BLOCKS;
+    if constexpr (TYPE == T_IQ2N) Halves<TYPE>::run(stage, g, t, xq_lane + s * SB * 256u, f0, f1);
+    else {
+        constexpr uint32_t pitch = FGeo<TYPE>::SLICE_BYTES / 16;
+        Halves<TYPE>::run(stage + g * pitch, stage + (8 + g) * pitch, SB * 2, t, xq_lane + s * SB * 256u, xsum_tok + s * SB * 8u, f0, f1);
+    }
 }
 
 // Down tile: 16 rows x K (K <= 512), fetched whole.
 template <uint32_t TYPE>
 __device__ __forceinline__ void issue_down_tile(const uint8_t *mat, uint32_t n_out, uint32_t nb, uint32_t row0, uint8_t *stage, uint64_t *bar,
                                              uint32_t lane) {
-    const uint32_t row_bytes = nb * FGeo<TYPE>::BLOCK_BYTES;
+    const uint32_t bytes = (nb >> 1) * FGeo<TYPE>::SLICE_BYTES;
     if (lane == 0) {
-        fbar_expect(bar, 16 * row_bytes);
-        fbulk(stage, mat + row0 * row_bytes, 16 * row_bytes, bar);
+        fbar_expect(bar, bytes);
+        fbulk(stage, mat + (row0 >> 4) * bytes, bytes, bar);
     }
 }
 template <uint32_t TYPE>
 __device__ __forceinline__ void consume_down_tile(const uint8_t *stage, uint32_t nb, const uint8_t *aq_lane,
                                                   const float2 *asc_tok, uint32_t g, uint32_t t, float &f0, float &f1) {
-    const uint32_t row_bytes = nb * FGeo<TYPE>::BLOCK_BYTES;
-    const uint16_t *d = reinterpret_cast<const uint16_t *>(stage + 4096);
-    HalvesS<TYPE>::run(stage + g * row_bytes, stage + (8 + g) * row_bytes, nb * 2, iq2_swizzle(g, nb), d + g * nb, d + (8 + g) * nb, nullptr, t,
-                       aq_lane, asc_tok, f0, f1);
+    if constexpr (TYPE == T_IQ2N) HalvesS<TYPE>::run(stage, g, t, aq_lane, asc_tok, f0, f1);              // nb = 2
+    else {
+        const uint32_t row_bytes = nb * 144u;
+        HalvesS<TYPE>::run(stage + g * row_bytes, stage + (8 + g) * row_bytes, nb * 2, t, aq_lane, asc_tok, f0, f1);
+    }
 }
 
 // Two int8 digits per value: v ~ dx * (q1 + q2 / 254), |v| <= 127 dx.  Rounding by the
@@ -1079,9 +1100,9 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
             for (uint32_t tile = sc; tile < (H >> 4); tile += NS)
                 for (uint32_t j = warp * 4 + lane; lane < 4 && j < n_src; j += FW * 4) {      // a few requests per warp: none of them falls behind
                     const Src s = srcs[j];
-                    const uint32_t rb = (s.shared ? IS >> 8 : I >> 8) * 144u;
+                    const uint32_t bytes = s.shared ? (IS >> 9) * FGeo<ST>::SLICE_BYTES : (I >> 9) * FGeo<RT>::SLICE_BYTES;
                     const uint8_t *mat = s.shared ? a.w[6].data : a.w[3].data + (uint64_t)s.expert * a.w[3].expert_bytes;
-                    fprefetch_l2(mat + tile * 16 * rb, 16 * rb);
+                    fprefetch_l2(mat + tile * bytes, bytes);
                 }
             const uint8_t *xq_lane = xq + g * p.kp + 8 * t;
             const int2 *xsum_tok = xsum + t * (H >> 5);
@@ -1325,15 +1346,14 @@ extern "C" void qw4sh_fused_scratch_sizes(const QW4ShLayer *l, size_t *aq_bytes,
 typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                 const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-// The tensor this path streams for resident tensor i: the tensor itself (Q4_K) or its expanded image (IQ2_XXS), whose
-// rows have the geometry of Q4_K rows (144 bytes per 256 columns).
+// The tensor this path streams for resident tensor i: the tensor itself (Q4_K) or its expanded image (IQ2_XXS).
 static DevTensor fused_view(const QW4ShLayer *l, int i) {
     DevTensor t = fdev(l->w[i]);
     const int holder = (i == 2 || i == 5) ? i - 1 : i;                     // gate and up share the gate's image
     if (t.type == T_IQ2_XXS && l->fused_alt[holder]) {
         t.data = (const uint8_t *)l->fused_alt[holder];
         t.type = T_IQ2N;
-        t.row_bytes = (t.k_storage >> 8) * 144u;
+        t.row_bytes = (t.k_storage >> 9) * (IQ2N_BLOCK / 16);
         t.expert_bytes = (uint64_t)t.row_bytes * t.n_out;
     }
     return t;
@@ -1347,7 +1367,7 @@ static int rows_map(const DevTensor &t, CUtensorMap *map) {
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &status) != cudaSuccess || !fn) return -1;
         encode = (EncodeTiled)fn;
     }
-    constexpr uint32_t slice = FGeo<T_Q4_K>::SLICE_BLOCKS * FGeo<T_Q4_K>::BLOCK_BYTES;
+    constexpr uint32_t slice = FGeo<T_Q4_K>::SLICE_BYTES / 16;
     const cuuint64_t dims[3] = {(cuuint64_t)t.row_bytes / 4, t.n_out, t.n_experts};
     const cuuint64_t strides[2] = {(cuuint64_t)t.row_bytes, t.expert_bytes};
     const cuuint32_t box[3] = {slice / 4, 8, 1}, elem[3] = {1, 1, 1};
@@ -1381,13 +1401,13 @@ extern "C" int qw4sh_fused_prepare(QW4ShLayer *l) {
         const bool pair = i == 1 || i == 4;
         const DevTensor src = fdev(l->w[i]);
         if (pair && (l->w[i + 1].n_out != src.n_out || l->w[i + 1].k_storage != src.k_storage || l->w[i + 1].n_experts != src.n_experts)) return 0;
-        const size_t bytes = (size_t)src.n_experts * src.n_out * (src.k_storage >> 9) * 288u * (pair ? 2 : 1);
+        const size_t bytes = (size_t)src.n_experts * src.n_out * (src.k_storage >> 9) * (IQ2N_BLOCK / 16) * (pair ? 2 : 1);
         cudaError_t e = cudaMalloc(&l->fused_alt[i], bytes);
         if (e == cudaSuccess) e = cudaMemset(l->fused_alt[i], 0, bytes);
         if (e == cudaSuccess) {
-            const uint64_t chunks = (uint64_t)src.n_experts * src.n_out * (src.k_storage >> 5);
-            iq2_expand_kernel<<<(unsigned)((chunks + 255) / 256), 256>>>(src, (uint8_t *)l->fused_alt[i], pair ? 0 : -1);
-            if (pair) iq2_expand_kernel<<<(unsigned)((chunks + 255) / 256), 256>>>(fdev(l->w[i + 1]), (uint8_t *)l->fused_alt[i], 1);
+            const uint64_t halves = (uint64_t)src.n_experts * src.n_out * (src.k_storage >> 7);
+            iq2_expand_kernel<<<(unsigned)((halves + 255) / 256), 256>>>(src, (uint8_t *)l->fused_alt[i], pair ? 0 : -1);
+            if (pair) iq2_expand_kernel<<<(unsigned)((halves + 255) / 256), 256>>>(fdev(l->w[i + 1]), (uint8_t *)l->fused_alt[i], 1);
             e = cudaDeviceSynchronize();
         }
         if (e != cudaSuccess) { qw4sh_fused_release(l); return -1; }
@@ -1395,8 +1415,9 @@ extern "C" int qw4sh_fused_prepare(QW4ShLayer *l) {
     }
     const int which[4] = {1, 2, 4, 5};
     for (int i = 0; i < 4; i++) {
-        alignas(64) CUtensorMap map;
-        if (rows_map(fused_view(l, which[i]), &map)) { qw4sh_fused_release(l); return -1; }
+        alignas(64) CUtensorMap map = {};
+        const DevTensor view = fused_view(l, which[i]);
+        if (view.type == T_Q4_K && rows_map(view, &map)) { qw4sh_fused_release(l); return -1; }
         memcpy(l->fused_maps[i], &map, sizeof map);
     }
     l->fused_maps_ready = 1;
