@@ -129,6 +129,8 @@ void qw4sh_set_only_step(int step);
 int qw4sh_prepare_mma(void);
 int qw4sh_stage_times(double *ms, uint64_t *forwards);
 int qw4sh_stream_sync(void *stream);
+int qw4sh_stream_query(void *stream);           /* 1 work pending, 0 none, -1 error */
+int qw4sh_event_query(void *event);             /* the same for an event */
 int qw4sh_device_sync(void);
 int qw4sh_event_create(void **event);
 void qw4sh_event_destroy(void *event);

@@ -841,13 +841,20 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
         // the CTA that leaves last clears the counters for the next launch
         __syncthreads();
         if (tid == 0) {
-            __threadfence();
+            if (a.status_mirror) __threadfence_system(); else __threadfence();      // results in host memory are out before the exit count
             leaving_last = atomicAdd(a.sync + S_EXITS, 1u) == gridDim.x - 1 ? 1u : 0u;
         }
         __syncthreads();
         if (leaving_last && tid < 8) { a.sync[tid] = 0; __threadfence(); }
-        // every CTA's error bits are in before its exit count: the last one hands the words to the host
-        if (leaving_last && tid < 4 && a.status_mirror) a.status_mirror[tid] = *reinterpret_cast<volatile uint32_t *>(a.status + tid);
+        // every CTA's error bits and results are in before its exit count: the last one hands the words to the host, which polls the first
+        if (leaving_last && tid == 0 && a.status_mirror) {
+            const volatile uint32_t *from = a.status;
+            volatile uint32_t *to = a.status_mirror;
+            const uint32_t bits = from[0];
+            to[1] = from[1]; to[2] = from[2]; to[3] = from[3];
+            __threadfence_system();
+            to[0] = bits;
+        }
     };
     if (blockIdx.x < NC) { chain_cta(a, smem); leave(); return; }
 

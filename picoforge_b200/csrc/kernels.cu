@@ -120,6 +120,17 @@ extern "C" int qw4sh_shared_stream(void **stream) {
     *stream = g_stream[device];
     return ensure_constants();
 }
+// 1 while work is pending, 0 when the stream has run dry, -1 on an error.
+extern "C" int qw4sh_stream_query(void *stream) {
+    const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+    if (e == cudaErrorNotReady) { (void)cudaGetLastError(); return 1; }
+    return e == cudaSuccess ? 0 : fail(e, "cudaStreamQuery");
+}
+extern "C" int qw4sh_event_query(void *event) {
+    const cudaError_t e = cudaEventQuery((cudaEvent_t)event);
+    if (e == cudaErrorNotReady) { (void)cudaGetLastError(); return 1; }
+    return e == cudaSuccess ? 0 : fail(e, "cudaEventQuery");
+}
 extern "C" int qw4sh_stream_sync(void *stream) { CU(cudaStreamSynchronize((cudaStream_t)stream)); return 0; }
 extern "C" int qw4sh_device_sync(void) { CU(cudaDeviceSynchronize()); return 0; }
 extern "C" int qw4sh_event_create(void **event) { cudaEvent_t e; CU(cudaEventCreate(&e)); *event = e; return 0; }

@@ -11,6 +11,11 @@
 #include <stdarg.h>
 #include <stdio.h>
 #include <pthread.h>
+#include <sched.h>
+#include <stdatomic.h>
+#include <sys/prctl.h>
+#include <time.h>
+#include <unistd.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -39,6 +44,9 @@ struct Qwen4MoeWork {
     QW4ShWork d;
     void *device_block;           /* one allocation carved into d.* */
     uint32_t *status_host;        /* pinned [4] */
+    unsigned char *stage;         /* pinned ring for the rows of larger host calls, from the first of them on */
+    size_t stage_bytes;
+    void *stage_event[8];
     unsigned char *pin;           /* pinned staging: x | y | ids | weights for small batches */
     QW4MoeObserver observer;
     void *observer_ctx;
@@ -314,6 +322,8 @@ void qwen4_moe_work_destroy(Qwen4MoeWork *w) {
     qw4sh_free(w->device_block);
     qw4sh_host_free(w->status_host);
     qw4sh_host_free(w->pin);
+    qw4sh_host_free(w->stage);
+    for (int i = 0; i < 8; i++) qw4sh_event_destroy(w->stage_event[i]);
     release(w->owner);
     free(w);
 }
@@ -604,6 +614,226 @@ Qwen4Status qw4cu_moe_work_sync_many(Qwen4MoeWork *const *works, size_t n, Qwen4
     return first == QW4_OK ? report(err, QW4_OK, "") : first;
 }
 
+/* ---- host rows ---------------------------------------------------------------------------
+ * A call with host views of more than a few rows spends more time moving them than the GPU spends on the layer when it is left to
+ * a scalar scan and pageable copies (333 rows of 2048: 280 us to scan, 300 us to copy in and out, 430 us on the GPU).  So
+ * the rows go through a ring of pinned slices: the calling thread and up to three helpers copy (and scan) slices in any order, the
+ * calling thread sends finished slices on in order and, on the way back, releases slices as their copies land.  The
+ * helpers live for one call (about 20 us to start, beside the calling thread's own first slice) and make no CUDA call; one that
+ * cannot be started is simply not there. */
+#define VECTORISED __attribute__((optimize("O3")))
+/* Nonzero when one of the n values is infinite or NaN: adding one to an exponent of all ones carries into the sign. */
+VECTORISED static uint32_t scan_floats(const uint32_t *restrict p, size_t n) {
+    uint32_t m = 0;
+    for (size_t i = 0; i < n; i++) m |= (p[i] & 0x7f800000u) + 0x00800000u;
+    return m & 0x80000000u;
+}
+static bool rows_finite(const float *p, size_t pitch, size_t rows, size_t cols) {
+    for (size_t r = 0; r < rows; r++) if (scan_floats((const uint32_t *)(p + r * pitch), cols)) return false;
+    return true;
+}
+enum { STAGE_BYTES = 4 << 20, SLICE_BYTES = 128 << 10, STAGE_EVENTS = 8, HELPERS = 3, HELPER_MIN_BYTES = 1 << 20 };
+typedef struct {
+    float *host;                                   /* the caller's rows */
+    size_t pitch, cols, rows, slice_rows;
+    unsigned char *stage;                          /* ring of pinned slices */
+    int slices, ring, group;                       /* ring = 4 groups; an event behind every group of copies */
+    bool in, scan;
+    atomic_int next, limit, nonfinite;             /* next slice to take; slices released; a bad value was seen */
+    atomic_int done[64];                           /* by slot: 1 + the last slice moved */
+} RowMove;
+typedef struct { RowMove in, out; atomic_int stage; } RowMoves;      /* stage 0: rows in; 1: rows out; 2: leave */
+
+static void plan_move(RowMove *m, Qwen4MoeWork *w, float *host, size_t pitch, size_t rows, size_t cols, bool in, bool scan) {
+    memset(m, 0, sizeof *m);
+    m->host = host; m->pitch = pitch; m->rows = rows; m->cols = cols; m->stage = w->stage; m->in = in; m->scan = scan;
+    m->slice_rows = SLICE_BYTES / (cols * 4) ? SLICE_BYTES / (cols * 4) : 1;
+    m->slices = (int)((rows + m->slice_rows - 1) / m->slice_rows);
+    const size_t slots = w->stage_bytes / (m->slice_rows * cols * 4);
+    m->group = slots > 64 ? 16 : (int)(slots / 4);
+    m->ring = m->group * 4;
+}
+static size_t slice_count(const RowMove *m, int s) {
+    const size_t first = (size_t)s * m->slice_rows;
+    return m->rows - first < m->slice_rows ? m->rows - first : m->slice_rows;
+}
+static unsigned char *slice_slot(const RowMove *m, int s) { return m->stage + (size_t)(s % m->ring) * m->slice_rows * m->cols * 4; }
+static bool slice_done(RowMove *m, int s) { return atomic_load(&m->done[s % m->ring]) > s; }
+/* Takes one released slice; false when there is none now. */
+static bool move_slice(RowMove *m) {
+    int s = atomic_load(&m->next);
+    do { if (s >= atomic_load(&m->limit)) return false; } while (!atomic_compare_exchange_weak(&m->next, &s, s + 1));
+    float *row = m->host + (size_t)s * m->slice_rows * m->pitch, *slot = (float *)slice_slot(m, s);
+    const size_t n = slice_count(m, s);
+    for (size_t r = 0; r < n; r++, row += m->pitch, slot += m->cols) {
+        if (m->scan && scan_floats((const uint32_t *)row, m->cols)) atomic_store(&m->nonfinite, 1);
+        if (m->in) memcpy(slot, row, m->cols * 4); else memcpy(row, slot, m->cols * 4);
+    }
+    atomic_store(&m->done[s % m->ring], s + 1);
+    return true;
+}
+static void *move_helper(void *arg) {
+    RowMoves *m = arg;
+    (void)prctl(PR_SET_TIMERSLACK, 1000ul, 0ul, 0ul, 0ul);           /* naps of this thread end when they should */
+    int idle = 0;
+    for (int stage; (stage = atomic_load(&m->stage)) != 2;) {
+        if (move_slice(stage ? &m->out : &m->in)) idle = 0;
+        else if (++idle < 50) sched_yield();
+        else { const struct timespec nap = {0, 20000}; nanosleep(&nap, NULL); }
+    }
+    return NULL;
+}
+/* All rows of `m` through the ring to or from dev.  0, or nonzero when a CUDA call failed. */
+static int run_move(RowMove *m, Qwen4MoeWork *w, float *dev) {
+    int copied = 0, recorded = 0, retired = 0, moved = 0;            /* slices copied by the GPU; groups recorded, seen done; slices moved, in order */
+    if (m->in) atomic_store(&m->limit, m->slices < m->ring ? m->slices : m->ring);
+    while (m->in ? copied < m->slices : moved < m->slices) {
+        while (copied < m->slices && (m->in ? slice_done(m, copied) : copied < m->ring || slice_done(m, copied - m->ring))) {
+            const size_t width = m->cols * 4, n = slice_count(m, copied);
+            float *rows = dev + (size_t)copied * m->slice_rows * m->cols;
+            unsigned char *slot = slice_slot(m, copied);
+            if (qw4sh_memcpy2d_async(m->in ? (void *)rows : slot, width * n, m->in ? slot : (void *)rows, width * n, width * n, 1, m->in, w->d.stream)) return -1;
+            if (++copied % m->group == 0 || copied == m->slices)
+                if (qw4sh_event_record(w->stage_event[recorded++ % STAGE_EVENTS], w->d.stream)) return -1;
+        }
+        if (retired < recorded && atomic_load(&m->limit) < m->slices) {
+            const int pending = qw4sh_event_query(w->stage_event[retired % STAGE_EVENTS]);
+            if (pending < 0) return -1;
+            if (!pending) {
+                const int limit = ++retired * m->group + (m->in ? m->ring : 0);
+                atomic_store(&m->limit, limit < m->slices ? limit : m->slices);
+            }
+        }
+        while (moved < m->slices && slice_done(m, moved)) moved++;
+        if (!move_slice(m) && m->in) sched_yield();
+    }
+    return 0;
+}
+/* The pinned ring and its events, made by the first call that needs them and kept with the workspace. */
+static int make_stage(Qwen4MoeWork *w, size_t cols) {
+    if (w->stage) return 0;
+    w->stage_bytes = cols * 4 * 8 > STAGE_BYTES ? cols * 4 * 8 : STAGE_BYTES;
+    w->stage = qw4sh_host_alloc(w->stage_bytes);
+    for (int i = 0; w->stage && i < STAGE_EVENTS; i++)
+        if (qw4sh_event_create(&w->stage_event[i])) return -1;
+    return w->stage ? 0 : -1;
+}
+/* Waits for the decode kernel's status words in host memory: they come behind its results and before the launch has wound up.  A look at the
+ * stream now and then catches a launch that never writes them. */
+static int wait_mirror(Qwen4MoeWork *w) {
+    volatile uint32_t *word = w->status_host;
+    for (uint32_t i = 1;; i++) {
+        if (*word != UINT32_MAX) { atomic_thread_fence(memory_order_acquire); return 0; }
+        if (i % 16384 == 0) {
+            const int pending = qw4sh_stream_query(w->d.stream);
+            if (pending <= 0) return pending;
+        }
+    }
+}
+
+static void copy_routes(Qwen4MoeRoutes *routes, size_t start, size_t n, size_t k, const uint32_t *ids, const float *weights) {
+    for (size_t row = 0; row < n; row++) {
+        memcpy(routes->ids.data + (start + row) * (routes->ids.row_stride_bytes / 4), ids + row * k, k * 4);
+        memcpy(routes->weights.data + (start + row) * (routes->weights.stride_bytes[0] / 4), weights + row * k, k * 4);
+    }
+}
+static int launch_layer(const Qwen4Moe *m, Qwen4MoeWork *w, const float *xs, size_t x_pitch, float *y, size_t n, size_t start, uint32_t *ids, float *weights) {
+    if (w->observer)                          /* stage by stage in the reference's order, every stage shown to the observer */
+        return qw4sh_observed_forward(&m->layer, &w->d, w->d.x, w->d.y, n, xs, x_pitch, start, w->observer, w->observer_ctx);
+    return qw4sh_layer_forward(&m->layer, &w->d, w->d.x, y, n, ids, weights, current_router_mode());
+}
+/* Up to a few rows: through the workspace's pinned block. */
+static Qwen4Status forward_few(const Qwen4Moe *m, Qwen4MoeWork *w, const float *xs, size_t x_pitch, float *ys, size_t y_pitch, size_t n, size_t start,
+                               Qwen4MoeRoutes *routes, Qwen4Error *err) {
+    const size_t h = m->c.hidden_size, k = m->c.top_k, x_bytes = n * h * 4, r_bytes = n * k * 4;
+    float *pin_x = (float *)w->pin, *pin_y = (float *)(w->pin + x_bytes);
+    uint32_t *pin_ids = (uint32_t *)(w->pin + 2 * x_bytes);
+    float *pin_w = (float *)(w->pin + 2 * x_bytes + r_bytes);
+    int rc = w->status_clean ? 0 : status_clear(w) || qw4sh_stream_sync(w->d.stream);      /* the words are set anew below */
+    w->status_clean = false;
+    for (size_t row = 0; row < n; row++) memcpy(pin_x + row * h, xs + row * x_pitch, h * 4);
+    rc |= qw4sh_memcpy2d_async(w->d.x, x_bytes, pin_x, x_bytes, x_bytes, 1, 1, w->d.stream);
+    /* the one-kernel decode path writes each result once and reads none: it stores straight into the pinned block
+     * (device-addressable) and hands over the status words itself, so nothing is copied back and no end of the stream is waited for */
+    const bool direct = !w->observer && qw4sh_takes_fused(&m->layer, &w->d, w->d.x, pin_y, n);
+    if (!rc && direct) {
+        w->status_host[0] = UINT32_MAX; w->status_host[1] = UINT32_MAX;
+        w->d.status_mirror = w->status_host;
+        rc = launch_layer(m, w, xs, x_pitch, pin_y, n, start, routes ? pin_ids : NULL, routes ? pin_w : NULL);
+        w->d.status_mirror = NULL;
+        if (!rc) rc = wait_mirror(w);
+        if (!rc && w->status_host[0] == UINT32_MAX)                 /* the launch fell back to the multi-kernel sequence: fetch the words */
+            rc = qw4sh_memcpy(w->status_host, w->d.status, 16, 0);
+    } else if (!rc) {
+        rc = launch_layer(m, w, xs, x_pitch, w->d.y, n, start, NULL, NULL);
+        if (!rc) rc = qw4sh_memcpy2d_async(w->status_host, 16, w->d.status, 16, 16, 1, 0, w->d.stream);
+        if (!rc) rc = qw4sh_memcpy2d_async(pin_y, x_bytes, w->d.y, x_bytes, x_bytes, 1, 0, w->d.stream);
+        if (!rc && routes) {
+            rc |= qw4sh_memcpy2d_async(pin_ids, r_bytes, w->d.ids, r_bytes, r_bytes, 1, 0, w->d.stream);
+            rc |= qw4sh_memcpy2d_async(pin_w, r_bytes, w->d.weights, r_bytes, r_bytes, 1, 0, w->d.stream);
+        }
+        if (!rc) rc = qw4sh_stream_sync(w->d.stream);
+    }
+    if (rc) return cuda_failure(err, "layer execution");
+    TRY(status_result(w, err));
+    w->status_clean = true;
+    for (size_t row = 0; row < n; row++) memcpy(ys + row * y_pitch, pin_y + row * h, h * 4);
+    if (routes) copy_routes(routes, start, n, k, pin_ids, pin_w);
+    return QW4_OK;
+}
+/* More rows: through the ring.  *rejected: a value of x is not finite (scan), nothing was launched. */
+static Qwen4Status forward_many(const Qwen4Moe *m, Qwen4MoeWork *w, const float *xs, size_t x_pitch, float *ys, size_t y_pitch, size_t n, size_t start,
+                                Qwen4MoeRoutes *routes, bool scan, bool *rejected, Qwen4Error *err) {
+    const size_t h = m->c.hidden_size, k = m->c.top_k, r_bytes = n * k * 4;
+    const bool pin_routes = routes && 2 * r_bytes <= PIN_BYTES;
+    uint32_t *pin_ids = (uint32_t *)w->pin;
+    float *pin_w = (float *)(w->pin + r_bytes);
+    if (make_stage(w, h)) return cuda_failure(err, "pinned rows");
+    RowMoves moves;
+    plan_move(&moves.in, w, (float *)xs, x_pitch, n, h, true, scan);
+    plan_move(&moves.out, w, ys, y_pitch, n, h, false, false);
+    atomic_init(&moves.stage, 0);
+    const long cpus = sysconf(_SC_NPROCESSORS_ONLN);
+    pthread_t helper[HELPERS];
+    int helpers = 0;
+    /* the first slices are released before the helpers start, so that they find work */
+    atomic_store(&moves.in.limit, moves.in.slices < moves.in.ring ? moves.in.slices : moves.in.ring);
+    for (; n * h * 4 >= HELPER_MIN_BYTES && helpers < HELPERS && helpers + 1 < cpus; helpers++)
+        if (pthread_create(&helper[helpers], NULL, move_helper, &moves)) break;
+    int rc = w->status_clean ? 0 : status_clear(w);
+    w->status_clean = false;
+    if (!rc) rc = run_move(&moves.in, w, w->d.x);
+    *rejected = !rc && atomic_load(&moves.in.nonfinite);
+    Qwen4Status st = QW4_OK;
+    if (!rc && !*rejected) {
+        atomic_store(&moves.stage, 1);
+        rc = launch_layer(m, w, xs, x_pitch, w->d.y, n, start, NULL, NULL);
+        if (!rc) rc = qw4sh_memcpy2d_async(w->status_host, 16, w->d.status, 16, 16, 1, 0, w->d.stream);
+        if (!rc && pin_routes) {
+            rc |= qw4sh_memcpy2d_async(pin_ids, r_bytes, w->d.ids, r_bytes, r_bytes, 1, 0, w->d.stream);
+            rc |= qw4sh_memcpy2d_async(pin_w, r_bytes, w->d.weights, r_bytes, r_bytes, 1, 0, w->d.stream);
+        }
+        if (!rc) rc = qw4sh_stream_sync(w->d.stream);
+        if (!rc && (st = status_result(w, err)) == QW4_OK) {
+            w->status_clean = true;
+            if (routes && !pin_routes) {
+                rc |= qw4sh_memcpy2d_async(routes->ids.data + start * (routes->ids.row_stride_bytes / 4), routes->ids.row_stride_bytes,
+                                           w->d.ids, k * 4, k * 4, n, 0, w->d.stream);
+                rc |= qw4sh_memcpy2d_async(routes->weights.data + start * (routes->weights.stride_bytes[0] / 4),
+                                           routes->weights.stride_bytes[0], w->d.weights, k * 4, k * 4, n, 0, w->d.stream);
+            }
+            if (!rc) rc = run_move(&moves.out, w, w->d.y);
+            if (pin_routes) copy_routes(routes, start, n, k, pin_ids, pin_w);
+        }
+    }
+    atomic_store(&moves.stage, 2);
+    for (int i = 0; i < helpers; i++) pthread_join(helper[i], NULL);
+    /* behind a rejected batch its copies, behind a good one a route copy to pageable memory */
+    if ((rc || *rejected || (routes && !pin_routes)) && qw4sh_stream_sync(w->d.stream)) rc = -1;
+    if (rc) { w->status_clean = false; return cuda_failure(err, "layer execution"); }
+    return st;
+}
+
 Qwen4Status qwen4_moe_forward(const Qwen4Moe *m, Qwen4F32 x, Qwen4F32Mut y, Qwen4MoeRoutes *routes,
                               Qwen4MoeWork *w, Qwen4Error *err) {
     if (!m || !w) return report(err, QW4_INVALID_ARGUMENT, "null forward handle");
@@ -631,78 +861,23 @@ Qwen4Status qwen4_moe_forward(const Qwen4Moe *m, Qwen4F32 x, Qwen4F32Mut y, Qwen
             if (spans_meet(spans[b], weights)) return raise(err, QW4_INVALID_ARGUMENT, "argument %zu overlaps weight tensor %zu", b, a);
     }
     /* Nonfinite input is rejected before any state is touched (src/qwen4_moe.c:411-413). */
-    for (size_t row = 0; row < t; row++) {
-        const float *p = x.data + row * (x.stride_bytes[0] / 4);
-        for (size_t col = 0; col < h; col++)
-            if (!isfinite(p[col])) return report(err, QW4_NONFINITE, "nonfinite input");
-    }
+    const size_t x_pitch = x.stride_bytes[0] / 4, y_pitch = y.stride_bytes[0] / 4;
+    const bool small_call = 2 * t * (h + k) * 4 <= PIN_BYTES;
+    const bool scan_on_copy = !small_call && t <= w->chunk;           /* one ring's pass: nothing but scratch is written before its end */
+    if (!scan_on_copy && !rows_finite(x.data, x_pitch, t, h)) return report(err, QW4_NONFINITE, "nonfinite input");
     if (!t) return report(err, QW4_OK, "");
     w->busy = true;
     Qwen4Status st = QW4_OK;
-    const bool observe = w->observer != NULL;
-    for (size_t start = 0; start < t && st == QW4_OK; start += w->chunk) {
+    bool rejected = false;
+    for (size_t start = 0; start < t && st == QW4_OK && !rejected; start += w->chunk) {
         const size_t n = t - start < w->chunk ? t - start : w->chunk;
-        const float *xs = x.data + start * (x.stride_bytes[0] / 4);
-        float *ys = y.data + start * (y.stride_bytes[0] / 4);
-        const size_t x_bytes = n * h * 4, r_bytes = n * k * 4;
-        const bool small = 2 * x_bytes + 2 * r_bytes <= PIN_BYTES;
-        float *pin_x = (float *)w->pin, *pin_y = (float *)(w->pin + x_bytes);
-        uint32_t *pin_ids = (uint32_t *)(w->pin + 2 * x_bytes);
-        float *pin_w = (float *)(w->pin + 2 * x_bytes + r_bytes);
-        int rc = w->status_clean ? 0 : status_clear(w);
-        w->status_clean = false;
-        if (small) {
-            for (size_t row = 0; row < n; row++) memcpy(pin_x + row * h, xs + row * (x.stride_bytes[0] / 4), h * 4);
-            rc |= qw4sh_memcpy2d_async(w->d.x, h * 4, pin_x, h * 4, h * 4, n, 1, w->d.stream);
-        } else rc |= qw4sh_memcpy2d_async(w->d.x, h * 4, xs, x.stride_bytes[0], h * 4, n, 1, w->d.stream);
-        /* the one-kernel decode path writes each y element once and reads none: it stores straight into the pinned
-         * staging (device-addressable), and the copy of y back drops out of the call */
-        const bool direct_y = small && !observe && qw4sh_takes_fused(&m->layer, &w->d, w->d.x, pin_y, n);
-        if (!rc && observe)                    /* stage by stage in the reference's order, every stage shown to the observer */
-            rc = qw4sh_observed_forward(&m->layer, &w->d, w->d.x, w->d.y, n, xs, x.stride_bytes[0] / 4, start, w->observer, w->observer_ctx);
-        else if (!rc) {
-            if (direct_y) {                   /* the kernel also hands over the status words itself */
-                w->status_host[0] = UINT32_MAX; w->status_host[1] = UINT32_MAX;
-                w->d.status_mirror = w->status_host;
-            }
-            rc = qw4sh_layer_forward(&m->layer, &w->d, w->d.x, direct_y ? pin_y : w->d.y, n, NULL, NULL, current_router_mode());
-            w->d.status_mirror = NULL;
-        }
-        if (!rc && !direct_y) rc = qw4sh_memcpy2d_async(w->status_host, 16, w->d.status, 16, 16, 1, 0, w->d.stream);
-        if (!rc && small) {
-            if (!direct_y) rc = qw4sh_memcpy2d_async(pin_y, h * 4, w->d.y, h * 4, h * 4, n, 0, w->d.stream);
-            if (routes) {
-                rc |= qw4sh_memcpy2d_async(pin_ids, k * 4, w->d.ids, k * 4, k * 4, n, 0, w->d.stream);
-                rc |= qw4sh_memcpy2d_async(pin_w, k * 4, w->d.weights, k * 4, k * 4, n, 0, w->d.stream);
-            }
-        }
-        if (!rc) rc = qw4sh_stream_sync(w->d.stream);
-        if (!rc && direct_y && w->status_host[0] == UINT32_MAX)        /* the launch fell back to the multi-kernel sequence: fetch the words */
-            rc = qw4sh_memcpy(w->status_host, w->d.status, 16, 0);
-        if (rc) { st = cuda_failure(err, "layer execution"); break; }
-        if ((st = status_result(w, err)) != QW4_OK) break;
-        w->status_clean = true;
-        if (small) {
-            for (size_t row = 0; row < n; row++) {
-                memcpy(ys + row * (y.stride_bytes[0] / 4), pin_y + row * h, h * 4);
-                if (routes) {
-                    memcpy(routes->ids.data + (start + row) * (routes->ids.row_stride_bytes / 4), pin_ids + row * k, k * 4);
-                    memcpy(routes->weights.data + (start + row) * (routes->weights.stride_bytes[0] / 4), pin_w + row * k, k * 4);
-                }
-            }
-        } else {
-            rc = qw4sh_memcpy2d_async(ys, y.stride_bytes[0], w->d.y, h * 4, h * 4, n, 0, w->d.stream);
-            if (routes) {
-                rc |= qw4sh_memcpy2d_async(routes->ids.data + start * (routes->ids.row_stride_bytes / 4), routes->ids.row_stride_bytes,
-                                           w->d.ids, k * 4, k * 4, n, 0, w->d.stream);
-                rc |= qw4sh_memcpy2d_async(routes->weights.data + start * (routes->weights.stride_bytes[0] / 4),
-                                           routes->weights.stride_bytes[0], w->d.weights, k * 4, k * 4, n, 0, w->d.stream);
-            }
-            if (!rc) rc = qw4sh_stream_sync(w->d.stream);
-            if (rc) { st = cuda_failure(err, "result copy"); break; }
-        }
+        const float *xs = x.data + start * x_pitch;
+        float *ys = y.data + start * y_pitch;
+        st = 2 * n * (h + k) * 4 <= PIN_BYTES ? forward_few(m, w, xs, x_pitch, ys, y_pitch, n, start, routes, err)
+                                              : forward_many(m, w, xs, x_pitch, ys, y_pitch, n, start, routes, scan_on_copy, &rejected, err);
     }
     w->busy = false;
+    if (rejected) return report(err, QW4_NONFINITE, "nonfinite input");
     if (st != QW4_OK) { w->failed = true; return st; }
     return report(err, QW4_OK, "");
 }
