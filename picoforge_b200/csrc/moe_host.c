@@ -23,6 +23,8 @@ _Static_assert(sizeof(float) == 4 && sizeof(uint32_t) == 4, "32-bit elements");
 _Static_assert(sizeof(Qwen4F32) == 88 && sizeof(QW4PackedLayout) == 64, "ABI layout");
 
 enum { CHUNK_TOKENS = 2048, PIN_BYTES = 256 * 1024 };
+/* host calls of more rows (forward_many): ring of pinned slices, helper threads and the bytes from which on they help */
+enum { STAGE_BYTES = 2 << 20, SLICE_BYTES = 32 << 10, STAGE_EVENTS = 8, HELPERS = 3, HELPER_MIN_BYTES = 1 << 20 };
 
 struct Qwen4Moe {
     Qwen4MoeConfig c;
@@ -44,9 +46,9 @@ struct Qwen4MoeWork {
     QW4ShWork d;
     void *device_block;           /* one allocation carved into d.* */
     uint32_t *status_host;        /* pinned [4] */
-    unsigned char *stage;         /* pinned ring for the rows of larger host calls, from the first of them on */
+    unsigned char *stage;         /* pinned ring for the rows of larger host calls */
     size_t stage_bytes;
-    void *stage_event[8];
+    void *stage_event[STAGE_EVENTS];
     unsigned char *pin;           /* pinned staging: x | y | ids | weights for small batches */
     QW4MoeObserver observer;
     void *observer_ctx;
@@ -323,11 +325,19 @@ void qwen4_moe_work_destroy(Qwen4MoeWork *w) {
     qw4sh_host_free(w->status_host);
     qw4sh_host_free(w->pin);
     qw4sh_host_free(w->stage);
-    for (int i = 0; i < 8; i++) qw4sh_event_destroy(w->stage_event[i]);
+    for (int i = 0; i < STAGE_EVENTS; i++) qw4sh_event_destroy(w->stage_event[i]);
     release(w->owner);
     free(w);
 }
 
+/* The pinned ring and its events. */
+static int make_stage(Qwen4MoeWork *w, size_t cols) {
+    w->stage_bytes = cols * 4 * 8 > STAGE_BYTES ? cols * 4 * 8 : STAGE_BYTES;
+    w->stage = qw4sh_host_alloc(w->stage_bytes);
+    for (int i = 0; w->stage && i < STAGE_EVENTS; i++)
+        if (qw4sh_event_create(&w->stage_event[i])) return -1;
+    return w->stage ? 0 : -1;
+}
 Qwen4Status qwen4_moe_work_create(const Qwen4Moe *m, size_t cap, size_t budget, Qwen4MoeWork **out, Qwen4Error *err) {
     if (out) *out = NULL;
     if (!out) return report(err, QW4_INVALID_ARGUMENT, "null workspace output");
@@ -344,7 +354,8 @@ Qwen4Status qwen4_moe_work_create(const Qwen4Moe *m, size_t cap, size_t budget, 
     w->pin = qw4sh_host_alloc(PIN_BYTES);
     w->d.graph_cache = qw4sh_graph_cache_create();
     if (!w->device_block || !w->status_host || !w->pin || !w->d.graph_cache || qw4sh_shared_stream(&w->d.stream) ||
-        qw4sh_event_create(&w->d.timer[0]) || qw4sh_event_create(&w->d.timer[1])) {
+        qw4sh_event_create(&w->d.timer[0]) || qw4sh_event_create(&w->d.timer[1]) ||
+        (2 * cap * (m->c.hidden_size + m->c.top_k) * 4 > PIN_BYTES && make_stage(w, m->c.hidden_size))) {
         Qwen4Status st = cuda_failure(err, "workspace allocation");
         qwen4_moe_work_destroy(w);
         return st;
@@ -632,7 +643,6 @@ static bool rows_finite(const float *p, size_t pitch, size_t rows, size_t cols) 
     for (size_t r = 0; r < rows; r++) if (scan_floats((const uint32_t *)(p + r * pitch), cols)) return false;
     return true;
 }
-enum { STAGE_BYTES = 4 << 20, SLICE_BYTES = 128 << 10, STAGE_EVENTS = 8, HELPERS = 3, HELPER_MIN_BYTES = 1 << 20 };
 typedef struct {
     float *host;                                   /* the caller's rows */
     size_t pitch, cols, rows, slice_rows;
@@ -683,20 +693,25 @@ static void *move_helper(void *arg) {
     }
     return NULL;
 }
-/* All rows of `m` through the ring to or from dev.  0, or nonzero when a CUDA call failed. */
+/* All rows of `m` through the ring to or from dev, a group of slices per copy (a copy costs the calling thread 3.6 us whatever its size).
+ * 0, or nonzero when a CUDA call failed. */
 static int run_move(RowMove *m, Qwen4MoeWork *w, float *dev) {
-    int copied = 0, recorded = 0, retired = 0, moved = 0;            /* slices copied by the GPU; groups recorded, seen done; slices moved, in order */
+    const int groups = (m->slices + m->group - 1) / m->group;
+    int copied = 0, retired = 0, moved = 0;                          /* groups copied by the GPU, groups seen done; slices moved, in order */
     if (m->in) atomic_store(&m->limit, m->slices < m->ring ? m->slices : m->ring);
-    while (m->in ? copied < m->slices : moved < m->slices) {
-        while (copied < m->slices && (m->in ? slice_done(m, copied) : copied < m->ring || slice_done(m, copied - m->ring))) {
-            const size_t width = m->cols * 4, n = slice_count(m, copied);
-            float *rows = dev + (size_t)copied * m->slice_rows * m->cols;
-            unsigned char *slot = slice_slot(m, copied);
-            if (qw4sh_memcpy2d_async(m->in ? (void *)rows : slot, width * n, m->in ? slot : (void *)rows, width * n, width * n, 1, m->in, w->d.stream)) return -1;
-            if (++copied % m->group == 0 || copied == m->slices)
-                if (qw4sh_event_record(w->stage_event[recorded++ % STAGE_EVENTS], w->d.stream)) return -1;
+    while (m->in ? copied < groups : moved < m->slices) {
+        while (moved < m->slices && slice_done(m, moved)) moved++;
+        /* in: the group's slices are in the ring; out: its slots are free again */
+        const int needed = m->in ? (copied + 1) * m->group : (copied + 1) * m->group - m->ring;
+        if (copied < groups && moved >= (needed < m->slices ? needed : m->slices)) {
+            const int first = copied * m->group;
+            const size_t row = (size_t)first * m->slice_rows, rows = m->rows - row < m->group * m->slice_rows ? m->rows - row : m->group * m->slice_rows;
+            const size_t bytes = rows * m->cols * 4;
+            void *there = dev + row * m->cols, *slot = slice_slot(m, first);
+            if (qw4sh_memcpy2d_async(m->in ? there : slot, bytes, m->in ? slot : there, bytes, bytes, 1, m->in, w->d.stream) ||
+                qw4sh_event_record(w->stage_event[copied++ % STAGE_EVENTS], w->d.stream)) return -1;
         }
-        if (retired < recorded && atomic_load(&m->limit) < m->slices) {
+        if (retired < copied && atomic_load(&m->limit) < m->slices) {
             const int pending = qw4sh_event_query(w->stage_event[retired % STAGE_EVENTS]);
             if (pending < 0) return -1;
             if (!pending) {
@@ -704,19 +719,9 @@ static int run_move(RowMove *m, Qwen4MoeWork *w, float *dev) {
                 atomic_store(&m->limit, limit < m->slices ? limit : m->slices);
             }
         }
-        while (moved < m->slices && slice_done(m, moved)) moved++;
         if (!move_slice(m) && m->in) sched_yield();
     }
     return 0;
-}
-/* The pinned ring and its events, made by the first call that needs them and kept with the workspace. */
-static int make_stage(Qwen4MoeWork *w, size_t cols) {
-    if (w->stage) return 0;
-    w->stage_bytes = cols * 4 * 8 > STAGE_BYTES ? cols * 4 * 8 : STAGE_BYTES;
-    w->stage = qw4sh_host_alloc(w->stage_bytes);
-    for (int i = 0; w->stage && i < STAGE_EVENTS; i++)
-        if (qw4sh_event_create(&w->stage_event[i])) return -1;
-    return w->stage ? 0 : -1;
 }
 /* Waits for the decode kernel's status words in host memory: they come behind its results and before the launch has wound up.  A look at the
  * stream now and then catches a launch that never writes them. */
@@ -788,7 +793,6 @@ static Qwen4Status forward_many(const Qwen4Moe *m, Qwen4MoeWork *w, const float 
     const bool pin_routes = routes && 2 * r_bytes <= PIN_BYTES;
     uint32_t *pin_ids = (uint32_t *)w->pin;
     float *pin_w = (float *)(w->pin + r_bytes);
-    if (make_stage(w, h)) return cuda_failure(err, "pinned rows");
     RowMoves moves;
     plan_move(&moves.in, w, (float *)xs, x_pitch, n, h, true, scan);
     plan_move(&moves.out, w, ys, y_pitch, n, h, false, false);
