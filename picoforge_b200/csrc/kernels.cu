@@ -397,13 +397,16 @@ __global__ void __launch_bounds__(256) router_fast_kernel(DevTensor router, DevT
 // separately rounded multiply and add when EXACT (the reference's order and bits,
 // src/qwen4_packed.c:164-173); outputs are independent chains, so sixteen of them interleave in
 // each thread.  Row `experts` is the shared expert's gate.
-// TI x TJ outputs per thread (tokens x router rows): a CTA of 256 threads covers 16 TI tokens x 16 TJ rows.  The kernel
-// is bound by shared-memory reads and issue slots (two instructions per multiply-add in the exact mode), so the tile
-// per thread stays as large as the batch allows while the grid still covers the SMs.  (Packed mul.rn.f32x2 / add.rn.f32x2
-// on token pairs was 15% faster but its sums were not the scalar ones in the last bit, so the exact mode stays scalar.)
+// TI x TJ outputs per thread (tokens x router rows): a CTA of 256 threads covers 16 TI tokens x 16 TJ rows.  The kernel is
+// bound by the FP32 pipes: a separately rounded multiply and add of three register operands each take 1.57 issue cycles a
+// warp, measured, so 64 x 64 outputs cost 100 cycles a column on an SM.  Two tokens at a time they cost less: a packed multiply (2.05
+// cycles, each half rounded like a scalar one) and, in place of the packed addition, which the assembler fuses with the multiply into
+// other last bits, a packed fma with a one that it cannot see through (2.88; p * 1 + sum is the rounded sum).
+// Logits of 1024 tokens x 513 rows x 2048: 114 us -> 102; of 333 tokens, with a grid that covers the SMs, 97 -> 75.
 template <bool EXACT, int TI, int TJ>
 __global__ void __launch_bounds__(256) router_gemm_kernel(DevTensor router, DevTensor srouter, const float *__restrict__ x, uint32_t tokens,
-                                                          float *__restrict__ logits, float *__restrict__ shared_logit, uint32_t *status) {
+                                                          float *__restrict__ logits, float *__restrict__ shared_logit, uint32_t *status, float one) {
+    static_assert(TI % 2 == 0, "tokens in pairs");
     // columns per stage: the narrower the tile of router rows, the less arithmetic a stage holds, so it covers more
     // columns to keep the global-memory round trip of the next stage hidden (two stages of shared memory, <= 45 KB)
     constexpr int BM = 16 * TI, BN = 16 * TJ, BK = TJ >= 2 ? 32 : 64, PASSES = BK / 16;
@@ -418,11 +421,14 @@ __global__ void __launch_bounds__(256) router_gemm_kernel(DevTensor router, DevT
     const float *xrow = load_x && gt < tokens ? x + (uint64_t)gt * K : nullptr;
     const float *wrow = !load_w ? nullptr : ge < experts ? (const float *)(router.data + (uint64_t)ge * router.row_bytes)
                                                           : (ge == experts ? (const float *)srouter.data : nullptr);
-    float acc[TI][TJ];
+    typedef unsigned long long u64;
+    auto twice = [](float v) { return (u64)__float_as_uint(v) << 32 | __float_as_uint(v); };
+    const u64 one2 = twice(one);
+    u64 acc2[TI / 2][TJ];
 #pragma unroll
-    for (int i = 0; i < TI; i++)
+    for (int i = 0; i < TI / 2; i++)
 #pragma unroll
-        for (int j = 0; j < TJ; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < TJ; j++) acc2[i][j] = 0;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 xa[PASSES], wa[PASSES];
 #pragma unroll
@@ -449,17 +455,28 @@ __global__ void __launch_bounds__(256) router_gemm_kernel(DevTensor router, DevT
         }
 #pragma unroll 16
         for (int kk = 0; kk < BK; kk++) {
-            float av[TI], bv[TJ];
+            u64 av[TI / 2], bv[TJ];
 #pragma unroll
-            for (int i = 0; i < TI; i++) av[i] = xs[b][kk][ty * TI + i];
+            for (int i = 0; i < TI / 2; i++) av[i] = *reinterpret_cast<const u64 *>(&xs[b][kk][ty * TI + 2 * i]);
 #pragma unroll
-            for (int j = 0; j < TJ; j++) bv[j] = ws[b][kk][tx * TJ + j];
+            for (int j = 0; j < TJ; j++) bv[j] = twice(ws[b][kk][tx * TJ + j]);
 #pragma unroll
-            for (int i = 0; i < TI; i++)
+            for (int i = 0; i < TI / 2; i++)
 #pragma unroll
-                for (int j = 0; j < TJ; j++) acc[i][j] = EXACT ? __fadd_rn(acc[i][j], __fmul_rn(bv[j], av[i])) : fmaf(bv[j], av[i], acc[i][j]);
+                for (int j = 0; j < TJ; j++) {
+                    u64 p;
+                    if (EXACT) {
+                        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(bv[j]), "l"(av[i]));
+                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[i][j]) : "l"(p), "l"(one2));
+                    } else asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[i][j]) : "l"(bv[j]), "l"(av[i]));
+                }
         }
     }
+    float acc[TI][TJ];
+#pragma unroll
+    for (int i = 0; i < TI; i++)
+#pragma unroll
+        for (int j = 0; j < TJ; j++) acc[i][j] = __uint_as_float((uint32_t)(acc2[i / 2][j] >> (32 * (i & 1))));
     bool bad = false;
 #pragma unroll
     for (int i = 0; i < TI; i++) {
@@ -1231,13 +1248,13 @@ static int launch_router(const QW4ShLayer *layer, const float *x, size_t tokens,
     } else if (tokens > 16 && router.k_logical % 64 == 0 && ((uintptr_t)x & 15u) == 0 && router.row_bytes % 16 == 0) {
 #define ROUTER_GEMM(TI, TJ) do { \
         const dim3 grid((unsigned)((tokens + 16 * TI - 1) / (16 * TI)), (rows + 16 * TJ - 1) / (16 * TJ)); \
-        if (mode == 0) router_gemm_kernel<true, TI, TJ><<<grid, 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status); \
-        else router_gemm_kernel<false, TI, TJ><<<grid, 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status); } while (0)
-        // four tokens per thread always (one 128-bit read serves four chains); fewer router rows per thread for
-        // smaller batches, so that the grid still covers the SMs
-        if (tokens >= 768) ROUTER_GEMM(4, 4);
-        else if (tokens >= 384) ROUTER_GEMM(4, 2);
-        else ROUTER_GEMM(4, 1);
+        if (mode == 0) router_gemm_kernel<true, TI, TJ><<<grid, 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status, 1.0f); \
+        else router_gemm_kernel<false, TI, TJ><<<grid, 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status, 1.0f); } while (0)
+        // the largest tile that still leaves a CTA for (nearly) every SM: 513 rows are seventeen tiles of 32 or nine of 64, so 32 tokens x
+        // 32 rows up to 256 tokens, 32 x 64 up to 512, then 64 x 64
+        if (tokens <= 256) ROUTER_GEMM(2, 2);
+        else if (tokens <= 512) ROUTER_GEMM(2, 4);
+        else ROUTER_GEMM(4, 4);
 #undef ROUTER_GEMM
         LAUNCHED("router_gemm_kernel");
     } else if (mode == 0) {
