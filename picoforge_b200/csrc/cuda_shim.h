@@ -74,6 +74,7 @@ typedef struct {
     void *groups32, *shared_groups32;  /* groups of <= 32 rows (16 bytes each): routed, shared */
     uint32_t *n_groups32;         /* [2]: routed, shared */
     uint32_t *dispatch_scratch;   /* [2 * experts * ceil(cap / 32) + experts]: token bitmaps, word prefixes, counts */
+    uint32_t *row_counts;         /* [experts] rows per expert, zero between launches */
     uint32_t *sync;               /* [256]: counters and phase clocks of the one-kernel decode path */
     void *fused_aq, *fused_asc;   /* one-kernel decode path: activation digits and their per-chunk scales */
     float *logits_fast;           /* one-kernel decode path: tree-summed logits [4, experts + 1 padded to 4] */

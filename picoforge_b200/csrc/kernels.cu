@@ -572,11 +572,15 @@ __global__ void __launch_bounds__(128) route_kernel(uint32_t experts, uint32_t k
 
 // Routes of a batch (experts <= 512, k <= 32), each CTA `per` tokens (route_rows above), and, where `offsets` is given, the
 // dispatch of all of them: the stable per-expert lists (src/qwen4_moe.c:285-301; order inside an expert by ascending pair) and
-// the groups of up to 2^group_log rows that the expert products walk.  The CTA that arrives last at an atomic counter builds them; no CTA
-// waits for another.  An expert takes a token at most once, so its list is a set of tokens: one bit per (expert, token)
-// in shared memory, a prefix count per word, and a pair's row is its expert's first row plus the bits below its token.
-// All of it is latency, not work (2048 tokens: 20480 pairs, 40 per thread), which is why it is one launch: 1024 tokens took 17 us to route
-// with a warp per token, 22 us in a clear and four launches for the lists and 4 us for the groups.
+// the groups of up to 2^group_log rows that the expert products walk.  An expert takes a token at most once, so its list is a set
+// of tokens: one bit per (expert, token) in shared memory, a prefix count per word, and a pair's row is its expert's first
+// row plus the bits below its token.
+//
+// All of it is latency, not work.  Up to 64 tokens it is one launch: the CTA that arrives last at an atomic counter builds the lists (no CTA
+// waits for another).  Beyond, one CTA's scattered stores and bit updates (a cycle each) would take longer than the launch
+// they save (15 us for 1024 tokens, 28 for 2048): the routing CTAs only count the experts' rows, and dispatch_kernel
+// places them, eight experts per CTA.  Before, 1024 tokens took 17 us to route with a warp per token, 22 us in a clear and four launches
+// for the lists and 4 us for the groups.
 struct Group4 { uint32_t expert, first, count, pad; };
 struct RouteArgs {
     const float *logits;
@@ -589,12 +593,13 @@ struct RouteArgs {
     uint32_t *status;
     uint32_t *offsets, *pair_to_row, *row_to_pair, *active;     // offsets nullptr: routes only
     Group4 *groups; uint32_t *n_groups, group_log;
-    Group4 *dense; uint32_t *n_dense;                           // the shared expert's groups: all rows in turn (or nullptr)
+    Group4 *dense; uint32_t *n_dense;                           // the shared expert's groups, all rows in turn (or nullptr): up to 64 tokens
     uint32_t *ticket;                                           // zero between launches
+    uint32_t *counts;                                           // rows per expert, zero between launches: more than 64 tokens
 };
 static size_t route_smem_bytes(size_t tokens, uint32_t per, bool dispatch) {
     const size_t route = sizeof(RouteShared) + (size_t)per * RT_PITCH * 4, words = ((tokens + 31) / 32) | 1;
-    const size_t lists = dispatch ? 512 * words * 6 : 0;
+    const size_t lists = dispatch && tokens <= 64 ? 512 * words * 6 : 0;
     return route > lists ? route : lists;
 }
 __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant__ RouteArgs a) {
@@ -602,7 +607,8 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
     __shared__ uint32_t s_last, wrows[16], wgroups[16], s_first[512];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, E = a.experts, k = a.k;
     const uint32_t row0 = blockIdx.x * a.per;
-    route_rows<16>(row0, min(a.per, a.tokens - row0), E, k, a.norm, true, reinterpret_cast<float *>(rb_smem + sizeof(RouteShared)),
+    const uint32_t rows = min(a.per, a.tokens - row0);
+    const uint32_t bad = route_rows<16>(row0, rows, E, k, a.norm, true, reinterpret_cast<float *>(rb_smem + sizeof(RouteShared)),
                    *reinterpret_cast<RouteShared *>(rb_smem), a.status, a.probs,
                    [&](uint32_t t, uint32_t e) { return __ldg(a.logits + (uint64_t)t * a.pitch + e); },
                    [&](uint32_t t, uint32_t slot, uint32_t id, float w) {
@@ -610,8 +616,11 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
                        a.ids[at] = id; a.weights[at] = w;
                        if (a.ids_out) a.ids_out[at] = id;
                        if (a.weights_out) a.weights_out[at] = w;
+                       if (a.counts) atomicAdd(a.counts + id, 1u);
                    });
-    if (!a.offsets) return;
+    if (a.counts)                                               // a row without routes has no pairs
+        for (uint32_t i = tid; i < rows * k; i += 512) if ((bad >> (i / k)) & 1u) a.ids[(uint64_t)row0 * k + i] = 0xffffffffu;
+    if (!a.offsets || a.counts) return;
     // ---- the CTA that arrives last does the dispatch for all tokens ----
     __threadfence();
     __syncthreads();
@@ -636,15 +645,15 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
     for (uint32_t w = 0; w < words; w++) { before[tid * pitch + w] = (uint16_t)count; count += __popc(bits[tid * pitch + w]); }
     const uint32_t per_group = 1u << a.group_log, n_groups = (count + per_group - 1) >> a.group_log;
     const uint32_t listed = n_groups | (count ? 1u << 20 : 0u);                                // groups, then experts with rows from bit 20
-    uint32_t rows = count, groups = listed;
+    uint32_t total = count, groups = listed;
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, rows, o), u = __shfl_up_sync(0xffffffffu, groups, o);
-        if (lane >= (uint32_t)o) { rows += v; groups += u; }
+        const uint32_t v = __shfl_up_sync(0xffffffffu, total, o), u = __shfl_up_sync(0xffffffffu, groups, o);
+        if (lane >= (uint32_t)o) { total += v; groups += u; }
     }
-    if (lane == 31) { wrows[warp] = rows; wgroups[warp] = groups; }
+    if (lane == 31) { wrows[warp] = total; wgroups[warp] = groups; }
     __syncthreads();
-    for (uint32_t w = 0; w < warp; w++) { rows += wrows[w]; groups += wgroups[w]; }
-    const uint32_t first = rows - count, at = groups - listed;
+    for (uint32_t w = 0; w < warp; w++) { total += wrows[w]; groups += wgroups[w]; }
+    const uint32_t first = total - count, at = groups - listed;
     s_first[tid] = first;
     if (tid < E) {
         a.offsets[tid] = first;
@@ -652,7 +661,7 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
         for (uint32_t j = 0; j < n_groups; j++)
             a.groups[(at & 0xfffffu) + j] = Group4{tid, first + (j << a.group_log), min(per_group, count - (j << a.group_log)), 0};
     }
-    if (tid == 511) { a.offsets[E] = rows; *a.n_groups = groups & 0xfffffu; a.active[0] = groups >> 20; }
+    if (tid == 511) { a.offsets[E] = total; *a.n_groups = groups & 0xfffffu; a.active[0] = groups >> 20; }
     if (a.dense) {
         const uint32_t n = (a.tokens + per_group - 1) >> a.group_log;
         for (uint32_t j = tid; j < n; j += 512) a.dense[j] = Group4{0, j << a.group_log, min(per_group, a.tokens - (j << a.group_log)), 0};
@@ -667,6 +676,75 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
             a.pair_to_row[q] = row; a.row_to_pair[row] = q;
         }
     }
+}
+
+// The lists of eight experts per CTA, from the rows' counts and ids that route_batch_kernel left.  Every CTA reads all counts (their scan
+// gives it the first rows of its experts) and all ids (coalesced, eight in flight per thread), keeps the pairs of its own
+// experts, and writes them in order of tokens.
+constexpr uint32_t DK_EXPERTS = 8, DK_WORDS = 64, DK_KEEP = DK_EXPERTS * DK_WORDS * 32;      // 2048 tokens; pairs of eight experts, at most
+__global__ void __launch_bounds__(512) dispatch_kernel(const __grid_constant__ RouteArgs a) {
+    extern __shared__ uint32_t kept[];                          // pair | own expert << 24
+    __shared__ uint32_t wrows[16], wgroups[16], bits[DK_EXPERTS][DK_WORDS + 1], before[DK_EXPERTS][DK_WORDS + 1], s_first[DK_EXPERTS], n_kept;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, E = a.experts, k = a.k, pairs = a.tokens * k;
+    const uint32_t own = blockIdx.x * DK_EXPERTS, words = (a.tokens + 31) / 32;
+    for (uint32_t i = tid; i < DK_EXPERTS * (DK_WORDS + 1); i += 512) (&bits[0][0])[i] = 0;
+    if (tid == 0) n_kept = 0;
+    const uint32_t count = tid < E ? __ldcg(a.counts + tid) : 0u;
+    __syncthreads();
+    for (uint32_t q0 = 0; q0 < pairs; q0 += 512 * 8) {
+        uint32_t id[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) { const uint32_t q = q0 + j * 512 + tid; id[j] = q < pairs ? __ldcg(a.ids + q) : 0xffffffffu; }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const uint32_t x = id[j] - own;
+            if (x < DK_EXPERTS && id[j] < E) {
+                const uint32_t q = q0 + j * 512 + tid, t = q / k;
+                atomicOr(&bits[x][t >> 5], 1u << (t & 31u));
+                kept[atomicAdd(&n_kept, 1u)] = q | x << 24;
+            }
+        }
+    }
+    const uint32_t per_group = 1u << a.group_log, n_groups = (count + per_group - 1) >> a.group_log;
+    const uint32_t listed = n_groups | (count ? 1u << 20 : 0u);
+    uint32_t total = count, groups = listed;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, total, o), u = __shfl_up_sync(0xffffffffu, groups, o);
+        if (lane >= (uint32_t)o) { total += v; groups += u; }
+    }
+    if (lane == 31) { wrows[warp] = total; wgroups[warp] = groups; }
+    __syncthreads();
+    for (uint32_t w = 0; w < warp; w++) { total += wrows[w]; groups += wgroups[w]; }
+    const uint32_t first = total - count, at = groups - listed;
+    if (tid - own < DK_EXPERTS && tid < E) {
+        s_first[tid - own] = first;
+        a.offsets[tid] = first;
+        if (count) a.active[1 + (at >> 20)] = tid;
+        for (uint32_t j = 0; j < n_groups; j++)
+            a.groups[(at & 0xfffffu) + j] = Group4{tid, first + (j << a.group_log), min(per_group, count - (j << a.group_log)), 0};
+    }
+    if (tid == 511 && blockIdx.x == 0) { a.offsets[E] = total; *a.n_groups = groups & 0xfffffu; a.active[0] = groups >> 20; }
+    if (warp < DK_EXPERTS) {                                    // prefix counts of an expert's words: one warp
+        uint32_t running = 0;
+        for (uint32_t w0 = 0; w0 < words; w0 += 32) {
+            const uint32_t c = w0 + lane < words ? __popc(bits[warp][w0 + lane]) : 0u;
+            uint32_t scan = c;
+            for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(0xffffffffu, scan, o); if (lane >= (uint32_t)o) scan += v; }
+            if (w0 + lane < words) before[warp][w0 + lane] = running + scan - c;
+            running += __shfl_sync(0xffffffffu, scan, 31);
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < n_kept; i += 512) {
+        const uint32_t q = kept[i] & 0xffffffu, x = kept[i] >> 24, t = q / k;
+        const uint32_t row = s_first[x] + before[x][t >> 5] + __popc(bits[x][t >> 5] & ((1u << (t & 31u)) - 1u));
+        a.pair_to_row[q] = row; a.row_to_pair[row] = q;
+    }
+    // the CTA that arrives last leaves the counts zero for the next launch: all have read them
+    __shared__ uint32_t s_last;
+    if (tid == 0) { __threadfence(); s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1 ? 1u : 0u; }
+    __syncthreads();
+    if (s_last) { if (tid < E) a.counts[tid] = 0; if (tid == 0) *a.ticket = 0; }
 }
 
 // ------------------------------------------------------------------------------------
@@ -1188,6 +1266,13 @@ static int launch_route_batch(RouteArgs &a, cudaStream_t stream) {
     if (!configured[device]) { if (allow_smem(route_batch_kernel, 220u * 1024u)) return -1; configured[device] = true; }
     route_batch_kernel<<<(a.tokens + a.per - 1) / a.per, 512, route_smem_bytes(a.tokens, a.per, a.offsets != nullptr), stream>>>(a);
     LAUNCHED("route_batch_kernel");
+    if (a.counts) {
+        static bool dispatch_configured[64] = {false};
+        if (!dispatch_configured[device]) { if (allow_smem(dispatch_kernel, DK_KEEP * 4)) return -1; dispatch_configured[device] = true; }
+        // an expert's list holds a token once at most
+        dispatch_kernel<<<(a.experts + DK_EXPERTS - 1) / DK_EXPERTS, 512, DK_EXPERTS * a.tokens * 4, stream>>>(a);
+        LAUNCHED("dispatch_kernel");
+    }
     return 0;
 }
 
@@ -1534,7 +1619,7 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
         (void)cudaGetLastError();
     }
     const bool prefill = prefill_path(layer, tokens), tc = prefill || tile_path(layer, tokens), mma = !tc && mma_path(layer, tokens);
-    const bool listed = (tc || mma) && E <= 512 && k <= 32 && T <= 2048;      // routes and lists in one launch
+    const bool listed = (tc || mma) && E <= 512 && k <= 32 && T <= DK_WORDS * 32;      // the lists come with the routes
     int rc, stage = 0;
 #define STAGE_MARK() do { if (timed) CU(cudaEventRecord(g_stage_event[stage++], stream)); } while (0)
     STAGE_MARK();
@@ -1574,7 +1659,7 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
     auto shared_branch = [&](int which) -> int {
         if (which == 0) {
             if (tc) { if ((rc = qw4sh_build_dense_tile_groups(T, work->shared_groups32, work->n_groups32 + 1, side))) return rc; }
-            else if (!listed && (rc = qw4sh_build_dense_groups(T, shared_groups, work->n_groups + 1, side))) return rc;
+            else if ((!listed || T > 64) && (rc = qw4sh_build_dense_groups(T, shared_groups, work->n_groups + 1, side))) return rc;
             return STEP(4) ? products(0, true, side) : 0;
         }
         if (mma && STEP(7) && (rc = qw4sh_quantize_rows(work->shared_act, T, layer->shared_inter, work->sq, work->sneg, work->ssum, work->sscale, side))) return rc;
@@ -1588,8 +1673,9 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
         a.ids = work->ids; a.weights = work->weights; a.ids_out = ids_out; a.weights_out = weights_out; a.status = work->status;
         a.offsets = work->offsets; a.pair_to_row = work->pair_to_row; a.row_to_pair = work->row_to_pair; a.active = work->active;
         a.groups = (Group4 *)(tc ? work->groups32 : work->groups); a.n_groups = tc ? work->n_groups32 : work->n_groups; a.group_log = tc ? 5 : 2;
-        if (mma) { a.dense = (Group4 *)shared_groups; a.n_dense = work->n_groups + 1; }
+        if (mma && T <= 64) { a.dense = (Group4 *)shared_groups; a.n_dense = work->n_groups + 1; }
         a.ticket = work->n_groups + 2;
+        if (T > 64) a.counts = work->row_counts;
         if (STEP(2) && (rc = launch_route_batch(a, stream))) return rc;
         STAGE_MARK(); STAGE_MARK();
         if (overlap && mma) {                         // shared groups are written by the same kernel

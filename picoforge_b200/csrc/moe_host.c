@@ -281,7 +281,7 @@ static Qwen4Status plan_work(const Qwen4Moe *m, size_t cap, size_t *chunk, Plan 
     const size_t g32 = pairs / 32 + e + 2;                   /* groups of <= 32 rows: at most pairs/32 + experts */
     size_t fused_aq = 0, fused_asc = 0, fused_fast = 0;
     qw4sh_fused_scratch_sizes(&m->layer, &fused_aq, &fused_asc, &fused_fast);
-    const size_t count[55] = {t * h, t * h, t * e, t * e, t, pairs, pairs, e + 1, pairs, pairs, e + 1,
+    const size_t count[56] = {t * h, t * h, t * e, t * e, t, pairs, pairs, e + 1, pairs, pairs, e + 1,
         pairs * i, t * si, t * h, 4,
         pairs * h, t * h,                                   /* 15 out, 16 shared_out */
         t * h / 2 + 8, t * h / 2 + 8, t * (h / 32 + 1) * 2, t,                 /* 17 xq, 18 xneg, 19 xsum, 20 xscale */
@@ -295,9 +295,10 @@ static Qwen4Status plan_work(const Qwen4Moe *m, size_t cap, size_t *chunk, Plan 
         g32 * 4 + (t / 32 + 2) * 4, 8,                      /* 46 groups of <= 32 rows (routed, then shared), 47 their counts */
         2 * e * (t / 32 + 1) + e + 8,                       /* 48 dispatch scratch */
         fused_aq / 4, fused_asc / 4, fused_fast / 4,        /* 49-51 one-kernel decode path */
-        t, pairs * (i / 128 + 1), t * (si / 128 + 1)};      /* 52-54 what undoes the scales of x, act, shared act */
+        t, pairs * (i / 128 + 1), t * (si / 128 + 1),       /* 52-54 what undoes the scales of x, act, shared act */
+        e};                                                 /* 55 rows per expert */
     size_t at = 0;
-    for (int j = 0; j < 55; j++) {
+    for (int j = 0; j < 56; j++) {
         if (count[j] > (SIZE_MAX >> 4)) return report(err, QW4_OVERFLOW, "scratch size overflow");
         plan->offset[j] = at;
         at += align256(count[j] * 4 + 4);
@@ -389,7 +390,7 @@ Qwen4Status qwen4_moe_work_create(const Qwen4Moe *m, size_t cap, size_t budget, 
     w->d.groups32 = base + plan.offset[46];
     w->d.shared_groups32 = (char *)w->d.groups32 + (pairs_of(m, chunk) / 32 + m->c.experts + 2) * 16;
     w->d.n_groups32 = (uint32_t *)(base + plan.offset[47]);
-    w->d.dispatch_scratch = (uint32_t *)(base + plan.offset[48]);
+    w->d.dispatch_scratch = (uint32_t *)(base + plan.offset[48]); w->d.row_counts = (uint32_t *)(base + plan.offset[55]);
     w->d.fused_aq = base + plan.offset[49]; w->d.fused_asc = base + plan.offset[50];
     w->d.logits_fast = (float *)(base + plan.offset[51]);
     if (qw4sh_prepare_mma()) {
