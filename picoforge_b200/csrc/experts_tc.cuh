@@ -708,27 +708,28 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
                 share[lane] = __float_as_uint(lane < grp.count ? __ldg(a.in_scale + my_pair / a.k_div) : 0.0f);
                 float *mine = hand + row + (row >> 4);
                 asm volatile("bar.sync 1, 256;" ::: "memory");                // the hand-over tile's previous content has been taken
-                if (m == 1)
+                // the gate's warps take the lower half of the tokens, the up's the upper: each hands over what the other needs
+                const uint32_t half = (grp.count + 7u) / 8u * 4u;
 #pragma unroll
-                    for (uint32_t n = 0; n < XTOK; n++) if (n < grp.count) mine[n * XPITCH] = acc[n];
+                for (uint32_t n = 0; n < XTOK; n++) if (n < grp.count && (n < half) == (m == 1)) mine[n * XPITCH] = acc[n];
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (m == 0)
 #pragma unroll
-                    for (uint32_t n4 = 0; n4 < XTOK; n4 += 4) {
-                        if (n4 >= grp.count) break;
-                        const float4 s4 = *reinterpret_cast<const float4 *>(share + n4);
-                        const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
+                for (uint32_t n4 = 0; n4 < XTOK; n4 += 4) {
+                    if (n4 >= grp.count) break;
+                    if ((n4 < half) != (m == 0)) continue;
+                    const float4 s4 = *reinterpret_cast<const float4 *>(share + n4);
+                    const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
-                        for (uint32_t i = 0; i < 4; i++) {
-                            const uint32_t n = n4 + i;
-                            if (n < grp.count) {
-                                const float g = acc[n] * sv[i], up = mine[n * XPITCH] * sv[i];
-                                const float e = __expf(-fabsf(g));
-                                const float sig = g >= 0.0f ? __fdividef(1.0f, 1.0f + e) : __fdividef(e, 1.0f + e);
-                                mine[n * XPITCH] = g * sig * up;
-                            }
+                    for (uint32_t i = 0; i < 4; i++) {
+                        const uint32_t n = n4 + i;
+                        if (n < grp.count) {
+                            const float own = acc[n] * sv[i], other = mine[n * XPITCH] * sv[i];
+                            const float g = m == 0 ? own : other, up = m == 0 ? other : own;
+                            const float e = __expf(-fabsf(g));
+                            mine[n * XPITCH] = g * __fdividef(g >= 0.0f ? 1.0f : e, 1.0f + e) * up;
                         }
                     }
+                }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 // eight threads a token, sixteen columns each: the tile's power of two, hi and lo, sums of eight columns
                 const uint32_t n = et >> 3, seg = et & 7u;
