@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
 // The lists of eight experts per CTA, from the rows' counts and ids that route_batch_kernel left.  Every CTA reads all counts (their scan
 // gives it the first rows of its experts) and all ids (coalesced, eight in flight per thread), keeps the pairs of its own
 // experts, and writes them in order of tokens.
-constexpr uint32_t DK_EXPERTS = 8, DK_WORDS = 64, DK_KEEP = DK_EXPERTS * DK_WORDS * 32;      // 2048 tokens; pairs of eight experts, at most
+constexpr uint32_t DK_EXPERTS = 8, DK_WORDS = 128, DK_KEEP = DK_EXPERTS * DK_WORDS * 32;     // 4096 tokens; pairs of eight experts, at most
 __global__ void __launch_bounds__(512) dispatch_kernel(const __grid_constant__ RouteArgs a) {
     extern __shared__ uint32_t kept[];                          // pair | own expert << 24
     __shared__ uint32_t wrows[16], wgroups[16], bits[DK_EXPERTS][DK_WORDS + 1], before[DK_EXPERTS][DK_WORDS + 1], s_first[DK_EXPERTS], n_kept;

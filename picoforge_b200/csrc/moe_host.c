@@ -22,7 +22,11 @@
 _Static_assert(sizeof(float) == 4 && sizeof(uint32_t) == 4, "32-bit elements");
 _Static_assert(sizeof(Qwen4F32) == 88 && sizeof(QW4PackedLayout) == 64, "ABI layout");
 
-enum { CHUNK_TOKENS = 2048, PIN_BYTES = 256 * 1024 };
+/* Tokens of one launch sequence.  The expert products work on groups of up to 32 rows of an expert and decode its weights once per group:
+ * with 512 experts and top-10, 2048 tokens make groups that are 62% full, 4096 tokens 83%, 8192 tokens 91%; the
+ * workspace grows in proportion (0.85 GB a layer at 4096), so the line is drawn at 4096.  Calls that take one sequence at most keep their
+ * limit of STEP_TOKENS. */
+enum { CHUNK_TOKENS = 4096, STEP_TOKENS = 2048, PIN_BYTES = 256 * 1024 };
 /* host calls of more rows (forward_many): ring of pinned slices, helper threads and the bytes from which on they help */
 enum { STAGE_BYTES = 2 << 20, SLICE_BYTES = 32 << 10, STAGE_EVENTS = 8, HELPERS = 3, HELPER_MIN_BYTES = 1 << 20 };
 
@@ -469,7 +473,7 @@ Qwen4Status qw4cu_moe_forward_hc_add_device(const Qwen4Moe *m, const float *x_de
     if (!m || !w) return report(err, QW4_INVALID_ARGUMENT, "null forward handle");
     if (tokens && (!residual_dev || !inject_dev)) return report(err, QW4_INVALID_ARGUMENT, "null hyper-connection view");
     if (!streams || streams > 64) return report(err, QW4_SHAPE, "hyper-connection streams out of range");
-    if (tokens > w->chunk) return report(err, QW4_CAPACITY, "batch exceeds one launch sequence (2048 rows)");
+    if (tokens > w->chunk || tokens > STEP_TOKENS) return report(err, QW4_CAPACITY, "batch exceeds one launch sequence (2048 rows)");
     w->d.hc_residual = residual_dev; w->d.hc_inject = inject_dev; w->d.hc_streams = (uint32_t)streams;
     const Qwen4Status st = qw4cu_moe_forward_device(m, x_dev, y_dev, tokens, NULL, NULL, w, err);
     w->d.hc_residual = NULL; w->d.hc_inject = NULL; w->d.hc_streams = 0;
@@ -482,7 +486,7 @@ static Qwen4Status piece_checks(const Qwen4Moe *m, Qwen4MoeWork *w, size_t rows,
     if (w->owner != m) return report(err, QW4_OWNER, "workspace belongs to another MoE");
     if (!m->alive || w->failed) return report(err, QW4_BAD_STATE, "inactive MoE/workspace; reset required");
     if (w->busy) return report(err, QW4_BUSY, "workspace executing");
-    if (rows > w->chunk || rows > w->cap) return report(err, QW4_CAPACITY, "batch exceeds the workspace (capacity, 2048 rows at most)");
+    if (rows > w->chunk || rows > w->cap || rows > STEP_TOKENS) return report(err, QW4_CAPACITY, "batch exceeds the workspace (capacity, 2048 rows at most)");
     use_current_stream(w);
     w->status_clean = false;
     return QW4_OK;
