@@ -1,0 +1,50 @@
+"""The layer at the sizes where its kernels' tiles end: the exact router's chain tiles (8, 16, 32, 64, 128 tokens) and GEMM
+tiles (256, 512), groups of 32 rows, the two ways of building the lists (64 tokens), short K rings and the widened formats, on
+device pointers and host views, against the CPU oracle: ids and weights bit for bit, y within 1e-3."""
+import numpy as np
+import pytest
+
+from picoforge_b200 import abi, synth
+from picoforge_b200.layer import MoeLayer
+
+pytestmark = pytest.mark.gpu
+
+Q4, Q2, IQ2, F32 = abi.Q4_K, abi.Q2_K, abi.IQ2_XXS, abi.F32
+
+
+@pytest.mark.parametrize("routed,down,shared,hidden,inter,physical,experts,top_k,tokens", [
+    (Q4, Q4, Q4, 256, 256, 256, 4, 2, 5),            # K of one block: rings shorter than their slots
+    (Q2, Q2, Q2, 512, 256, 256, 3, 2, 8),
+    (IQ2, IQ2, Q4, 1536, 512, 512, 40, 10, 9),       # 41 router rows: a ragged last tile
+    (IQ2, Q2, F32, 1536, 384, 512, 16, 4, 16),        # the checkpoint's mixture: stored padding, a widened shared expert
+    (IQ2, Q2, F32, 512, 640, 768, 33, 6, 17),
+    (Q2, Q2, Q4, 2560, 256, 256, 24, 8, 32),         # K beyond one pass of the chain ring
+    (Q4, Q4, F32, 512, 256, 256, 5, 1, 33),           # top-1; groups of 32 and 1 rows in the shared expert
+    (Q4, Q4, Q4, 512, 256, 256, 2, 2, 64),           # every expert takes every token: two full groups each
+    (Q4, Q4, Q4, 512, 256, 256, 2, 2, 65),           # the first size with a launch of its own for the lists
+    (Q2, Q2, Q2, 512, 512, 512, 7, 3, 128),
+    (IQ2, IQ2, Q4, 512, 512, 512, 96, 10, 129),     # the first size of the router GEMM
+    (Q4, Q4, Q4, 512, 256, 256, 512, 10, 257),
+    (IQ2, Q2, F32, 512, 384, 512, 130, 8, 513),
+])
+def test_layer_at_tile_edges(gpu, routed, down, shared, hidden, inter, physical, experts, top_k, tokens):
+    import oracle
+    spec = synth.make_layer(7000 + tokens, routed_type=routed, down_type=down, shared_type=shared, hidden=hidden, inter=inter, shared_inter=256,
+                            down_physical=physical, experts=experts, top_k=top_k)
+    x = synth.activations(7000 + tokens, tokens, hidden)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    with MoeLayer(gpu, spec, tokens) as layer:
+        y, ids, weights = layer.forward(x)
+        y2, ids2, weights2 = layer.forward(x)
+        bad = x.copy()
+        bad[tokens - 1, hidden - 1] = np.inf
+        with pytest.raises(abi.MoeError):
+            layer.forward(bad)                       # found while the rows are staged: nothing is written, the workspace stays usable
+        y3, _, _ = layer.forward(x)
+    np.testing.assert_array_equal(ids, want["ids"])
+    np.testing.assert_array_equal(weights, want["weights"])
+    assert np.abs(y - want["y"]).max() <= 1e-3
+    np.testing.assert_array_equal(y2, y)             # deterministic
+    np.testing.assert_array_equal(y3, y)
+    np.testing.assert_array_equal(ids2, ids)
+    np.testing.assert_array_equal(weights2, weights)
