@@ -431,6 +431,9 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
     xtc_before();
     __syncthreads();
     xtc_after();
+    // The down product is launched while gate/up still runs: its CTAs move in as those leave, and fetch and dequantise weights (the groups are
+    // older than both) until the activation rows, which alone wait for gate/up's end, hold them up.
+    if (MODE == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr uint32_t tmem = 0;                                            // all 512 columns are this CTA's
     const uint32_t n_items = *a.n_groups * a.tiles;
 
@@ -481,6 +484,7 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
         // ---------------- activation rows: hi by one warp, lo by the other ----------------
         // eight lanes take the 128 bytes of a row, so an instruction touches four lines of the cache and not thirty-two
         const uint32_t part = warp - R::ACT, piece = lane & 7u, sub = lane >> 3;
+        if (MODE == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
         constexpr uint32_t LAG = 2;                                           // steps between a copy's issue and its hand-over
         uint32_t n = 0, un = 0;
         bool ok = true;

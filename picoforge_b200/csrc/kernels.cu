@@ -344,6 +344,7 @@ __global__ void __launch_bounds__(ROWS * TOK) router_chain_kernel(DevTensor rout
             if (tid < 32 && c + STAGES < chunks) { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); issue(c + STAGES); }
         }
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");              // the routing may move in; not before: its CTAs would keep others off the SMs
     const uint32_t e = e0 + er, t = t0 + tc;
     if (e <= experts && t < tokens && alive) {
         if (!finite_f32(sum)) atomicOr(status, QW4SH_ERR_NONFINITE);
@@ -472,6 +473,7 @@ __global__ void __launch_bounds__(256) router_gemm_kernel(DevTensor router, DevT
                 }
         }
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");              // the routing may move in; not before: its CTAs would keep others off the SMs
     float acc[TI][TJ];
 #pragma unroll
     for (int i = 0; i < TI; i++)
@@ -607,6 +609,7 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
     __shared__ uint32_t s_last, wrows[16], wgroups[16], s_first[512];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, E = a.experts, k = a.k;
     const uint32_t row0 = blockIdx.x * a.per;
+    asm volatile("griddepcontrol.wait;" ::: "memory");                          // launched while the router drains
     const uint32_t rows = min(a.per, a.tokens - row0);
     const uint32_t bad = route_rows<16>(row0, rows, E, k, a.norm, true, reinterpret_cast<float *>(rb_smem + sizeof(RouteShared)),
                    *reinterpret_cast<RouteShared *>(rb_smem), a.status, a.probs,
@@ -618,6 +621,7 @@ __global__ void __launch_bounds__(512) route_batch_kernel(const __grid_constant_
                        if (a.weights_out) a.weights_out[at] = w;
                        if (a.counts) atomicAdd(a.counts + id, 1u);
                    });
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (a.counts)                                               // a row without routes has no pairs
         for (uint32_t i = tid; i < rows * k; i += 512) if ((bad >> (i / k)) & 1u) a.ids[(uint64_t)row0 * k + i] = 0xffffffffu;
     if (!a.offsets || a.counts) return;
@@ -689,6 +693,7 @@ __global__ void __launch_bounds__(512) dispatch_kernel(const __grid_constant__ R
     const uint32_t own = blockIdx.x * DK_EXPERTS, words = (a.tokens + 31) / 32;
     for (uint32_t i = tid; i < DK_EXPERTS * (DK_WORDS + 1); i += 512) (&bits[0][0])[i] = 0;
     if (tid == 0) n_kept = 0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t count = tid < E ? __ldcg(a.counts + tid) : 0u;
     __syncthreads();
     for (uint32_t q0 = 0; q0 < pairs; q0 += 512 * 8) {
@@ -1254,6 +1259,16 @@ static int sm_count() {
         g_sm_count[device] = 148;
     return g_sm_count[device];
 }
+// A launch that may begin before the one ahead of it in the stream has ended; its kernel waits (griddepcontrol.wait) before it
+// touches what that one wrote.
+static cudaError_t launch_behind(void (*kernel)(RouteArgs), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const RouteArgs &a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization; attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
 // Tokens per CTA: as few as cover the SMs once, sixteen at most (one lane of a warp sums one row, and one warp ranks one).
 static int launch_route_batch(RouteArgs &a, cudaStream_t stream) {
     static bool configured[64] = {false};
@@ -1264,13 +1279,13 @@ static int launch_route_batch(RouteArgs &a, cudaStream_t stream) {
     CU(cudaGetDevice(&device));
     if (device < 0 || device >= 64) return fail(cudaErrorInvalidDevice, "device index");
     if (!configured[device]) { if (allow_smem(route_batch_kernel, 220u * 1024u)) return -1; configured[device] = true; }
-    route_batch_kernel<<<(a.tokens + a.per - 1) / a.per, 512, route_smem_bytes(a.tokens, a.per, a.offsets != nullptr), stream>>>(a);
+    CU(launch_behind(route_batch_kernel, (a.tokens + a.per - 1) / a.per, 512, route_smem_bytes(a.tokens, a.per, a.offsets != nullptr), stream, a));
     LAUNCHED("route_batch_kernel");
     if (a.counts) {
         static bool dispatch_configured[64] = {false};
         if (!dispatch_configured[device]) { if (allow_smem(dispatch_kernel, DK_KEEP * 4)) return -1; dispatch_configured[device] = true; }
         // an expert's list holds a token once at most
-        dispatch_kernel<<<(a.experts + DK_EXPERTS - 1) / DK_EXPERTS, 512, DK_EXPERTS * a.tokens * 4, stream>>>(a);
+        CU(launch_behind(dispatch_kernel, (a.experts + DK_EXPERTS - 1) / DK_EXPERTS, 512, DK_EXPERTS * a.tokens * 4, stream, a));
         LAUNCHED("dispatch_kernel");
     }
     return 0;
@@ -1647,8 +1662,13 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
         float *out = shared ? work->shared_out : work->out;
         if (tc) {
             const QW4ShSplit *act = shared ? &work->split_shared : &work->split_act;
+            const uint32_t items = (shared ? (T + 31) / 32 : T * k) * (mode ? w0->n_out / 256 : w0->n_out / 128);      // most that there can be
+            // a few rows' shared expert is still on its (at most sixteen) SMs when the routed gate/up starts: that one leaves them out, because its
+            // CTAs have their items from the start and those that come late end late
+            const uint32_t beside = (T + 31) / 32 * (H / 256), room = !shared && mode == 0 && overlap && beside <= 16 ? (uint32_t)ctas - beside : (uint32_t)ctas;
             return qw4sh_expert_tc(mode, prefill, w0, w1, shared ? work->shared_groups32 : work->groups32, work->n_groups32 + (shared ? 1 : 0), r2p, k_div,
-                                   mode ? act : &work->split_x, mode ? nullptr : act, mode ? out : nullptr, work->status, ctas, strm);
+                                   mode ? act : &work->split_x, mode ? nullptr : act, mode ? out : nullptr, work->status,
+                                   (int)(items < room ? items : room), strm);
         }
         const int8_t *q = mode == 0 ? work->xq : shared ? work->sq : work->aq, *neg = mode == 0 ? work->xneg : shared ? work->sneg : work->aneg;
         const int *sums = mode == 0 ? work->xsum : shared ? work->ssum : work->asum;
