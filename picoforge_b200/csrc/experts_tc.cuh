@@ -23,10 +23,15 @@
 // activation traffic from L2, and the two tiles take turns on the tensor pipe, so one is read back while the other is
 // multiplied.  CTAs are persistent and walk the item list with a stride.
 //
-// Warps (20):
-//   0-3, 4-7    dequantise tile 0 / 1 (TMEM lane = weight row), 64 columns at a time into a ring of three A slots per tile
-//   8-11, 12-15 read tile 0 / 1 back (tcgen05.ld), scale, accumulate; SwiGLU + split of the activation, or the store
-//   16          TMA of the packed rows; 17: tcgen05.mma issue; 18, 19: activation rows (cp.async gathers of hi and lo)
+// Measured, routed experts of 1024 tokens: Q4_K (Zipf) gate/up 484 -> 151 us, down 275 -> 97; Q2_K gate/up 579 -> 188 us.  A
+// step (128 columns of both tiles) takes about 1500 cycles where its MMAs take 528 and its dequantising 560: the rest is the
+// hand-over between the two (barrier answers behind the shared-memory and TMEM traffic, 100 to 200 cycles each way, and two A
+// slots per tile are all that TMEM holds beside the accumulators).
+//
+// Warps (21; 25 for IQ2_XXS, whose dequantiser takes three sets of four):
+//   0-7         dequantise: each set of four takes (step, tile) pairs in turn (TMEM lane = weight row), 128 columns at a time into two A slots per tile
+//   next 8      read tile 0 / 1 back (tcgen05.ld), scale, accumulate; SwiGLU + split of the activation, or the store
+//   next 1      TMA of the packed rows;  next 2: tcgen05.mma issue, one warp per tile;  last 2: activation rows (cp.async gathers of hi and lo)
 //
 // A unit is the span of columns between two read-backs: 256 (mode 0: a block, one row scale per token) or 128 (mode 1: the
 // activation of a token has one power of two per 128 columns, because those come out of different CTAs).  The minima of a
@@ -603,7 +608,7 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
         }
     } else if (warp < R::EPI) {
         // ---------------- dequantise: packed bytes -> exact halves in TMEM ----------------
-        // three sets of four warps take turns at the (step, tile) pairs: pair w goes to set w % 3 and to A slot w & 3
+        // the sets of four warps take turns at the (step, tile) pairs
         const uint32_t set = warp >> 2, row = (warp & 3u) * 32 + lane, quad = ((warp & 3u) * 32) << 16, nb = a.w0.k_storage >> 8;
         constexpr uint32_t STPS = STCH / CPS;                                 // steps per stage
         const uint32_t steps = a.units * SPU, stages = (steps + STPS - 1) / STPS, spare = stages * STPS - steps;
