@@ -28,7 +28,7 @@ _Static_assert(sizeof(Qwen4F32) == 88 && sizeof(QW4PackedLayout) == 64, "ABI lay
  * limit of STEP_TOKENS. */
 enum { CHUNK_TOKENS = 4096, STEP_TOKENS = 2048, PIN_BYTES = 256 * 1024 };
 /* host calls of more rows (forward_many): ring of pinned slices, helper threads and the bytes from which on they help */
-enum { STAGE_BYTES = 2 << 20, SLICE_BYTES = 32 << 10, STAGE_EVENTS = 8, HELPERS = 3, HELPER_MIN_BYTES = 1 << 20 };
+enum { STAGE_BYTES = 2 << 20, SLICE_BYTES = 32 << 10, STAGE_EVENTS = 8, HELPERS = 5, HELPER_MIN_BYTES = 1 << 20 };
 
 struct Qwen4Moe {
     Qwen4MoeConfig c;
@@ -633,10 +633,10 @@ Qwen4Status qw4cu_moe_work_sync_many(Qwen4MoeWork *const *works, size_t n, Qwen4
 /* ---- host rows ---------------------------------------------------------------------------
  * A call with host views of more than a few rows spends more time moving them than the GPU spends on the layer when it is left to
  * a scalar scan and pageable copies (333 rows of 2048: 280 us to scan, 300 us to copy in and out, 430 us on the GPU).  So
- * the rows go through a ring of pinned slices: the calling thread and up to three helpers copy (and scan) slices in any order, the
+ * the rows go through a ring of pinned slices: the calling thread and up to five helpers copy (and scan) slices in any order, the
  * calling thread sends finished slices on in order and, on the way back, releases slices as their copies land.  The
  * helpers live for one call (about 20 us to start, beside the calling thread's own first slice) and make no CUDA call; one that
- * cannot be started is simply not there. */
+ * cannot be started is simply not there.  333 rows: 1364 us before, 835 with three helpers, 785 with five, 805 with seven. */
 #define VECTORISED __attribute__((optimize("O3")))
 /* Nonzero when one of the n values is infinite or NaN: adding one to an exponent of all ones carries into the sign. */
 VECTORISED static uint32_t scan_floats(const uint32_t *restrict p, size_t n) {
