@@ -241,7 +241,8 @@ size_t qw4cu_moe_device_bytes(const Qwen4Moe *moe);
 size_t qw4cu_moe_work_device_bytes(const Qwen4MoeWork *work);
 
 /* Forward on device pointers: x_dev [tokens, hidden] and y_dev [tokens, hidden] are dense
- * FP32 in HBM; ids_dev [tokens, k] and weights_dev [tokens, k] may be NULL.  Enqueues on
+ * FP32 in HBM, aligned to a float (on a 16-byte boundary the kernels use wider loads, and the
+ * one-kernel decode path is open only there); ids_dev [tokens, k] and weights_dev [tokens, k] may be NULL.  Enqueues on
  * the library's stream (one per device, shared by all workspaces) and returns without waiting; errors found by the kernels are
  * reported by qw4cu_moe_work_sync. */
 Qwen4Status qw4cu_moe_forward_device(const Qwen4Moe *moe, const float *x_dev, float *y_dev,

@@ -440,6 +440,7 @@ __global__ void __launch_bounds__(NT, 1) grouped_mma_kernel(const GroupedArgs a)
 // row_list (optional): CTA b handles row row_list[*row_begin + b] (row_begin null: 0), and only while that index is
 // below *row_end (the rows an expert-parallel rank's experts actually received, out of a launch sized for the most
 // there can be).
+template <bool ALIGNED>
 __global__ void __launch_bounds__(128) quantize_rows_kernel(const float *__restrict__ x, uint32_t pitch, uint32_t k, int8_t *__restrict__ xq,
                                                             int8_t *__restrict__ xneg, int *__restrict__ xsum, float *__restrict__ xscale,
                                                             const uint32_t *__restrict__ row_list, const uint32_t *__restrict__ row_begin,
@@ -449,10 +450,10 @@ __global__ void __launch_bounds__(128) quantize_rows_kernel(const float *__restr
     if (row_list && listed >= *row_end) return;
     const uint32_t row = row_list ? row_list[listed] : blockIdx.x;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, items = k >> 2;
-    const float4 *src = reinterpret_cast<const float4 *>(x + (uint64_t)row * pitch);
+    const float *src = x + (uint64_t)row * pitch;
     float amax = 0.0f;
     for (uint32_t i = tid; i < items; i += 128) {
-        const float4 v = src[i];
+        const float4 v = load_quad<ALIGNED>(src + 4 * i);
         amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
     for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(128) quantize_rows_kernel(const float *__restr
     for (uint32_t i0 = 0; i0 < items; i0 += 128) {                      // items is a multiple of 8: whole groups of eight lanes
         const uint32_t i = i0 + tid;
         const bool live = i < items;
-        const float4 v4 = live ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 v4 = live ? load_quad<ALIGNED>(src + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float vv[4] = {v4.x, v4.y, v4.z, v4.w};
         uint32_t ra[4], rb[4];
 #pragma unroll
@@ -703,14 +704,14 @@ extern "C" const uint8_t *qw4sh_lut_image(void) { return lut_image(); }
 extern "C" int qw4sh_quantize_rows_pitched(const float *x, uint32_t pitch, uint32_t rows, uint32_t k, int8_t *xq, int8_t *xneg, int *xsum,
                                            float *xscale, void *stream) {
     if (!rows) return 0;
-    quantize_rows_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>(x, pitch, k, xq, xneg, xsum, xscale, nullptr, nullptr, nullptr);
+    (rows_aligned(x, pitch) ? quantize_rows_kernel<true> : quantize_rows_kernel<false>)<<<rows, 128, 0, (cudaStream_t)stream>>>(x, pitch, k, xq, xneg, xsum, xscale, nullptr, nullptr, nullptr);
     return qw4sh_note_launch("quantize_rows_kernel");
 }
 extern "C" int qw4sh_quantize_rows_listed(const float *x, uint32_t pitch, uint32_t max_rows, uint32_t k, const uint32_t *row_list,
                                           const uint32_t *row_begin, const uint32_t *row_end, int8_t *xq, int8_t *xneg, int *xsum, float *xscale,
                                           void *stream) {
     if (!max_rows) return 0;
-    quantize_rows_kernel<<<max_rows, 128, 0, (cudaStream_t)stream>>>(x, pitch, k, xq, xneg, xsum, xscale, row_list, row_begin, row_end);
+    (rows_aligned(x, pitch) ? quantize_rows_kernel<true> : quantize_rows_kernel<false>)<<<max_rows, 128, 0, (cudaStream_t)stream>>>(x, pitch, k, xq, xneg, xsum, xscale, row_list, row_begin, row_end);
     return qw4sh_note_launch("quantize_rows_kernel");
 }
 extern "C" int qw4sh_quantize_rows(const float *x, uint32_t rows, uint32_t k, int8_t *xq, int8_t *xneg, int *xsum, float *xscale, void *stream) {

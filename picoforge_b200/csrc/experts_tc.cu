@@ -25,13 +25,14 @@ __global__ void __launch_bounds__(XRole<T_Q4_K>::THREADS, 1) prefill_tc_kernel(c
 
 // x [rows][k], `pitch` floats apart -> fp16 hi / lo of x * 2^e (the kernel's column order), sums over 16 columns (hi / lo),
 // and 2^-e per row; e puts the row's largest value into [512, 1024).  One CTA of 128 threads per row, 16 columns a thread.
+template <bool ALIGNED>
 __global__ void __launch_bounds__(128) split_rows_kernel(const float *__restrict__ x, uint32_t pitch, uint32_t k, __half *__restrict__ hi, __half *__restrict__ lo,
                                                          __half *__restrict__ sum_hi, __half *__restrict__ sum_lo, float *__restrict__ scale) {
     __shared__ float red[4];
     const uint32_t r = blockIdx.x, segs = k >> 4, tid = threadIdx.x;
-    const float4 *src = reinterpret_cast<const float4 *>(x + (uint64_t)r * pitch);
+    const float *src = x + (uint64_t)r * pitch;
     float top = 0.0f;
-    for (uint32_t i = tid; i < segs * 4; i += 128) { const float4 v = src[i]; top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); }
+    for (uint32_t i = tid; i < segs * 4; i += 128) { const float4 v = load_quad<ALIGNED>(src + 4 * i); top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); }
     for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     if ((tid & 31u) == 0) red[tid >> 5] = top;
     __syncthreads();
@@ -43,7 +44,7 @@ __global__ void __launch_bounds__(128) split_rows_kernel(const float *__restrict
         float sum = 0.0f;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const float4 p = src[s * 4 + 2 * h], q = src[s * 4 + 2 * h + 1];
+            const float4 p = load_quad<ALIGNED>(src + s * 16 + 8 * h), q = load_quad<ALIGNED>(src + s * 16 + 8 * h + 4);
             const float v[8] = {p.x * up, p.y * up, p.z * up, p.w * up, q.x * up, q.y * up, q.z * up, q.w * up};
             uint32_t a[4], b[4];
 #pragma unroll
@@ -231,7 +232,7 @@ extern "C" int qw4sh_tile_supported(const QW4ShTensor *w) { return w->tc_format 
 // ---- launches -----------------------------------------------------------------------------------
 extern "C" int qw4sh_split_rows(const float *x, uint32_t pitch, uint32_t rows, uint32_t k, const QW4ShSplit *to, void *stream) {
     if (!rows) return 0;
-    split_rows_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>(x, pitch, k, (__half *)to->hi, (__half *)to->lo, (__half *)to->sum_hi, (__half *)to->sum_lo, to->scale);
+    (rows_aligned(x, pitch) ? split_rows_kernel<true> : split_rows_kernel<false>)<<<rows, 128, 0, (cudaStream_t)stream>>>(x, pitch, k, (__half *)to->hi, (__half *)to->lo, (__half *)to->sum_hi, (__half *)to->sum_lo, to->scale);
     return qw4sh_note_launch("split_rows_kernel");
 }
 // Groups of <= 32 rows (16-byte records {expert, first row, rows, 0}) for qw4sh_expert_tc: from the expert-sorted lists, or

@@ -119,6 +119,15 @@ __device__ inline float decode_value(const DevTensor &t, uint32_t expert, uint32
     }
 }
 
+// Four consecutive floats of a caller's row.  A caller's arrays are dense FP32 with the alignment of a float and no more, so a kernel
+// that reads them 128 bits at a time takes the 128-bit load only where the launch found the base and the pitch on the 16-byte grid
+// (rows_aligned); four scalar loads otherwise.
+template <bool ALIGNED> __device__ __forceinline__ float4 load_quad(const float *p) {
+    if (ALIGNED) return *reinterpret_cast<const float4 *>(p);
+    return make_float4(p[0], p[1], p[2], p[3]);
+}
+static inline bool rows_aligned(const float *base, uint64_t pitch) { return ((uintptr_t)base & 15u) == 0 && pitch % 4 == 0; }
+
 // The hyper-connection add that follows the layer (picoforge src/qwen4_base.c:160-176, fused into the down
 // epilogue by the reference's GPU path, src/qwen4_moe_internal.h:55-58): for each of the `streams` residual
 // streams, residual[t, h, c] += inject[t, h] * y[t, c], the product and the sum rounded separately.  Called by

@@ -355,6 +355,7 @@ __global__ void __launch_bounds__(ROWS * TOK) router_chain_kernel(DevTensor rout
 
 // Fast: one warp per router row, lanes stride K with 128-bit loads, tree sum.  Up to 8 tokens
 // per pass share the weight reads.
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256) router_fast_kernel(DevTensor router, DevTensor srouter, const float *__restrict__ x,
                                                           uint32_t tokens, float *__restrict__ logits,
                                                           float *__restrict__ shared_logit, uint32_t *status) {
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(256) router_fast_kernel(DevTensor router, DevT
                 const float4 wv = *reinterpret_cast<const float4 *>(w + k);
 #pragma unroll
                 for (int r = 0; r < 8; r++) if ((uint32_t)r < nt) {
-                    const float4 xv = *reinterpret_cast<const float4 *>(x + (uint64_t)(t0 + r) * k_total + k);
+                    const float4 xv = load_quad<ALIGNED>(x + (uint64_t)(t0 + r) * k_total + k);
                     acc[r] = fmaf(wv.x, xv.x, fmaf(wv.y, xv.y, fmaf(wv.z, xv.z, fmaf(wv.w, xv.w, acc[r]))));
                 }
             }
@@ -1066,7 +1067,7 @@ constexpr int GU_TILE = 16;           // output rows per CTA
 // act[pair, n] = silu(gate_e[n] . x) * (up_e[n] . x) for every pair routed to expert e.
 // grid = (ceil(inter / GU_TILE), groups); group g of the grid is expert active[1 + g].
 // row_to_pair == nullptr means one group holding rows 0..tokens-1 of x (the shared expert).
-template <uint32_t TYPE>
+template <uint32_t TYPE, bool ALIGNED>
 __global__ void __launch_bounds__(GU_WARPS * 32) gate_up_kernel(DevTensor gate, DevTensor up, const float *__restrict__ x,
                                                                 uint32_t hidden, const uint32_t *__restrict__ offsets,
                                                                 const uint32_t *__restrict__ row_to_pair,
@@ -1094,7 +1095,7 @@ __global__ void __launch_bounds__(GU_WARPS * 32) gate_up_kernel(DevTensor gate, 
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (r < nr) {
                 const uint32_t src_row = row_to_pair ? row_to_pair[first + r0 + r] / k_div : r0 + r;
-                v = *reinterpret_cast<const float4 *>(x + (uint64_t)src_row * hidden + c4 * 4);
+                v = load_quad<ALIGNED>(x + (uint64_t)src_row * hidden + c4 * 4);
             }
             *reinterpret_cast<float4 *>(gu_smem + r * x_pitch + xs_index(c4 * 4)) = v;
         }
@@ -1368,7 +1369,7 @@ static int launch_router(const QW4ShLayer *layer, const float *x, size_t tokens,
         LAUNCHED("router_exact_kernel");
     } else {
         const unsigned ty = (unsigned)((tokens + 7) / 8);
-        router_fast_kernel<<<dim3((rows + 7) / 8, ty > 64 ? 64 : ty), 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status);
+        (rows_aligned(x, router.k_logical) ? router_fast_kernel<true> : router_fast_kernel<false>)<<<dim3((rows + 7) / 8, ty > 64 ? 64 : ty), 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status);
         LAUNCHED("router_fast_kernel");
     }
     return 0;
@@ -1381,8 +1382,9 @@ static int launch_gate_up(const DevTensor &gate, const DevTensor &up, const floa
     if (up.type != gate.type || hidden % 4) type = GENERIC;
     const size_t smem = (size_t)GU_ROWS * xs_floats(hidden) * sizeof(float);
     const dim3 grid((gate.n_out + GU_TILE - 1) / GU_TILE, groups);
-#define GU_CASE(T) case T: if (allow_smem(gate_up_kernel<T>, smem)) return -1; \
-    gate_up_kernel<T><<<grid, GU_WARPS * 32, smem, stream>>>(gate, up, x, hidden, offsets, row_to_pair, active, k_div, tokens, act, status); break;
+#define GU_CASE(T) case T: { const auto kernel = rows_aligned(x, hidden) ? gate_up_kernel<T, true> : gate_up_kernel<T, false>; \
+    if (allow_smem(kernel, smem)) return -1; \
+    kernel<<<grid, GU_WARPS * 32, smem, stream>>>(gate, up, x, hidden, offsets, row_to_pair, active, k_div, tokens, act, status); break; }
     switch (type) {
         GU_CASE(T_Q4_K) GU_CASE(T_Q2_K) GU_CASE(T_IQ2_XXS)
     default: {
