@@ -307,7 +307,9 @@ Qwen4Status qw4cu_moe_work_sync_many(Qwen4MoeWork *const *works, size_t n, Qwen4
  *            the shared expert of these tokens on a second stream;
  *   experts  rows_all_dev: the rows of all ranks in rank order [tokens_total, row floats]; own_first:
  *            index of this rank's first token in it; partial_dev [tokens_total, hidden] receives the
- *            partial sums.  y of a token = sum over ranks of its partial rows. */
+ *            partial sums.  y of a token = sum over ranks of its partial rows.
+ * rows_local_dev, rows_all_dev and partial_dev start on 16-byte boundaries (QW4_STRIDE otherwise); x_dev and y_dev
+ * need only a float's alignment. */
 typedef struct QW4CuEp QW4CuEp;
 Qwen4Status qw4cu_moe_create_sharded(const Qwen4MoeConfig *config, const Qwen4MoeWeights *weights,
                                      uint32_t first_expert, uint32_t local_experts, Qwen4Moe **out,

@@ -40,6 +40,7 @@
 #include <string.h>
 
 #include "cuda_shim.h"
+#include "formats.cuh"
 
 extern "C" int qw4sh_note_launch(const char *name);
 extern "C" int qw4sh_fail_text(const char *text);
@@ -48,13 +49,14 @@ namespace qw4 {
 
 // ---- kernels ---------------------------------------------------------------------------------------------
 // Row t of the message: x[t, 0..hidden) | ids[t, 0..k) as words | weights[t, 0..k); k padded to a multiple of 4.
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256) ep_pack_kernel(const float *__restrict__ x, const uint32_t *__restrict__ ids,
                                                       const float *__restrict__ weights, uint32_t hidden, uint32_t k, uint32_t kp,
                                                       float *__restrict__ msg, uint32_t pitch) {
     const uint32_t t = blockIdx.x;
-    const float4 *src = reinterpret_cast<const float4 *>(x + (uint64_t)t * hidden);
+    const float *src = x + (uint64_t)t * hidden;
     float4 *dst = reinterpret_cast<float4 *>(msg + (uint64_t)t * pitch);
-    for (uint32_t i = threadIdx.x; i < hidden / 4; i += 256) dst[i] = src[i];
+    for (uint32_t i = threadIdx.x; i < hidden / 4; i += 256) dst[i] = load_quad<ALIGNED>(src + 4 * i);
     uint32_t *tail = reinterpret_cast<uint32_t *>(msg + (uint64_t)t * pitch + hidden);
     for (uint32_t s = threadIdx.x; s < 2 * kp; s += 256) {
         uint32_t word = 0xffffffffu;
@@ -203,7 +205,7 @@ extern "C" uint32_t qw4sh_ep_row_floats(uint32_t hidden, uint32_t k) { return hi
 extern "C" int qw4sh_ep_pack_rows(const float *x, const uint32_t *ids, const float *weights, uint32_t tokens, uint32_t hidden, uint32_t k,
                                   float *msg, void *stream) {
     if (!tokens) return 0;
-    ep_pack_kernel<<<tokens, 256, 0, (cudaStream_t)stream>>>(x, ids, weights, hidden, k, (k + 3) & ~3u, msg, qw4sh_ep_row_floats(hidden, k));
+    (rows_aligned(x, hidden) ? ep_pack_kernel<true> : ep_pack_kernel<false>)<<<tokens, 256, 0, (cudaStream_t)stream>>>(x, ids, weights, hidden, k, (k + 3) & ~3u, msg, qw4sh_ep_row_floats(hidden, k));
     return qw4sh_note_launch("ep_pack_kernel");
 }
 extern "C" int qw4sh_ep_local_ids(const float *msg, uint32_t hidden, uint32_t k, uint32_t tokens, uint32_t experts, uint32_t first,

@@ -1839,7 +1839,6 @@ static bool shared_on_mma(const QW4ShLayer *layer) {
 static int ep_shared_begin(const QW4ShLayer *layer, const QW4ShWork *work, const float *x, size_t tokens) {
     if (!tokens) return 0;
     const bool tiles = g_tile_path != 0 && tc_shared(layer);
-    if (!tiles && !shared_on_mma(layer)) return fail(cudaErrorNotSupported, "expert-parallel step: no tensor-core kernel takes the shared expert");
     cudaStream_t stream = (cudaStream_t)work->stream, side;
     cudaEvent_t *ev;
     int rc;
@@ -1878,6 +1877,9 @@ static int ep_shared_begin(const QW4ShLayer *layer, const QW4ShWork *work, const
 // packed into msg_local, the shared expert started beside.
 extern "C" int qw4sh_ep_begin(const QW4ShLayer *layer, const QW4ShWork *work, const float *x, size_t tokens, float *msg_local, int router_mode) {
     if (!tokens) return 0;
+    // asked before the first launch: the packing of rows, too, counts on the shapes that these kernels take (hidden % 256 == 0)
+    if (!(g_tile_path != 0 && tc_shared(layer)) && !shared_on_mma(layer))
+        return fail(cudaErrorNotSupported, "expert-parallel step: no tensor-core kernel takes the shared expert");
     int rc;
     if ((rc = qw4sh_ep_trace_mark(0, work->stream))) return rc;
     if ((rc = launch_router(layer, x, tokens, work->logits, work->shared_logit, work->status, router_mode, (cudaStream_t)work->stream))) return rc;

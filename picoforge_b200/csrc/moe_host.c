@@ -536,6 +536,7 @@ Qwen4Status qw4cu_moe_ep_begin_device(const Qwen4Moe *m, const float *x_dev, siz
                                       float *weights_dev, Qwen4MoeWork *w, Qwen4Error *err) {
     TRY(piece_checks(m, w, tokens_local, err));
     if (tokens_local && (!x_dev || !rows_local_dev)) return report(err, QW4_INVALID_ARGUMENT, "null device view");
+    if (tokens_local && (uintptr_t)rows_local_dev % 16) return report(err, QW4_STRIDE, "exchange rows: not aligned to 16 bytes");
     if (qw4sh_ep_begin(&m->layer, &w->d, x_dev, tokens_local, rows_local_dev, current_router_mode())) return cuda_failure(err, "route and pack");
     const size_t bytes = tokens_local * m->c.top_k * 4;
     if (tokens_local && ids_dev && qw4sh_memcpy2d_async(ids_dev, bytes, w->d.ids, bytes, bytes, 1, 2, w->d.stream)) return cuda_failure(err, "ids copy");
@@ -547,6 +548,7 @@ Qwen4Status qw4cu_moe_ep_experts_device(const Qwen4Moe *m, const float *rows_all
                                         Qwen4MoeWork *w, Qwen4Error *err) {
     TRY(piece_checks(m, w, tokens_total, err));
     if (tokens_total && (!rows_all_dev || !partial_dev)) return report(err, QW4_INVALID_ARGUMENT, "null device view");
+    if (tokens_total && ((uintptr_t)rows_all_dev % 16 || (uintptr_t)partial_dev % 16)) return report(err, QW4_STRIDE, "exchange rows or partial sums: not aligned to 16 bytes");
     const size_t own = w->shared_tokens;
     w->shared_tokens = 0;
     if (own_first > tokens_total || own > tokens_total - own_first) return report(err, QW4_RANGE, "own tokens outside the gathered batch");

@@ -83,3 +83,46 @@ def test_fast_router_off_the_16_byte_grid(gpu):
                     np.testing.assert_array_equal(a, b)
     finally:
         gpu.lib.qw4cu_set_router_mode(0)
+
+
+def test_expert_parallel_rows_off_the_16_byte_grid(gpu):
+    """x and y of the expert-parallel step may start anywhere a float may; the exchange rows and partial sums, which kernels of this
+    library write for kernels of this library, are refused off a 16-byte boundary, and a layer that the step has no kernel for
+    before anything is launched."""
+    import sys
+    from pathlib import Path
+    sys.path.insert(0, str(Path(__file__).resolve().parent))
+    import cases
+    from picoforge_b200.expert_parallel import Communicator, EpLayer
+    lib, err = gpu.lib, abi.Qwen4Error()
+    spec = synth.make_layer(8300, routed_type=Q2, shared_type=Q4, hidden=512, inter=256, shared_inter=256, experts=16, top_k=4)
+    x = synth.activations(8300, 9, 512)
+    layer, comm = EpLayer(gpu, spec, 9, 1, 0), Communicator(gpu, 0, 1)
+    pitch = lib.qw4cu_ep_row_floats(layer.layer.moe)
+    d_x, d_y, d_rows = lib.qw4cu_malloc(x.nbytes + 16), lib.qw4cu_malloc(x.nbytes + 16), lib.qw4cu_malloc(9 * pitch * 4 + 16)
+    try:
+        got = []
+        for shift in (0, 4, 12):
+            assert lib.qw4cu_upload(d_x + shift, x.ctypes.data, x.nbytes) == 0
+            layer.forward(comm, d_x + shift, d_y + shift)
+            layer.sync()
+            y = np.empty_like(x)
+            assert lib.qw4cu_download(y.ctypes.data, d_y + shift, y.nbytes) == 0
+            got.append((y, *layer.routes()))
+        for moved in got[1:]:
+            for a, b in zip(moved, got[0]):
+                np.testing.assert_array_equal(a, b)
+        moe, work = layer.layer.moe, layer.layer.work
+        assert lib.qw4cu_moe_ep_begin_device(moe, d_x, 9, d_rows + 4, None, None, work, C.byref(err)) == abi.STRIDE
+        assert lib.qw4cu_moe_ep_experts_device(moe, d_rows + 8, 9, 0, d_y, work, C.byref(err)) == abi.STRIDE
+        assert lib.qw4cu_moe_ep_experts_device(moe, d_rows, 9, 0, d_y + 4, work, C.byref(err)) == abi.STRIDE
+        odd = cases.float_layer(8301, hidden=10)              # rows of 40 bytes: every other one lies off the grid
+        with MoeLayer(gpu, odd, 6) as generic:
+            launches = lib.qw4cu_launch_count()
+            assert lib.qw4cu_moe_ep_begin_device(generic.moe, d_x, 3, d_rows, None, None, generic.work, C.byref(err)) == abi.GPU_ERROR
+        assert lib.qw4cu_launch_count() == launches
+    finally:
+        layer.close()
+        comm.close()
+        for p in (d_x, d_y, d_rows):
+            lib.qw4cu_free(p)
