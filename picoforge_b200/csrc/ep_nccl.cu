@@ -182,7 +182,10 @@ __global__ void __launch_bounds__(32) ep_wait_kernel(const uint32_t *flags_local
     }
     atomicOr(status, QW4SH_ERR_STATE);
 }
-// y[i] = sum over ranks, in rank order, of that rank's partial row of this rank's token.
+// y[i] = sum over ranks, in rank order, of that rank's partial row of this rank's token.  y is the caller's: off the 16-byte grid it
+// is stored float by float.  (The transport must not hang on y: a rank that left for the library's collective while its
+// peers meet at their epochs would leave both sides waiting.)
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256) ep_pull_sum_kernel(PeerTable pt, float *__restrict__ y, uint32_t quads, uint32_t rank, uint32_t world) {
     for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < quads; i += gridDim.x * 256) {
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -190,7 +193,8 @@ __global__ void __launch_bounds__(256) ep_pull_sum_kernel(PeerTable pt, float *_
             const float4 v = __ldcv(reinterpret_cast<const float4 *>(pt.partial[r]) + (uint64_t)rank * quads + i);
             sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
         }
-        reinterpret_cast<float4 *>(y)[i] = sum;
+        if (ALIGNED) reinterpret_cast<float4 *>(y)[i] = sum;
+        else { float *at = y + (uint64_t)i * 4; at[0] = sum.x; at[1] = sum.y; at[2] = sum.z; at[3] = sum.w; }
     }
 }
 
@@ -448,17 +452,24 @@ extern "C" int qw4sh_ep_all_gather(QW4ShEp *ep, size_t floats_per_rank, uint32_t
     }
     return nccl_check(g_nccl.all_gather(ep->msg_local, ep->msg_all, floats_per_rank, NCCL_FLOAT, ep->comm, (cudaStream_t)stream), "ncclAllGather");
 }
+// y [floats] = sum over `world` ranks, in rank order, of partial[r][rank * floats ..]; floats % 4 == 0, world <= EP_MAX_WORLD.
+extern "C" int qw4sh_ep_pull_sum(const float *const *partial, float *y, size_t floats, int rank, int world, void *stream) {
+    PeerTable table = {};
+    for (int r = 0; r < world && r < EP_MAX_WORLD; r++) table.partial[r] = partial[r];
+    const uint32_t quads = (uint32_t)(floats / 4), blocks = (quads + 255) / 256;
+    (rows_aligned(y, 4) ? ep_pull_sum_kernel<true> : ep_pull_sum_kernel<false>)<<<blocks < 592 ? blocks : 592, 256, 0, (cudaStream_t)stream>>>(
+        table, y, quads, (uint32_t)rank, (uint32_t)world);
+    return qw4sh_note_launch("ep_pull_sum_kernel");
+}
 // reduce-scatter (sum) of the partial rows: partial [world * tokens_local, hidden] -> y [tokens_local, hidden]
 extern "C" int qw4sh_ep_reduce_scatter(QW4ShEp *ep, float *y, size_t floats_per_rank, uint32_t *status, void *stream) {
     if (ep->world == 1) { CU(cudaMemcpyAsync(y, ep->partial, floats_per_rank * 4, cudaMemcpyDeviceToDevice, (cudaStream_t)stream)); return 0; }
-    if (ep->peer && floats_per_rank % 4 == 0 && floats_per_rank / 4 < (1u << 31) && ((uintptr_t)y & 15u) == 0) {
-        const uint32_t quads = (uint32_t)(floats_per_rank / 4), blocks = (quads + 255) / 256;
+    if (ep->peer && floats_per_rank % 4 == 0 && floats_per_rank / 4 < (1u << 31)) {
         ep_signal_partial_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(ep->table, (uint32_t)ep->rank, (uint32_t)ep->world, ep->state);
         qw4sh_note_launch("ep_signal_partial_kernel");
         ep_wait_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(ep->flags, EP_FLAG_PARTIAL, &ep->state->epoch_partial, (uint32_t)ep->rank, (uint32_t)ep->world, EP_WAIT_POLLS, status);
         qw4sh_note_launch("ep_wait_kernel");
-        ep_pull_sum_kernel<<<blocks < 592 ? blocks : 592, 256, 0, (cudaStream_t)stream>>>(ep->table, y, quads, (uint32_t)ep->rank, (uint32_t)ep->world);
-        return qw4sh_note_launch("ep_pull_sum_kernel");
+        return qw4sh_ep_pull_sum(ep->table.partial, y, floats_per_rank, ep->rank, ep->world, stream);
     }
     return nccl_check(g_nccl.reduce_scatter(ep->partial, y, floats_per_rank, NCCL_FLOAT, NCCL_SUM, ep->comm, (cudaStream_t)stream), "ncclReduceScatter");
 }

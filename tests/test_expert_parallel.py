@@ -205,3 +205,36 @@ def test_sharded_layer_over_nccl_on_two_gpus(gpu, routed):
     ids = np.concatenate([results[r][1] for r in range(world)])
     np.testing.assert_array_equal(ids, want["ids"])
     assert np.abs(y - want["y"]).max() <= 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("world,quads", [(2, 1), (3, 257), (8, 700)])
+def test_pulled_partial_sums_wherever_y_starts(gpu, world, quads):
+    """The peer transport's reduce-scatter is the same kernel for every y (a rank's y must not decide which transport it takes: its
+    peers would wait for it in the other one): sums in rank order, on and off the 16-byte grid.  The ranks' buffers are local here."""
+    import ctypes as C
+    lib = gpu.lib
+    lib.qw4sh_ep_pull_sum.argtypes = [C.POINTER(C.c_void_p), C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_void_p]
+    floats, rank = 4 * quads, world - 1
+    partial = np.random.default_rng(world).standard_normal((world, world * floats)).astype(np.float32)
+    want = np.zeros(floats, np.float32)
+    for r in range(world):
+        want += partial[r, rank * floats:(rank + 1) * floats]
+    d_partial = [lib.qw4cu_malloc(partial[0].nbytes) for _ in range(world)]
+    d_y = lib.qw4cu_malloc(floats * 4 + 32)
+    try:
+        for r in range(world):
+            assert lib.qw4cu_upload(d_partial[r], partial[r].ctypes.data, partial[r].nbytes) == 0
+        for shift in (0, 4, 8, 12):
+            guard = np.full(floats + 8, 7.0, np.float32)
+            assert lib.qw4cu_upload(d_y, guard.ctypes.data, guard.nbytes) == 0
+            assert lib.qw4sh_ep_pull_sum((C.c_void_p * world)(*d_partial), d_y + shift, floats, rank, world, None) == 0
+            assert lib.qw4cu_device_synchronize() == 0
+            got = np.empty_like(guard)
+            assert lib.qw4cu_download(got.ctypes.data, d_y, got.nbytes) == 0
+            at = shift // 4
+            np.testing.assert_array_equal(got[at:at + floats], want)
+            assert (got[:at] == 7.0).all() and (got[at + floats:] == 7.0).all()
+    finally:
+        for p in d_partial + [d_y]:
+            lib.qw4cu_free(p)
