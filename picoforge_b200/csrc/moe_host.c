@@ -4,6 +4,7 @@
  *
  * The entry points mirror picoforge src/qwen4_moe.h:13-27 (see include/qwen4_moe_b200.h).
  */
+#define _GNU_SOURCE                                   /* CPU_COUNT */
 #include "../../include/qwen4_moe_b200.h"
 #include "cuda_shim.h"
 
@@ -12,6 +13,7 @@
 #include <stdio.h>
 #include <pthread.h>
 #include <sched.h>
+#include <signal.h>
 #include <stdatomic.h>
 #include <sys/prctl.h>
 #include <time.h>
@@ -61,8 +63,8 @@ struct Qwen4MoeWork {
 typedef struct { uintptr_t first, end; } Span;
 
 /* ---- errors --------------------------------------------------------------------------- */
-/* Fills *err (when given) and hands the code back, so that `return raise(...)` reads as one step. */
-static Qwen4Status raise(Qwen4Error *err, Qwen4Status code, const char *format, ...) {
+/* Fills *err (when given) and hands the code back, so that `return fail_with(...)` reads as one step. */
+static Qwen4Status fail_with(Qwen4Error *err, Qwen4Status code, const char *format, ...) {
     if (!err) return code;
     memset(err, 0, sizeof *err);
     err->code = code;
@@ -74,9 +76,9 @@ static Qwen4Status raise(Qwen4Error *err, Qwen4Status code, const char *format, 
     va_end(args);
     return code;
 }
-#define report(err, code, text) raise((err), (code), "%s", (text))
+#define report(err, code, text) fail_with((err), (code), "%s", (text))
 static Qwen4Status cuda_failure(Qwen4Error *err, const char *what) {
-    return raise(err, QW4_GPU_ERROR, "%s: %s", what, qw4sh_last_error());
+    return fail_with(err, QW4_GPU_ERROR, "%s: %s", what, qw4sh_last_error());
 }
 #define TRY(call) do { Qwen4Status st_ = (call); if (st_ != QW4_OK) return st_; } while (0)
 
@@ -108,26 +110,26 @@ typedef struct {
 
 static Qwen4Status region_span(const Region *r, Span *span, Qwen4Error *err) {
     *span = (Span){0, 0};
-    if (r->cols > SIZE_MAX / r->elem) return raise(err, QW4_OVERFLOW, "%s: a row does not fit size_t", r->name);
+    if (r->cols > SIZE_MAX / r->elem) return fail_with(err, QW4_OVERFLOW, "%s: a row does not fit size_t", r->name);
     const size_t row = r->cols * r->elem;
-    if (r->pitch < row || r->pitch % r->elem) return raise(err, QW4_STRIDE, "%s: row pitch %zu cannot hold %zu-byte rows", r->name, r->pitch, row);
+    if (r->pitch < row || r->pitch % r->elem) return fail_with(err, QW4_STRIDE, "%s: row pitch %zu cannot hold %zu-byte rows", r->name, r->pitch, row);
     if (r->rows == 0 || row == 0) return QW4_OK;              /* nothing to address */
-    if (r->rows - 1 > (SIZE_MAX - row) / r->pitch) return raise(err, QW4_OVERFLOW, "%s: extent does not fit size_t", r->name);
+    if (r->rows - 1 > (SIZE_MAX - row) / r->pitch) return fail_with(err, QW4_OVERFLOW, "%s: extent does not fit size_t", r->name);
     const size_t extent = (r->rows - 1) * r->pitch + row;
     if (extent == 0) return QW4_OK;
-    if (r->capacity < extent) return raise(err, QW4_CAPACITY, "%s: %zu bytes declared, %zu needed", r->name, r->capacity, extent);
-    if (r->base == NULL) return raise(err, QW4_INVALID_ARGUMENT, "%s: null data for a nonempty view", r->name);
+    if (r->capacity < extent) return fail_with(err, QW4_CAPACITY, "%s: %zu bytes declared, %zu needed", r->name, r->capacity, extent);
+    if (r->base == NULL) return fail_with(err, QW4_INVALID_ARGUMENT, "%s: null data for a nonempty view", r->name);
     const uintptr_t at = (uintptr_t)r->base;
-    if (at % r->elem) return raise(err, QW4_STRIDE, "%s: data not aligned to %zu bytes", r->name, r->elem);
-    if (extent > UINTPTR_MAX - at) return raise(err, QW4_OVERFLOW, "%s: address range wraps", r->name);
+    if (at % r->elem) return fail_with(err, QW4_STRIDE, "%s: data not aligned to %zu bytes", r->name, r->elem);
+    if (extent > UINTPTR_MAX - at) return fail_with(err, QW4_OVERFLOW, "%s: address range wraps", r->name);
     *span = (Span){at, at + extent};
     return QW4_OK;
 }
 /* A rank-2 token-major FP32 view [rows, cols] (Qwen4F32 and Qwen4F32Mut share the layout). */
 static Qwen4Status f32_span(const char *name, const float *data, size_t capacity, size_t rank, const size_t *dim, const size_t *stride,
                             size_t rows, size_t cols, Span *span, Qwen4Error *err) {
-    if (rank != 2 || dim[0] != rows || dim[1] != cols) return raise(err, QW4_SHAPE, "%s: want a [%zu, %zu] matrix", name, rows, cols);
-    if (stride[1] != sizeof(float)) return raise(err, QW4_STRIDE, "%s: last axis must be dense", name);
+    if (rank != 2 || dim[0] != rows || dim[1] != cols) return fail_with(err, QW4_SHAPE, "%s: want a [%zu, %zu] matrix", name, rows, cols);
+    if (stride[1] != sizeof(float)) return fail_with(err, QW4_STRIDE, "%s: last axis must be dense", name);
     const Region r = {name, data, capacity, rows, cols, stride[0], sizeof(float)};
     return region_span(&r, span, err);
 }
@@ -141,14 +143,14 @@ static bool spans_meet(Span a, Span b) { return a.first < b.end && b.first < a.e
 static Qwen4Status all_apart(const Span *spans, size_t n, Qwen4Error *err) {
     for (size_t i = 1; i < n; i++)
         for (size_t j = 0; j < i; j++)
-            if (spans_meet(spans[i], spans[j])) return raise(err, QW4_INVALID_ARGUMENT, "arguments %zu and %zu share memory", j, i);
+            if (spans_meet(spans[i], spans[j])) return fail_with(err, QW4_INVALID_ARGUMENT, "arguments %zu and %zu share memory", j, i);
     return QW4_OK;
 }
 static Qwen4Status check_config(const Qwen4MoeConfig *c, Qwen4Error *err) {
-    if (!c) return raise(err, QW4_INVALID_ARGUMENT, "config pointer is null");
+    if (!c) return fail_with(err, QW4_INVALID_ARGUMENT, "config pointer is null");
     const bool sized = c->hidden_size && c->experts && c->intermediate && c->shared_intermediate;
     const bool routable = c->top_k >= 1 && c->top_k <= c->experts;
-    if (!sized || !routable || c->down_physical < c->intermediate) return raise(err, QW4_RANGE, "MoE dimensions out of range");
+    if (!sized || !routable || c->down_physical < c->intermediate) return fail_with(err, QW4_RANGE, "MoE dimensions out of range");
     return QW4_OK;
 }
 
@@ -638,7 +640,8 @@ Qwen4Status qw4cu_moe_work_sync_many(Qwen4MoeWork *const *works, size_t n, Qwen4
  * the rows go through a ring of pinned slices: the calling thread and up to five helpers copy (and scan) slices in any order, the
  * calling thread sends finished slices on in order and, on the way back, releases slices as their copies land.  The
  * helpers live for one call (about 20 us to start, beside the calling thread's own first slice) and make no CUDA call; one that
- * cannot be started is simply not there.  333 rows: 1364 us before, 835 with three helpers, 785 with five, 805 with seven. */
+ * cannot be started is simply not there.  No signal of the process is handled on them, and there are no more of them than the
+ * calling thread has cores beside its own.  333 rows: 1364 us before, 835 with three helpers, 785 with five, 805 with seven. */
 #define VECTORISED __attribute__((optimize("O3")))
 /* Nonzero when one of the n values is infinite or NaN: adding one to an exponent of all ones carries into the sign. */
 VECTORISED static uint32_t scan_floats(const uint32_t *restrict p, size_t n) {
@@ -699,6 +702,26 @@ static void *move_helper(void *arg) {
         else { const struct timespec nap = {0, 20000}; nanosleep(&nap, NULL); }
     }
     return NULL;
+}
+/* Cores that the calling thread, and with it its helpers, may run on: a process pinned to one of a hundred has one. */
+static int usable_cores(void) {
+    cpu_set_t set;
+    if (!sched_getaffinity(0, sizeof set, &set)) return CPU_COUNT(&set);
+    return (int)sysconf(_SC_NPROCESSORS_ONLN);         /* more processors than the set holds */
+}
+/* Starts up to `most` helpers; how many there are.  They inherit a mask that blocks every signal sent to the process, so that a handler
+ * (of a timer, of SIGINT) runs where the host program expects it, never on a thread it has not made; faults of a helper's own copies
+ * stay open. */
+static int start_helpers(pthread_t *helper, int most, RowMoves *moves) {
+    static const int own_faults[] = {SIGSEGV, SIGBUS, SIGFPE, SIGILL, SIGTRAP, SIGABRT};
+    sigset_t blocked, before;
+    sigfillset(&blocked);
+    for (size_t i = 0; i < sizeof own_faults / sizeof *own_faults; i++) sigdelset(&blocked, own_faults[i]);
+    if (pthread_sigmask(SIG_SETMASK, &blocked, &before)) return 0;
+    int n = 0;
+    while (n < most && !pthread_create(&helper[n], NULL, move_helper, moves)) n++;
+    pthread_sigmask(SIG_SETMASK, &before, NULL);
+    return n;
 }
 /* All rows of `m` through the ring to or from dev, a group of slices per copy (a copy costs the calling thread 3.6 us whatever its size).
  * 0, or nonzero when a CUDA call failed. */
@@ -804,13 +827,14 @@ static Qwen4Status forward_many(const Qwen4Moe *m, Qwen4MoeWork *w, const float 
     plan_move(&moves.in, w, (float *)xs, x_pitch, n, h, true, scan);
     plan_move(&moves.out, w, ys, y_pitch, n, h, false, false);
     atomic_init(&moves.stage, 0);
-    const long cpus = sysconf(_SC_NPROCESSORS_ONLN);
     pthread_t helper[HELPERS];
     int helpers = 0;
     /* the first slices are released before the helpers start, so that they find work */
     atomic_store(&moves.in.limit, moves.in.slices < moves.in.ring ? moves.in.slices : moves.in.ring);
-    for (; n * h * 4 >= HELPER_MIN_BYTES && helpers < HELPERS && helpers + 1 < cpus; helpers++)
-        if (pthread_create(&helper[helpers], NULL, move_helper, &moves)) break;
+    if (n * h * 4 >= HELPER_MIN_BYTES) {
+        const int cores = usable_cores();
+        helpers = start_helpers(helper, cores - 1 < HELPERS ? cores - 1 : HELPERS, &moves);
+    }
     int rc = w->status_clean ? 0 : status_clear(w);
     w->status_clean = false;
     if (!rc) rc = run_move(&moves.in, w, w->d.x);
@@ -860,7 +884,7 @@ Qwen4Status qwen4_moe_forward(const Qwen4Moe *m, Qwen4F32 x, Qwen4F32Mut y, Qwen
     TRY(F32_SPAN("y", y, t, h, &spans[1], err));
     if (routes) {
         TRY(F32_SPAN("route weights", routes->weights, t, k, &spans[2], err));
-        if (routes->ids.rows != t || routes->ids.cols != k) return raise(err, QW4_SHAPE, "route ids: want a [%zu, %zu] matrix", t, k);
+        if (routes->ids.rows != t || routes->ids.cols != k) return fail_with(err, QW4_SHAPE, "route ids: want a [%zu, %zu] matrix", t, k);
         TRY(u32_span("route ids", routes->ids, &spans[3], err));
         ns = 4;
     }
@@ -869,7 +893,7 @@ Qwen4Status qwen4_moe_forward(const Qwen4Moe *m, Qwen4F32 x, Qwen4F32Mut y, Qwen
         if (!m->host[a].span.data) continue;                        /* created from a file: no host bytes are borrowed */
         const Span weights = {(uintptr_t)m->host[a].span.data, (uintptr_t)m->host[a].span.data + m->host[a].layout.tensor_bytes};
         for (size_t b = 0; b < ns; b++)
-            if (spans_meet(spans[b], weights)) return raise(err, QW4_INVALID_ARGUMENT, "argument %zu overlaps weight tensor %zu", b, a);
+            if (spans_meet(spans[b], weights)) return fail_with(err, QW4_INVALID_ARGUMENT, "argument %zu overlaps weight tensor %zu", b, a);
     }
     /* Nonfinite input is rejected before any state is touched (src/qwen4_moe.c:411-413). */
     const size_t x_pitch = x.stride_bytes[0] / 4, y_pitch = y.stride_bytes[0] / 4;
@@ -937,7 +961,7 @@ Qwen4Status qwen4_moe_route(const Qwen4MoeConfig *c, Qwen4F32 logits, Qwen4MoeRo
     TRY(F32_SPAN("logits", logits, t, e, &spans[0], err));
     TRY(F32_SPAN("probabilities", probabilities, t, e, &spans[1], err));
     TRY(F32_SPAN("route weights", routes.weights, t, k, &spans[2], err));
-    if (routes.ids.rows != t || routes.ids.cols != k) return raise(err, QW4_SHAPE, "route ids: want a [%zu, %zu] matrix", t, k);
+    if (routes.ids.rows != t || routes.ids.cols != k) return fail_with(err, QW4_SHAPE, "route ids: want a [%zu, %zu] matrix", t, k);
     TRY(u32_span("route ids", routes.ids, &spans[3], err));
     TRY(all_apart(spans, 4, err));
     if (!t) return report(err, QW4_OK, "");
@@ -993,7 +1017,7 @@ Qwen4Status qw4_moe_group_pairs(const Qwen4MoeConfig *c, Qwen4U32Mut ids, QW4Moe
         {"row_to_pair", g.row_to_pair, g.row_to_pair_capacity_bytes, 1, pairs, 0, sizeof(size_t)}};
     for (size_t a = 0; a < 4; a++) {
         Region r = lists[a];
-        if (r.cols > SIZE_MAX / r.elem) return raise(err, QW4_OVERFLOW, "%s: byte count does not fit size_t", r.name);
+        if (r.cols > SIZE_MAX / r.elem) return fail_with(err, QW4_OVERFLOW, "%s: byte count does not fit size_t", r.name);
         r.pitch = r.cols * r.elem;                          /* one dense row */
         TRY(region_span(&r, &spans[a + 1], err));
     }
