@@ -177,8 +177,9 @@ Qwen4Status qwen4_moe_create(const Qwen4MoeConfig *config, const Qwen4MoeWeights
 void qwen4_moe_destroy(Qwen4Moe *moe);
 
 /* Replaces qwen4_moe_work_size (src/qwen4_moe.h:16-17, src/qwen4_moe.c:106-111).
- * Reports the HOST bytes of a workspace (metadata plus pinned staging for routes); the
- * device scratch it also owns is reported by qw4cu_moe_work_device_bytes. */
+ * Reports the HOST bytes of a workspace: metadata, a pinned block of 256 KB for small host calls
+ * and, where token_cap rows do not fit it, a pinned ring of 2 MB (eight rows, if those are more)
+ * for larger ones.  The device scratch it also owns is reported by qw4cu_moe_work_device_bytes. */
 Qwen4Status qwen4_moe_work_size(const Qwen4Moe *moe, size_t token_cap, size_t *bytes,
                                 Qwen4Error *err);
 

@@ -314,12 +314,21 @@ static Qwen4Status plan_work(const Qwen4Moe *m, size_t cap, size_t *chunk, Plan 
     return QW4_OK;
 }
 
+/* Bytes of the pinned ring: none where every host call of the workspace goes through the pinned block (forward_few). */
+static size_t stage_bytes_of(const Qwen4Moe *m, size_t chunk) {
+    const size_t h = m->c.hidden_size, eight_rows = 8 * h * 4;
+    if (2 * chunk * (h + m->c.top_k) * 4 <= PIN_BYTES) return 0;
+    return eight_rows > STAGE_BYTES ? eight_rows : STAGE_BYTES;
+}
+/* Everything a workspace holds in host memory: metadata, pinned block, status words, ring. */
+static size_t host_bytes_of(const Qwen4Moe *m, size_t chunk) { return sizeof(Qwen4MoeWork) + PIN_BYTES + 64 + stage_bytes_of(m, chunk); }
+
 Qwen4Status qwen4_moe_work_size(const Qwen4Moe *m, size_t cap, size_t *bytes, Qwen4Error *err) {
     if (!bytes) return report(err, QW4_INVALID_ARGUMENT, "null size output");
     *bytes = 0;
     Plan plan; size_t chunk;
     TRY(plan_work(m, cap, &chunk, &plan, err));
-    *bytes = sizeof(Qwen4MoeWork) + PIN_BYTES + 64;
+    *bytes = host_bytes_of(m, chunk);
     return report(err, QW4_OK, "");
 }
 
@@ -337,9 +346,9 @@ void qwen4_moe_work_destroy(Qwen4MoeWork *w) {
     free(w);
 }
 
-/* The pinned ring and its events. */
-static int make_stage(Qwen4MoeWork *w, size_t cols) {
-    w->stage_bytes = cols * 4 * 8 > STAGE_BYTES ? cols * 4 * 8 : STAGE_BYTES;
+/* The pinned ring and its events, made with the workspace: a forward allocates nothing. */
+static int make_stage(Qwen4MoeWork *w, size_t bytes) {
+    w->stage_bytes = bytes;
     w->stage = qw4sh_host_alloc(w->stage_bytes);
     for (int i = 0; w->stage && i < STAGE_EVENTS; i++)
         if (qw4sh_event_create(&w->stage_event[i])) return -1;
@@ -350,7 +359,7 @@ Qwen4Status qwen4_moe_work_create(const Qwen4Moe *m, size_t cap, size_t budget, 
     if (!out) return report(err, QW4_INVALID_ARGUMENT, "null workspace output");
     Plan plan; size_t chunk;
     TRY(plan_work(m, cap, &chunk, &plan, err));
-    const size_t host_bytes = sizeof(Qwen4MoeWork) + PIN_BYTES + 64;
+    const size_t host_bytes = host_bytes_of(m, chunk), ring = stage_bytes_of(m, chunk);
     if (budget < host_bytes) return report(err, QW4_CAPACITY, "workspace budget too small");
     Qwen4MoeWork *w = calloc(1, sizeof *w);
     if (!w) return report(err, QW4_OOM, "workspace metadata");
@@ -362,7 +371,7 @@ Qwen4Status qwen4_moe_work_create(const Qwen4Moe *m, size_t cap, size_t budget, 
     w->d.graph_cache = qw4sh_graph_cache_create();
     if (!w->device_block || !w->status_host || !w->pin || !w->d.graph_cache || qw4sh_shared_stream(&w->d.stream) ||
         qw4sh_event_create(&w->d.timer[0]) || qw4sh_event_create(&w->d.timer[1]) ||
-        (2 * cap * (m->c.hidden_size + m->c.top_k) * 4 > PIN_BYTES && make_stage(w, m->c.hidden_size))) {
+        (ring && make_stage(w, ring))) {
         Qwen4Status st = cuda_failure(err, "workspace allocation");
         qwen4_moe_work_destroy(w);
         return st;

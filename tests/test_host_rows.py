@@ -56,3 +56,11 @@ def test_no_more_threads_than_the_caller_has_cores(harness, cores):
         pytest.skip("fewer cores here")
     wrong, threads, _, _ = run(harness, "rows", 333, 2048, 0, 0, 10, cores=mine[:cores])
     assert wrong == 0 and threads == cores
+
+
+@pytest.mark.parametrize("cap,hidden", [(1, 2048), (15, 2048), (16, 2048), (8192, 2048), (2**62, 2048), (64, 8), (2, 200000)])
+def test_a_workspace_stays_within_the_host_bytes_it_asks_for(harness, cap, hidden):
+    asked, held, refused = run(harness, "budget", cap, hidden)
+    assert held <= asked
+    assert asked - held <= 64                                  # and asks for little more than that
+    assert refused == 10                                       # QW4_CAPACITY with one byte less
