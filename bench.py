@@ -15,7 +15,8 @@ One JSON line is printed by rank 0:
   roofline   the dominant kernel's algorithmic weight bytes / its event-timed duration
   layer      the whole layer's weight bytes touched / step time, against the HBM peak
   cpu_baseline  the reference's own CPU MoE path timed here on the host cores
-`--impl reference` times only that CPU path and prints the same line shape.
+`--impl reference` times only that CPU path and prints the same line shape; without the reference's own
+objects it prints {"impl": "reference", "unavailable": ...} (the port below is this project's code).
 
 With N > 1 (torchrun, one rank per GPU) every rank runs its own replica of that batch (single-token
 decode stays on one GPU: independent replicas, no collective on the data path, weak scaling).
@@ -404,6 +405,11 @@ def main():
 
     if args.impl == "reference":
         if rank != 0:
+            return
+        import oracle
+        if not oracle.reference_available():
+            # this project's restatement of the reference is a checker, not the reference: no number of its goes under that name
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's own CPU objects (oracle/_ref) are not built: its sources are not mounted"}))
             return
         name = args.workload if args.workload in ("c0", "c1", "c2") else "c1"
         desc, tokens, specs, x = workload(name, 1)
