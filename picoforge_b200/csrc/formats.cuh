@@ -11,7 +11,7 @@
 //   Q4_K     unchanged: block b of row n at (n * nb + b) * 144; 144 = 9 * 16 bytes.
 //   Q2_K     [rows*nb][64 B codes] | [rows*nb][16 B scale/min bytes] | [rows*nb][d, dmin f16]
 //   IQ2_XXS  [rows][nb*8 groups x 8 B] | [rows*nb][d f16]; inside a row, 8-byte group c is
-//            stored at position c ^ ((row & 3) << 2) (rows of two or more blocks), so that the
+//            stored at position c ^ ((row & 3) << 2) (rows of an even number of blocks), so that the
 //            four rows a half-warp reads together fall in different shared-memory banks when
 //            whole row tiles are copied to shared memory unchanged
 //   others   unchanged (F32, F16, BF16, Q8_0, MXFP4).
@@ -47,8 +47,9 @@ __device__ __forceinline__ uint32_t load_u32(const uint8_t *p) { return *reinter
 
 __device__ __forceinline__ uint32_t iq2_magnitude(uint32_t level) { return 8u + 17u * level + (level >> 1); }
 
-// Position swizzle of IQ2_XXS groups inside a row of the resident image.
-__host__ __device__ __forceinline__ uint32_t iq2_swizzle(uint32_t row, uint32_t nb) { return nb >= 2 ? (row & 3u) << 2 : 0u; }
+// Position swizzle of IQ2_XXS groups inside a row of the resident image.  It permutes runs of sixteen groups, two blocks; the last eight
+// groups of a row of three blocks would land in the next row's.
+__host__ __device__ __forceinline__ uint32_t iq2_swizzle(uint32_t row, uint32_t nb) { return nb & 1u ? 0u : (row & 3u) << 2; }
 
 // 8th sign of an IQ2_XXS vector: parity of the seven stored ones.
 __device__ __forceinline__ uint32_t iq2_signs8(uint32_t seven) { return seven | ((__popc(seven) & 1u) << 7); }

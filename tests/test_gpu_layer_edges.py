@@ -48,3 +48,21 @@ def test_layer_at_tile_edges(gpu, routed, down, shared, hidden, inter, physical,
     np.testing.assert_array_equal(y3, y)
     np.testing.assert_array_equal(ids2, ids)
     np.testing.assert_array_equal(weights2, weights)
+
+
+@pytest.mark.parametrize("hidden,inter", [(256, 768), (768, 256), (1280, 512)])
+def test_iq2_rows_of_an_odd_number_of_blocks(gpu, hidden, inter):
+    """The resident image of IQ2_XXS rows of three and five blocks decodes to the oracle's bits, and the layer computes with it."""
+    import oracle
+    spec = synth.make_layer(7800 + hidden, routed_type=IQ2, shared_type=Q4, hidden=hidden, inter=inter, shared_inter=256, experts=8, top_k=3)
+    x = synth.activations(7800 + hidden, 6, hidden)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    with MoeLayer(gpu, spec, 6) as layer:
+        for tensor in (1, 2, 3):
+            k, _, rows, experts = spec.shapes()[tensor]
+            raw = oracle.decode_rows(IQ2, spec.tensors[tensor], rows * experts, k).reshape(experts, rows, k)
+            for expert in (0, experts - 1):
+                np.testing.assert_array_equal(layer.decode_rows(tensor, expert, 0, rows).view(np.uint32), raw[expert].view(np.uint32))
+        y, ids, _ = layer.forward(x)
+    np.testing.assert_array_equal(ids, want["ids"])
+    assert np.abs(y - want["y"]).max() <= 1e-3
