@@ -668,7 +668,10 @@ extern "C" int qw4sh_mma_supported(const QW4ShTensor *w, int mode) {
     if (w->type != T_Q4_K && w->type != T_IQ2_XXS) return 0;
     if (w->k_storage % 256 || w->k_storage > KMAX || w->k_logical != w->k_storage) return 0;
     if (w->n_out % (mode == 0 ? 32 : 256)) return 0;
-    return 1;
+    // two stages of a unit beside the activations: 32 gate and up rows fit up to K = 2048 (Q4_K) and 3072 (IQ2_XXS), 256 down rows up to 512 and 1024
+    const uint32_t k = w->k_storage;
+    return (w->type == T_Q4_K ? mode == 0 ? make_plan<T_Q4_K, 0>(k) : make_plan<T_Q4_K, 1>(k)
+                              : mode == 0 ? make_plan<T_IQ2_XXS, 0>(k) : make_plan<T_IQ2_XXS, 1>(k)).n_stages >= 2;
 }
 
 template <uint32_t TYPE, int MODE>

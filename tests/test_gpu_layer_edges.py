@@ -66,3 +66,29 @@ def test_iq2_rows_of_an_odd_number_of_blocks(gpu, hidden, inter):
         y, ids, _ = layer.forward(x)
     np.testing.assert_array_equal(ids, want["ids"])
     assert np.abs(y - want["y"]).max() <= 1e-3
+
+
+@pytest.mark.parametrize("routed,hidden,inter,kernel", [
+    (IQ2, 1024, 1024, "grouped_mma_kernel"),         # the most down columns of the four-row kernels
+    (IQ2, 512, 1280, "gate_up_kernel"),               # one more block: no pair of blocks for the tcgen05 products either
+    (IQ2, 512, 1536, "expert_tile_kernel"),
+    (IQ2, 3328, 256, "gate_up_kernel"),               # beyond their gate and up columns
+    (Q4, 2304, 256, "expert_tile_kernel"),
+])
+def test_layers_around_the_four_row_kernels_largest_rows(gpu, routed, hidden, inter, kernel):
+    """A layer whose rows do not fit the four-row kernels' shared memory twice goes elsewhere, whatever path is preferred."""
+    import oracle
+    spec = synth.make_layer(7700 + inter, routed_type=routed, shared_type=Q4, hidden=hidden, inter=inter, shared_inter=256, experts=6, top_k=2)
+    x = synth.activations(7700 + inter, 6, hidden)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    try:
+        with MoeLayer(gpu, spec, 6) as layer:
+            for path in (-1, 1):
+                gpu.lib.qw4cu_set_expert_path(path)
+                gpu.lib.qw4cu_launch_log_begin()
+                y, ids, _ = layer.forward(x)
+                assert kernel in gpu.launch_names()
+                np.testing.assert_array_equal(ids, want["ids"])
+                assert np.abs(y - want["y"]).max() <= 1e-3
+    finally:
+        gpu.lib.qw4cu_set_expert_path(-1)
