@@ -108,7 +108,7 @@ __device__ inline float decode_value(const DevTensor &t, uint32_t expert, uint32
         const uint64_t blocks = (uint64_t)t.n_out * nb, block = (uint64_t)row * nb + (column >> 8);
         const uint32_t lane = column & 255u, slot = (lane & 31u) >> 3;
         const uint8_t *group = mat + ((uint64_t)row * nb * 8u + ((((column >> 8) * 8u) + (lane >> 5)) ^ iq2_swizzle(row, nb))) * 8u;
-        const uint32_t bits = load_u32(group + 4);
+        const uint32_t bits = load_u16(group + 4) | load_u16(group + 6) << 16;      // an expert starts on an even byte, no more (66 bytes a block)
         const uint32_t signs = iq2_signs8((bits >> (7 * slot)) & 127u);
         const uint32_t level = (c_iq2_levels[group[slot]] >> (2 * (lane & 7u))) & 3u;
         const float d = half_bits_to_float((uint16_t)load_u16(mat + blocks * 64u + block * 2u));

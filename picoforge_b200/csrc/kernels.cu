@@ -953,7 +953,9 @@ extern "C" int qw4sh_group_large(uint32_t experts, uint32_t k, size_t tokens, co
 // Activations sit in shared memory with 4 floats of padding after every 32 (index
 // k + 4*(k/32)) so that 128-bit reads by consecutive lanes fall in distinct banks.
 // ------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t xs_index(uint32_t k) { return k + ((k >> 5) << 2); }
+__host__ __device__ __forceinline__ uint32_t xs_index(uint32_t k) { return k + ((k >> 5) << 2); }
+// floats from one such row to the next: on the 16-byte grid whatever k is
+__host__ __device__ __forceinline__ uint32_t xs_pitch(uint32_t k) { return (xs_index(k) + 7u) & ~3u; }
 
 template <uint32_t TYPE> struct Unit;
 
@@ -1076,7 +1078,7 @@ __global__ void __launch_bounds__(GU_WARPS * 32) gate_up_kernel(DevTensor gate, 
     extern __shared__ __align__(16) float gu_smem[];
     __shared__ uint16_t levels_lut[256];
     const uint32_t inter = gate.n_out, nb = gate.k_storage >> 8, units = gate.k_storage >> 5;
-    const uint32_t x_pitch = xs_index(hidden) + 4;
+    const uint32_t x_pitch = xs_pitch(hidden);
     uint32_t expert = 0, first = 0, count = tokens;
     if (row_to_pair) {
         if (blockIdx.y >= active[0]) return;
@@ -1201,7 +1203,7 @@ __global__ void __launch_bounds__(DR_WARPS * 32) down_reduce_kernel(DevTensor do
     extern __shared__ __align__(16) float dr_smem[];
     __shared__ uint16_t levels_lut[256];
     const uint32_t t = blockIdx.y, hidden = down.n_out, inter = down.k_logical, sinter = sdown.k_logical;
-    const uint32_t a_pitch = xs_index(inter) + 4;
+    const uint32_t a_pitch = xs_pitch(inter);
     float *sa = dr_smem + (uint64_t)k * a_pitch;
     if (RT == T_IQ2_XXS || ST == T_IQ2_XXS) for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) levels_lut[i] = c_iq2_levels[i];
     for (uint32_t i = threadIdx.x; i < k * inter; i += blockDim.x) {
@@ -1240,10 +1242,13 @@ __global__ void __launch_bounds__(DR_WARPS * 32) down_reduce_kernel(DevTensor do
 // Launch helpers
 // ------------------------------------------------------------------------------------
 static const uint32_t GENERIC = 0xffffffffu;
-static uint32_t kernel_type(uint32_t type, uint32_t k_storage) {
-    return ((type == T_Q4_K || type == T_Q2_K || type == T_IQ2_XXS) && k_storage % 256 == 0) ? type : GENERIC;
+// The format whose units the CUDA-core kernels read, or GENERIC, one value at a time: units are whole runs of eight columns, so the
+// logical ones must end with a run, and 64-bit loads, so every expert must start on an 8-byte boundary (a Q2_K block has 84 bytes, an
+// IQ2_XXS block 66).
+static uint32_t kernel_type(const DevTensor &t) {
+    const bool packed = t.type == T_Q4_K || t.type == T_Q2_K || t.type == T_IQ2_XXS;
+    return packed && t.k_storage % 256 == 0 && t.k_logical % 8 == 0 && (t.n_experts == 1 || t.expert_bytes % 8 == 0) ? t.type : GENERIC;
 }
-static size_t xs_floats(size_t k) { return k + ((k >> 5) << 2) + 4; }
 
 template <typename Kernel>
 static int allow_smem(Kernel kernel, size_t smem) {
@@ -1378,9 +1383,9 @@ static int launch_router(const QW4ShLayer *layer, const float *x, size_t tokens,
 static int launch_gate_up(const DevTensor &gate, const DevTensor &up, const float *x, uint32_t hidden, const uint32_t *offsets,
                           const uint32_t *row_to_pair, const uint32_t *active, uint32_t k_div, uint32_t tokens, uint32_t groups,
                           float *act, uint32_t *status, cudaStream_t stream) {
-    uint32_t type = kernel_type(gate.type, gate.k_storage);
+    uint32_t type = kernel_type(gate);
     if (up.type != gate.type || hidden % 4) type = GENERIC;
-    const size_t smem = (size_t)GU_ROWS * xs_floats(hidden) * sizeof(float);
+    const size_t smem = (size_t)GU_ROWS * xs_pitch(hidden) * sizeof(float);
     const dim3 grid((gate.n_out + GU_TILE - 1) / GU_TILE, groups);
 #define GU_CASE(T) case T: { const auto kernel = rows_aligned(x, hidden) ? gate_up_kernel<T, true> : gate_up_kernel<T, false>; \
     if (allow_smem(kernel, smem)) return -1; \
@@ -1401,7 +1406,7 @@ template <uint32_t RT>
 static int launch_down_st(uint32_t st, const DevTensor &down, const DevTensor &sdown, const float *act, const float *shared_act,
                           const uint32_t *ids, const float *weights, const float *shared_logit, uint32_t k, uint32_t tokens,
                           float *y, float *routed, uint32_t *status, cudaStream_t stream) {
-    const size_t smem = ((size_t)k * xs_floats(down.k_logical) + xs_floats(sdown.k_logical)) * sizeof(float);
+    const size_t smem = ((size_t)k * xs_pitch(down.k_logical) + xs_pitch(sdown.k_logical)) * sizeof(float);
     const dim3 grid((down.n_out + DR_TILE - 1) / DR_TILE, tokens);
 #define DR_CASE(S) case S: if (allow_smem(down_reduce_kernel<RT, S>, smem)) return -1; \
     down_reduce_kernel<RT, S><<<grid, DR_WARPS * 32, smem, stream>>>(down, sdown, act, shared_act, ids, weights, shared_logit, k, y, routed, status); break;
@@ -1419,7 +1424,7 @@ static int launch_down_st(uint32_t st, const DevTensor &down, const DevTensor &s
 static int launch_down(const DevTensor &down, const DevTensor &sdown, const float *act, const float *shared_act,
                        const uint32_t *ids, const float *weights, const float *shared_logit, uint32_t k, uint32_t tokens,
                        float *y, float *routed, uint32_t *status, cudaStream_t stream) {
-    const uint32_t rt = kernel_type(down.type, down.k_storage), st = kernel_type(sdown.type, sdown.k_storage);
+    const uint32_t rt = kernel_type(down), st = kernel_type(sdown);
     switch (rt) {
     case T_Q4_K: return launch_down_st<T_Q4_K>(st, down, sdown, act, shared_act, ids, weights, shared_logit, k, tokens, y, routed, status, stream);
     case T_Q2_K: return launch_down_st<T_Q2_K>(st, down, sdown, act, shared_act, ids, weights, shared_logit, k, tokens, y, routed, status, stream);

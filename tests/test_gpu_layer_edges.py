@@ -92,3 +92,30 @@ def test_layers_around_the_four_row_kernels_largest_rows(gpu, routed, hidden, in
                 assert np.abs(y - want["y"]).max() <= 1e-3
     finally:
         gpu.lib.qw4cu_set_expert_path(-1)
+
+
+@pytest.mark.parametrize("routed,shared,inter,physical,shared_inter", [
+    (Q2, F32, 5, 256, 7),                # experts that start four bytes off an 8-byte boundary; logical columns that end inside a run of eight
+    (IQ2, F32, 5, 256, 7),               # two bytes off
+    (IQ2, F32, 6, 256, 7),
+    (Q2, IQ2, 12, 256, 256),             # experts on the boundary, a last run of four
+    (F32, Q4, 5, 5, 256),                # rows of five activations ahead of one that is read 128 bits at a time
+    (F32, Q2, 7, 7, 256),
+])
+def test_packed_layers_off_the_units(gpu, routed, shared, inter, physical, shared_inter):
+    import oracle
+    spec = synth.make_layer(7600 + inter, routed_type=routed, shared_type=shared, hidden=256, inter=inter, shared_inter=shared_inter, down_physical=physical,
+                            experts=5, top_k=2)
+    x = synth.activations(7600 + inter, 6, 256)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    with MoeLayer(gpu, spec, 6) as layer:
+        for tensor in (1, 3):
+            k, _, rows, experts = spec.shapes()[tensor]
+            raw = oracle.decode_rows(spec.types[tensor], spec.tensors[tensor], rows * experts, k).reshape(experts, rows, k)
+            for expert in range(experts):
+                np.testing.assert_array_equal(layer.decode_rows(tensor, expert, 0, rows).view(np.uint32), raw[expert].view(np.uint32))
+        for tokens in (1, 6):
+            y, ids, weights = layer.forward(x[:tokens])
+            np.testing.assert_array_equal(ids, want["ids"][:tokens])
+            np.testing.assert_array_equal(weights, want["weights"][:tokens])
+            assert np.abs(y - want["y"][:tokens]).max() <= 1e-3
