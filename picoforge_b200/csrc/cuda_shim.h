@@ -64,7 +64,7 @@ typedef struct {
     float *shared_out;            /* [cap, hidden] */
     /* int8 digit images of the three activation matrices (quantize_rows): x [cap rows of
      * hidden], act [cap*k rows of inter], shared_act [cap rows of shared_inter] */
-    int8_t *xq, *xneg, *aq, *aneg, *sq, *sneg;   /* [rows, 2, K] digits and negated digits */
+    int8_t *xq, *xneg, *aq, *aneg, *sq, *sneg;   /* [rows, 2, K] digits and negated digits: where split_*.hi and .lo of the same rows lie */
     int *xsum, *asum, *ssum;      /* [rows, K / 32, 2] digit sums per 32-column chunk */
     float *xscale, *ascale, *sscale;  /* [rows] */
     void *groups, *shared_groups; /* [cap * k], [cap / 4 + 1] groups of <= 4 rows (16 bytes each) */

@@ -103,16 +103,16 @@ int qw4sh_layer_forward(const QW4ShLayer *layer, const QW4ShWork *work, const fl
     return 0;
 }
 
-/* A handle of `experts` experts with F32 tensors of `hidden` columns whose bytes nobody reads. */
-static Qwen4Moe *make_moe(size_t h, size_t experts, size_t k) {
-    static float bytes[1 << 20];
-    const size_t shape[8][3] = {{h, experts, 1}, {h, 1, experts}, {h, 1, experts}, {1, h, experts}, {h, 1, 1}, {h, 1, 1}, {1, h, 1}, {h, 1, 1}};
+/* A handle of `experts` experts with F32 tensors of h columns, i intermediate, whose bytes nobody reads. */
+static Qwen4Moe *make_moe(size_t h, size_t experts, size_t k, size_t i) {
+    static float bytes[16];
+    const size_t shape[8][3] = {{h, experts, 1}, {h, i, experts}, {h, i, experts}, {i, h, experts}, {h, i, 1}, {h, i, 1}, {i, h, 1}, {h, 1, 1}};
     QW4PackedCpuView v[8];
-    for (int i = 0; i < 8; i++) {
-        const size_t row = shape[i][0] * 4, expert = row * shape[i][1], tensor = expert * shape[i][2];
-        v[i] = (QW4PackedCpuView){{(const unsigned char *)bytes, tensor}, {0, shape[i][0], shape[i][0], shape[i][1], shape[i][2], row, expert, tensor}};
+    for (int a = 0; a < 8; a++) {
+        const size_t row = shape[a][0] * 4, expert = row * shape[a][1], tensor = expert * shape[a][2];
+        v[a] = (QW4PackedCpuView){{(const unsigned char *)bytes, tensor}, {0, shape[a][0], shape[a][0], shape[a][1], shape[a][2], row, expert, tensor}};
     }
-    const Qwen4MoeConfig c = {(uint32_t)h, (uint32_t)experts, (uint32_t)k, 1, 1, 1, true, {0, 0, 0}};
+    const Qwen4MoeConfig c = {(uint32_t)h, (uint32_t)experts, (uint32_t)k, (uint32_t)i, (uint32_t)i, (uint32_t)i, true, {0, 0, 0}};
     const Qwen4MoeWeights w = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
     Qwen4Moe *m = NULL;
     Qwen4Error err;
@@ -136,7 +136,7 @@ static Qwen4F32Mut view_mut(float *p, size_t rows, size_t cols, size_t pitch) {
 
 /* budget CAP HIDDEN: the bytes asked for, the bytes held at the most, the status with one byte less. */
 static int budget(size_t cap, size_t h) {
-    Qwen4Moe *m = make_moe(h, 16, 4);
+    Qwen4Moe *m = make_moe(h, 16, 4, 1);
     size_t asked = 0;
     Qwen4MoeWork *work = NULL;
     Qwen4Error err;
@@ -150,7 +150,7 @@ static int budget(size_t cap, size_t h) {
 }
 /* rows TOKENS HIDDEN XPAD YPAD CALLS: wrong values, threads seen, threads with open signal masks, whether the caller's mask changed. */
 static int rows(size_t t, size_t h, size_t xpad, size_t ypad, int calls) {
-    Qwen4Moe *m = make_moe(h, 16, 4);
+    Qwen4Moe *m = make_moe(h, 16, 4, 1);
     size_t asked = 0, wrong = 0;
     Qwen4MoeWork *work = NULL;
     Qwen4Error err;
@@ -183,9 +183,22 @@ static int rows(size_t t, size_t h, size_t xpad, size_t ypad, int calls) {
     free(x); free(y); free(w); free(ids);
     return host_bytes_live ? 5 : 0;
 }
+/* device CAP HIDDEN EXPERTS TOPK INTER: bytes of the workspace's device block. */
+static int device(size_t cap, size_t h, size_t e, size_t k, size_t i) {
+    Qwen4Moe *m = make_moe(h, e, k, i);
+    size_t chunk;
+    Plan plan;
+    Qwen4Error err;
+    if (plan_work(m, cap, &chunk, &plan, &err)) return 3;
+    printf("%zu\n", plan.total);
+    qwen4_moe_destroy(m);
+    return 0;
+}
 int main(int argc, char **argv) {
     if (argc == 4 && !strcmp(argv[1], "budget")) return budget(strtoul(argv[2], NULL, 10), strtoul(argv[3], NULL, 10));
     if (argc == 7 && !strcmp(argv[1], "rows"))
         return rows(strtoul(argv[2], NULL, 10), strtoul(argv[3], NULL, 10), strtoul(argv[4], NULL, 10), strtoul(argv[5], NULL, 10), atoi(argv[6]));
+    if (argc == 7 && !strcmp(argv[1], "device"))
+        return device(strtoul(argv[2], NULL, 10), strtoul(argv[3], NULL, 10), strtoul(argv[4], NULL, 10), strtoul(argv[5], NULL, 10), strtoul(argv[6], NULL, 10));
     return 1;
 }

@@ -238,3 +238,27 @@ def test_pulled_partial_sums_wherever_y_starts(gpu, world, quads):
     finally:
         for p in d_partial + [d_y]:
             lib.qw4cu_free(p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("routed,shared", [(16, 12), (12, 16)])
+def test_a_step_with_its_halves_on_different_kernels(gpu, routed, shared):
+    """768 columns: IQ2_XXS tensors (whole pairs of blocks a stage) stay on the four-row kernels where Q4_K ones take the tcgen05
+    products, so one step holds rows of x as digits and as halves at once."""
+    import oracle
+    from picoforge_b200 import synth
+    from picoforge_b200.expert_parallel import EpLayer, forward_emulated
+    spec = synth.make_layer(330 + routed, routed_type=routed, shared_type=shared, experts=16, top_k=4, hidden=768, inter=256, shared_inter=256)
+    x = synth.activations(330, 24, 768)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    layers = [EpLayer(gpu, spec.shard(r * 8, 8), 12, 2, r) for r in range(2)]
+    try:
+        gpu.lib.qw4cu_launch_log_begin()
+        ys = forward_emulated(gpu, layers, [x[:12], x[12:]])
+        names = gpu.launch_names()
+    finally:
+        for layer in layers:
+            layer.close()
+    assert "expert_tile_kernel" in names
+    assert ("grouped_mma_kernel" in names) == (routed == 16)
+    assert np.abs(np.concatenate(ys) - want["y"]).max() <= 1e-3

@@ -119,3 +119,32 @@ def test_packed_layers_off_the_units(gpu, routed, shared, inter, physical, share
             np.testing.assert_array_equal(ids, want["ids"][:tokens])
             np.testing.assert_array_equal(weights, want["weights"][:tokens])
             assert np.abs(y - want["y"][:tokens]).max() <= 1e-3
+
+
+@pytest.mark.parametrize("routed,shared,tokens", [(IQ2, Q4, 40), (Q4, Q4, 96), (Q4, Q4, 7)])
+def test_one_workspace_through_every_path_in_turn(gpu, routed, shared, tokens):
+    """The four-row kernels' digits and the tcgen05 products' halves lie in the same rows of the workspace: each path gives the same
+    bits before and after the others have used it."""
+    spec = synth.make_layer(7900 + tokens, routed_type=routed, shared_type=shared, hidden=512, inter=512, shared_inter=256, experts=24, top_k=6)
+    x = synth.activations(7900 + tokens, tokens, 512)
+    paths = {"expert_tile_kernel": (-1, 1), "grouped_mma_kernel": (1, 0), "gate_up_kernel": (0, -1)}      # expert path, tile path
+    seen = {}
+    try:
+        with MoeLayer(gpu, spec, tokens) as layer:
+            for turn in range(2):
+                for kernel, (expert, tile) in paths.items():
+                    gpu.lib.qw4cu_set_expert_path(expert)
+                    gpu.lib.qw4cu_set_tile_path(tile)
+                    gpu.lib.qw4cu_set_prefill_path(0)
+                    gpu.lib.qw4cu_launch_log_begin()
+                    y, ids, _ = layer.forward(x)
+                    assert kernel in gpu.launch_names()
+                    if turn:
+                        np.testing.assert_array_equal(y, seen[kernel])
+                    seen[kernel] = y
+    finally:
+        gpu.lib.qw4cu_set_expert_path(-1)
+        gpu.lib.qw4cu_set_tile_path(-1)
+        gpu.lib.qw4cu_set_prefill_path(-1)
+    for kernel in paths:
+        assert np.abs(seen[kernel] - seen["gate_up_kernel"]).max() <= 1e-3

@@ -64,3 +64,13 @@ def test_a_workspace_stays_within_the_host_bytes_it_asks_for(harness, cap, hidde
     assert held <= asked
     assert asked - held <= 64                                  # and asks for little more than that
     assert refused == 10                                       # QW4_CAPACITY with one byte less
+
+
+def test_digits_and_halves_of_a_row_share_their_room(harness):
+    """4096 tokens of the benchmark's layer: x, act and shared act as halves (4 bytes a value) and not as digits beside them."""
+    cap, h, e, k, i = 4096, 2048, 512, 10, 512
+    bytes_, = run(harness, "device", cap, h, e, k, i)
+    values = cap * h + cap * k * i + cap * i                   # x, routed and shared activations
+    # staging, logits, outputs and the like; the halves; their sums and scales (an eighth to a quarter of the values' count, in words)
+    rest = 4 * (2 * cap * h + 2 * cap * e + cap * k * h + cap * h + cap * k * i + cap * i)
+    assert rest + 4 * values < bytes_ < rest + 4 * values + values + (8 << 20)
