@@ -305,7 +305,8 @@ Qwen4Status qw4cu_moe_work_sync_many(Qwen4MoeWork *const *works, size_t n, Qwen4
  * own (or one process that plays several ranks):
  *   begin    routes x [tokens_local, hidden], writes this rank's exchange rows to rows_local_dev
  *            [tokens_local, row floats] (and ids / weights [tokens_local, k] if not NULL) and starts
- *            the shared expert of these tokens on a second stream;
+ *            the shared expert of these tokens on a second stream, which reads x until `experts` has been
+ *            waited for;
  *   experts  rows_all_dev: the rows of all ranks in rank order [tokens_total, row floats]; own_first:
  *            index of this rank's first token in it; partial_dev [tokens_total, hidden] receives the
  *            partial sums.  y of a token = sum over ranks of its partial rows.

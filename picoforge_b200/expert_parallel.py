@@ -123,14 +123,15 @@ def forward_emulated(api: abi.MoeApi, layers: list[EpLayer], xs: list[np.ndarray
     hidden = layers[0].spec.hidden
     pitch = lib.qw4cu_ep_row_floats(layers[0].layer.moe)
     rows_all = np.empty((world * per, pitch), np.float32)
-    d_x, d_rows = lib.qw4cu_malloc(per * hidden * 4), lib.qw4cu_malloc(per * pitch * 4)
+    d_x = [lib.qw4cu_malloc(per * hidden * 4) for _ in layers]       # one each: a rank's shared expert reads its x until its experts have joined it
+    d_rows = lib.qw4cu_malloc(per * pitch * 4)
     d_all, d_partial = lib.qw4cu_malloc(world * per * pitch * 4), lib.qw4cu_malloc(world * per * hidden * 4)
     try:
         # every rank's begin (and with it the start of its shared expert) comes before any rank's experts
         for r, layer in enumerate(layers):
             x = np.ascontiguousarray(xs[r], np.float32)
-            assert lib.qw4cu_upload(d_x, x.ctypes.data, x.nbytes) == 0
-            layer.begin(d_x, d_rows)
+            assert lib.qw4cu_upload(d_x[r], x.ctypes.data, x.nbytes) == 0
+            layer.begin(d_x[r], d_rows)
             layer.sync()
             block = rows_all[r * per:(r + 1) * per]
             assert lib.qw4cu_download(block.ctypes.data, d_rows, block.nbytes) == 0
@@ -144,7 +145,7 @@ def forward_emulated(api: abi.MoeApi, layers: list[EpLayer], xs: list[np.ndarray
             total += partial
         return [total[r * per:(r + 1) * per].astype(np.float32) for r in range(world)]
     finally:
-        for pointer in (d_x, d_rows, d_all, d_partial):
+        for pointer in (*d_x, d_rows, d_all, d_partial):
             lib.qw4cu_free(pointer)
 
 
