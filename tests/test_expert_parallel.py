@@ -116,8 +116,7 @@ def test_shard_bytes_equal_the_slice_of_the_whole_tensor():
 @pytest.mark.parametrize("routed,world,tokens", [(12, 4, 16), (16, 2, 6), (10, 4, 32), (10, 2, 160), (12, 1, 24)])
 def test_sharded_layer_matches_the_oracle_with_the_ranks_played_in_one_process(gpu, routed, world, tokens):
     """`world` ranks share one GPU; the all-gather is a concatenation and the reduce-scatter a sum on the host.
-    Q4_K and IQ2_XXS shards take the four-row grouped kernels, Q2_K (and more than 64 tokens) the tile kernels;
-    80 own tokens per rank put the shared expert on the tile kernels too."""
+    All three formats take the tcgen05 products, shared expert included; these batches' lists are built with the foreign ids masked out."""
     import oracle
     from picoforge_b200 import abi, synth
     from picoforge_b200.expert_parallel import EpLayer, forward_emulated
@@ -262,3 +261,29 @@ def test_a_step_with_its_halves_on_different_kernels(gpu, routed, shared):
     assert "expert_tile_kernel" in names
     assert ("grouped_mma_kernel" in names) == (routed == 16)
     assert np.abs(np.concatenate(ys) - want["y"]).max() <= 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("routed,world,tokens", [(12, 4, 516), (10, 2, 1022)])
+def test_large_batches_slice_the_lists_of_all_pairs(gpu, routed, world, tokens):
+    """More than 2048 pairs: the bitmap dispatch sorts all of them, and a rank's experts are a contiguous slice of that order."""
+    import oracle
+    from picoforge_b200 import synth
+    from picoforge_b200.expert_parallel import EpLayer, forward_emulated
+    spec = synth.make_layer(340 + routed, routed_type=routed, shared_type=12, experts=32, top_k=4, hidden=256, inter=256, shared_inter=256)
+    x = synth.activations(340, tokens, 256)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    per, epr = tokens // world, 32 // world
+    layers = [EpLayer(gpu, spec.shard(r * epr, epr), per, world, r) for r in range(world)]
+    try:
+        gpu.lib.qw4cu_launch_log_begin()
+        ys = forward_emulated(gpu, layers, [x[r * per:(r + 1) * per] for r in range(world)])
+        names = gpu.launch_names()
+        ids = np.concatenate([layer.routes()[0] for layer in layers])
+    finally:
+        for layer in layers:
+            layer.close()
+    assert names.count("ep_active_slice_kernel") == world
+    np.testing.assert_array_equal(ids, want["ids"])
+    exact = want["y"].astype(np.float64)                       # FP32 sums in another order: 3e-6 of RMS(y), as on one device
+    assert np.sqrt(np.mean((np.concatenate(ys) - exact) ** 2)) <= 1e-5 * np.sqrt(np.mean(exact ** 2))

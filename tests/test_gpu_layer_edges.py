@@ -148,3 +148,48 @@ def test_one_workspace_through_every_path_in_turn(gpu, routed, shared, tokens):
         gpu.lib.qw4cu_set_prefill_path(-1)
     for kernel in paths:
         assert np.abs(seen[kernel] - seen["gate_up_kernel"]).max() <= 1e-3
+
+
+@pytest.mark.parametrize("routed,down,shared,hidden,inter,physical,tokens", [
+    (Q4, Q4, Q4, 2048, 512, 512, 40),
+    (Q4, Q4, Q4, 2048, 512, 512, 96),
+    (Q2, Q2, Q2, 2048, 512, 512, 7),
+    (Q2, Q2, Q4, 512, 256, 256, 96),
+    (IQ2, IQ2, IQ2, 2048, 512, 512, 96),
+    (IQ2, Q2, F32, 2560, 640, 768, 4),               # the checkpoint's mixture, its shared expert widened
+    (IQ2, Q2, F32, 2560, 640, 768, 96),
+])
+def test_tcgen05_products_keep_fp32_accuracy(gpu, routed, down, shared, hidden, inter, physical, tokens):
+    """Exact integer codes against activations in fp16 hi + lo: RMS error within 1e-5 of RMS(y) in every format.
+
+    Two FP32 results that add K <= 2560 products in other orders differ by about sqrt(K / 3) roundings of 2^-24, 1.7e-6, in each of
+    gate, up and down: 3e-6 together (2.0e-6 to 3.0e-6 measured).  The halves add 2^-22 per value.  Activations without their
+    low half would be off by 2^-12, int8 digits by 2^-16 (5e-5 of RMS(y)); a bit lost from a code or a scale by far more."""
+    import oracle
+    spec = synth.make_layer(7500 + tokens, routed_type=routed, down_type=down, shared_type=shared, hidden=hidden, inter=inter, shared_inter=inter,
+                            down_physical=physical, experts=32, top_k=6)
+    x = synth.activations(7500 + tokens, tokens, hidden)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    with MoeLayer(gpu, spec, tokens) as layer:
+        gpu.lib.qw4cu_launch_log_begin()
+        y, ids, _ = layer.forward(x)
+        assert {"expert_tile_kernel", "prefill_tc_kernel"} & set(gpu.launch_names())
+    np.testing.assert_array_equal(ids, want["ids"])
+    exact = want["y"].astype(np.float64)
+    assert np.sqrt(np.mean((y - exact) ** 2)) <= 1e-5 * np.sqrt(np.mean(exact ** 2))
+
+
+@pytest.mark.parametrize("routed,tokens", [(Q4, 2048), (Q2, 2049), (Q4, 4096), (Q2, 4097), (Q4, 4500)])
+def test_long_prompts(gpu, routed, tokens):
+    """Lists of more than 64 words of 32 tokens an expert, the last word full or of one token, and a second launch sequence of one
+    token or of 404."""
+    import oracle
+    spec = synth.make_layer(7400 + tokens, routed_type=routed, shared_type=routed, hidden=256, inter=256, shared_inter=256, experts=40, top_k=3)
+    x = synth.activations(7400 + tokens, tokens, 256)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    with MoeLayer(gpu, spec, tokens) as layer:
+        y, ids, weights = layer.forward(x)
+    np.testing.assert_array_equal(ids, want["ids"])
+    np.testing.assert_array_equal(weights, want["weights"])
+    exact = want["y"].astype(np.float64)
+    assert np.sqrt(np.mean((y - exact) ** 2)) <= 1e-5 * np.sqrt(np.mean(exact ** 2))

@@ -1,4 +1,4 @@
-"""The tile kernels (groups of up to 16 rows per expert on the int8 tensor cores) against the CPU
+"""The tcgen05 products under their general name (expert_tile_kernel: groups of up to 32 rows per expert) against the CPU
 oracle and against the four-row grouped kernels: route ids bit-exact, y within 1e-3 (max abs)."""
 import sys
 from pathlib import Path
@@ -29,12 +29,12 @@ def _forward(gpu, spec, x, tile):
 
 
 @pytest.mark.parametrize("routed,shared,tokens,experts,top_k", [
-    (12, 12, 5, 64, 10),      # one ragged column tile
+    (12, 12, 5, 64, 10),      # groups of one to five rows
     (16, 12, 16, 64, 10),     # IQ2_XXS routed + Q4_K shared
-    (12, 16, 33, 64, 6),      # dense shared groups of 16 + 16 + 1
-    (16, 16, 64, 16, 4),      # every expert sees several column tiles; groups split at 16 rows
-    (16, 12, 100, 64, 10),    # beyond the small-batch dispatch: bitmap dispatch + tile kernels
-    (10, 12, 7, 64, 10),      # Q2_K routed: scales folded into the codes, minima through a second MMA
+    (12, 16, 33, 64, 6),      # dense shared groups of 32 + 1
+    (16, 16, 64, 16, 4),      # about 16 rows an expert: groups of either width
+    (16, 12, 100, 64, 10),    # beyond 64 tokens: lists by a launch of their own
+    (10, 12, 7, 64, 10),      # Q2_K routed: scales folded into the codes, minima through a second accumulator
     (10, 10, 40, 32, 6),      # Q2_K everywhere
     (10, 12, 130, 64, 10),
 ])
@@ -73,7 +73,7 @@ def test_tile_kernels_at_config_shapes(gpu):
 
 
 def test_skewed_routing_fills_whole_groups(gpu):
-    """A router that sends every token to the same experts: each list splits into full 16-row groups."""
+    """A router that sends every token to the same experts: each list splits into a full group of 32 rows and one of 16."""
     import oracle
     from picoforge_b200 import abi, synth
     spec = synth.make_layer(11, routed_type=abi.IQ2_XXS, shared_type=abi.Q4_K, experts=64, top_k=4)
