@@ -359,10 +359,11 @@ float qw4cu_moe_work_timer_elapsed_ms(Qwen4MoeWork *work);
  * captured into a CUDA graph and later identical calls replay it. */
 void qw4cu_set_graph_mode(int on);
 int qw4cu_get_graph_mode(void);
-/* Which expert kernels run.  -1 (default): batches of up to 64 tokens use the tensor-core
- * grouped kernels (groups of <= 4 rows, int8 MMA on the raw codes) when every expert tensor is
- * Q4_K or IQ2_XXS, everything else the CUDA-core kernels.  0: CUDA-core kernels only.  1:
- * tensor-core grouped kernels for any batch size the formats allow. */
+/* Which expert kernels run.  -1 (default): the tcgen05 products and the four-row kernels as
+ * qw4cu_set_tile_path says, the CUDA-core kernels for formats and shapes that neither takes.
+ * 0: CUDA-core kernels only.  1: the four-row grouped kernels (groups of <= 4 rows, int8 MMA on the
+ * raw codes) for any batch beyond the one-kernel decode path whose expert tensors are all Q4_K or
+ * IQ2_XXS and fit them, except what qw4cu_set_prefill_path names. */
 void qw4cu_set_expert_path(int path);
 /* One-kernel decode path (no counterpart in the reference): batches of up to four tokens whose
  * expert tensors are all Q4_K or IQ2_XXS run the whole layer as one persistent kernel, one CTA
@@ -384,15 +385,16 @@ void qw4cu_set_expert_path(int path);
  * run the experts a second time.  qw4cu_set_decode_wrong_speculation(1) makes every later launch
  * speculate a wrong expert for its first token (test aid for that repair path; 0 restores). */
 void qw4cu_set_fused_decode(int mode);
-/* Tensor-core prefill path (no counterpart in the reference): batches of more than 64 tokens whose
- * expert tensors are all Q4_K run gate/up and down as grouped GEMMs on tcgen05 tensor cores with
- * TMEM accumulators (groups of <= 32 token rows per expert, exact integer codes as fp16 operands,
- * activations split into fp16 hi + lo).  -1 (default): used whenever the layer fits; 0: never. */
+/* The tcgen05 products (no counterpart in the reference): gate/up and down as grouped GEMMs on tcgen05
+ * tensor cores with TMEM accumulators (groups of <= 32 token rows per expert, exact integer codes as fp16
+ * operands, activations split into fp16 hi + lo).  They are one kernel under two names: batches of more
+ * than 64 tokens whose expert tensors are all Q4_K launch it as prefill_tc_kernel (-1, default), or as
+ * expert_tile_kernel like everything else (0).  The arithmetic is the same. */
 void qw4cu_set_prefill_path(int path);
-/* Tile kernels: the same tcgen05 products (weights dequantised into TMEM once per group of <= 32 rows of an expert, activations as
- * fp16 hi + lo) under their general name, for every format.
- * -1 (default): every batch beyond the one-kernel decode path that the prefill name does not cover, except IQ2_XXS layers at up to
- * 64 rows, which the four-row kernels serve faster; 0: never; 1: every batch of more than four rows. */
+/* The same products under their general name, for every format.  -1 (default): every batch beyond the one-kernel decode path that
+ * the prefill name does not cover, except IQ2_XXS layers at up to 64 tokens, which the four-row kernels serve faster where the tokens
+ * spread evenly over the experts (slower where they crowd onto few: 1 is worth a try there); 0: never; 1: every batch of more
+ * than four tokens. */
 void qw4cu_set_tile_path(int path);
 /* Profiling aid of the tensor-core prefill kernels: device_words is a device array of 64 x 8 bytes (NULL: off).
  * CTA 0 of every later launch stores the SM cycles its roles (0 epilogue, 1 dequantise, 2 TMA, 3 MMA issue,

@@ -5,8 +5,11 @@
 //   router_logits  x -> logits [T,E] and the shared-expert gate logit [T]
 //   route          softmax, top-k, renormalise -> ids, weights [T,k]
 //   group          stable per-expert pair lists (dispatch)
-//   gate_up        act[pair] = silu(gate_e x) * (up_e x), weights dequantised in registers
-//   down_reduce    y[t] = sum_s w[t,s] (down_e act[pair]) + sigmoid(slogit[t]) (sdown sact[t])
+//   gate/up        act[pair] = silu(gate_e x) * (up_e x)
+//   down           out[pair] = down_e act[pair]
+//   combine        y[t] = sum_s w[t,s] out[t,s] + sigmoid(slogit[t]) (sdown sact[t])
+// The products are experts_tc.cu's (tcgen05), experts_mma.cu's (four rows of an expert at a time) or, for every format and shape,
+// the CUDA-core kernels below, which do the combine with the down product; layer_launches chooses.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -1334,7 +1337,8 @@ static int launch_router(const QW4ShLayer *layer, const float *x, size_t tokens,
     const bool aligned = ((uintptr_t)x & 15u) == 0 && router.k_logical % 4 == 0 && router.row_bytes % 16 == 0 && ((uintptr_t)router.data & 15u) == 0 &&
                          ((uintptr_t)srouter.data & 15u) == 0;
     if (mode == 0 && tokens <= 128 && aligned) {
-        // the tile: as many chains per CTA as leave one CTA per SM (513 rows)
+        // the tile: as many chains per CTA as leave about one CTA per SM.  Worked out for the 513 rows of both layer shapes; a layer of
+        // fewer experts gets the same tile, and a smaller grid.
 #define ROUTER_CHAIN(ROWS, TOK, STAGES) do { \
         static bool configured[64] = {false}; \
         const size_t smem = (size_t)STAGES * rc_stage_bytes(ROWS + TOK); \
@@ -1357,7 +1361,7 @@ static int launch_router(const QW4ShLayer *layer, const float *x, size_t tokens,
         if (mode == 0) router_gemm_kernel<true, TI, TJ><<<grid, 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status, 1.0f); \
         else router_gemm_kernel<false, TI, TJ><<<grid, 256, 0, stream>>>(router, srouter, x, (uint32_t)tokens, logits, shared_logit, status, 1.0f); } while (0)
         // the largest tile that still leaves a CTA for (nearly) every SM: 513 rows are seventeen tiles of 32 or nine of 64, so 32 tokens x
-        // 32 rows up to 256 tokens, 32 x 64 up to 512, then 64 x 64
+        // 32 rows up to 256 tokens, 32 x 64 up to 512, then 64 x 64 (as above: fewer experts, a smaller grid)
         if (tokens <= 256) ROUTER_GEMM(2, 2);
         else if (tokens <= 512) ROUTER_GEMM(2, 4);
         else ROUTER_GEMM(4, 4);
@@ -1544,7 +1548,7 @@ extern "C" void qw4sh_set_only_step(int step) { g_only_step = step; }
 static int g_expert_path = -1;                     // -1 auto, 0 CUDA-core kernels, 1 tensor-core grouped kernels
 extern "C" void qw4sh_set_expert_path(int path) { g_expert_path = path; }
 
-// Token batches up to this size take the decode path (groups of <= 4 rows on int8 MMA).
+// Token batches up to this size may take the four-row kernels by themselves (see tile_path), and have their lists built by the routing launch.
 static const size_t MMA_MAX_TOKENS = 64;
 
 static bool mma_path(const QW4ShLayer *layer, size_t tokens) {
@@ -1577,8 +1581,12 @@ static bool tile_path(const QW4ShLayer *layer, size_t tokens) {
     if (g_tile_path == 0 || g_expert_path == 0 || (g_tile_path > 0 && tokens <= 4)) return false;
     if (g_tile_path < 0) {
         if (prefill_path(layer, tokens)) return false;
-        // IQ2_XXS at up to 64 rows: two table reads for eight weights bound its dequantiser (2000 cycles for 128 columns of 256
-        // rows), and with a row or two per expert the four-row kernel's int8 table form is faster (23 tokens: 158 against 176 us)
+        // IQ2_XXS at up to 64 tokens: two table reads for eight weights bound its dequantiser (2000 cycles for 128 columns of 256
+        // rows), and where tokens spread evenly over 512 experts, a row or two to each, the four-row kernel's int8 table form is
+        // the faster one.  us a layer, four-row against tcgen05: 5 tokens 78 / 77, 16 130 / 132, 23 152 / 163, 32 177 / 188, 64 247 / 272,
+        // 96 302 / 306, 128 338 / 325.  Where they crowd onto few experts (Zipf 1.1) it is the slower one from the start, since a
+        // group is four rows: 5 tokens 68 / 60, 23 102 / 85, 64 162 / 102.  The host knows the tokens and not their routes, so the line
+        // is drawn for the even case.
         if (mma_path(layer, tokens) && (g_expert_path == 1 || layer->w[1].type == T_IQ2_XXS)) return false;
     }
     return tc_routed(layer) && tc_shared(layer);
