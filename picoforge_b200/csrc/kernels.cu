@@ -1256,7 +1256,8 @@ static uint32_t kernel_type(const DevTensor &t) {
 template <typename Kernel>
 static int allow_smem(Kernel kernel, size_t smem) {
     if (smem > 227u * 1024u) return fail(cudaErrorInvalidValue, "shape needs more shared memory than one CTA has");
-    if (smem > 48u * 1024u) CU(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // beyond 48 KB, which the kernel's own static arrays count towards (a few KB at most)
+    if (smem > 40u * 1024u) CU(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return 0;
 }
 

@@ -193,3 +193,22 @@ def test_long_prompts(gpu, routed, tokens):
     np.testing.assert_array_equal(weights, want["weights"])
     exact = want["y"].astype(np.float64)
     assert np.sqrt(np.mean((y - exact) ** 2)) <= 1e-5 * np.sqrt(np.mean(exact ** 2))
+
+
+@pytest.mark.parametrize("top_k,inter,shared_inter", [(16, 640, 512), (16, 640, 256), (33, 256, 256)])
+def test_down_rows_around_48_kb_of_shared_memory(gpu, top_k, inter, shared_inter):
+    """The CUDA-core down kernel holds a token's activations: (16, 640, 512) are 48,656 bytes, which with its table are more than
+    the 48 KB that a launch gets unasked."""
+    import oracle
+    spec = synth.make_layer(7300 + inter, routed_type=Q4, down_type=IQ2, shared_type=Q4, hidden=768, inter=inter, shared_inter=shared_inter,
+                            down_physical=(inter + 255) // 256 * 256, experts=40, top_k=top_k)
+    x = synth.activations(7300 + inter, 9, 768)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    gpu.lib.qw4cu_set_expert_path(0)
+    try:
+        with MoeLayer(gpu, spec, 9) as layer:
+            y, ids, _ = layer.forward(x)
+    finally:
+        gpu.lib.qw4cu_set_expert_path(-1)
+    np.testing.assert_array_equal(ids, want["ids"])
+    assert np.abs(y - want["y"]).max() <= 1e-3
