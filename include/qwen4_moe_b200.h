@@ -530,7 +530,7 @@ void *qw4cu_malloc(size_t bytes);
 void qw4cu_free(void *device_pointer);
 void *qw4cu_host_alloc(size_t bytes);            /* pinned host memory */
 void qw4cu_host_free(void *host_pointer);
-int qw4cu_upload(void *device_dst, const void *host_src, size_t bytes);
+int qw4cu_upload(void *device_dst, const void *host_src, size_t bytes);    /* there when the call returns */
 int qw4cu_download(void *host_dst, const void *device_src, size_t bytes);
 /* Writes `bytes` of a scratch buffer larger than L2 so that the next kernel starts cold. */
 int qw4cu_flush_l2(void);

@@ -98,8 +98,11 @@ extern "C" void *qw4sh_host_alloc(size_t bytes) {
     return p;
 }
 extern "C" void qw4sh_host_free(void *p) { if (p) cudaFreeHost(p); }
+// cudaMemcpy from pageable memory returns when the last piece has been staged, before it has arrived, and the library's stream does not
+// wait for the default one that it travels on: so this waits for it.
 extern "C" int qw4sh_memcpy(void *dst, const void *src, size_t bytes, int to_device) {
     if (bytes) CU(cudaMemcpy(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost));
+    if (bytes && to_device) CU(cudaStreamSynchronize(cudaStreamLegacy));
     return 0;
 }
 extern "C" int qw4sh_memcpy2d_async(void *dst, size_t dst_pitch, const void *src, size_t src_pitch,
@@ -205,8 +208,7 @@ extern "C" int qw4sh_upload_tensor(const void *host, size_t bytes, uint32_t type
         cudaFree(staging);
         if (e != cudaSuccess) { cudaFree(image); return fail(e, "regroup"); }
     } else if (bytes) {
-        cudaError_t e = cudaMemcpy(image, host, bytes, cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) { cudaFree(image); return fail(e, "cudaMemcpy weights"); }
+        if (qw4sh_memcpy(image, host, bytes, 1)) { cudaFree(image); return -1; }
     }
     *device = image;
     return 0;

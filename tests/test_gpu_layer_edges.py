@@ -212,3 +212,27 @@ def test_down_rows_around_48_kb_of_shared_memory(gpu, top_k, inter, shared_inter
         gpu.lib.qw4cu_set_expert_path(-1)
     np.testing.assert_array_equal(ids, want["ids"])
     assert np.abs(y - want["y"]).max() <= 1e-3
+
+
+def test_an_upload_has_arrived_when_the_call_returns(gpu):
+    """A megabyte and a row from pageable memory: the row travels as a piece of its own, and the library's stream does not wait for the
+    stream that it travels on."""
+    import ctypes as C
+    lib, err = gpu.lib, abi.Qwen4Error()
+    spec = synth.make_layer(7200, routed_type=Q4, shared_type=Q4, hidden=512, inter=256, shared_inter=256, experts=16, top_k=4)
+    tokens, k = 513, spec.top_k
+    d_x, d_ids = lib.qw4cu_malloc(tokens * 2048), lib.qw4cu_malloc(tokens * k * 4)
+    try:
+        with MoeLayer(gpu, spec, tokens) as layer:
+            for turn in range(40):
+                x = synth.activations(7200 + turn, tokens, 512)
+                assert lib.qw4cu_upload(d_x, x.ctypes.data, x.nbytes) == 0
+                assert lib.qw4cu_moe_route_device(layer.moe, d_x, tokens, d_ids, None, layer.work, C.byref(err)) == abi.OK
+                assert lib.qw4cu_moe_work_sync(layer.work, C.byref(err)) == abi.OK
+                ids = np.empty((tokens, k), np.uint32)
+                assert lib.qw4cu_download(ids.ctypes.data, d_ids, ids.nbytes) == 0
+                _, want, _ = layer.forward(x)
+                np.testing.assert_array_equal(ids, want, err_msg=f"turn {turn}")
+    finally:
+        lib.qw4cu_free(d_x)
+        lib.qw4cu_free(d_ids)
