@@ -10,7 +10,10 @@
 //   Q4_K      the 4-bit codes ARE the A operand (nibbles masked out of the packed bytes);
 //             sum(code * x) comes from mma.m16n8k32.s8, and the 6-bit sub-block scale and min
 //             are applied to the int32 sums with integer multiply-adds
-//   IQ2_XXS   the codebook vector (eight int8 magnitudes) and the byte masks of its sign word
+//   IQ2_XXS   from the expanded image where the layer holds one (iq2n.cuh): level and sign of a weight are a nibble that a byte
+//             permute turns into the signed magnitude.  Bound by instructions in either form, and the reads of the packed one came on
+//             top: a layer of 23 tokens 151 us on the packed image and 129 on this one, of 64 tokens 245 and 199, evenly spread
+//             tokens; the sums are added in the same order, so the results are the same bits.  From the packed image elsewhere: the codebook vector (eight int8 magnitudes) and the byte masks of its sign word
 //             come from bank-conflict-free shared-memory tables; a negative weight is
 //             (v ^ 0xff) + 1 per byte, two integer operations per four weights; the 4-bit
 //             group scale multiplies the int32 sums
@@ -32,6 +35,7 @@
 
 #include "cuda_shim.h"
 #include "formats.cuh"
+#include "iq2n.cuh"
 
 namespace qw4 {
 
@@ -103,6 +107,7 @@ struct GroupedArgs {
     uint32_t k_div;                    // input row = pair / k_div
     QuantRows in;
     const uint8_t *lut;                // IQ2_XXS tables image, LUT_BYTES
+    const uint8_t *expanded;           // the expanded image of w0 (gate and up in one): [expert][rows of a block][blocks of 512 columns]
     float *out;                        // [pairs][n_out]
     uint32_t *status;
 };
@@ -123,6 +128,12 @@ template <> struct Fmt<T_IQ2_XXS> {
     __host__ __device__ static uint32_t pitch(uint32_t nb) { return nb * 64; }   // rows are swizzled in the image
 };
 
+template <> struct Fmt<T_IQ2N> {
+    static constexpr uint32_t BLOCK_BYTES = 0;                           // not by rows: whole blocks of sixteen rows x 512 columns, one span a unit
+    static constexpr bool NEEDS_LUT = false;
+    __host__ __device__ static uint32_t pitch(uint32_t) { return 0; }
+};
+
 // Shared-memory plan (byte offsets), the same on host and device.
 struct Plan {
     uint32_t bars, lut, bslot, bslot_bytes, xq, xneg, xsum, meta, partial, stages, stage_bytes, total;
@@ -134,7 +145,7 @@ __host__ __device__ inline Plan make_plan(uint32_t k_storage) {
     const uint32_t nb = k_storage / 256;
     p.unit_rows = MODE == 0 ? 32 : 256;                                 // two row tiles per warp and unit, so that the barriers and the
                                                                          // partial-sum exchange of a unit are paid half as often
-    p.matrices = MODE == 0 ? 2 : 1;
+    p.matrices = MODE == 0 && TYPE != T_IQ2N ? 2 : 1;
     p.kp = k_storage + 32;
     p.pitch = Fmt<TYPE>::pitch(nb);
     uint32_t at = 0;
@@ -152,6 +163,7 @@ __host__ __device__ inline Plan make_plan(uint32_t k_storage) {
     at = (at + 127) & ~127u;
     p.dsec = p.unit_rows * p.pitch;                                      // IQ2_XXS: fp16 d after the payload rows
     uint32_t per_matrix = p.unit_rows * p.pitch + (TYPE == T_IQ2_XXS ? ((p.unit_rows * nb * 2 + 15) & ~15u) : 0);
+    if (TYPE == T_IQ2N) per_matrix = (MODE == 0 ? p.unit_rows / 8 : p.unit_rows / 16) * (k_storage / 512) * IQ2N_BLOCK;
     p.per_matrix = (per_matrix + 127) & ~127u;
     p.stage_bytes = p.per_matrix * p.matrices;
     p.stages = at;
@@ -246,11 +258,48 @@ template <> struct Consume<T_IQ2_XXS> {
     }
 };
 
+// One half (128 columns) of a block of the expanded image: rows g and g + 8 of it.
+template <> struct Consume<T_IQ2N> {
+    __device__ static __forceinline__ void half_block(const uint8_t *block, const Plan &p, const uint8_t *act, uint32_t half, uint32_t g, uint32_t t, float (&facc)[2]) {
+        const uint32_t h = half & 3u;
+        const uint8_t *lv = block + 512u * h + 32u * g + 8u * t, *sg = block + IQ2N_SIGNS + 256u * h + 16u * g + 4u * t, *sc = block + IQ2N_SCALES + 16u * g + 4u * h,
+                      *dd = block + IQ2N_D + 4u * g + 2u * (h >> 1), *xq = act + p.xq + g * p.kp + half * 128u + 8u * t;
+        const uint2 l0 = *reinterpret_cast<const uint2 *>(lv), l1 = *reinterpret_cast<const uint2 *>(lv + 256);
+        const uint32_t g0 = *reinterpret_cast<const uint32_t *>(sg), g1 = *reinterpret_cast<const uint32_t *>(sg + 128);
+        const uint32_t s0 = *reinterpret_cast<const uint32_t *>(sc), s1 = *reinterpret_cast<const uint32_t *>(sc + 128);
+        const uint32_t c0[4] = {iq2n_select<0>(l0, g0), iq2n_select<1>(l0, g0), iq2n_select<2>(l0, g0), iq2n_select<3>(l0, g0)};
+        const uint32_t c1[4] = {iq2n_select<0>(l1, g1), iq2n_select<1>(l1, g1), iq2n_select<2>(l1, g1), iq2n_select<3>(l1, g1)};
+        int iacc[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint2 bq = *reinterpret_cast<const uint2 *>(xq + j * 32);
+            int c[4];
+            mma_s8_zero(c, __byte_perm(IQ2N_LO, IQ2N_HI, c0[j]), __byte_perm(IQ2N_LO, IQ2N_HI, c1[j]),
+                        __byte_perm(IQ2N_LO, IQ2N_HI, c0[j] >> 16), __byte_perm(IQ2N_LO, IQ2N_HI, c1[j] >> 16), bq.x, bq.y);
+            const int k0 = (int)((s0 >> (8 * j)) & 0xffu), k1 = (int)((s1 >> (8 * j)) & 0xffu);               // 2 * scale + 1
+            iacc[0] += c[0] * k0; iacc[1] += c[1] * k0; iacc[2] += c[2] * k1; iacc[3] += c[3] * k1;
+        }
+        const float d0 = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t *>(dd))) * 0.125f;
+        const float d1 = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t *>(dd + 32))) * 0.125f;
+        const float lo = 1.0f / 254.0f;
+        facc[0] += d0 * fmaf((float)iacc[1], lo, (float)iacc[0]);
+        facc[1] += d1 * fmaf((float)iacc[3], lo, (float)iacc[2]);
+    }
+};
+
 // Producer: stage one unit (unit_rows rows of each matrix).
-template <uint32_t TYPE>
+template <uint32_t TYPE, int MODE>
 __device__ __forceinline__ void produce_unit(const GroupedArgs &a, const Plan &p, uint8_t *stage, uint64_t *full, uint32_t expert,
                                              uint32_t row0, uint32_t lane) {
     const uint32_t nb = a.w0.k_storage >> 8, rows = p.unit_rows;
+    if (TYPE == T_IQ2N) {                                                // gate and up rows (or down rows) of the unit lie in one span
+        if (lane == 0) {
+            const uint32_t bytes = (MODE == 0 ? rows / 8 : rows / 16) * (nb >> 1) * IQ2N_BLOCK;
+            mbar_expect_tx(full, bytes);
+            bulk_copy(stage, a.expanded + ((uint64_t)expert * (a.w0.n_out / rows) + row0 / rows) * bytes, bytes, full);
+        }
+        return;
+    }
     const uint32_t row_bytes = nb * Fmt<TYPE>::BLOCK_BYTES;
     const bool contiguous = p.pitch == row_bytes;
     if (lane == 0) mbar_expect_tx(full, p.matrices * (rows * row_bytes + (TYPE == T_IQ2_XXS ? rows * nb * 2 : 0)));
@@ -337,7 +386,7 @@ __global__ void __launch_bounds__(NT, 1) grouped_mma_kernel(const GroupedArgs a)
             if (lane == 0 && u - u_begin >= p.n_stages) alive = mbar_wait(&empty[stage], phase ^ 1u, a.status);
             alive = __shfl_sync(0xffffffffu, alive, 0);
             if (!alive) break;
-            produce_unit<TYPE>(a, p, smem + p.stages + stage * p.stage_bytes, &full[stage], grp.expert,
+            produce_unit<TYPE, MODE>(a, p, smem + p.stages + stage * p.stage_bytes, &full[stage], grp.expert,
                                (u % units_per_group) * p.unit_rows, lane);
             if (++stage == p.n_stages) { stage = 0; phase ^= 1u; }
         }
@@ -371,7 +420,15 @@ __global__ void __launch_bounds__(NT, 1) grouped_mma_kernel(const GroupedArgs a)
         alive = __shfl_sync(0xffffffffu, alive, 0);
         const uint8_t *st = smem + p.stages + stage * p.stage_bytes;
         float facc[2] = {0.0f, 0.0f}, facc2[2] = {0.0f, 0.0f};
-        if (MODE == 0) {                                                 // warp = (matrix, k-slice of 8), both row tiles of the unit
+        if constexpr (TYPE == T_IQ2N) {
+            // gate/up: warp = (two of the unit's four blocks of 8 gate + 8 up rows, k-slice of 8); down: (row tile of 8, k-slice of 2)
+            const uint32_t nb5 = nb >> 1, rt = MODE == 0 ? (warp & 1u) * 2 : warp & 7u, next = MODE == 0 ? 1 : 8, slices = MODE == 0 ? 8 : 2;
+            if (alive)
+                for (uint32_t h = MODE == 0 ? warp >> 1 : warp >> 3; h < halves; h += slices) {
+                    Consume<TYPE>::half_block(st + (rt * nb5 + (h >> 2)) * IQ2N_BLOCK, p, act, h, g, t, facc);
+                    Consume<TYPE>::half_block(st + ((rt + next) * nb5 + (h >> 2)) * IQ2N_BLOCK, p, act, h, g, t, facc2);
+                }
+        } else if (MODE == 0) {                                          // warp = (matrix, k-slice of 8), both row tiles of the unit
             const uint32_t m = warp & 1u, ks = warp >> 1;
             if (alive)
                 for (uint32_t h = ks; h < halves; h += 8) {
@@ -403,7 +460,12 @@ __global__ void __launch_bounds__(NT, 1) grouped_mma_kernel(const GroupedArgs a)
                 const uint32_t row = tid >> 2, tok = tid & 3u;
                 float gsum = 0.0f, usum = 0.0f;
 #pragma unroll
-                for (int ks = 0; ks < 8; ks++) { gsum += part[(2 * ks) * 128 + tid]; usum += part[(2 * ks + 1) * 128 + tid]; }
+                for (int ks = 0; ks < 8; ks++) {
+                    if (TYPE == T_IQ2N) {                                // a block of 8 + 8 rows: gate in the first 32 values of a row tile, up in the next
+                        const float *from = part + (2 * ks + (row >> 4)) * 128 + ((row >> 3) & 1u) * 64 + (tid & 31u);
+                        gsum += from[0]; usum += from[32];
+                    } else { gsum += part[(2 * ks) * 128 + tid]; usum += part[(2 * ks + 1) * 128 + tid]; }
+                }
                 if (tok < count) {
                     const float dx = tokscale[tok];
                     gsum *= dx; usum *= dx;
@@ -685,17 +747,21 @@ static int launch_grouped(const GroupedArgs &a, int ctas, cudaStream_t stream) {
 }
 
 // mode 0: gate+up (w0, w1) -> out = act [pairs][n_out]; mode 1: down (w0) -> out [pairs][n_out].
-// Input rows are the quantised rows of quantize_rows (row = pair / k_div).
+// Input rows are the quantised rows of quantize_rows (row = pair / k_div).  expanded: the expanded image of an IQ2_XXS w0 (and w1), or nullptr.
 extern "C" int qw4sh_grouped_mma(int mode, const QW4ShTensor *w0, const QW4ShTensor *w1, const void *groups, const uint32_t *n_groups,
                                  const uint32_t *row_to_pair, uint32_t k_div, const int8_t *digits, const int8_t *negated,
-                                 const int *sums, const float *scale, float *out, uint32_t *status, int ctas, void *stream) {
+                                 const int *sums, const float *scale, float *out, uint32_t *status, int ctas, void *stream, const void *expanded) {
     GroupedArgs a;
     a.w0 = dev(*w0); a.w1 = dev(w1 ? *w1 : *w0);
     a.groups = (const VGroup *)groups; a.n_groups = n_groups; a.row_to_pair = row_to_pair; a.k_div = k_div;
     a.in.digits = digits; a.in.negated = negated; a.in.sums = sums; a.in.scale = scale;
-    a.lut = nullptr; a.out = out; a.status = status;
-    if (w0->type == T_IQ2_XXS && !(a.lut = lut_image())) return -3;
+    a.lut = nullptr; a.out = out; a.status = status; a.expanded = (const uint8_t *)expanded;
     cudaStream_t s = (cudaStream_t)stream;
+    // the expanded image where the layer holds one and two of its units fit (gate/up: K up to 2560; down: 512); always the faster one
+    if (w0->type == T_IQ2_XXS && expanded && w0->k_storage % 512 == 0 &&
+        (mode == 0 ? make_plan<T_IQ2N, 0>(w0->k_storage) : make_plan<T_IQ2N, 1>(w0->k_storage)).n_stages >= 2)
+        return mode == 0 ? launch_grouped<T_IQ2N, 0>(a, ctas, s) : launch_grouped<T_IQ2N, 1>(a, ctas, s);
+    if (w0->type == T_IQ2_XXS && !(a.lut = lut_image())) return -3;
     if (w0->type == T_Q4_K) return mode == 0 ? launch_grouped<T_Q4_K, 0>(a, ctas, s) : launch_grouped<T_Q4_K, 1>(a, ctas, s);
     return mode == 0 ? launch_grouped<T_IQ2_XXS, 0>(a, ctas, s) : launch_grouped<T_IQ2_XXS, 1>(a, ctas, s);
 }

@@ -1537,7 +1537,7 @@ extern "C" int qw4sh_stage_times(double *ms, uint64_t *forwards) {
 extern "C" int qw4sh_mma_supported(const QW4ShTensor *w, int mode);
 extern "C" int qw4sh_grouped_mma(int mode, const QW4ShTensor *w0, const QW4ShTensor *w1, const void *groups, const uint32_t *n_groups,
                                  const uint32_t *row_to_pair, uint32_t k_div, const int8_t *digits, const int8_t *negated,
-                                 const int *sums, const float *scale, float *out, uint32_t *status, int ctas, void *stream);
+                                 const int *sums, const float *scale, float *out, uint32_t *status, int ctas, void *stream, const void *expanded);
 extern "C" int qw4sh_quantize_rows(const float *x, uint32_t rows, uint32_t k, int8_t *xq, int8_t *xneg, int *xsum, float *xscale, void *stream);
 extern "C" int qw4sh_combine(const float *out, const float *shared_out, const float *weights, const float *shared_logit, uint32_t k,
                              uint32_t hidden, uint32_t tokens, float *y, float *routed, uint32_t *status, float *hc_residual,
@@ -1584,12 +1584,11 @@ static bool tile_path(const QW4ShLayer *layer, size_t tokens) {
     if (g_tile_path == 0 || g_expert_path == 0 || (g_tile_path > 0 && tokens <= 4)) return false;
     if (g_tile_path < 0) {
         if (prefill_path(layer, tokens)) return false;
-        // IQ2_XXS at up to 64 tokens: two table reads for eight weights bound its dequantiser (2000 cycles for 128 columns of 256
-        // rows), and where tokens spread evenly over 512 experts, a row or two to each, the four-row kernel's int8 table form is
-        // the faster one.  us a layer, four-row against tcgen05: 5 tokens 78 / 77, 16 130 / 132, 23 152 / 163, 32 177 / 188, 64 247 / 272,
-        // 96 302 / 306, 128 338 / 325.  Where they crowd onto few experts (Zipf 1.1) it is the slower one from the start, since a
-        // group is four rows: 5 tokens 68 / 60, 23 102 / 85, 64 162 / 102.  The host knows the tokens and not their routes, so the line
-        // is drawn for the even case.
+        // IQ2_XXS at up to 64 tokens: table reads bound its dequantiser (1480 cycles for 128 columns of 256 rows), and where tokens
+        // spread evenly over 512 experts, a row or two to each, the four-row kernels on the expanded image are the faster ones.  us a
+        // layer, four-row against tcgen05: 5 tokens 70 / 75, 8 81 / 90, 16 113 / 128, 23 129 / 159, 32 149 / 182, 64 199 / 252.  Where
+        // they crowd onto few experts (Zipf 1.1) they are the slower ones, since a group is four rows: 5 tokens 63 / 59, 23 91 / 81,
+        // 64 138 / 93.  The host knows the tokens and not their routes, so the line is drawn for the even case.
         if (mma_path(layer, tokens) && (g_expert_path == 1 || layer->w[1].type == T_IQ2_XXS)) return false;
     }
     return tc_routed(layer) && tc_shared(layer);
@@ -1692,7 +1691,7 @@ static int layer_launches(const QW4ShLayer *layer, const QW4ShWork *work, const 
         const int *sums = mode == 0 ? work->xsum : shared ? work->ssum : work->asum;
         const float *scale = mode == 0 ? work->xscale : shared ? work->sscale : work->ascale;
         return qw4sh_grouped_mma(mode, w0, w1, shared ? (void *)shared_groups : work->groups, work->n_groups + (shared ? 1 : 0), r2p, k_div, q, neg,
-                                 sums, scale, mode ? out : shared ? work->shared_act : work->act, work->status, ctas, strm);
+                                 sums, scale, mode ? out : shared ? work->shared_act : work->act, work->status, ctas, strm, layer->fused_alt[(shared ? 4 : 1) + (mode ? 2 : 0)]);
     };
     auto shared_branch = [&](int which) -> int {
         if (which == 0) {
@@ -1880,10 +1879,10 @@ static int ep_shared_begin(const QW4ShLayer *layer, const QW4ShWork *work, const
         if ((rc = qw4sh_quantize_rows(x, T, H, xq, xneg, xsum, xscale, side))) return rc;
         if ((rc = qw4sh_build_dense_groups(T, work->shared_groups, work->n_groups + 3, side))) return rc;
         if ((rc = qw4sh_grouped_mma(0, &layer->w[4], &layer->w[5], work->shared_groups, work->n_groups + 3, nullptr, 1, xq, xneg, xsum, xscale,
-                                    work->shared_act, work->status, ctas, side))) return rc;
+                                    work->shared_act, work->status, ctas, side, nullptr))) return rc;
         if ((rc = qw4sh_quantize_rows(work->shared_act, T, layer->shared_inter, work->sq, work->sneg, work->ssum, work->sscale, side))) return rc;
         if ((rc = qw4sh_grouped_mma(1, &layer->w[6], nullptr, work->shared_groups, work->n_groups + 3, nullptr, 1, work->sq, work->sneg, work->ssum,
-                                    work->sscale, work->shared_out, work->status, ctas, side))) return rc;
+                                    work->sscale, work->shared_out, work->status, ctas, side, nullptr))) return rc;
     }
     CU(cudaEventRecord(ev[3], side));
     return 0;
@@ -1973,13 +1972,13 @@ extern "C" int qw4sh_ep_experts(const QW4ShLayer *layer, const QW4ShWork *work, 
     } else {
         if ((rc = qw4sh_build_groups(offsets, active, work->groups, work->n_groups, stream))) return rc;
         if ((rc = qw4sh_grouped_mma(0, &layer->w[1], &layer->w[2], work->groups, work->n_groups, work->row_to_pair, k, work->xq, work->xneg,
-                                    work->xsum, work->xscale, work->act, work->status, ctas, stream))) return rc;
+                                    work->xsum, work->xscale, work->act, work->status, ctas, stream, nullptr))) return rc;
         if ((rc = qw4sh_ep_trace_mark(6, stream))) return rc;
         if ((rc = qw4sh_quantize_rows_listed(work->act, layer->inter, T * k, layer->inter, work->row_to_pair, row_begin, row_end, work->aq, work->aneg,
                                              work->asum, work->ascale, stream))) return rc;
         if ((rc = qw4sh_ep_trace_mark(7, stream))) return rc;
         if ((rc = qw4sh_grouped_mma(1, &layer->w[3], nullptr, work->groups, work->n_groups, work->row_to_pair, 1, work->aq, work->aneg,
-                                    work->asum, work->ascale, work->out, work->status, ctas, stream))) return rc;
+                                    work->asum, work->ascale, work->out, work->status, ctas, stream, nullptr))) return rc;
     }
     if ((rc = qw4sh_ep_trace_mark(8, stream))) return rc;
     if (own) {
