@@ -32,7 +32,8 @@
 //   C  streaming CTA sc owns 16 columns of y: its warps split the sources (shared expert +
 //      distinct routed experts), each runs the 16 x K down tile on the tensor cores against the
 //      digits of the pair's activation, scales by the route weight (or the sigmoid gate), and the
-//      partial sums are added in warp order: y is deterministic.
+//      partial sums are added in warp order: y is deterministic.  The digits and the first tiles are
+//      fetched under the comparison of the routes; a repair drops them.
 //
 // The kernel is launched as a normal grid of one CTA per SM with programmatic stream
 // serialisation: the next layer's launch may begin while this one drains, and everything that
@@ -53,7 +54,7 @@
 
 namespace qw4 {
 
-constexpr int FW = 12;                          // warps per CTA
+constexpr int FW = 12;                          // warps per CTA (with sixteen a Q4_K token takes 24.5 us a layer, with twelve 24.1; four tokens the same)
 constexpr int FT = FW * 32;
 constexpr int FTOK = 4;                         // tokens per launch
 constexpr int FMAXK = 16;                       // top-k limit
@@ -92,6 +93,7 @@ struct FusedArgs {
     uint32_t *status;
     uint32_t partial_slices;                    // capacity of the partial-sum buffer (slices per CTA)
     uint32_t chain_ctas;                        // NC
+    uint32_t clear;                             // see make_fplan
     long long t0;                               // (device side) this CTA's clock at its start
     HcAdd hc;                                   // hyper-connection add applied where y is written (residual nullptr: none)
     uint32_t *status_mirror;                    // pinned host words [4] that receive the status words at the end, or nullptr
@@ -104,7 +106,8 @@ struct Src {
     __device__ __forceinline__ uint32_t slot(uint32_t t) const { return (slots >> (8 * t)) & 0xffu; }
 };
 
-// Shared-memory plan of a streaming CTA (byte offsets), the same on host and device.  `region` is
+// Shared-memory plan of a streaming CTA (byte offsets), the same on host and device.  `clear`: phase C keeps clear of the digit image of x, so that
+// its first copies may be under way while it is still open whether phase B has to run again.  `region` is
 // reused by the three phases; the digit image of x lives at its start through phases A and B.
 struct FPlan {
     uint32_t bars, ids, wts, idx, wtx, misc, tokmask, slotmap, src, region, total;
@@ -114,7 +117,7 @@ struct FPlan {
     uint32_t zs, ring, partial;                 // phase B
     uint32_t aq, ap, asc, tiles, cpartial;      // phase C
 };
-__host__ __device__ inline FPlan make_fplan(uint32_t hidden, uint32_t inter_max, uint32_t rows_c, uint32_t partial_slices) {
+__host__ __device__ inline FPlan make_fplan(uint32_t hidden, uint32_t inter_max, uint32_t rows_c, uint32_t partial_slices, bool clear) {
     FPlan p;
     uint32_t at = 0;
     p.bars = at; at += 512;
@@ -145,7 +148,7 @@ __host__ __device__ inline FPlan make_fplan(uint32_t hidden, uint32_t inter_max,
     if (b < head + FTOK * FZP * 4) b = head + FTOK * FZP * 4;
     p.partial = b; b += partial_slices * 256;
     // phase C
-    uint32_t c = 0;
+    uint32_t c = clear ? head : 0;
     p.ap = inter_max + 32;
     p.aq = c; c += rows_c * 2 * p.ap;
     c = (c + 127) & ~127u;
@@ -242,19 +245,15 @@ __device__ __forceinline__ uint32_t lds_ring_u16(uint32_t a) {
 }
 // Thread 0 waits until *counter >= expected (bounded); the verdict reaches every thread.
 // False (CTA-uniform) when the wait ran out.
-__device__ __forceinline__ bool wait_counter(const uint32_t *counter, uint32_t expected, uint32_t *status, uint32_t *flag_smem) {
+__device__ __forceinline__ bool wait_counter(const uint32_t *counter, uint32_t expected, uint32_t *status) {
+    int ok = 1;
     if (threadIdx.x == 0) {
-        uint32_t ok = 1;
         const long long start = clock64();
         while (fld_acquire(counter) < expected) {
             if (clock64() - start > (1ll << 31)) { atomicOr(status, QW4SH_ERR_STATE); ok = 0; break; }
         }
-        *flag_smem = ok;
     }
-    __syncthreads();
-    const bool ok = *flag_smem != 0;
-    __syncthreads();
-    return ok;
+    return __syncthreads_and(ok) != 0;
 }
 // All threads' earlier global writes are ordered before one release increment.
 __device__ __forceinline__ void arrive_counter(uint32_t *counter) {
@@ -676,7 +675,6 @@ __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + p.bars);              // [CSTG]
     uint64_t *empty = full + CSTG;                                             // [CSTG]
     uint64_t *xbar = empty + CSTG;
-    uint32_t *misc_u = reinterpret_cast<uint32_t *>(smem + p.misc);
     const bool exact = a.router_mode != 1;
     if (tid < CSTG) { fbar_init(&full[tid], 1); fbar_init(&empty[tid], T); }
     if (tid == CSTG) fbar_init(xbar, 1);
@@ -773,7 +771,7 @@ __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
     // ---- routing of token `cta` ----
     const uint32_t waited = exact ? S_CHAIN : S_FAST;
     const uint32_t expected = exact ? a.chain_ctas : gridDim.x - a.chain_ctas;
-    bool ok = wait_counter(a.sync + waited, expected, a.status, misc_u);
+    bool ok = wait_counter(a.sync + waited, expected, a.status);
     if (ok) {
         const float *from = exact ? a.logits + (uint64_t)cta * E : a.logits_fast + (uint64_t)cta * a.fast_pitch;
         if (!exact) {
@@ -835,7 +833,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
 
     const uint32_t T = a.tokens, H = a.hidden, E = a.experts, k = a.top_k, I = a.inter, IS = a.shared_inter;
     const uint32_t pairs = T * k, rows_c = pairs + T, imax = I > IS ? I : IS;
-    const FPlan p = make_fplan(H, imax, rows_c, a.partial_slices);
+    const FPlan p = make_fplan(H, imax, rows_c, a.partial_slices, a.clear != 0);
     const uint32_t warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t sc = blockIdx.x - NC, NS = gridDim.x - NC;
     uint64_t *ringbar = reinterpret_cast<uint64_t *>(smem + p.bars);           // [FW][FNS], four single ones, then [FW][FNC]
@@ -973,7 +971,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
     arrive_counter(a.sync + S_FAST);                                          // (its CTA barrier also orders the reads of xf before the digits' consts)
     digitise_rows(reinterpret_cast<const float *>(xf), p.xf_pitch >> 2, T, H, misc_f, xq, p.kp, xsum, H >> 5, xconsts);
     CLOCK(3);
-    if (!wait_counter(a.sync + S_FAST, NS, a.status, misc_u)) return;
+    if (!wait_counter(a.sync + S_FAST, NS, a.status)) return;
     CLOCK(4);
     MARK(0);
 
@@ -1002,8 +1000,44 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
     CLOCK(5);
 
     uint32_t ring_count = 0;                                                   // slices this warp has pushed through its ring
+    // phase C: this warp's sources and (tile, source) steps, the next one to issue, steps and digit images read before (a repaired step comes here
+    // twice), and whether its first copies are on their way
+    uint8_t *aq = region + p.aq, *tiles = region + p.tiles + warp * FNC * FSTAGE;
+    float2 *asc = reinterpret_cast<float2 *>(region + p.asc);
+    uint32_t n_src = 0, my_src = 0, steps = 0, next_tile = 0, next_src = 0, tiles_read = 0, digits_read = 0;
+    bool begun = false;
+    auto issue_down = [&](uint32_t n) {                                        // in step order; the phase has ring barriers of its own
+        const uint32_t tile = next_tile, j = next_src, at = tiles_read + n;
+        next_src += FW;
+        if (next_src >= n_src) { next_src = warp; next_tile += NS; }
+        const Src s = srcs[j];
+        uint8_t *stage = tiles + (at % FNC) * FSTAGE;
+        if (s.shared) issue_down_tile<ST>(a.w[6].data, H, IS >> 8, tile * 16, stage, &tilebar[at % FNC], lane);
+        else issue_down_tile<RT>(a.w[3].data + (uint64_t)s.expert * a.w[3].expert_bytes, H, I >> 8, tile * 16, stage, &tilebar[at % FNC], lane);
+    };
+    const bool down_here = sc < (H >> 4);
+    auto begin_down = [&]() {                                                  // behind a CTA barrier: phase B's use of the region is over
+        if (!down_here || !lists_ok) return;
+        asm volatile("fence.proxy.async;" ::: "memory");                          // the digits were written through the generic proxy, by other CTAs
+        fproxy_fence();
+        const uint32_t aq_bytes = rows_c * 2u * p.ap, asc_bytes = rows_c * (imax >> 5) * 8u;
+        if (tid == 0) {
+            fbar_expect(abar, aq_bytes + asc_bytes);
+            fbulk(aq, a.aq, aq_bytes, abar);
+            fbulk(asc, a.asc, asc_bytes, abar);
+        }
+        alive = __all_sync(0xffffffffu, alive);
+        if (alive) for (uint32_t n = 0; n < FNC && n < steps; n++) issue_down(n);
+    };
+    auto drain_down = [&]() {                                                  // what begin_down sent for has landed, and is not wanted
+        if (!down_here || !lists_ok) return;
+        bool landed = fbar_wait(abar, digits_read & 1u, a.status);
+        const uint32_t sent = alive ? min(steps, (uint32_t)FNC) : 0;
+        for (uint32_t n = 0; n < sent; n++) landed &= fbar_wait(&tilebar[(tiles_read + n) % FNC], ((tiles_read + n) / FNC) & 1u, a.status);
+        digits_read++; tiles_read += sent;
+        alive = __all_sync(0xffffffffu, alive && landed);
+    };
     uint64_t *bar = ringbar + warp * FNS;
-    uint32_t n_src = 0;
     const uint32_t gs = IS >> 5, gr = I >> 5;                                  // granules (32 activation columns) per expert
     const uint32_t nbh = H >> 8;
     const uint32_t spu_s = nbh / FGeo<ST>::SLICE_BLOCKS, spu_r = nbh / FGeo<RT>::SLICE_BLOCKS;
@@ -1023,19 +1057,23 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 }
                 __syncwarp();
                 if (lane == 0) { Src s0; s0.expert = 0xffffu; s0.mask = (uint8_t)((1u << T) - 1u); s0.shared = 1; s0.slots = 0; srcs[0] = s0; }
-                uint32_t running = 1;
-#pragma unroll 4
-                for (uint32_t c = 0; c < (E + 31) / 32; c++) {
-                    const uint32_t e = c * 32 + lane;
-                    const bool has = e < E && tokmask[e] != 0;
-                    const uint32_t any = __ballot_sync(0xffffffffu, has);
-                    if (has) {
-                        Src sn; sn.expert = (uint16_t)e; sn.mask = tokmask[e]; sn.shared = 0;
-                        sn.slots = *reinterpret_cast<const uint32_t *>(slotmap + e * 4);
-                        srcs[running + __popc(any & ((1u << lane) - 1u))] = sn;
-                    }
-                    running += __popc(any);
+                // lane = sixteen experts in turn: which of them have tokens, the experts before them, then their entries one by one (one or two a lane;
+                // a ballot for every 32 experts took 3.2 k cycles, this half of that)
+                uint32_t mine = 0;
+                const uint4 marks = reinterpret_cast<const uint4 *>(tokmask)[lane];
+                const uint32_t word[4] = {marks.x, marks.y, marks.z, marks.w};
+#pragma unroll
+                for (uint32_t i = 0; i < 16; i++) mine |= ((word[i >> 2] >> (8 * (i & 3u))) & 0xffu ? 1u : 0u) << i;
+                uint32_t running = __popc(mine);
+                for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(0xffffffffu, running, o); if (lane >= (uint32_t)o) running += v; }
+                uint32_t at = 1 + running - __popc(mine);
+                for (uint32_t left = mine; left; left &= left - 1, at++) {
+                    const uint32_t e = lane * 16 + __ffs(left) - 1;
+                    Src sn; sn.expert = (uint16_t)e; sn.mask = tokmask[e]; sn.shared = 0;
+                    sn.slots = *reinterpret_cast<const uint32_t *>(slotmap + e * 4);
+                    srcs[at] = sn;
                 }
+                running = 1 + __shfl_sync(0xffffffffu, running, 31);
                 if (lane == 0) misc_u[2] = running;
             }
             __syncthreads();
@@ -1158,16 +1196,28 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
         CLOCK(8);
         __threadfence();
         arrive_counter(a.sync + (attempt ? S_ACT1 : S_ACT0));
-        if (!wait_counter(a.sync + (attempt ? S_ACT1 : S_ACT0), NS, a.status, misc_u)) return;
+        if (!wait_counter(a.sync + (attempt ? S_ACT1 : S_ACT0), NS, a.status)) return;
+        // ---- the first copies of phase C, which needs the activations alone: under the comparison below.  The digits and each warp's first tiles come
+        // from memory in 1.8 k cycles (one token) to 2.6 k (four), and behind the comparison nothing hid them: 97.6 -> 96.1 us for four Q4_K layers with
+        // one token, 154.0 -> 150.0 for four IQ2_XXS layers with four, together with the lists above.  (The products as well, before the routes are
+        // known, made it slower: their weights then arrive while the chains still read the router.) ----
+        my_src = n_src > warp ? (n_src - 1 - warp) / FW + 1 : 0;
+        steps = sc < (H >> 4) && lists_ok ? my_src * (((H >> 4) - sc + NS - 1) / NS) : 0;
+        next_tile = sc; next_src = warp;
+        begun = a.clear || attempt == 1;
+        if (begun) begin_down();
         if (attempt == 1) break;
-        if (!wait_counter(a.sync + S_ROUTED, T, a.status, misc_u)) return;
+        if (!wait_counter(a.sync + S_ROUTED, T, a.status)) { if (begun) drain_down(); return; }
         CLOCK(9);
         MARK(2);
-        if (fld_acquire(a.sync + S_ROUTE_FAIL)) { leave(); return; }             // a nonfinite logit: y stays untouched
         // ---- the exact routes against the speculation ----
         if (tid < pairs) { ids_x[tid] = __ldcg(a.ids + tid); wts_x[tid] = __ldcg(a.weights + tid); }
         if (tid < T) misc_f[4 + tid] = a.router_mode == 1 ? misc_f[4 + tid] : __ldcg(a.shared_logit + tid);
-        __syncthreads();
+        if (__syncthreads_or(tid == 0 && fld_acquire(a.sync + S_ROUTE_FAIL))) {        // a nonfinite logit: y stays untouched
+            if (begun) drain_down();
+            leave();
+            return;
+        }
         bool same = lists_ok;
         if (lists_ok && tid < pairs) same = ((tokmask[ids_x[tid]] >> (tid / k)) & 1u) != 0;   // k distinct ids on both sides: contained = equal
         same = __syncthreads_and(same);
@@ -1177,6 +1227,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
             break;
         }
         // repair: phase B again with the exact ids (every CTA takes this branch together: same data, same test)
+        if (begun) drain_down();
         if (tid < pairs) { ids_s[tid] = ids_x[tid]; wts_s[tid] = wts_x[tid]; }
         if (sc == 0 && tid == 0) atomicAdd(a.sync + S_REPAIRS, 1u);             // repaired launches since the workspace was cleared (diagnostic)
         lists_ok = __syncthreads_and(alive);
@@ -1185,36 +1236,15 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
 
     // ================================ phase C ================================
     if (sc < (H >> 4) && lists_ok) {
-        uint8_t *aq = region + p.aq;
-        float2 *asc = reinterpret_cast<float2 *>(region + p.asc);
-        uint8_t *tiles = region + p.tiles + warp * FNC * FSTAGE;
         float2 *cpartial = reinterpret_cast<float2 *>(region + p.cpartial);
-        const uint32_t my_src = n_src > warp ? (n_src - 1 - warp) / FW + 1 : 0;
         const uint32_t n_tiles = ((H >> 4) - sc + NS - 1) / NS;
-        const uint32_t steps = my_src * n_tiles;
-        uint32_t next_tile = sc, next_src = warp;                              // issues come in step order: the next step's tile and source
-        auto issue = [&](uint32_t n) {                                         // this phase has ring barriers of its own, counted from zero
-            const uint32_t tile = next_tile, j = next_src;
-            next_src += FW;
-            if (next_src >= n_src) { next_src = warp; next_tile += NS; }
-            const Src s = srcs[j];
-            uint8_t *stage = tiles + (n % FNC) * FSTAGE;
-            if (s.shared) issue_down_tile<ST>(a.w[6].data, H, IS >> 8, tile * 16, stage, &tilebar[n % FNC], lane);
-            else issue_down_tile<RT>(a.w[3].data + (uint64_t)s.expert * a.w[3].expert_bytes, H, I >> 8, tile * 16, stage, &tilebar[n % FNC], lane);
-        };
-        bool ok = __syncthreads_and(alive);                                    // also: phase B's use of the region is over
-        if (ok) {
-            asm volatile("fence.proxy.async;" ::: "memory");                      // the digits were written through the generic proxy, by other CTAs
-            fproxy_fence();
-            const uint32_t aq_bytes = rows_c * 2u * p.ap, asc_bytes = rows_c * (imax >> 5) * 8u;
-            if (tid == 0) {
-                fbar_expect(abar, aq_bytes + asc_bytes);
-                fbulk(aq, a.aq, aq_bytes, abar);
-                fbulk(asc, a.asc, asc_bytes, abar);
-            }
-            for (uint32_t n = 0; n < FNC && n < steps; n++) issue(n);
-            ok = __syncthreads_and(fbar_wait(abar, 0, a.status));
+        if (!begun) {
+            __syncthreads();                                                   // phase B's use of the region is over
+            begin_down();
         }
+        bool ok = __syncthreads_and(alive);
+        if (ok) ok = __syncthreads_and(fbar_wait(abar, digits_read & 1u, a.status));
+        if (!ok) drain_down();
         alive = ok;
         CLOCK(11);
         uint32_t n = 0;
@@ -1231,9 +1261,10 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 const uint32_t row_t = s.shared ? pairs + (t < T ? t : 0) : (live_t ? t * k + s.slot(t) : 0);
                 const uint8_t *aq_lane = aq + (2 * row_g + (g & 1u)) * p.ap + 8 * t;
                 const float2 *asc_tok = asc + row_t * (imax >> 5);
-                if (alive) alive = fbar_wait(&tilebar[n % FNC], (n / FNC) & 1u, a.status);
+                const uint32_t at = tiles_read + n;
+                if (alive) alive = fbar_wait(&tilebar[at % FNC], (at / FNC) & 1u, a.status);
                 alive = __all_sync(0xffffffffu, alive);
-                const uint8_t *stage = tiles + (n % FNC) * FSTAGE;
+                const uint8_t *stage = tiles + (at % FNC) * FSTAGE;
                 float f0 = 0.0f, f1 = 0.0f;
                 if (alive) {
                     if (s.shared) consume_down_tile<ST>(stage, IS >> 8, aq_lane, asc_tok, g, t, f0, f1);
@@ -1241,7 +1272,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 }
                 __syncwarp();
                 fproxy_fence();
-                if (alive && n + FNC < steps) issue(n + FNC);
+                if (alive && n + FNC < steps) issue_down(n + FNC);
                 if (live_t) {
                     const float coef = s.shared ? fast_sigmoid(misc_f[4 + t]) : wts_s[t * k + s.slot(t)];
                     acc0 = fmaf(coef, f0, acc0); acc1 = fmaf(coef, f1, acc1);
@@ -1310,9 +1341,13 @@ static uint32_t partial_capacity(const QW4ShLayer *l, size_t tokens, uint32_t st
     return per_cta * 4 * (spu_s > spu_r ? spu_s : spu_r);
 }
 
-static FPlan plan_for(const QW4ShLayer *l, size_t tokens, uint32_t streaming) {
-    const uint32_t imax = l->inter > l->shared_inter ? l->inter : l->shared_inter;
-    return make_fplan(l->hidden, imax, (uint32_t)tokens * l->top_k + (uint32_t)tokens, partial_capacity(l, tokens, streaming));
+// Phase C clear of the digit image of x where there is room: everywhere but at hidden 4096 with four tokens and more than fifteen experts each, where
+// the two lie over each other and phase C's first copies wait for the comparison.
+static FPlan plan_for(const QW4ShLayer *l, size_t tokens, uint32_t streaming, bool *clear) {
+    const uint32_t imax = l->inter > l->shared_inter ? l->inter : l->shared_inter, rows = (uint32_t)tokens * l->top_k + (uint32_t)tokens;
+    const FPlan p = make_fplan(l->hidden, imax, rows, partial_capacity(l, tokens, streaming), true);
+    *clear = p.total <= 227u * 1024u - 1024u;
+    return *clear ? p : make_fplan(l->hidden, imax, rows, partial_capacity(l, tokens, streaming), false);
 }
 
 // Bytes of the workspace arrays the kernel needs beyond the common ones (for `cap` tokens, at most FTOK used).
@@ -1438,7 +1473,8 @@ extern "C" int qw4sh_fused_supported(const QW4ShLayer *l, size_t tokens, const f
     if (grid < 1 || (uint32_t)grid <= nc) return 0;
     const uint32_t streaming = (uint32_t)grid - nc;
     if (streaming * FRMAX < l->experts + 1) return 0;
-    if (plan_for(l, tokens, streaming).total > 227u * 1024u || make_cplan(H).total > 227u * 1024u) return 0;
+    bool clear;
+    if (plan_for(l, tokens, streaming, &clear).total > 227u * 1024u || make_cplan(H).total > 227u * 1024u) return 0;
     return 1;
 }
 
@@ -1489,7 +1525,9 @@ extern "C" int qw4sh_fused_decode(const QW4ShLayer *layer, const QW4ShWork *work
     const uint32_t streaming = (uint32_t)sm_count - chain_ctas(layer, tokens, 0);     // the same split in every mode (plans, capacity)
     a.chain_ctas = (uint32_t)sm_count - streaming;
     a.partial_slices = partial_capacity(layer, tokens, streaming);
-    const FPlan p = plan_for(layer, tokens, streaming);
+    bool clear;
+    const FPlan p = plan_for(layer, tokens, streaming, &clear);
+    a.clear = clear;
     const CPlan c = make_cplan(layer->hidden);
     const uint32_t smem = p.total > c.total ? p.total : c.total;
     if (smem > 227u * 1024u - 1024u) return -4;

@@ -114,3 +114,30 @@ def test_nonfinite_logit_leaves_outputs_untouched(gpu):
             layer.forward(x)
         assert info.value.status == abi.NONFINITE
         layer.reset()
+
+
+@pytest.mark.parametrize("routed,tokens,top_k", [(12, 4, 15), (12, 4, 16), (16, 4, 16), (16, 1, 16)])
+def test_first_down_copies_at_the_largest_hidden_size(gpu, routed, tokens, top_k):
+    """Hidden 4096: with four tokens and sixteen experts each, shared memory has no room for the down
+    phase beside the digits of x, and its first copies wait for the comparison of the routes; with
+    fifteen, or one token, they are under way before it and are taken in and dropped by a repair."""
+    import oracle
+    from picoforge_b200 import synth
+    from picoforge_b200.layer import MoeLayer
+    spec = synth.make_layer(900 + routed + top_k, routed_type=routed, shared_type=12, hidden=4096, experts=64, top_k=top_k)
+    x = synth.activations(900 + tokens, tokens, 4096)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    repairs = C.c_uint32()
+    with MoeLayer(gpu, spec, tokens) as layer:
+        for wrong in (0, 1, 0):
+            gpu.lib.qw4cu_set_decode_wrong_speculation(wrong)
+            gpu.lib.qw4cu_launch_log_begin()
+            try:
+                y, ids, weights = layer.forward(x)
+            finally:
+                gpu.lib.qw4cu_set_decode_wrong_speculation(0)
+            assert gpu.launch_names() == ["fused_decode_kernel"]
+            np.testing.assert_array_equal(ids, want["ids"])
+            np.testing.assert_array_equal(weights, want["weights"])
+            assert np.abs(y - want["y"]).max() <= Y_TOLERANCE
+        assert gpu.lib.qw4cu_decode_repairs(layer.work, C.byref(repairs)) == 0 and repairs.value == 1
