@@ -255,7 +255,7 @@ __device__ __forceinline__ bool wait_counter(const uint32_t *counter, uint32_t e
     }
     return __syncthreads_and(ok) != 0;
 }
-// All threads' earlier global writes are ordered before one release increment.
+// All threads' earlier global writes are ordered before one release increment (the barrier puts them before it, and a release is cumulative).
 __device__ __forceinline__ void arrive_counter(uint32_t *counter) {
     __syncthreads();
     if (threadIdx.x == 0) fred_release(counter);
@@ -622,23 +622,22 @@ __device__ __forceinline__ float fast_sigmoid(float v) {
     return v >= 0.0f ? __fdividef(1.0f, 1.0f + e) : __fdividef(e, 1.0f + e);
 }
 
-// The k largest of one row of logits by VALUE (ties to the lower id), one warp; the row is turned
-// read into ordered integer keys (its memory then serves as scratch).  `extra`: choose k + 1 and put the last one in slot k - 1 (a
+// The k largest of one row of logits by VALUE (ties to the lower id), one warp.  The row is read straight from global memory into ordered integer
+// keys: through a bulk copy into shared memory the same round trip took 1.8 k cycles instead of 0.7 (90.4 against 93.4 us for four Q4_K layers of one
+// token).  cand: 256 words of scratch.  `extra`: choose k + 1 and put the last one in slot k - 1 (a
 // deliberately wrong set, for the test of the repair path).  Returns false on a nonfinite logit.
-__device__ __forceinline__ bool speculate_row(float *zs, uint32_t E, uint32_t k, bool extra, uint32_t *ids_s, uint32_t lane) {
+__device__ __forceinline__ bool speculate_row(const float *logits, uint32_t *cand, uint32_t E, uint32_t k, bool extra, uint32_t *ids_s, uint32_t lane) {
     constexpr int PL = FMAXE / 32;
     uint32_t key[PL];
     bool bad = false;
 #pragma unroll
     for (int i = 0; i < PL; i++) {
         const uint32_t e = lane + 32u * i;
-        const uint32_t u = e < E ? __float_as_uint(zs[e]) : 0u;
+        const uint32_t u = e < E ? __float_as_uint(__ldcg(logits + e)) : 0u;
         bad |= e < E && (u & 0x7f800000u) == 0x7f800000u;
         key[i] = e < E ? ((u & 0x80000000u) ? ~u : (u | 0x80000000u)) : 0u;      // monotone in the value, never 0
     }
     if (__any_sync(0xffffffffu, bad)) return false;
-    __syncwarp();
-    uint32_t *cand = reinterpret_cast<uint32_t *>(zs);                          // the row is in registers now
     const uint32_t want = extra && k < E ? k + 1 : k;
     uint32_t *out = extra ? cand + 128 : ids_s;
     if (!warp_topk<PL>(key, lane, want, cand, out, nullptr)) warp_topk_sequential<PL>(key, lane, want, out, nullptr);
@@ -788,7 +787,6 @@ __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
                             }) == 0;
     }
     if (!ok && tid == 0) atomicOr(a.sync + S_ROUTE_FAIL, 1u);
-    __threadfence();
     arrive_counter(a.sync + S_ROUTED);
     MARK(1);
 }
@@ -841,7 +839,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
     uint64_t *tilebar = ringbar + FW * FNS + 4 + (threadIdx.x >> 5) * FNC;     // this warp's barriers of the down phase
     static_assert((FW * FNS + 4 + FW * FNC) * 8 <= 512, "the barrier block is 512 bytes");
     uint64_t *lutbar = rowbar + 1;
-    uint64_t *xbar = lutbar + 1;                                               // x rows (phase A), then the fast logits (phase B)
+    uint64_t *xbar = lutbar + 1;                                               // x rows (phase A)
     uint64_t *abar = xbar + 1;                                                 // activation digits (phase C)
     uint32_t *ids_s = reinterpret_cast<uint32_t *>(smem + p.ids);              // the ids phase B works with
     float *wts_s = reinterpret_cast<float *>(smem + p.wts);                    // exact weights in the order of ids_s
@@ -968,6 +966,9 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
         a.logits_fast[(uint64_t)(tid % FTOK) * a.fast_pitch + sc + (tid / FTOK) * NS] = v;
     }
     CLOCK(2);
+    if (tid < FMAXE / 4) reinterpret_cast<uint32_t *>(tokmask)[tid] = 0;      // for the lists
+    static_assert(FMAXE / 4 <= FT, "one word a thread");
+    if (tid == 0) misc_u[1] = 1;                                               // the guess is usable
     arrive_counter(a.sync + S_FAST);                                          // (its CTA barrier also orders the reads of xf before the digits' consts)
     digitise_rows(reinterpret_cast<const float *>(xf), p.xf_pitch >> 2, T, H, misc_f, xq, p.kp, xsum, H >> 5, xconsts);
     CLOCK(3);
@@ -977,24 +978,13 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
 
     // ================================ phase B ================================
     float *zs = reinterpret_cast<float *>(region + p.zs);
-    if (warp == 0 && alive) {
-        asm volatile("fence.proxy.async;" ::: "memory");                          // generic-proxy writes (the logits; phase A's use of this memory) before the copy
-        if (lane == 0) fbar_expect(xbar, T * a.fast_pitch * 4u);
-        __syncwarp();
-        if (lane < T) fbulk(zs + lane * FZP, a.logits_fast + (uint64_t)lane * a.fast_pitch, a.fast_pitch * 4u, xbar);
-    }
-    if (alive) alive = fbar_wait(xbar, 1, a.status);                           // second use of this barrier: phase parity 1
-    CLOCK(13);
-    if (tid == 0) misc_u[1] = 1;
-    __syncthreads();
     if (warp < T) {
-        if (a.router_mode == 1 && lane == 0) misc_f[4 + warp] = zs[warp * FZP + E];     // the shared router's tree sum
-        CLOCK(14);
-        const bool fine = speculate_row(zs + warp * FZP, E, k, a.router_mode == 2 && warp == 0, ids_s + warp * k, lane);
+        const float *logits = a.logits_fast + (uint64_t)warp * a.fast_pitch;
+        if (a.router_mode == 1 && lane == 0) misc_f[4 + warp] = __ldcg(logits + E);     // the shared router's tree sum
+        const bool fine = speculate_row(logits, reinterpret_cast<uint32_t *>(zs + warp * FZP), E, k, a.router_mode == 2 && warp == 0, ids_s + warp * k, lane);
         if (!fine && lane == 0) misc_u[1] = 0;
         CLOCK(15);
     }
-    __syncthreads();
     const bool all_alive = __syncthreads_and(alive);
     bool lists_ok = misc_u[1] != 0 && all_alive;
     CLOCK(5);
@@ -1047,9 +1037,6 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
         if (lists_ok) {
             if (warp == 0) {                                                   // one warp, warp-level synchronisation only
 #pragma unroll 1
-                for (uint32_t i = lane; i < FMAXE / 4; i += 32) reinterpret_cast<uint32_t *>(tokmask)[i] = 0;
-                __syncwarp();
-#pragma unroll 1
                 for (uint32_t pr = lane; pr < pairs; pr += 32) {
                     const uint32_t e = ids_s[pr], tok = pr / k;
                     atomicOr(reinterpret_cast<uint32_t *>(tokmask) + (e >> 2), (1u << tok) << (8 * (e & 3u)));
@@ -1058,7 +1045,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 __syncwarp();
                 if (lane == 0) { Src s0; s0.expert = 0xffffu; s0.mask = (uint8_t)((1u << T) - 1u); s0.shared = 1; s0.slots = 0; srcs[0] = s0; }
                 // lane = sixteen experts in turn: which of them have tokens, the experts before them, then their entries one by one (one or two a lane;
-                // a ballot for every 32 experts took 3.2 k cycles, this half of that)
+                // a ballot for every 32 experts took 3.2 k cycles, this 1.1 k)
                 uint32_t mine = 0;
                 const uint4 marks = reinterpret_cast<const uint4 *>(tokmask)[lane];
                 const uint32_t word[4] = {marks.x, marks.y, marks.z, marks.w};
@@ -1136,7 +1123,8 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 const uint8_t *stage = ring + (at % FNS) * FSTAGE;
                 float f0 = 0.0f, f1 = 0.0f;
                 if (alive) {
-                    if (sh) consume_unit_slice<ST>(stage, nbh, s, xq_lane, xsum_tok, g, t, f0, f1);
+                    // one copy of the code where the formats are the same: what a phase costs at one token is partly its code's first fetch
+                    if (RT != ST && sh) consume_unit_slice<ST>(stage, nbh, s, xq_lane, xsum_tok, g, t, f0, f1);
                     else consume_unit_slice<RT>(stage, nbh, s, xq_lane, xsum_tok, g, t, f0, f1);
                 }
                 partial[(warp + i * FW) * 32 + lane] = make_float2(f0, f1);
@@ -1148,7 +1136,8 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
             CLOCK(7);
             MARK(1);
             __syncthreads();
-            // granules: slices added in order, SwiGLU, digit pairs with one scale per chunk
+            // granules: slices added in order (the four units' sums side by side, or each read's latency shows: 89.3 against 90.4 us), SwiGLU, digit
+            // pairs with one scale per chunk
 #pragma unroll 1
             for (uint32_t gl = warp; gl < g1 - g0; gl += FW) {
                 const bool sh = gl < n_shg;
@@ -1158,19 +1147,19 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 const uint32_t chunk = sh ? gi : (gi - gs) % gr;
                 const bool live = t < T && ((sr.mask >> t) & 1u);
                 const uint32_t row = sh ? pairs + t : t * k + sr.slot(t);
-                float v[4];
+                float v[4], f0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, f1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 float m = 0.0f;
-                bool whole = true;
+                const uint32_t n0 = sh ? gl * 4 * spu_s : n_shu * spu_s + (gl * 4 - n_shu) * spu_r;
+                const bool whole = n0 + 4 * spu <= slices;                         // beyond the partial buffer: never for supported shapes
+                const float2 *from = partial + n0 * 32 + lane;
+#pragma unroll 1
+                for (uint32_t s = 0; s < spu && whole; s++)
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; u++) { const float2 q = from[(u * spu + s) * 32]; f0[u] += q.x; f1[u] += q.y; }
+                const float dx = misc_f[t];
 #pragma unroll
                 for (uint32_t u = 0; u < 4; u++) {
-                    const uint32_t ul = gl * 4 + u;
-                    const uint32_t n0 = sh ? ul * spu_s : n_shu * spu_s + (ul - n_shu) * spu_r;
-                    whole &= n0 + spu <= slices;                                   // beyond the partial buffer (never for supported shapes)
-                    float f0 = 0.0f, f1 = 0.0f;
-#pragma unroll 1
-                    for (uint32_t s = 0; s < spu && whole; s++) { const float2 q = partial[(n0 + s) * 32 + lane]; f0 += q.x; f1 += q.y; }
-                    const float dx = misc_f[t];
-                    const float gate = f0 * dx, upv = f1 * dx;
+                    const float gate = f0[u] * dx, upv = f1[u] * dx;
                     v[u] = live ? gate * fast_sigmoid(gate) * upv : 0.0f;
                     m = fmaxf(m, fabsf(v[u]));
                 }
@@ -1194,7 +1183,6 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
             }
         }
         CLOCK(8);
-        __threadfence();
         arrive_counter(a.sync + (attempt ? S_ACT1 : S_ACT0));
         if (!wait_counter(a.sync + (attempt ? S_ACT1 : S_ACT0), NS, a.status)) return;
         // ---- the first copies of phase C, which needs the activations alone: under the comparison below.  The digits and each warp's first tiles come
@@ -1211,9 +1199,15 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
         CLOCK(9);
         MARK(2);
         // ---- the exact routes against the speculation ----
-        if (tid < pairs) { ids_x[tid] = __ldcg(a.ids + tid); wts_x[tid] = __ldcg(a.weights + tid); }
-        if (tid < T) misc_f[4 + tid] = a.router_mode == 1 ? misc_f[4 + tid] : __ldcg(a.shared_logit + tid);
-        if (__syncthreads_or(tid == 0 && fld_acquire(a.sync + S_ROUTE_FAIL))) {        // a nonfinite logit: y stays untouched
+        // all words in one round trip (thread 0's acquire above and the barrier behind it order them for every thread); ids, logits and the flag one
+        // after another took 2.5 k cycles, this 1.4 k: 93.3 against 96.4 us, four IQ2_XXS tokens 146.9 against 150.8
+        const bool takes_logit = tid >= 64 && tid < 64 + T && a.router_mode != 1;
+        const uint32_t my_id = tid < pairs ? __ldcg(a.ids + tid) : 0;
+        const float my_weight = tid < pairs ? __ldcg(a.weights + tid) : takes_logit ? __ldcg(a.shared_logit + tid - 64) : 0.0f;
+        const uint32_t failed = tid == FT - 1 ? __ldcg(a.sync + S_ROUTE_FAIL) : 0;
+        if (tid < pairs) { ids_x[tid] = my_id; wts_x[tid] = my_weight; }
+        if (takes_logit) misc_f[4 + tid - 64] = my_weight;
+        if (__syncthreads_or(failed != 0)) {                                          // a nonfinite logit: y stays untouched
             if (begun) drain_down();
             leave();
             return;
@@ -1229,6 +1223,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
         // repair: phase B again with the exact ids (every CTA takes this branch together: same data, same test)
         if (begun) drain_down();
         if (tid < pairs) { ids_s[tid] = ids_x[tid]; wts_s[tid] = wts_x[tid]; }
+        if (tid < FMAXE / 4) reinterpret_cast<uint32_t *>(tokmask)[tid] = 0;
         if (sc == 0 && tid == 0) atomicAdd(a.sync + S_REPAIRS, 1u);             // repaired launches since the workspace was cleared (diagnostic)
         lists_ok = __syncthreads_and(alive);
     }
@@ -1267,8 +1262,8 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 const uint8_t *stage = tiles + (at % FNC) * FSTAGE;
                 float f0 = 0.0f, f1 = 0.0f;
                 if (alive) {
-                    if (s.shared) consume_down_tile<ST>(stage, IS >> 8, aq_lane, asc_tok, g, t, f0, f1);
-                    else consume_down_tile<RT>(stage, I >> 8, aq_lane, asc_tok, g, t, f0, f1);
+                    if (RT != ST && s.shared) consume_down_tile<ST>(stage, IS >> 8, aq_lane, asc_tok, g, t, f0, f1);
+                    else consume_down_tile<RT>(stage, (s.shared ? IS : I) >> 8, aq_lane, asc_tok, g, t, f0, f1);
                 }
                 __syncwarp();
                 fproxy_fence();
@@ -1283,11 +1278,9 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
             if (tid < 64) {                                                    // rows g (threads 0-31) and g + 8 (32-63), warps added in order
                 const uint32_t l = tid & 31u, gg = l >> 2, tt = l & 3u, hi = tid >> 5;
                 float sum = 0.0f;
-#pragma unroll 1
-                for (uint32_t w = 0; w < FW; w++) {
-                    const float2 v = cpartial[w * 32 + l];
-                    sum += hi ? v.y : v.x;
-                }
+                const float *from = reinterpret_cast<const float *>(cpartial) + 2 * l + hi;
+#pragma unroll
+                for (uint32_t w = 0; w < FW; w++) sum += from[w * 64];
                 if (tt < T && alive) {
                     if (!finite_f32(sum)) atomicOr(a.status, QW4SH_ERR_NONFINITE);
                     a.y[(uint64_t)tt * H + tile * 16 + hi * 8 + gg] = sum;

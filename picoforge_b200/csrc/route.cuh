@@ -72,7 +72,7 @@ __device__ __forceinline__ uint32_t topk_bound(const uint32_t (&key)[PL], uint32
 #pragma unroll
     for (int i = 0; i < PL; i++) m = max(m, key[i]);
     uint32_t ahead = 0;                                                     // lanes whose maximum beats this lane's
-#pragma unroll
+#pragma unroll 8                                                              // all 32 at once: 1% slower in the decode kernel, whose code is fetched cold
     for (int j = 0; j < 32; j++) {
         const uint32_t v = __shfl_sync(0xffffffffu, m, j);
         ahead += (v > m || (v == m && (uint32_t)j < lane)) ? 1u : 0u;
@@ -212,10 +212,9 @@ __device__ __forceinline__ uint32_t route_rows(uint32_t row0, uint32_t rows, uin
     if (tid < 32) s.table[tid] = c_exp2_table[tid];
     if (tid == 0) s.bad = 0;
     const uint32_t per_row = NW / rows, r = warp / per_row, sub = warp % per_row;          // warps on one row (rows <= NW)
-    float m = -CUDART_INF_F;
+    float m = -CUDART_INF_F, z[PL];
     bool bad = false;
     if (r < rows) {
-        float z[PL];
 #pragma unroll
         for (int i = 0; i < PL; i++) { const uint32_t e = lane + 32u * i; z[i] = e < E ? load(row0 + r, e) : -CUDART_INF_F; }
 #pragma unroll
@@ -229,7 +228,10 @@ __device__ __forceinline__ uint32_t route_rows(uint32_t row0, uint32_t rows, uin
 #pragma unroll 1
         for (uint32_t i = sub; i < PL; i += per_row) {
             const uint32_t e = lane + 32u * i;
-            es[r * RT_PITCH + e] = e < E && !bad ? expf_libm_table(__fsub_rn(load(row0 + r, e), m), s.table) : 0.0f;
+            float zi = z[0];                                     // register i: sixteen selects, where a second read of the logit is a round trip to L2
+#pragma unroll
+            for (int j = 1; j < PL; j++) zi = i == (uint32_t)j ? z[j] : zi;
+            es[r * RT_PITCH + e] = e < E && !bad ? expf_libm_table(__fsub_rn(zi, m), s.table) : 0.0f;
         }
     __syncthreads();
     const uint32_t bad_rows = s.bad;
