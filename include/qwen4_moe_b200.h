@@ -374,7 +374,8 @@ void qw4cu_set_expert_path(int path);
  * route weights are always the exact mode's.  -1 (default): used whenever the layer fits it; 0:
  * never (the multi-kernel sequence runs instead).  A layer that fits this path holds, for each of
  * its IQ2_XXS expert tensors, a second resident image made at create (3-bit codes, 3.3 bits per
- * weight: the kernel streams that one; same decoded values); qw4cu_moe_device_bytes counts it.
+ * weight: the kernel streams that one, and the four-row kernels read it too; same decoded values);
+ * qw4cu_moe_device_bytes counts it.
  * A layer created while mode 0 is in force gets neither the image nor the path, whatever the mode later.
  * qw4cu_decode_phase_clocks copies the SM clock that the first streaming CTA of the workspace's
  * last one-kernel launch read at its phase boundaries into clocks[0..12] (start, x staged, fast
@@ -403,7 +404,8 @@ void qw4cu_prefill_debug(void *device_words);
 int qw4cu_decode_phase_clocks(const Qwen4MoeWork *work, uint64_t clocks[16]);
 int qw4cu_decode_repairs(const Qwen4MoeWork *work, uint32_t *count);
 /* Profiling aid: the first `words` (<= 1024) 32-bit words of the one-kernel path's counter block: counters,
- * phase clocks, and from word 256 four marks per CTA (cycles since that CTA started). */
+ * phase clocks, and from word 256 four marks per CTA (cycles since that CTA started; zeros unless the
+ * library was built with QW4_PHASE_MARKS, since the marks cost the kernel 1%). */
 int qw4cu_decode_debug_words(const Qwen4MoeWork *work, uint32_t *out, size_t words);
 void qw4cu_set_decode_wrong_speculation(int on);
 /* Profiling aid: launch only one step of the small-batch sequence on later forwards, so that a
@@ -432,7 +434,7 @@ size_t qw4cu_launch_log(char *out, size_t cap);
 Qwen4Status qw4cu_moe_decode_rows(const Qwen4Moe *moe, uint32_t tensor, size_t expert,
                                   size_t row0, size_t rows, float *out, size_t out_elements,
                                   Qwen4Error *err);
-/* The same from the EXPANDED image that the one-kernel decode path streams for an IQ2_XXS expert tensor
+/* The same from the EXPANDED image that the one-kernel decode path and the four-row kernels stream for an IQ2_XXS expert tensor
  * (tensor 1-6); QW4_UNSUPPORTED when the tensor has none (another format, or a layer that does not fit
  * that path). */
 Qwen4Status qw4cu_moe_decode_rows_expanded(const Qwen4Moe *moe, uint32_t tensor, size_t expert,
