@@ -37,7 +37,7 @@ typedef struct {
      * qw4sh_fused_prepare once the images are resident; ready = 0 when the layer does not fit that path */
     unsigned char fused_maps[4][128];
     int fused_maps_ready;
-    /* the same path: expanded images (3-bit codes) of the IQ2_XXS expert tensors, owned by the layer */
+    /* the same path: expanded images (3-bit codes) of the IQ2_XXS expert tensors, owned by the layer; the four-row kernels read them too */
     void *fused_alt[8];
     size_t fused_alt_bytes;
 } QW4ShLayer;
@@ -224,7 +224,7 @@ void qw4sh_tile_release(QW4ShLayer *layer);
 void qw4sh_set_tile_path(int path);         /* -1 automatic (default), 0 never, 1 every batch of > 4 rows */
 void qw4sh_set_prefill_path(int path);      /* -1 automatic (default), 0 never */
 /* Profiling aid: device array of 64 x 8 bytes (or NULL); CTA 0 of later launches stores the cycles its five roles spent in
- * their waits: [32 * mode + 4 * role + kind], kind 3 = the role's total. */
+ * waits that were not over at once: [32 * mode + 4 * role + kind], kind 3 = the role's total. */
 void qw4sh_prefill_debug(void *device_words);
 int qw4sh_split_rows(const float *x, uint32_t pitch, uint32_t rows, uint32_t k, const QW4ShSplit *to, void *stream);
 int qw4sh_build_tile_groups(const uint32_t *offsets, const uint32_t *active, void *groups, uint32_t *n_groups, void *stream);
