@@ -269,15 +269,18 @@ __device__ __forceinline__ __half2 xbytes2(uint32_t v, uint32_t i, uint32_t j) {
 // word(): what the read-back multiplies by, {d, dmin} or a float.
 template <uint32_t F> struct XDeq;
 
-// Codes masked out in place ARE halves, subnormal ones: a code at bit b of its half is code * 2^(b - 24), and times s * 2^(4 - b) it
-// becomes s * code * 2^-20, exactly; the 2^20 goes to the FP32 scale of the read-back.  One logic operation with an immediate (one
+// Codes masked out in place ARE halves, subnormal ones: a code at bit b of its half is code * 2^(b - 24), and times s * 2^(10 - b) it
+// becomes s * code * 2^-14, exactly; the 2^14 goes to the FP32 scale of the read-back.  One logic operation with an immediate (one
 // cycle a warp instruction; with three registers two) and one multiply (two cycles) per two weights.
-constexpr float XUP = 1048576.0f;
+// 2^-14 makes every operand that is not zero a normal half.  With 2^-20 the multipliers come out of one fused multiply-add instead of a
+// subtraction and a product, but the operands (all of Q2_K's, many of Q4_K's) are subnormal: as exact, yet the tensor core then adds the
+// same products with other last bits (1e-7 of the result on Q2_K, 1.6e-8 on Q4_K; with 2^-14 the same bits whatever else the kernel
+// does).  RMS error of y against 64 bits, 2^-14 and 2^-20: Q2_K 1.5435e-6 and 1.5425e-6 (1024 tokens), 1.9594e-6 and 1.9586e-6 (7), Q4_K
+// 1.6450e-6 and 1.6452e-6 (64), 2.0619e-6 and 2.0622e-6 (333, rows with outliers); time the same within its spread.
+constexpr float XUP = 16384.0f;
 __device__ __forceinline__ uint32_t xfold(uint32_t bits, __half2 mul) { return xu32(__hmul2(xh2(bits), mul)); }
-// byte i of `v` (at most 63) times `up`, in both halves: out of 1024 + byte with one fused multiply-add
-__device__ __forceinline__ __half2 xscaled(uint32_t v, uint32_t i, float up) {
-    return __hfma2(xh2(__byte_perm(v, 0x64646464u, 0x4040u | i | (i << 8))), __float2half2_rn(up), __float2half2_rn(-1024.0f * up));
-}
+// byte i of `v` (at most 63) times `up` (a power of two), in both halves
+__device__ __forceinline__ __half2 xscaled(uint32_t v, uint32_t i, float up) { return __hmul2(xbytes2(v, i, i), __float2half2_rn(up)); }
 
 template <> struct XDeq<T_Q4_K> {
     uint4 h;
@@ -294,7 +297,7 @@ template <> struct XDeq<T_Q4_K> {
     template <int SP, int P> __device__ __forceinline__ void part(uint32_t (&v)[16]) {
         constexpr uint32_t mask = P & 1 ? 0x00f000f0u : 0x000f000fu;         // low nibbles are columns 0-31 of 64, high ones 32-63
         const uint32_t sc = SP ? (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3f3f3f3fu;
-        const __half2 mul = xscaled(sc, P, P & 1 ? 1.0f : 16.0f);
+        const __half2 mul = xscaled(sc, P, P & 1 ? 64.0f : 1024.0f);
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const uint32_t q = w[8 * (P >> 1) + j];
@@ -332,7 +335,7 @@ template <> struct XDeq<T_Q2_K> {
     }
     template <int SP, int P> __device__ __forceinline__ void part(uint32_t (&v)[16]) {
         constexpr uint32_t r = P & 1, mask = 0x00030003u << (2 * P);         // bit pair P of the bytes, in place
-        constexpr float up = P == 0 ? 16.0f : P == 1 ? 4.0f : P == 2 ? 1.0f : 0.25f;
+        constexpr float up = P == 0 ? 1024.0f : P == 1 ? 256.0f : P == 2 ? 64.0f : 16.0f;
         const uint32_t word = q[2 * SP + (P >> 1)] & 0x0f0f0f0fu;
         const __half2 ma = xscaled(word, 2 * r, up), mb = xscaled(word, 2 * r + 1, up);
 #pragma unroll
