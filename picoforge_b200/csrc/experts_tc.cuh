@@ -429,7 +429,8 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
     static_assert(8 * (2 * Fm::STAGES + 4 * NB + 6) <= 512, "barrier block");
     volatile uint32_t *dead = reinterpret_cast<volatile uint32_t *>(smem + XM_TMEM + 8);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    // items whose apart-lying scales are held: more than the stages reach ahead (a stage holds at least one block of a row)
+    // items whose apart-lying scales are held: four where the rows are short enough, else two (rows of 9 to 16 blocks); four are more than the
+    // stages reach ahead, two are not where an item is one or two stages of four (see the TMA warp)
     const uint32_t ring_mask = (a.w0.k_storage >> 8) <= 8 ? 3u : 1u;
     const bool prof = a.debug && blockIdx.x == 0;
     uint32_t w0 = 0, w1 = 0, w2 = 0;                                        // cycles spent in this role's waits
@@ -493,6 +494,12 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
         for (uint32_t it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
             const uint32_t expert = next_expert, row0 = (it % a.tiles) * STEP;
             if (it + gridDim.x < n_items) next_expert = a.groups[(it + gridDim.x) / a.tiles].expert;
+            // Where two items' scales are held and an item is so few stages that the stages alone would reach a third one (few logical columns of
+            // long stored rows), these scales wait until the item before the last has been dequantised.  Its last stage is its slot's latest use.
+            if (Fm::SIDE && ring_mask == 1 && steps + 1 < Fm::STAGES && issued >= 2 * steps) {
+                const uint32_t last = issued - steps - 1;
+                if (!(ok = xbar_wait<200>(w_empty + 8 * (last % Fm::STAGES), (last / Fm::STAGES) & 1u, dead, a.status, w0))) break;
+            }
             for (uint32_t s = 0; s < steps; s++) {
                 if (!(ok = xbar_wait<200>(w_empty + 8 * st, ph ^ 1u, dead, a.status, w0))) break;
                 const uint32_t bar = w_full + 8 * st;

@@ -204,6 +204,33 @@ def test_tcgen05_products_keep_fp32_accuracy(gpu, routed, down, shared, hidden, 
     assert error <= 3e-6
 
 
+@pytest.mark.parametrize("routed,down,hidden,inter,physical", [
+    (Q4, Q4, 256, 128, 256),              # one unit an item, more than eight items a CTA: the rings of groups, pairs and scales at their tightest
+    (Q2, Q2, 256, 128, 256),
+    (IQ2, IQ2, 512, 128, 512),
+    (Q2, Q2, 256, 128, 2304),             # scales of two items held, an item one stage of four
+    (Q2, Q2, 256, 384, 4096),             # two stages
+    (IQ2, Q2, 512, 640, 2560),            # three: the first that cannot run ahead of its scales
+])
+def test_many_short_items_a_cta(gpu, routed, down, hidden, inter, physical):
+    """64 experts with 640 rows each: 1280 groups, and as many or twice as many items of the down product on 148 CTAs."""
+    import oracle
+    tokens = 4096
+    spec = synth.make_layer(7550 + physical, routed_type=routed, down_type=down, shared_type=Q4, hidden=hidden, inter=inter, shared_inter=256,
+                            down_physical=physical, experts=64, top_k=10, fabricated=True)
+    x = synth.activations(7550, tokens, hidden)
+    want = oracle.forward(spec, x, threads=synth.threads())
+    with MoeLayer(gpu, spec, tokens) as layer:
+        gpu.lib.qw4cu_launch_log_begin()
+        y, ids, _ = layer.forward(x)
+        assert {"expert_tile_kernel", "prefill_tc_kernel"} & set(gpu.launch_names())
+        y2, _, _ = layer.forward(x)
+    np.testing.assert_array_equal(ids, want["ids"])
+    np.testing.assert_array_equal(y2, y)
+    exact = want["y"].astype(np.float64)
+    assert np.sqrt(np.mean((y - exact) ** 2)) <= 1e-5 * np.sqrt(np.mean(exact ** 2))
+
+
 def _with_scales(blocks, gguf_type, doubled):
     """Copies of Q4_K / Q2_K blocks whose integer scales fit one bit less than the format has; plain: with twice
     the super-scale; `doubled`: with those scales times two, the same weights bit for bit."""
