@@ -399,13 +399,17 @@ void qw4cu_set_prefill_path(int path);
 void qw4cu_set_tile_path(int path);
 /* Profiling aid of the tensor-core prefill kernels: device_words is a device array of 64 x 8 bytes (NULL: off).
  * CTA 0 of every later launch stores the SM cycles its roles (0 epilogue, 1 dequantise, 2 TMA, 3 MMA issue,
- * 4 activation loader) spent waiting, at [32 * mode + 4 * role + kind]; kind 3 is the role's whole run. */
+ * 4 activation loader) spent waiting, at [32 * mode + 4 * role + kind]; kind 3 is the role's whole run.  Waits that are
+ * over at the first question (about a hundred cycles each) are not counted: two clock readings a wait would be in every role's way. */
 void qw4cu_prefill_debug(void *device_words);
 int qw4cu_decode_phase_clocks(const Qwen4MoeWork *work, uint64_t clocks[16]);
 int qw4cu_decode_repairs(const Qwen4MoeWork *work, uint32_t *count);
 /* Profiling aid: the first `words` (<= 1024) 32-bit words of the one-kernel path's counter block: counters,
- * phase clocks, and from word 256 four marks per CTA (cycles since that CTA started; zeros unless the
- * library was built with QW4_PHASE_MARKS, since the marks cost the kernel 1%). */
+ * phase clocks, and from word 256 four marks per CTA (cycles since that CTA started), which launches store
+ * while qw4cu_set_decode_marks(1) is in force: they cost the kernel 1%, so they are off by default (and then zeros).  A streaming
+ * CTA's: expert sets' counter passed, gate/up slices done, second counter passed and routes received, end; a chain CTA's:
+ * chains done, routes published, x staged, cycles its chains waited for router rows. */
+void qw4cu_set_decode_marks(int on);
 int qw4cu_decode_debug_words(const Qwen4MoeWork *work, uint32_t *out, size_t words);
 void qw4cu_set_decode_wrong_speculation(int on);
 /* Profiling aid: launch only one step of the small-batch sequence on later forwards, so that a

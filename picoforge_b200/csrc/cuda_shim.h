@@ -181,6 +181,7 @@ int qw4sh_fused_phase_clocks(const QW4ShWork *work, uint64_t clocks[16]);
 /* Launches of this workspace whose speculated expert sets had to be repaired (since it was cleared). */
 int qw4sh_fused_repairs(const QW4ShWork *work, uint32_t *count);
 void qw4sh_set_wrong_speculation(int on);
+void qw4sh_set_decode_marks(int on);
 void qw4sh_fused_scratch_sizes(const QW4ShLayer *layer, size_t *aq_bytes, size_t *asc_bytes, size_t *fast_bytes);
 
 /* Stable per-expert lists of plain rows (one id per row; 0xffffffff: none), one CTA. */

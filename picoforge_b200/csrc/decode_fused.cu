@@ -649,18 +649,11 @@ __device__ __forceinline__ bool speculate_row(const float *logits, uint32_t *can
 }
 
 // CLOCK: SM clock of the first streaming CTA at a phase boundary.  MARK: cycles since its own start, for every CTA
-// (words S_MARKS + 4 * cta + i of the sync array); built in with QW4_PHASE_MARKS only, because its stores by every CTA cost 0.7 us in four
-// Q4_K layers of one token (83.8 against 83.1) and 1.9 in four IQ2_XXS layers of four (140.9 against 139.0).
-#ifdef QW4_NO_PHASE_CLOCKS
-#define CLOCK(i) do { } while (0)
-#else
+// (words S_MARKS + 4 * cta + i of the sync array), by kernels of their own (MARKS) that are launched on request: stored at every launch the
+// marks cost 0.7 us in four Q4_K layers of one token (83.8 against 83.1) and 1.9 in four IQ2_XXS layers of four (140.9 against 139.0), and a
+// switch among the arguments costs as much without storing any (88.0 against 87.4, 143.1 against 142.2).
 #define CLOCK(i) do { if (clocked) clocks[i] = clock64(); } while (0)
-#endif
-#ifdef QW4_PHASE_MARKS
-#define MARK_CYCLES(i, cycles) do { if (threadIdx.x == 0) a.sync[S_MARKS + 4 * blockIdx.x + (i)] = (uint32_t)(cycles); } while (0)
-#else
-#define MARK_CYCLES(i, cycles) do { } while (0)
-#endif
+#define MARK_CYCLES(i, cycles) do { if (MARKS && threadIdx.x == 0) a.sync[S_MARKS + 4 * blockIdx.x + (i)] = (uint32_t)(cycles); } while (0)
 #define MARK(i) MARK_CYCLES(i, clock64() - a.t0)
 
 // ---- chain CTA -----------------------------------------------------------------------------------
@@ -672,6 +665,7 @@ __device__ __forceinline__ bool speculate_row(const float *logits, uint32_t *can
 // the next sixteen columns while the products of the current ones are added.  (Before: 64-column chunks through a
 // 16-stage cp.async ring, with a barrier wait and exposed read latency per chunk: 20 k cycles with resident
 // rows, 35 k when the rows came from HBM.)
+template <bool MARKS>
 __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
     const uint32_t T = a.tokens, H = a.hidden, E = a.experts, k = a.top_k;
     const CPlan p = make_cplan(H);
@@ -797,7 +791,7 @@ __device__ __forceinline__ void chain_cta(FusedArgs &a, uint8_t *smem) {
 }
 
 // ---- the kernel ---------------------------------------------------------------------------------
-template <uint32_t RT, uint32_t ST>
+template <uint32_t RT, uint32_t ST, bool MARKS>
 __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_constant__ FusedArgs args, const __grid_constant__ CUtensorMap map_g,
                                                              const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_sg,
                                                              const __grid_constant__ CUtensorMap map_su) {
@@ -832,7 +826,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
             to[0] = bits;
         }
     };
-    if (blockIdx.x < NC) { chain_cta(a, smem); leave(); return; }
+    if (blockIdx.x < NC) { chain_cta<MARKS>(a, smem); leave(); return; }
 
     const uint32_t T = a.tokens, H = a.hidden, E = a.experts, k = a.top_k, I = a.inter, IS = a.shared_inter;
     const uint32_t pairs = T * k, rows_c = pairs + T, imax = I > IS ? I : IS;
@@ -1327,6 +1321,9 @@ extern "C" void qw4sh_set_fused_decode(int mode) { g_fused_mode = mode; }
 static int g_wrong_speculation = 0;
 extern "C" void qw4sh_set_wrong_speculation(int on) { g_wrong_speculation = on ? 1 : 0; }
 
+static int g_marks = 0;
+extern "C" void qw4sh_set_decode_marks(int on) { g_marks = on ? 1 : 0; }
+
 static bool fused_type(uint32_t type) { return type == T_Q4_K || type == T_IQ2_XXS; }
 static uint32_t slice_blocks(uint32_t) { return FGeo<T_Q4_K>::SLICE_BLOCKS; }          // both formats of this path: 512 columns per slice
 
@@ -1483,18 +1480,18 @@ extern "C" int qw4sh_fused_supported(const QW4ShLayer *l, size_t tokens, const f
     return 1;
 }
 
-template <uint32_t RT, uint32_t ST>
-static int launch_fused(const FusedArgs &a, const QW4ShLayer *layer, uint32_t smem, int grid, cudaStream_t stream) {
+template <uint32_t RT, uint32_t ST, bool MARKS>
+static int launch_fused_as(const FusedArgs &a, const QW4ShLayer *layer, uint32_t smem, int grid, cudaStream_t stream) {
     static bool configured[64] = {false};                 // per device: the attribute and the residency check
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
     if (!configured[device]) {
-        e = cudaFuncSetAttribute(fused_decode_kernel<RT, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
+        e = cudaFuncSetAttribute(fused_decode_kernel<RT, ST, MARKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
         if (e != cudaSuccess) return (int)e;
         // the grid barriers need every CTA resident: one per SM, and an SM must take one
         int resident = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fused_decode_kernel<RT, ST>, FT, 227 * 1024 - 1024);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fused_decode_kernel<RT, ST, MARKS>, FT, 227 * 1024 - 1024);
         if (e != cudaSuccess) return (int)e;
         if (resident < 1) return (int)cudaErrorCooperativeLaunchTooLarge;
         configured[device] = true;
@@ -1506,9 +1503,13 @@ static int launch_fused(const FusedArgs &a, const QW4ShLayer *layer, uint32_t sm
     cfg.attrs = attr; cfg.numAttrs = 1;
     alignas(64) CUtensorMap maps[4];
     memcpy(maps, layer->fused_maps, sizeof maps);
-    e = cudaLaunchKernelEx(&cfg, fused_decode_kernel<RT, ST>, a, maps[0], maps[1], maps[2], maps[3]);
+    e = cudaLaunchKernelEx(&cfg, fused_decode_kernel<RT, ST, MARKS>, a, maps[0], maps[1], maps[2], maps[3]);
     if (e != cudaSuccess) return (int)e;
     return qw4sh_note_launch("fused_decode_kernel");
+}
+template <uint32_t RT, uint32_t ST>
+static int launch_fused(const FusedArgs &a, const QW4ShLayer *layer, uint32_t smem, int grid, cudaStream_t stream) {
+    return g_marks ? launch_fused_as<RT, ST, true>(a, layer, smem, grid, stream) : launch_fused_as<RT, ST, false>(a, layer, smem, grid, stream);
 }
 
 extern "C" int qw4sh_fused_decode(const QW4ShLayer *layer, const QW4ShWork *work, const float *x, float *y, size_t tokens,

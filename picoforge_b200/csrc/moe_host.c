@@ -1133,6 +1133,7 @@ void qw4cu_set_tile_path(int path) { qw4sh_set_tile_path(path); }
 void qw4cu_prefill_debug(void *device_words) { qw4sh_prefill_debug(device_words); }
 int qw4cu_decode_phase_clocks(const Qwen4MoeWork *w, uint64_t clocks[16]) { return w ? qw4sh_fused_phase_clocks(&w->d, clocks) : -1; }
 void qw4cu_set_decode_wrong_speculation(int on) { qw4sh_set_wrong_speculation(on); }
+void qw4cu_set_decode_marks(int on) { qw4sh_set_decode_marks(on); }
 int qw4cu_decode_debug_words(const Qwen4MoeWork *w, uint32_t *out, size_t words) { return w && out && words <= 1024 ? qw4sh_memcpy(out, w->d.sync, words * 4, 0) : -1; }
 int qw4cu_decode_repairs(const Qwen4MoeWork *w, uint32_t *count) { return w && count ? qw4sh_fused_repairs(&w->d, count) : -1; }
 int qw4cu_stage_times(double *ms, uint64_t *forwards) { return qw4sh_stage_times(ms, forwards); }

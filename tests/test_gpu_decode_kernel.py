@@ -141,3 +141,31 @@ def test_first_down_copies_at_the_largest_hidden_size(gpu, routed, tokens, top_k
             np.testing.assert_array_equal(weights, want["weights"])
             assert np.abs(y - want["y"]).max() <= Y_TOLERANCE
         assert gpu.lib.qw4cu_decode_repairs(layer.work, C.byref(repairs)) == 0 and repairs.value == 1
+
+
+def test_marks_are_stored_on_request(gpu):
+    """Four marks a CTA while they are asked for, none before, and the same results either way."""
+    from picoforge_b200 import synth
+    from picoforge_b200.layer import MoeLayer
+    spec = synth.make_layer(670, routed_type=16, shared_type=12, experts=64, top_k=10)
+    x = synth.activations(670, 4)
+    words = (C.c_uint32 * 1024)()
+
+    def marks(layer):
+        assert gpu.lib.qw4cu_decode_debug_words(layer.work, words, 1024) == 0
+        return np.array(words[256:], np.int64).reshape(-1, 4)
+
+    with MoeLayer(gpu, spec, 4) as layer:
+        y, _, _ = layer.forward(x)
+        assert not marks(layer).any()
+        gpu.lib.qw4cu_set_decode_marks(1)
+        try:
+            marked, _, _ = layer.forward(x)
+        finally:
+            gpu.lib.qw4cu_set_decode_marks(0)
+        seen = marks(layer)
+    np.testing.assert_array_equal(marked, y)
+    chains = 4                                       # one a token: the 65 router rows need three
+    streaming = seen[chains:][seen[chains:].any(axis=1)]
+    assert len(streaming) > 100 and (seen[:chains, 1] > seen[:chains, 0]).all() and (seen[:chains, 1] > 0).all()
+    assert (np.diff(streaming, axis=1) > 0).all() and (streaming > 0).all() and (streaming < 10**7).all()
