@@ -407,7 +407,7 @@ int qw4cu_decode_repairs(const Qwen4MoeWork *work, uint32_t *count);
 /* Profiling aid: the first `words` (<= 1024) 32-bit words of the one-kernel path's counter block: counters,
  * phase clocks, and from word 256 four marks per CTA (cycles since that CTA started), which launches store
  * while qw4cu_set_decode_marks(1) is in force: they cost the kernel 1%, so they are off by default (and then zeros).  A streaming
- * CTA's: expert sets' counter passed, gate/up slices done, second counter passed and routes received, end; a chain CTA's:
+ * CTA's: first counter passed, gate/up slices done, second counter passed and routes received, end; a chain CTA's:
  * chains done, routes published, x staged, cycles its chains waited for router rows. */
 void qw4cu_set_decode_marks(int on);
 int qw4cu_decode_debug_words(const Qwen4MoeWork *work, uint32_t *out, size_t words);

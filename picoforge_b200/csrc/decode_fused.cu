@@ -54,7 +54,7 @@
 
 namespace qw4 {
 
-constexpr int FW = 12;                          // warps per CTA (with sixteen a Q4_K token takes 24.5 us a layer, with twelve 24.1; four tokens the same)
+constexpr int FW = 12;                          // warps per CTA (with sixteen a Q4_K token took 2% longer, four IQ2_XXS tokens the same)
 constexpr int FT = FW * 32;
 constexpr int FTOK = 4;                         // tokens per launch
 constexpr int FMAXK = 16;                       // top-k limit
@@ -64,6 +64,7 @@ constexpr int FRMAX = 4;                        // router rows per streaming CTA
 constexpr int FNS = 2;                          // ring stages per warp, gate/up phase (three stages fit and were measured: no faster)
 constexpr int FNC = 2;                          // ring stages per warp, down phase
 constexpr uint32_t FSTAGE = 4608;               // bytes per ring stage: sixteen rows x 512 columns (4608 of Q4_K, 3392 of the expanded IQ2_XXS image)
+constexpr uint32_t FSMEM = 226 * 1024;          // most dynamic shared memory of a launch: an SM's 227 KB less a kilobyte for static variables
 constexpr uint32_t FZP = FMAXE + 4;             // pitch of a logit row in shared memory (floats)
 constexpr int CROWS = 32;                       // router rows per chain CTA (lane = row).  64 rows (two chain warps per token, nine
                                                 // chain CTAs) evened out the streaming CTAs' shares but ran the chains at 42 k cycles
@@ -845,7 +846,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
     uint32_t *ids_x = reinterpret_cast<uint32_t *>(smem + p.idx);              // the exact routes as published
     float *wts_x = reinterpret_cast<float *>(smem + p.wtx);
     float *misc_f = reinterpret_cast<float *>(smem + p.misc);                  // [0..3] x maxima then scales, [4..7] shared logits
-    uint32_t *misc_u = reinterpret_cast<uint32_t *>(smem + p.misc) + 16;       // [0] wait flag, [1] spec ok, [2] sources, [3] verify, [4..19] chunk counts
+    uint32_t *misc_u = reinterpret_cast<uint32_t *>(smem + p.misc) + 16;       // [1] the guess is usable, [2] sources
     uint8_t *tokmask = smem + p.tokmask, *slotmap = smem + p.slotmap;
     Src *srcs = reinterpret_cast<Src *>(smem + p.src);
     uint8_t *region = smem + p.region;
@@ -1051,7 +1052,7 @@ __global__ void __launch_bounds__(FT, 1) fused_decode_kernel(const __grid_consta
                 __syncwarp();
                 if (lane == 0) { Src s0; s0.expert = 0xffffu; s0.mask = (uint8_t)((1u << T) - 1u); s0.shared = 1; s0.slots = 0; srcs[0] = s0; }
                 // lane = sixteen experts in turn: which of them have tokens, the experts before them, then their entries one by one (one or two a lane;
-                // a ballot for every 32 experts took 3.2 k cycles, this 1.1 k)
+                // a ballot for every 32 experts took 3.2 k cycles, this 1.1 k with one token and 1.4 k with four)
                 uint32_t mine = 0;
                 const uint4 marks = reinterpret_cast<const uint4 *>(tokmask)[lane];
                 const uint32_t word[4] = {marks.x, marks.y, marks.z, marks.w};
@@ -1348,7 +1349,7 @@ static uint32_t partial_capacity(const QW4ShLayer *l, size_t tokens, uint32_t st
 static FPlan plan_for(const QW4ShLayer *l, size_t tokens, uint32_t streaming, bool *clear) {
     const uint32_t imax = l->inter > l->shared_inter ? l->inter : l->shared_inter, rows = (uint32_t)tokens * l->top_k + (uint32_t)tokens;
     const FPlan p = make_fplan(l->hidden, imax, rows, partial_capacity(l, tokens, streaming), true);
-    *clear = p.total <= 227u * 1024u - 1024u;
+    *clear = p.total <= FSMEM;
     return *clear ? p : make_fplan(l->hidden, imax, rows, partial_capacity(l, tokens, streaming), false);
 }
 
@@ -1476,7 +1477,7 @@ extern "C" int qw4sh_fused_supported(const QW4ShLayer *l, size_t tokens, const f
     const uint32_t streaming = (uint32_t)grid - nc;
     if (streaming * FRMAX < l->experts + 1) return 0;
     bool clear;
-    if (plan_for(l, tokens, streaming, &clear).total > 227u * 1024u || make_cplan(H).total > 227u * 1024u) return 0;
+    if (plan_for(l, tokens, streaming, &clear).total > FSMEM || make_cplan(H).total > FSMEM) return 0;
     return 1;
 }
 
@@ -1487,11 +1488,11 @@ static int launch_fused_as(const FusedArgs &a, const QW4ShLayer *layer, uint32_t
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
     if (!configured[device]) {
-        e = cudaFuncSetAttribute(fused_decode_kernel<RT, ST, MARKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
+        e = cudaFuncSetAttribute(fused_decode_kernel<RT, ST, MARKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FSMEM);
         if (e != cudaSuccess) return (int)e;
         // the grid barriers need every CTA resident: one per SM, and an SM must take one
         int resident = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fused_decode_kernel<RT, ST, MARKS>, FT, 227 * 1024 - 1024);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fused_decode_kernel<RT, ST, MARKS>, FT, FSMEM);
         if (e != cudaSuccess) return (int)e;
         if (resident < 1) return (int)cudaErrorCooperativeLaunchTooLarge;
         configured[device] = true;
@@ -1536,7 +1537,7 @@ extern "C" int qw4sh_fused_decode(const QW4ShLayer *layer, const QW4ShWork *work
     a.clear = clear;
     const CPlan c = make_cplan(layer->hidden);
     const uint32_t smem = p.total > c.total ? p.total : c.total;
-    if (smem > 227u * 1024u - 1024u) return -4;
+    if (smem > FSMEM) return -4;
     cudaStream_t s = (cudaStream_t)work->stream;
     if (rt == T_Q4_K) return st == T_Q4_K ? launch_fused<T_Q4_K, T_Q4_K>(a, layer, smem, sm_count, s) : launch_fused<T_Q4_K, T_IQ2N>(a, layer, smem, sm_count, s);
     return st == T_Q4_K ? launch_fused<T_IQ2N, T_Q4_K>(a, layer, smem, sm_count, s) : launch_fused<T_IQ2N, T_IQ2N>(a, layer, smem, sm_count, s);

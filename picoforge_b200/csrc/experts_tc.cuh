@@ -618,7 +618,7 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
         const uint32_t items = __reduce_max_sync(0xffffffffu, n_items), units = a.units;
         const uint32_t m = warp - R::MMA;
         uint32_t n = 0, un = 0;
-        bool ok = true, ready = false;
+        bool ok = true;
         uint32_t next_count = blockIdx.x < items ? a.groups[blockIdx.x / a.tiles].count : 0u;          // asked for an item ahead
         for (uint32_t it = blockIdx.x; it < items && ok; it += gridDim.x) {
             const uint32_t tok = __any_sync(0xffffffffu, next_count > 16) ? 32u : 16u;
@@ -629,10 +629,8 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
 #pragma unroll 1
                 for (uint32_t c = 0; c < SPU; c++, n++) {
                     const uint32_t slot = n & (NB - 1), ph = (n >> NBLOG) & 1u;
-                    if (!ready) {
-                        if (!(ok = wait(full + 8 * (slot * 2 + m), ph, w0))) break;
-                        if (c == 0 && !(ok = wait(q_bar, q_ph, w2))) break;                      // the unit before last has been read
-                    }
+                    if (!(ok = wait(full + 8 * (slot * 2 + m), ph, w0))) break;
+                    if (c == 0 && !(ok = wait(q_bar, q_ph, w2))) break;                          // the unit before last has been read
                     xtc_after();
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     const uint64_t bd = b_desc + slot * (BSTEP >> 4);
@@ -659,7 +657,6 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
                         }
                     }
                     if (el) xtc_commit(done + 8 * (slot * 2 + m));
-                    
                 }
             }
         }

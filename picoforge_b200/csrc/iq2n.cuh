@@ -9,8 +9,9 @@ namespace qw4 {
 // resident image, made at create (iq2_expand_kernel): every weight as a 2-bit level and a sign bit, laid out for their lanes.  2.06 bits per
 // weight become 3.31, and in exchange a lane turns eight weights into MMA operands with shifts, masks and two byte permutes against an
 // 8-byte table held in two registers (the codebook and sign look-ups of the packed form cost four shared-memory reads per eight weights
-// and bound both kernels).  Decoded values are the same bits.  The decode kernel's weight phases are bound by the bytes they stream: with
-// whole 4-bit codes (4.5 bits per weight, one shift and two permutes) four tokens read 65 MB and took 39.3 us a layer.
+// and bound both kernels).  Decoded values are the same bits.  In the decode kernel a warp spends most of a slice in its MMA loop and HBM
+// is a third busy; the bytes still count: with whole 4-bit codes (4.5 bits per weight, one shift and two permutes) four tokens read 65 MB a
+// layer instead of 49 and four layers took 162.7 us instead of 153.9.
 //
 // Block of sixteen rows x 512 columns, 3392 bytes: a slice of a gate/up unit (8 gate rows, 8 up rows) or a down tile.  With row r, half h
 // (128 columns) and lane t of the consumer (columns 128 h + 32 j + 8 t .. + 7 of chunk j):

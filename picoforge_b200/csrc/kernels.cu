@@ -1563,8 +1563,9 @@ static bool mma_path(const QW4ShLayer *layer, size_t tokens) {
 }
 
 // Every layer whose six expert tensors fit the tensor-core products (experts_tc.cu) runs on them, whatever the batch: large
-// all-Q4_K batches under one name (prefill), everything else under the other (tile).  The four-row grouped kernels stay for
-// callers that ask for them (qw4cu_set_tile_path(0), qw4cu_set_expert_path(1)); the CUDA-core kernels for the rest.
+// all-Q4_K batches under one name (prefill), everything else under the other (tile).  The four-row grouped kernels serve IQ2_XXS
+// layers at 5 to 64 tokens (see tile_path) and callers that ask for them (qw4cu_set_tile_path(0), qw4cu_set_expert_path(1)); the CUDA-core
+// kernels the rest.
 static int g_prefill_path = -1;                    // -1 automatic, 0 never
 extern "C" void qw4sh_set_prefill_path(int path) { g_prefill_path = path; }
 static int g_tile_path = -1;                       // -1 automatic, 0 never, 1 whenever the types allow
@@ -1588,7 +1589,8 @@ static bool tile_path(const QW4ShLayer *layer, size_t tokens) {
         // spread evenly over 512 experts, a row or two to each, the four-row kernels on the expanded image are the faster ones.  us a
         // layer, four-row against tcgen05: 5 tokens 70 / 75, 8 81 / 90, 16 113 / 128, 23 129 / 159, 32 149 / 182, 64 199 / 252.  Where
         // they crowd onto few experts (Zipf 1.1) they are the slower ones, since a group is four rows: 5 tokens 63 / 59, 23 91 / 81,
-        // 64 138 / 93.  The host knows the tokens and not their routes, so the line is drawn for the even case.
+        // 64 138 / 93.  The line is drawn by the number of tokens alone and for the even case, so crowded layers pay for it; the routes,
+        // which would tell the two apart, are known on the device before the products start, but nothing there chooses between them.
         if (mma_path(layer, tokens) && (g_expert_path == 1 || layer->w[1].type == T_IQ2_XXS)) return false;
     }
     return tc_routed(layer) && tc_shared(layer);
@@ -1849,6 +1851,8 @@ static bool shared_on_mma(const QW4ShLayer *layer) {
            qw4sh_mma_supported(&layer->w[6], 1);
 }
 
+// The four-row products of the expert-parallel step read IQ2_XXS from the packed image: they run only where the tcgen05 products are switched off
+// or do not take the tensors, and what those do not take of IQ2_XXS (rows of an odd number of blocks) has no expanded image either.
 // The shared expert of `tokens` own tokens, on the side stream: it needs only x, so it runs under the exchange.
 // Its converted x lives in the LAST rows of the buffers (rows 0 .. total-1 belong to the gathered rows).
 static int ep_shared_begin(const QW4ShLayer *layer, const QW4ShWork *work, const float *x, size_t tokens) {
