@@ -356,7 +356,8 @@ int qw4cu_moe_work_timer_end(Qwen4MoeWork *work);
 float qw4cu_moe_work_timer_elapsed_ms(Qwen4MoeWork *work);
 /* Launch strategy of qw4cu_moe_forward_device.  0 (default): kernels are launched one by
  * one.  1: the second identical call on a workspace (same layer, pointers, token count) is
- * captured into a CUDA graph and later identical calls replay it. */
+ * captured into a CUDA graph and later identical calls replay it.  A capture takes all that is enqueued on the stream
+ * meanwhile: with 1, calls of several threads must not overlap (with 0 they may, a workspace each). */
 void qw4cu_set_graph_mode(int on);
 int qw4cu_get_graph_mode(void);
 /* Which expert kernels run.  -1 (default): the tcgen05 products and the four-row kernels as

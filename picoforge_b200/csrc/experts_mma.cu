@@ -31,6 +31,7 @@
 // Every wait on an mbarrier is bounded: after about a second the kernel records
 // QW4SH_ERR_STATE, stops computing and runs out of its loops without hanging.
 #include <cuda_runtime.h>
+#include <pthread.h>
 #include <stdint.h>
 
 #include "cuda_shim.h"
@@ -704,6 +705,7 @@ __global__ void build_dense_groups_kernel(uint32_t tokens, VGroup *groups, uint3
 using namespace qw4;
 
 extern "C" int qw4sh_note_launch(const char *name);      // kernels.cu: counts the launch, checks the error
+extern "C" int qw4sh_allow_smem(const void *kernel, size_t smem);
 
 static DevTensor dev(const QW4ShTensor &s) {
     DevTensor t;
@@ -713,17 +715,19 @@ static DevTensor dev(const QW4ShTensor &s) {
 }
 
 static uint8_t *g_lut[64] = {nullptr};
+static pthread_mutex_t g_lut_lock = PTHREAD_MUTEX_INITIALIZER;          // one maker, and nobody launches on an image that is still being made
 static const uint8_t *lut_image() {
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
-    if (!g_lut[device]) {
-        uint8_t *p = nullptr;
-        if (cudaMalloc(&p, LUT_BYTES) != cudaSuccess) return nullptr;
+    pthread_mutex_lock(&g_lut_lock);
+    uint8_t *p = g_lut[device];
+    if (!p && cudaMalloc(&p, LUT_BYTES) == cudaSuccess) {
         build_lut_kernel<<<24, 256>>>(p);
-        if (qw4sh_note_launch("build_lut_kernel") || cudaDeviceSynchronize() != cudaSuccess) { cudaFree(p); return nullptr; }
+        if (qw4sh_note_launch("build_lut_kernel") || cudaDeviceSynchronize() != cudaSuccess) { cudaFree(p); p = nullptr; }
         g_lut[device] = p;
     }
-    return g_lut[device];
+    pthread_mutex_unlock(&g_lut_lock);
+    return p;
 }
 
 extern "C" int qw4sh_mma_supported(const QW4ShTensor *w, int mode) {
@@ -740,8 +744,8 @@ template <uint32_t TYPE, int MODE>
 static int launch_grouped(const GroupedArgs &a, int ctas, cudaStream_t stream) {
     const Plan p = make_plan<TYPE, MODE>(a.w0.k_storage);
     if (p.n_stages < 2) return -2;
-    cudaError_t e = cudaFuncSetAttribute(grouped_mma_kernel<TYPE, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.total);
-    if (e != cudaSuccess) return (int)e;
+    const int rc = qw4sh_allow_smem((const void *)grouped_mma_kernel<TYPE, MODE>, p.total);
+    if (rc) return rc;
     grouped_mma_kernel<TYPE, MODE><<<ctas, NT, p.total, stream>>>(a);
     return qw4sh_note_launch("grouped_mma_kernel");
 }

@@ -12,6 +12,7 @@
 // the CUDA-core kernels below, which do the combine with the down product; layer_launches chooses.
 #include <cuda_runtime.h>
 #include <math_constants.h>
+#include <pthread.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
@@ -33,11 +34,17 @@ static int fail(cudaError_t e, const char *where) {
     return (int)e ? (int)e : -1;
 }
 #define CU(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) return fail(e_, #call); } while (0)
-// Names of the kernels launched since qw4sh_launch_log_begin (string literals; the first LOG_CAP are kept).
+// Held by whoever looks for, or makes, what the library makes on first use: once for a device and all threads.
+static pthread_mutex_t g_first_use = PTHREAD_MUTEX_INITIALIZER;
+struct FirstUse {
+    FirstUse() { pthread_mutex_lock(&g_first_use); }
+    ~FirstUse() { pthread_mutex_unlock(&g_first_use); }
+};
 extern "C" int qw4sh_fail_text(const char *text) {
     snprintf(g_error, sizeof g_error, "%s", text);
     return -1;
 }
+// Names of the kernels launched since qw4sh_launch_log_begin (string literals; the first LOG_CAP are kept).
 static const unsigned LOG_CAP = 512;
 static const char *g_log[LOG_CAP];
 static unsigned g_log_n = LOG_CAP;                // full: logging off until the first begin
@@ -122,6 +129,7 @@ extern "C" int qw4sh_shared_stream(void **stream) {
     int device = 0;
     CU(cudaGetDevice(&device));
     if (device < 0 || device >= 64) return fail(cudaErrorInvalidDevice, "device index");
+    FirstUse first;
     if (!g_stream[device]) CU(cudaStreamCreateWithFlags(&g_stream[device], cudaStreamNonBlocking));
     *stream = g_stream[device];
     return ensure_constants();
@@ -1255,12 +1263,27 @@ static uint32_t kernel_type(const DevTensor &t) {
     return packed && t.k_storage % 256 == 0 && t.k_logical % 8 == 0 && (t.n_experts == 1 || t.expert_bytes % 8 == 0) ? t.type : GENERIC;
 }
 
+// The most dynamic shared memory that launches of a kernel may ask for on this device: raised to `smem`, never lowered.  It stays with the kernel
+// and not with a launch, so a smaller launch that set it to its own size could take it from under a larger one of another thread.
+extern "C" int qw4sh_allow_smem(const void *kernel, size_t smem) {
+    static struct { const void *kernel; int device; size_t smem; } have[512];
+    static unsigned n = 0;
+    int device = 0;
+    CU(cudaGetDevice(&device));
+    FirstUse first;
+    unsigned i = 0;
+    while (i < n && (have[i].kernel != kernel || have[i].device != device)) i++;
+    if (i < n && have[i].smem >= smem) return 0;
+    CU(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (i == n && n < sizeof have / sizeof have[0]) { have[n].kernel = kernel; have[n].device = device; n++; }
+    if (i < n) have[i].smem = smem;
+    return 0;
+}
 template <typename Kernel>
 static int allow_smem(Kernel kernel, size_t smem) {
     if (smem > 227u * 1024u) return fail(cudaErrorInvalidValue, "shape needs more shared memory than one CTA has");
     // beyond 48 KB, which the kernel's own static arrays count towards (a few KB at most)
-    if (smem > 40u * 1024u) CU(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return 0;
+    return smem > 40u * 1024u ? qw4sh_allow_smem((const void *)kernel, smem) : 0;
 }
 
 static int g_sm_count[64] = {0};
@@ -1602,10 +1625,9 @@ static int side_stream(cudaStream_t *stream, cudaEvent_t **events) {
     int device = 0;
     CU(cudaGetDevice(&device));
     if (device < 0 || device >= 64) return fail(cudaErrorInvalidDevice, "device index");
-    if (!g_side_stream[device]) {
-        CU(cudaStreamCreateWithFlags(&g_side_stream[device], cudaStreamNonBlocking));
-        for (int i = 0; i < 4; i++) CU(cudaEventCreateWithFlags(&g_side_event[device][i], cudaEventDisableTiming));
-    }
+    FirstUse first;
+    for (int i = 0; i < 4; i++) if (!g_side_event[device][i]) CU(cudaEventCreateWithFlags(&g_side_event[device][i], cudaEventDisableTiming));
+    if (!g_side_stream[device]) CU(cudaStreamCreateWithFlags(&g_side_stream[device], cudaStreamNonBlocking));
     *stream = g_side_stream[device]; *events = g_side_event[device];
     return 0;
 }
@@ -1618,10 +1640,9 @@ static int aux_stream(cudaStream_t *stream, cudaEvent_t **events) {
     int device = 0;
     CU(cudaGetDevice(&device));
     if (device < 0 || device >= 64) return fail(cudaErrorInvalidDevice, "device index");
-    if (!g_aux_stream[device]) {
-        CU(cudaStreamCreateWithFlags(&g_aux_stream[device], cudaStreamNonBlocking));
-        for (int i = 0; i < 2; i++) CU(cudaEventCreateWithFlags(&g_aux_event[device][i], cudaEventDisableTiming));
-    }
+    FirstUse first;
+    for (int i = 0; i < 2; i++) if (!g_aux_event[device][i]) CU(cudaEventCreateWithFlags(&g_aux_event[device][i], cudaEventDisableTiming));
+    if (!g_aux_stream[device]) CU(cudaStreamCreateWithFlags(&g_aux_stream[device], cudaStreamNonBlocking));
     *stream = g_aux_stream[device]; *events = g_aux_event[device];
     return 0;
 }
