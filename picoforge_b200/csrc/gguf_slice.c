@@ -235,8 +235,9 @@ static Qwen4Status read_slice(const char *path, uint32_t layer, Mapping *m, QW4C
         for (uint32_t d = 0; d < t->rank; d++)
             if (t->shape[d] != shape[j][d]) return fail(err, QW4_SHAPE, t->name, "tensor shape differs from the metadata", 0, 0);
         if ((j == 0 || j == 7) && t->type != 0) return fail(err, QW4_TYPE, t->name, "router tensors are F32", 0, 0);
+        if (t->file_offset > m->size - data_offset || t->bytes > m->size - data_offset - t->file_offset)       /* a sum could wrap */
+            return fail(err, QW4_FORMAT, t->name, "tensor runs past the file", 0, data_offset + t->file_offset);
         t->file_offset += data_offset;
-        if (t->file_offset > m->size || t->bytes > m->size - t->file_offset) return fail(err, QW4_FORMAT, t->name, "tensor runs past the file", 0, t->file_offset);
         size_t block = 1, bytes = 1;
         (void)format_of(t->type, &block, &bytes);
         QW4PackedLayout *l = &out->layout[j];

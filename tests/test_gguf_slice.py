@@ -133,6 +133,21 @@ def test_malformed_files_are_statuses(tmp_path):
     assert got.config.hidden_size == 0 and got.tensor[0].bytes == 0               # nothing left behind on error
 
 
+def test_an_offset_that_wraps_is_refused(tmp_path):
+    """A payload offset so large that adding the data section's start comes out inside the file again."""
+    import struct
+    api = abi.product()
+    path = tmp_path / "m.gguf"
+    gguf_fixture.write_layer(path, _spec())
+    blob = bytearray(path.read_bytes())
+    name = b"blk.0.ffn_gate_inp.weight"
+    at = blob.index(name) + len(name) + 4 + 2 * 8 + 4                            # rank, two dimensions, type
+    blob[at:at + 8] = struct.pack("<Q", 2**64 - 32)
+    path.write_bytes(bytes(blob))
+    status, _, err = _describe(api, path)
+    assert status == abi.FORMAT and b"past the file" in err.detail
+
+
 @pytest.mark.gpu
 def test_layer_created_from_a_file_equals_one_created_from_memory(gpu, tmp_path):
     import oracle
