@@ -494,9 +494,10 @@ __device__ __forceinline__ void expert_tc_body(const XMaps &maps, const XArgs &a
         for (uint32_t it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
             const uint32_t expert = next_expert, row0 = (it % a.tiles) * STEP;
             if (it + gridDim.x < n_items) next_expert = a.groups[(it + gridDim.x) / a.tiles].expert;
-            // Where two items' scales are held and an item is so few stages that the stages alone would reach a third one (few logical columns of
-            // long stored rows), these scales wait until the item before the last has been dequantised.  Its last stage is its slot's latest use.
-            if (Fm::SIDE && ring_mask == 1 && steps + 1 < Fm::STAGES && issued >= 2 * steps) {
+            // Where two items' scales are held and an item is so few stages that the stages alone would reach a third one (down with few logical
+            // columns of long stored rows), these scales wait until the item before the last has been dequantised.  Its last stage is its slot's
+            // latest use.  (Gate/up stores what it multiplies: nine stages where two are held.  Asking there as well cost a layer of seven tokens 0.4%.)
+            if (MODE == 1 && Fm::SIDE && ring_mask == 1 && steps + 1 < Fm::STAGES && issued >= 2 * steps) {
                 const uint32_t last = issued - steps - 1;
                 if (!(ok = xbar_wait<200>(w_empty + 8 * (last % Fm::STAGES), (last / Fm::STAGES) & 1u, dead, a.status, w0))) break;
             }
